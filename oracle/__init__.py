@@ -49,7 +49,7 @@ def build(with_ref: bool | None = None) -> None:
     """Compile the restatement, and the reference shims if the sources exist."""
     targets = ["port"]
     if with_ref is None:
-        with_ref = bool(REFERENCE_SRC) and os.path.isdir(REFERENCE_SRC)
+        with_ref = bool(REFERENCE_SRC) and os.path.isdir(os.path.join(REFERENCE_SRC, "flens"))
     if with_ref:
         targets.append("ref")
     extra = [f"REF={REFERENCE_SRC}"] if with_ref and REFERENCE_SRC else []
