@@ -92,6 +92,16 @@ Workspace *workspace_side(cudaStream_t stream);
 int workspace_flags(cudaStream_t stream, int n, unsigned long long **flags,
                     unsigned long long *epoch);
 
+// Scratch for one sequence of launches on `stream`, taken from and given back
+// to a device's memory pool in stream order (cudaMallocAsync), so calls on the
+// same stream from several threads have their own.  The pool keeps at most
+// kScratchKeep bytes between synchronisations and is destroyed at unload.
+// nullptr when there is no memory (the last error is not set: the callers have
+// a way without).  *status: the stream's device status word.
+constexpr size_t kScratchKeep = (size_t)2 << 30;
+void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status);
+void scratch_release(void *p, cudaStream_t stream);
+
 int num_sms();                 // SM count of the current device
 int device_id();               // current device ordinal
 
@@ -207,6 +217,23 @@ namespace fg {
 int dgemm_launch(char transA, char transB, int m, int n, int k, double alpha,
                  const double *A, int ldA, const double *B, int ldB,
                  double beta, double *C, int ldC, cudaStream_t stream);
+
+// dgemm on the FP64 pipe whatever the size, without scratch memory.
+int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
+                      int ldA, const double *B, int ldB, double beta, double *C, int ldC,
+                      cudaStream_t stream);
+
+// The product on the tensor cores by exact residues (mod_gemm.cu), tri 0 all
+// of C, 1/2 its lower/upper triangle; kErrUnsupported (nothing launched) when
+// mod_gemm_wins is false, the stream is being captured or no scratch memory
+// is to be had.  dgemm_flagged_launch: the FP64 kernel on the blocks it
+// refused.
+bool mod_gemm_wins(int m, int n, int k, int tri);
+int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
+                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s);
+int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
+                         int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
+                         const uint8_t *flag, int flag_ld, cudaStream_t stream);
 
 // dgemm with one triangular operand stored full (explicit zeros): kr 1/2 =
 // op(A) upper/lower, 3/4 = op(B) upper/lower; the zero k blocks are skipped.

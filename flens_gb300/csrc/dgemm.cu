@@ -79,12 +79,16 @@ struct SlabLoader {
 // nonzero (the skipped terms are exact zeros): 1 op(A) upper (k >= row),
 // 2 op(A) lower (k <= row), 3 op(B) upper (k <= column), 4 op(B) lower
 // (k >= column).
-template <typename T, bool TA, bool TB, int TRI = 0, int KR = 0, int TM = BM, int TN = BN>
+// FLAG: only the tiles of the 128 x 256 blocks of C whose byte in `flag`
+// (column-major, flag_ld block rows) is set: what the residue product
+// (mod_gemm.cu) left to FP64.
+template <typename T, bool TA, bool TB, int TRI = 0, int KR = 0, int TM = BM, int TN = BN, bool FLAG = false>
 __global__ void __launch_bounds__(256)
 dgemm_fma_kernel(int m, int n, int k, T alpha,
                  const T *__restrict__ A, int ldA,
                  const T *__restrict__ B, int ldB,
-                 T beta, T *__restrict__ C, int ldC) {
+                 T beta, T *__restrict__ C, int ldC, const uint8_t *__restrict__ flag = nullptr,
+                 int flag_ld = 0) {
     constexpr int RI = TM / 16, RJ = TN / 16;
     __shared__ T As[2][BK][TM + PAD];
     __shared__ T Bs[2][BK][TN + PAD];
@@ -92,6 +96,7 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
     if (TRI == 1 && m0 + TM <= n0) return;       // tile strictly above the diagonal
     if (TRI == 2 && n0 + TN <= m0) return;       // tile strictly below the diagonal
+    if (FLAG && !flag[m0 / 128 + flag_ld * (n0 / 256)]) return;
 
     SlabLoader<T, !TA, TM, 256> la;
     SlabLoader<T, TB, TN, 256> lb;
@@ -707,6 +712,11 @@ int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const dou
     }
     const bool lower = uplo == 'L' || uplo == 'l';
     const bool nt = trans == 'N' || trans == 'n';
+    if (k > 0 && alpha != 0.0) {
+        const int st = mod_gemm_launch(nt ? 'N' : 'T', nt ? 'T' : 'N', n, n, k, alpha, A, ldA, B, ldB, beta, C, ldC,
+                                       lower ? 1 : 2, stream);
+        if (st != kErrUnsupported) return st;
+    }
     const dim3 grid(ceil_div(n, BM), ceil_div(n, BN));
     if (grid.y > 65535) {
         set_last_error("syrk: n=%d too large for one launch", n);
@@ -739,8 +749,47 @@ int dsyrk_launch(char uplo, char trans, int n, int k, double alpha, const double
 int dgemm_launch(char transA, char transB, int m, int n, int k, double alpha,
                  const double *A, int ldA, const double *B, int ldB,
                  double beta, double *C, int ldC, cudaStream_t stream) {
+    if (m > 0 && n > 0 && alpha != 0.0) {
+        const int st = mod_gemm_launch(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, 0, stream);
+        if (st != kErrUnsupported) return st;
+    }
+    return dgemm_fp64_launch(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream);
+}
+
+int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
+                      int ldA, const double *B, int ldB, double beta, double *C, int ldC,
+                      cudaStream_t stream) {
     return gemm_launch_t<double>(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC,
                                  stream);
+}
+
+// The FP64 kernel on the flagged 128 x 256 blocks of C only (tri 1/2: within
+// the lower/upper triangle): the tiles a residue product refused.
+int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
+                         int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
+                         const uint8_t *flag, int flag_ld, cudaStream_t stream) {
+    const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
+    KTimer kt(kFamGemm, stream, 0.0, 0.0);
+    const dim3 g64(ceil_div(m, BM), ceil_div(n, BN)), g32(ceil_div(m, 32), ceil_div(n, 32));
+    const bool small = (long long)g64.x * g64.y < 4LL * num_sms();
+#define FG_FL(TA_, TB_, TRI_)                                                                              \
+    do {                                                                                                   \
+        if (small)                                                                                         \
+            dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32, true><<<g32, 256, 0, stream>>>(            \
+                m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld);                              \
+        else                                                                                               \
+            dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, BM, BN, true><<<g64, 256, 0, stream>>>(            \
+                m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld);                              \
+    } while (0)
+#define FG_FLT(TA_, TB_) do { if (tri == 1) FG_FL(TA_, TB_, 1); else if (tri == 2) FG_FL(TA_, TB_, 2); else FG_FL(TA_, TB_, 0); } while (0)
+    if (!ta && !tb) FG_FL(false, false, 0);      // a triangle's product has one transposed operand
+    else if (ta && !tb) FG_FLT(true, false);
+    else if (!ta && tb) FG_FLT(false, true);
+    else FG_FL(true, true, 0);
+#undef FG_FLT
+#undef FG_FL
+    FG_CUDA(cudaGetLastError());
+    return kOk;
 }
 
 int sgemm_launch(char transA, char transB, int m, int n, int k, float alpha, const float *A,

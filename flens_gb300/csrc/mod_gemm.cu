@@ -1,0 +1,874 @@
+// mod_gemm.cu -- the FP64 GEMM on the tensor cores, by exact residues.
+//
+// C <- beta*C + alpha*op(A)*op(B), the large products of dgemm / syrk and of
+// the LU and Cholesky updates (cxxblas/level3/gemm.tcc:42-190, syrk.tcc:42-90).
+// GB300's FP64 pipe issues 2 FMAs per clock per SM (1.26 TFLOP/s); its tensor
+// cores have no FP64 kind but add BF16 products of small integers exactly.
+// The product is therefore formed in a residue number system (the scheme of
+// Ozaki, Uchino and Imamura, "Ozaki Scheme II", 2025, with moduli and bounds
+// of our own):
+//
+//  1. exponents: 2^e_i bounds row i of op(A), 2^f_j column j of op(B).
+//  2. residues: a_ik is rounded to the integer X_ik = rint(a_ik 2^(beta-e_i)),
+//     |X| <= 2^beta, and stored as its NM = 17 centred residues modulo
+//     pairwise coprime p <= 256 (exact in BF16); likewise op(B).  beta is the
+//     largest with 2^(2 beta) k <= P/4, P = prod p ~ 2^133, at most 61: 61 for
+//     k <= 512, 59 for k = 4096 -- 6 to 8 bits more than FP64's significand.
+//  3. products: one BF16 tensor-core GEMM per modulus.  |r r'| <= 2^14, so the
+//     FP32 sums of 1024 products are exact integers; longer k is cut into such
+//     chunks whose residues are added.  17 products where the digit form
+//     (split_gemm.cu) needs 36 to 45, and every (modulus, tile) is a work item
+//     of its own, so small outputs fill the GPU too.
+//  4. reconstruction: X Y mod P from the residues (the operand residues of
+//     op(A) already carry the inverse weights), in 160-bit integers with
+//     dp4a, then ONE rounding to FP64, and C as the FP64 kernel forms it.
+//
+// No less accurate than FP64 arithmetic, by a check on the data: an 18th
+// product of the magnitudes (rounded down to BF16) bounds Q_ij = sum_k
+// |a_ik||b_kj| 2^(-e_i-f_j) from below.  Rounding the operands changes c_ij by
+// at most 2^-beta k 2^(e_i+f_j); a tile is accepted only if k/Q_ij <= 2^(beta-51)
+// for all its elements with Q_ij != 0, that is, if that change is below
+// 4 * 2^-53 * (|A||B|)_ij -- FP64's own bound is k * 2^-53 * (|A||B|)_ij.
+// Uniform data needs k/Q = 2^2, LU and Cholesky updates up to 2^7, the limit
+// is 2^8 to 2^10.  Tiles of graded data beyond that, and tiles with
+// non-finite rows or exponents outside +-450, are left to the FP64 kernel,
+// which runs last and skips all others: no readback, the call stays
+// asynchronous.
+#include "tcgen05.cuh"
+
+#include <cuda_bf16.h>
+
+#include <cmath>
+#include <cstdlib>
+
+namespace fg {
+namespace {
+
+constexpr int NM = 17;                       // moduli
+constexpr int NP = NM + 1;                   // operand planes: residues, magnitudes
+constexpr int NG = (NM + 3) / 4;             // dp4a groups of moduli
+constexpr int NL = 17;                       // base-256 limbs of P
+constexpr int kPrime[NM] = {256, 255, 253, 251, 247, 241, 239, 233, 229,
+                            227, 223, 217, 211, 199, 197, 193, 191};
+constexpr int MT = tc::BM, NT = 256;         // output tile
+constexpr int KBLK = 64;                     // k of one operand stage (128 bytes of BF16)
+constexpr int CHUNK = 1024;                  // 2^14 * 1024 = 2^24: exact FP32 sums
+constexpr int kExpLimit = 450;
+constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23: adds round to integers
+
+struct ResConst {                            // operand side, per modulus
+    float p[NM], ip[NM];
+    float ca[NM][4], cb[NM][4];              // 2^(16 t) (times the CRT inverse for A) mod p
+};
+struct CrtConst {
+    uint32_t w[NG][NL];                      // byte l of P/p_i, four moduli per word
+    uint32_t qw[NG];                         // round(2^14 / p_i)
+    int P[NL];
+};
+struct Consts {
+    ResConst res;
+    CrtConst crt;
+    int log2P;
+};
+
+int centred(int x, int p) {
+    x %= p;
+    if (x < 0) x += p;
+    return 2 * x > p ? x - p : x;
+}
+
+Consts make_consts() {
+    Consts c{};
+    // P in base 256
+    int P[NL + 1] = {1};
+    for (int i = 0; i < NM; ++i) {
+        int carry = 0;
+        for (int l = 0; l <= NL; ++l) {
+            const int v = P[l] * kPrime[i] + carry;
+            P[l] = v & 255;
+            carry = v >> 8;
+        }
+    }
+    int top = NL;
+    while (P[top] == 0) --top;
+    c.log2P = 8 * top;
+    for (int v = P[top]; v > 1; v >>= 1) ++c.log2P;
+    for (int l = 0; l < NL; ++l) c.crt.P[l] = P[l];
+    for (int i = 0; i < NM; ++i) {
+        const int p = kPrime[i];
+        int W[NL], rem = 0, wmod = 0;
+        for (int l = NL - 1; l >= 0; --l) {
+            const int v = rem * 256 + P[l];
+            W[l] = v / p;
+            rem = v % p;
+        }
+        for (int l = NL - 1; l >= 0; --l) wmod = (wmod * 256 + W[l]) % p;
+        int y = 1;
+        while ((wmod * y) % p != 1) ++y;
+        for (int l = 0; l < NL; ++l) c.crt.w[i / 4][l] |= (uint32_t)W[l] << (8 * (i % 4));
+        c.crt.qw[i / 4] |= (uint32_t)((2 * 16384 + p) / (2 * p)) << (8 * (i % 4));
+        c.res.p[i] = (float)p;
+        c.res.ip[i] = 1.0f / (float)p;
+        int b = 1;
+        for (int t = 0; t < 4; ++t) {
+            c.res.cb[i][t] = (float)centred(b, p);
+            c.res.ca[i][t] = (float)centred(b * y, p);
+            b = b * (65536 % p) % p;
+        }
+    }
+    return c;
+}
+const Consts &consts() {
+    static const Consts c = make_consts();
+    return c;
+}
+
+// One operand as the kernels see it: R rows of op(X) along k.
+struct Operand {
+    const double *X;
+    int ld, R, rcontig;                      // rcontig: element (r, k) at X[r + k ld], else X[k + r ld]
+    unsigned *key;                           // row maxima: high word of |x|
+    __nv_bfloat16 *planes;                   // NP planes of R rows x Kp
+};
+
+// e with max|x| < 2^e from the row key; ok = false: non-finite or out of range.
+__device__ __forceinline__ int key_exp(unsigned key, bool &ok) {
+    const int e = (int)(key >> 20) - 1022;
+    ok = key == 0u || (e >= -kExpLimit && e <= kExpLimit);
+    return key == 0u ? 0 : e;
+}
+
+__device__ __forceinline__ unsigned mag_key(double v) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    const unsigned hi = (unsigned)(b >> 32);
+    return hi ? hi : ((unsigned)b ? 1u : 0u);
+}
+
+// ------------------------------------------------------------ exponents --
+// Row maxima of |x| (as high words) by integer atomicMax into zeroed keys.
+// A block takes 64 rows x 128 k (rows contiguous) or 8 rows x 1024 k.
+// Bound: HBM, one read of each operand.
+constexpr int EX_K0 = 128, EX_K1 = 1024;
+__host__ __device__ inline int exp_blocks(int R, int K, int rcontig) {
+    return rcontig ? ((R + 63) / 64) * ((K + EX_K0 - 1) / EX_K0) : ((R + 7) / 8) * ((K + EX_K1 - 1) / EX_K1);
+}
+
+__global__ void __launch_bounds__(256)
+mod_exp_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Operand ob, int K, int blocksA) {
+    const bool isB = (int)blockIdx.x >= blocksA;
+    const Operand &o = isB ? ob : oa;
+    const int b = isB ? blockIdx.x - blocksA : blockIdx.x;
+    if (o.rcontig) {
+        __shared__ unsigned sm[4][64];
+        const int rb = (o.R + 63) / 64;
+        const int x = threadIdx.x & 63, y = threadIdx.x >> 6;
+        const int r = (b % rb) * 64 + x, k0 = (b / rb) * EX_K0;
+        unsigned m = 0u;
+        if (r < o.R) {
+            const double *p = o.X + (size_t)r + (size_t)k0 * o.ld;
+            const int kn = min(EX_K0, K - k0);
+#pragma unroll 8
+            for (int k = y; k < kn; k += 4) m = max(m, mag_key(p[(size_t)k * o.ld]));
+        }
+        sm[y][x] = m;
+        __syncthreads();
+        if (y == 0 && r < o.R) {
+            m = max(max(m, sm[1][x]), max(sm[2][x], sm[3][x]));
+            if (m) atomicMax(&o.key[r], m);
+        }
+    } else {
+        const int rb = (o.R + 7) / 8;
+        const int lane = threadIdx.x & 31;
+        const int r = (b % rb) * 8 + (threadIdx.x >> 5), k0 = (b / rb) * EX_K1;
+        if (r >= o.R) return;
+        const double *p = o.X + (size_t)k0 + (size_t)r * o.ld;
+        const int kn = min(EX_K1, K - k0);
+        unsigned m = 0u;
+#pragma unroll 8
+        for (int k = lane; k < kn; k += 32) m = max(m, mag_key(p[k]));
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0 && m) atomicMax(&o.key[r], m);
+    }
+}
+
+// ------------------------------------------------------------- residues --
+// X = rint(v 2^(bits - e)) as an integer, from the bits of v.
+__device__ __forceinline__ long long fixed_point(double v, int e, int bits) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    int ex = (int)((u >> 52) & 0x7FF);
+    long long m = (long long)(u & 0xFFFFFFFFFFFFFull);
+    if (ex) m |= 1ll << 52;
+    else ex = 1;
+    const int sh = ex - 1075 + bits - e;         // <= bits - 53 <= 8
+    if (sh >= 0) m <<= sh;
+    else if (sh > -55) m = (m + (1ll << (-sh - 1))) >> -sh;
+    else m = 0;
+    return (long long)u < 0 ? -m : m;
+}
+
+// |v| 2^-e rounded down to BF16's 8 significant bits; values below 2^-60 are
+// raised to it, so that products of nonzeros stay nonzero in the sum.
+__device__ __forceinline__ float magnitude(double v, int e) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+    if (u == 0ull) return 0.0f;
+    int ex = (int)(u >> 52) - 1023 - e;          // v in [2^ex, 2^(ex+1)) 2^e
+    if (ex < -60) return __uint_as_float((127u - 60u) << 23);
+    const unsigned mant = (unsigned)(u >> 45) & 0x7Fu;
+    return __uint_as_float(((unsigned)(ex + 127) << 23) | (mant << 16));
+}
+
+// A block turns 32 rows x 64 k of one operand into its NP planes.  The tile is
+// staged through shared memory so that both the FP64 reads and the BF16
+// writes (16 lanes x 8 bytes = one 128-byte line per row) are coalesced; a
+// thread holds 4 consecutive k, each as four signed 16-bit pieces in FP32, so
+// a residue is 4 FMAs (exact: |sum| < 2^24) and 3 operations of reduction.
+// Bound: 8 bytes read and 36 written per element, about 130 FP32 operations.
+__global__ void __launch_bounds__(256)
+mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Operand ob, int K, int Kp,
+                   int bits, int blocksA, const __grid_constant__ ResConst rc) {
+    __shared__ __align__(16) double tile[32][66];
+    const bool isB = (int)blockIdx.x >= blocksA;
+    const Operand &o = isB ? ob : oa;
+    const int b = isB ? blockIdx.x - blocksA : blockIdx.x;
+    const int rb = (o.R + 31) / 32;
+    const int r0 = (b % rb) * 32, k0 = (b / rb) * KBLK;
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    if (o.rcontig) {
+        const int r = r0 + lane;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int k = wy + 8 * i;
+            tile[lane][k] = (r < o.R && k0 + k < K) ? o.X[(size_t)r + (size_t)(k0 + k) * o.ld] : 0.0;
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int rr = wy + 8 * (i >> 1), k = lane + 32 * (i & 1);
+            tile[rr][k] = (r0 + rr < o.R && k0 + k < K) ? o.X[(size_t)(k0 + k) + (size_t)(r0 + rr) * o.ld] : 0.0;
+        }
+    }
+    __syncthreads();
+    const size_t plane = (size_t)o.R * Kp;
+#pragma unroll 1
+    for (int h = 0; h < 2; ++h) {
+        const int rr = (threadIdx.x >> 4) + 16 * h, kq = (threadIdx.x & 15) * 4;
+        const int r = r0 + rr;
+        if (r >= o.R) continue;
+        bool ok;
+        const int e = key_exp(o.key[r], ok);
+        float x[4][4], mg[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double d = ok ? tile[rr][kq + i] : 0.0;
+            mg[i] = magnitude(d, e);
+            long long v = fixed_point(d, e, bits);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int piece = (int)(short)(v & 0xFFFF);
+                x[i][t] = (float)piece;
+                v = (v - piece) >> 16;
+            }
+        }
+        __nv_bfloat16 *out = o.planes + (size_t)r * Kp + (k0 + kq);
+        auto put = [&](const float (&f)[4]) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+            uint2 w;
+            w.x = *(const unsigned *)&lo;
+            w.y = *(const unsigned *)&hi;
+            *(uint2 *)out = w;
+            out += plane;
+        };
+#pragma unroll
+        for (int j = 0; j < NM; ++j) {
+            const float *c = isB ? rc.cb[j] : rc.ca[j];
+            const float c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
+            float f[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float s = fmaf(x[i][3], c3, fmaf(x[i][2], c2, fmaf(x[i][1], c1, x[i][0] * c0)));
+                const float q = fmaf(s, rc.ip[j], kMagic) - kMagic;
+                f[i] = fmaf(-q, rc.p[j], s);
+            }
+            put(f);
+        }
+        put(mg);
+    }
+}
+
+// ------------------------------------------------------------- products --
+// Tiles of the output: all of them in bands (tc::tile_origin), or the ones
+// that meet one triangle (tri 1: lower, 2: upper), column by column.
+struct TileMap {
+    int M, N, tm, tn, tri, ntiles;
+};
+TileMap make_tiles(int M, int N, int tri) {
+    TileMap t{M, N, ceil_div(M, MT), ceil_div(N, NT), tri, 0};
+    if (!tri) t.ntiles = t.tm * t.tn;
+    for (int j = 0; tri && j < t.tn; ++j) {
+        const int first = tri == 1 ? 2 * j : 0, last = tri == 1 ? t.tm : (2 * j + 2 < t.tm ? 2 * j + 2 : t.tm);
+        if (last > first) t.ntiles += last - first;
+    }
+    return t;
+}
+__device__ __forceinline__ void tile_at(const TileMap &tm, int t, int &m0, int &n0) {
+    if (!tm.tri) {
+        tc::tile_origin(t, tm.tm, tm.tn, NT, m0, n0);
+        return;
+    }
+    m0 = n0 = 0;
+    for (int j = 0; j < tm.tn; ++j) {
+        const int first = tm.tri == 1 ? 2 * j : 0;
+        const int cnt = (tm.tri == 1 ? tm.tm : min(2 * j + 2, tm.tm)) - first;
+        if (t < cnt) {
+            m0 = (first + t) * MT;
+            n0 = j * NT;
+            return;
+        }
+        if (cnt > 0) t -= cnt;
+    }
+}
+
+struct ModArgs {
+    TileMap tiles;
+    int nkb;                                  // 64-deep k blocks
+    float qmin;                               // smallest accepted Q
+    uint8_t *res;                             // residues [modulus][tile][16-column group][row][16]
+    uint8_t *flag;                            // per tile (row tile + tm * column tile): 1 = left to FP64
+    const unsigned *keyA, *keyB;
+    float p[NM], ip[NM];
+};
+
+constexpr int STAGES = 4;
+constexpr uint32_t A_BYTES = MT * 128, B_BYTES = NT * 128;
+constexpr size_t MOD_SMEM = 1024 + (size_t)STAGES * (A_BYTES + B_BYTES) + 256;
+
+// Persistent, one CTA per SM; a work item is (plane, tile), the magnitude
+// plane first.  Same roles as tc::tc_kernel (TMA producer, MMA issuer, eight
+// epilogue warps over two TMEM accumulators); a residue plane runs one
+// accumulator per 1024 of k.  Epilogue: 6 FP32 operations per element reduce
+// the integer sum to a centred residue, 4 are packed per word, and a warp
+// stores 512 contiguous bytes per 16 columns.  MULTI (more than one chunk)
+// keeps the running residue sums of the thread's 128 elements packed in 64
+// registers.  Bound: the BF16 tensor pipe (0.65 us of epilogue against 2.6 us of
+// MMAs per item at k = 512).
+template <bool MULTI>
+__global__ void __launch_bounds__(tc::THREADS, 1)
+mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                   const __grid_constant__ ModArgs a, int *__restrict__ status) {
+    using namespace tc;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint8_t *sA = smem;
+    uint8_t *sB = smem + STAGES * fg::A_BYTES;
+    uint64_t *full = (uint64_t *)(sB + STAGES * fg::B_BYTES);
+    uint64_t *empty = full + STAGES;
+    uint64_t *tfull = empty + STAGES;
+    uint64_t *tempty = tfull + 2;
+    uint32_t *tmem_slot = (uint32_t *)(tempty + 2);
+    __shared__ int s_abort;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int M = a.tiles.M, N = a.tiles.N, ntiles = a.tiles.ntiles;
+    const int nitems = ntiles * NP;
+    constexpr int CB = CHUNK / KBLK;             // k blocks per chunk
+    const int nch = MULTI ? (a.nkb + CB - 1) / CB : 1;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&tfull[b], 1);
+            mbar_init(&tempty[b], EPI_WARPS);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                         smem_u32(tmem_slot)),
+                     "r"(512u)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int q = 0, issued = 0;
+            bool ok = true;
+            for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+                const int pl = it / ntiles, plane = pl == 0 ? NM : pl - 1;
+                int m0, n0;
+                tile_at(a.tiles, it - pl * ntiles, m0, n0);
+                const int ya = plane * M + m0, yb = plane * N + n0;
+                for (int k = 0; k < a.nkb; ++k, ++q) {
+                    const int s = q % STAGES;
+                    const uint32_t ph = (uint32_t)(q / STAGES) & 1u;
+                    if (s_abort || !mbar_wait(&empty[s], ph ^ 1u, status)) {
+                        s_abort = 1;
+                        ok = false;
+                        break;
+                    }
+                    mbar_expect_tx(&full[s], fg::A_BYTES + fg::B_BYTES);
+                    tma_load_2d(&tmA, &full[s], sA + s * fg::A_BYTES, k * KBLK, ya);
+                    tma_load_2d(&tmB, &full[s], sB + s * fg::B_BYTES, k * KBLK, yb);
+                    ++issued;
+                }
+            }
+            if (!ok) {
+                // let the copies already issued land before the CTA can exit
+                for (int r = (issued > STAGES ? issued - STAGES : 0); r < issued; ++r)
+                    mbar_wait(&full[r % STAGES], (uint32_t)(r / STAGES) & 1u, status);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = idesc_for(kTcBF16, MT, NT);
+            int q = 0, i = 0;
+            bool ok = true;
+            for (int it = blockIdx.x; it < nitems && ok; it += gridDim.x) {
+                const bool mag = it < ntiles;
+                const int chunks = mag ? 1 : nch;
+                for (int c = 0; c < chunks && ok; ++c, ++i) {
+                    const int nk = (!MULTI || mag) ? a.nkb : min(CB, a.nkb - c * CB);
+                    const int b = i & 1;
+                    const uint32_t acc = tmem + (uint32_t)(b * NT);
+                    if (!mbar_wait(&tempty[b], ((uint32_t)(i >> 1) & 1u) ^ 1u, status)) {
+                        s_abort = 1;
+                        ok = false;
+                        break;
+                    }
+                    fence_after();
+                    for (int k = 0; k < nk; ++k, ++q) {
+                        const int s = q % STAGES;
+                        const uint32_t ph = (uint32_t)(q / STAGES) & 1u;
+                        if (s_abort || !mbar_wait(&full[s], ph, status)) {
+                            s_abort = 1;
+                            ok = false;
+                            break;
+                        }
+                        fence_after();
+                        const uint32_t a0 = smem_u32(sA + s * fg::A_BYTES);
+                        const uint32_t b0 = smem_u32(sB + s * fg::B_BYTES);
+#pragma unroll
+                        for (int kk = 0; kk < 4; ++kk)
+                            umma<kTcBF16>(acc, sdesc_sw128(a0 + kk * 32), sdesc_sw128(b0 + kk * 32), idesc,
+                                          (k | kk) != 0 ? 1u : 0u);
+                        umma_commit(&empty[s]);
+                    }
+                    if (ok) umma_commit(&tfull[b]);
+                }
+            }
+        }
+    } else {
+        const int quarter = warp & 3;                // TMEM lane quarter this warp may access
+        const int half = (warp - 2) >> 2;            // column half
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        const int rl = quarter * 32 + lane;          // tile row
+        int i = 0;
+        bool live = true;
+        for (int it = blockIdx.x; it < nitems && live; it += gridDim.x) {
+            const int pl = it / ntiles, t = it - pl * ntiles;
+            int m0, n0;
+            tile_at(a.tiles, t, m0, n0);
+            const bool mag = pl == 0;
+            const int chunks = mag ? 1 : nch;
+            const float p = mag ? 1.0f : a.p[mag ? 0 : pl - 1], ip = mag ? 1.0f : a.ip[mag ? 0 : pl - 1];
+            uint8_t *out = mag ? nullptr
+                               : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 16;
+            uint32_t st[MULTI ? 64 : 1];
+            bool bad = false;
+            for (int c = 0; c < chunks; ++c, ++i) {
+                const int b = i & 1;
+                if (!mbar_wait(&tfull[b], (uint32_t)(i >> 1) & 1u, status)) {
+                    s_abort = 1;
+                    live = false;
+                    break;
+                }
+                fence_after();
+                const uint32_t base = tmem + (uint32_t)(b * NT) + lanes;
+                const bool lastc = c == chunks - 1;
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) {
+                    const int c0 = half * 128 + cc * 32;
+                    if (n0 + c0 >= N) break;         // uniform across the warp
+                    uint32_t r[32];
+                    tmem_ld32(base + (uint32_t)c0, r);
+                    if (mag) {
+                        bool okr = true, okc = true;
+                        if (m0 + rl < M) key_exp(a.keyA[m0 + rl], okr);
+                        if (n0 + c0 + lane < N) key_exp(a.keyB[n0 + c0 + lane], okc);
+                        bad |= !okr | !okc;
+                        if (m0 + rl < M) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) {
+                                const float q = __uint_as_float(r[j]);
+                                bad |= n0 + c0 + j < N && q < a.qmin && q != 0.0f;
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) {
+                            const float v = __uint_as_float(r[j]);
+                            const float q = fmaf(v, ip, kMagic) - kMagic;
+                            float f = fmaf(-q, p, v);
+                            if (!MULTI && f > 127.0f) f -= p;
+                            r[j] = __float_as_uint(f + (MULTI ? kMagic + 256.0f : kMagic));
+                        }
+                        if (MULTI) {
+                            // residues + 256 in 16-bit fields: no carries for 127 chunks
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                const uint32_t w = __byte_perm(r[2 * j], r[2 * j + 1], 0x5410) & 0x03FF03FFu;
+                                st[cc * 16 + j] = c == 0 ? w : st[cc * 16 + j] + w;
+                            }
+                            if (lastc) {
+                                const float off = 256.0f * (float)chunks;
+#pragma unroll
+                                for (int j = 0; j < 32; ++j) {
+                                    const uint32_t w = st[cc * 16 + j / 2];
+                                    const float v = (float)(int)((j & 1) ? w >> 16 : w & 0xFFFFu) - off;
+                                    const float q = fmaf(v, ip, kMagic) - kMagic;
+                                    float f = fmaf(-q, p, v);
+                                    if (f > 127.0f) f -= p;
+                                    r[j] = __float_as_uint(f + kMagic);
+                                }
+                            }
+                        }
+                        if (lastc) {
+#pragma unroll
+                            for (int g = 0; g < 2; ++g) {
+                                uint4 w;
+                                uint32_t *wp = (uint32_t *)&w;
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    const uint32_t *s4 = &r[g * 16 + u * 4];
+                                    wp[u] = __byte_perm(__byte_perm(s4[0], s4[1], 0x0040),
+                                                        __byte_perm(s4[2], s4[3], 0x0040), 0x5410);
+                                }
+                                *(uint4 *)(out + (size_t)(c0 / 16 + g) * (MT * 16)) = w;
+                            }
+                        }
+                    }
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0)
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tempty[b]))
+                                 : "memory");
+                if (s_abort) {
+                    live = false;
+                    break;
+                }
+            }
+            if (mag && __any_sync(0xffffffffu, bad) && lane == 0)
+                a.flag[m0 / MT + a.tiles.tm * (n0 / NT)] = 1;
+        }
+    }
+    fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u)
+                     : "memory");
+    }
+}
+
+// ------------------------------------------------------- reconstruction --
+__device__ __forceinline__ int dp4a_su(uint32_t a, uint32_t b, int c) {
+    int d;
+    asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+    return d;
+}
+
+// The integer sum r_i P/p_i mod P, centred, times 2^ex, rounded once (to
+// nearest, ties to even) to FP64, on the integer pipe.
+__device__ __forceinline__ double crt_value(const uint32_t (&g)[NG], const CrtConst &k, int ex) {
+    int q = 8192;
+#pragma unroll
+    for (int i = 0; i < NG; ++i) q = dp4a_su(g[i], k.qw[i], q);
+    q >>= 14;
+    int s[NL];
+#pragma unroll
+    for (int l = 0; l < NL; ++l) {
+        int v = -q * k.P[l];
+#pragma unroll
+        for (int i = 0; i < NG; ++i) v = dp4a_su(g[i], k.w[i][l], v);
+        s[l] = v;
+    }
+    uint32_t w[5];
+    long long acc = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        acc += (long long)(s[4 * i] + (s[4 * i + 1] << 8)) + ((long long)(s[4 * i + 2] + (s[4 * i + 3] << 8)) << 16);
+        w[i] = (uint32_t)acc;
+        acc >>= 32;
+    }
+    const int top = (int)acc + s[16];
+    w[4] = (uint32_t)top;
+    const uint32_t neg = (uint32_t)(top >> 31);
+    // magnitude: (w ^ neg) - neg
+    unsigned long long c = neg & 1u;
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        c += w[i] ^ neg;
+        w[i] = (uint32_t)c;
+        c >>= 32;
+    }
+    // leading word into w[4]
+    int e = ex + 160;                             // value = 0.w4 w3 ... 2^e
+    uint32_t sticky = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (w[4] == 0u) {
+            w[4] = w[3];
+            w[3] = w[2];
+            w[2] = w[1];
+            w[1] = w[0];
+            w[0] = 0u;
+            e -= 32;
+        }
+    }
+    if (w[4] == 0u) return 0.0;
+    const int z = __clz((int)w[4]);
+    const uint32_t h = __funnelshift_l(w[3], w[4], z), l = __funnelshift_l(w[2], w[3], z);
+    sticky = (w[2] << z) | w[1] | w[0];           // z < 32
+    e -= z;
+    unsigned long long m = ((unsigned long long)h << 32) | l;          // leading bit 63
+    const unsigned long long rest = m & 0x7FFull;
+    m >>= 11;                                     // 53 bits
+    const bool up = rest > 0x400ull || (rest == 0x400ull && (sticky || (m & 1ull)));
+    // e in [-900 - 122, 900 + 160]: always a normal number; the carry of the
+    // rounding moves into the exponent field by itself
+    const unsigned long long bits = ((unsigned long long)(e + 1021) << 52) + m + (up ? 1ull : 0ull) +
+                                    ((unsigned long long)(neg & 1u) << 63);
+    return __longlong_as_double((long long)bits);
+}
+
+// C from the residues.  A block takes 32 columns of a tile (8 blocks per tile), a
+// thread one row x 16 columns: its 17 residue loads are 16 bytes each,
+// contiguous over the warp, and C is read and written along columns, a warp
+// per 256 bytes.  About 230 integer operations per element; 17 bytes of residues and
+// 16 of C move.
+__global__ void __launch_bounds__(256)
+mod_crt_kernel(const __grid_constant__ TileMap tiles, const uint8_t *__restrict__ res,
+               const uint8_t *__restrict__ flag, const unsigned *__restrict__ keyA,
+               const unsigned *__restrict__ keyB, int bits2, double alpha, double beta,
+               double *__restrict__ C, int ldC, const __grid_constant__ CrtConst k) {
+    const int t = blockIdx.x >> 3, part = blockIdx.x & 7;
+    int m0, n0;
+    tile_at(tiles, t, m0, n0);
+    if (flag[m0 / MT + tiles.tm * (n0 / NT)]) return;     // left to the FP64 kernel
+    const int rl = threadIdx.x & 127, cg = part * 2 + (threadIdx.x >> 7);
+    const int row = m0 + rl, col0 = n0 + cg * 16;
+    if (row >= tiles.M || col0 >= tiles.N) return;
+    if (tiles.tri == 1 && row < col0) return;
+    if (tiles.tri == 2 && row > col0 + 15) return;
+    const size_t tile_bytes = (size_t)MT * NT;
+    const uint8_t *src = res + (size_t)t * tile_bytes + (size_t)cg * (MT * 16) + (size_t)rl * 16;
+    bool ok;
+    const int ea = key_exp(keyA[row], ok) - bits2;
+    const bool beta1 = beta == 1.0;
+    uint4 w[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) w[i] = __ldcs((const uint4 *)(src + (size_t)i * tiles.ntiles * tile_bytes));
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        uint32_t x[NM];
+#pragma unroll
+        for (int i = 0; i < NM; ++i) x[i] = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+            const int col = col0 + u * 4 + v;
+            if (col >= tiles.N) continue;
+            if (tiles.tri == 1 && row < col) continue;
+            if (tiles.tri == 2 && row > col) continue;
+            uint32_t g[NG];
+#pragma unroll
+            for (int i = 0; i + 3 < NM; i += 4) {
+                const uint32_t lo = __byte_perm(x[i], x[i + 1], v | ((4 + v) << 4));
+                const uint32_t hi = __byte_perm(x[i + 2], x[i + 3], v | ((4 + v) << 4));
+                g[i / 4] = __byte_perm(lo, hi, 0x5410);
+            }
+            g[NG - 1] = (x[NM - 1] >> (8 * v)) & 0xFFu;
+            const double s = crt_value(g, k, ea + key_exp(keyB[col], ok));
+            double *c = C + (size_t)row + (size_t)col * ldC;
+            const double cv = *c;
+            *c = fma(alpha, s, beta1 ? cv : beta * cv);
+        }
+    }
+}
+static_assert(NM % 4 == 1, "the last residue group holds one modulus");
+
+size_t up256(size_t b) { return (b + 255) / 256 * 256; }
+
+struct Layout {
+    size_t keyA, keyB, flag, zeroed, planesA, planesB, res, total;
+};
+Layout layout_for(int m, int n, int Kp, const TileMap &t) {
+    Layout l{};
+    l.keyA = 0;
+    l.keyB = up256((size_t)m * 4);
+    l.flag = l.keyB + up256((size_t)n * 4);
+    l.zeroed = l.flag + up256((size_t)t.tm * t.tn);
+    l.planesA = l.zeroed;
+    l.planesB = l.planesA + up256((size_t)NP * m * Kp * 2);
+    l.res = l.planesB + up256((size_t)NP * n * Kp * 2);
+    l.total = l.res + (size_t)NM * t.ntiles * MT * NT;
+    return l;
+}
+
+constexpr int kBlkK = 4096, kBlkMN = 4096;        // one block product at most: 1.5 GB of scratch
+
+// One block product in the scratch `ws` (layout_for(m, n, Kp, tiles).total bytes).
+int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int ldA,
+              const double *B, int ldB, double beta, double *C, int ldC, int tri, char *ws, int *status,
+              cudaStream_t s) {
+    const Consts &cs = consts();
+    const int Kp = ceil_div(k, KBLK) * KBLK;
+    const TileMap tiles = make_tiles(m, n, tri);
+    const Layout l = layout_for(m, n, Kp, tiles);
+    int lk = 0;
+    while ((1 << lk) < k) ++lk;
+    int bits = (cs.log2P - 2 - lk) / 2;
+    if (bits > 61) bits = 61;
+    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (__nv_bfloat16 *)(ws + l.planesA)};
+    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (__nv_bfloat16 *)(ws + l.planesB)};
+    FG_CUDA(cudaMemsetAsync(ws, 0, l.zeroed, s));
+    {
+        KTimer kt(kFamAux, s, 0.0, 8.0 * k * ((double)m + n));
+        const int ba = exp_blocks(m, k, oa.rcontig), bb = exp_blocks(n, k, ob.rcontig);
+        mod_exp_kernel<<<ba + bb, 256, 0, s>>>(oa, ob, k, ba);
+        FG_CUDA(cudaGetLastError());
+    }
+    {
+        KTimer kt(kFamAux, s, 0.0, (8.0 + 2.0 * NP) * Kp * ((double)m + n));
+        const int ba = ceil_div(m, 32) * (Kp / KBLK), bb = ceil_div(n, 32) * (Kp / KBLK);
+        mod_residue_kernel<<<ba + bb, 256, 0, s>>>(oa, ob, k, Kp, bits, ba, cs.res);
+        FG_CUDA(cudaGetLastError());
+    }
+    CUtensorMap ma, mb;
+    int rc = tc::make_kmajor_map(&ma, kTcBF16, oa.planes, NP * m, Kp, Kp, MT);
+    if (rc == kOk) rc = tc::make_kmajor_map(&mb, kTcBF16, ob.planes, NP * n, Kp, Kp, NT);
+    if (rc != kOk) return rc;
+    ModArgs a{};
+    a.tiles = tiles;
+    a.nkb = Kp / KBLK;
+    a.qmin = (float)(k * ldexp(1.0, 51 - bits));
+    a.res = (uint8_t *)(ws + l.res);
+    a.flag = (uint8_t *)(ws + l.flag);
+    a.keyA = oa.key;
+    a.keyB = ob.key;
+    for (int i = 0; i < NM; ++i) {
+        a.p[i] = cs.res.p[i];
+        a.ip[i] = cs.res.ip[i];
+    }
+    const int items = tiles.ntiles * NP, sms = num_sms();
+    const int grid = items < sms ? items : sms;
+    {
+        KTimer kt(kFamGemm, s, 2.0 * (tri ? 0.5 : 1.0) * m * (double)n * k,
+                  8.0 * ((double)m * k + (double)k * n + 2.0 * m * n));
+        static DeviceOnce once1, onceN;
+        if (Kp <= CHUNK) {
+            if ((rc = set_smem_once(once1, (const void *)mod_product_kernel<false>, (int)MOD_SMEM)) != kOk) return rc;
+            mod_product_kernel<false><<<grid, tc::THREADS, MOD_SMEM, s>>>(ma, mb, a, status);
+        } else {
+            if ((rc = set_smem_once(onceN, (const void *)mod_product_kernel<true>, (int)MOD_SMEM)) != kOk) return rc;
+            mod_product_kernel<true><<<grid, tc::THREADS, MOD_SMEM, s>>>(ma, mb, a, status);
+        }
+        FG_CUDA(cudaGetLastError());
+    }
+    {
+        KTimer kt(kFamAux, s, 0.0, (NM + 16.0) * m * (double)n);
+        mod_crt_kernel<<<tiles.ntiles * 8, 256, 0, s>>>(tiles, a.res, a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta,
+                                                        C, ldC, cs.crt);
+        FG_CUDA(cudaGetLastError());
+    }
+    // tiles the check refused
+    return dgemm_flagged_launch(ta ? 'T' : 'N', tb ? 'T' : 'N', m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, tri,
+                                a.flag, tiles.tm, s);
+}
+
+int g_mode = -1;
+bool mod_enabled() {
+    // FLENS_GB300_DGEMM=fma|dmma selects an FP64-pipe kernel for every product
+    if (g_mode < 0) {
+        const char *e = getenv("FLENS_GB300_DGEMM");
+        g_mode = (e && *e) ? 0 : 1;
+    }
+    return g_mode == 1;
+}
+
+}  // namespace
+
+// Estimated microseconds of the two routes, from measurements at the sizes
+// named: the FP64 kernel runs at 1.1 TFLOP/s; a residue product costs its
+// launches, its work items in waves over the SMs (5.2 ns per unit of k and
+// tile), 50 bytes of operand traffic per element and 40 per element of C.
+bool mod_gemm_wins(int m, int n, int k, int tri) {
+    if (n <= 16 || m <= 16 || k < 32 || !mod_enabled()) return false;
+    const double half = tri ? 0.5 : 1.0;
+    const double fp64 = half * 2.0 * m * (double)n * k / 1.1e6;
+    if (fp64 < 40.0) return false;
+    const int sms = num_sms() > 0 ? num_sms() : 1;
+    const double items = ceil(half * ceil_div(m, MT) * ceil_div(n, NT) * (double)NP / sms);
+    const double mod = 30.0 + items * (1.0 + 0.0052 * k) + 50.0e-6 / 3.0 * k * ((double)m + n) +
+                       half * 40.0e-6 / 3.0 * m * (double)n;
+    return mod < 0.9 * fp64;
+}
+
+// C <- beta*C + alpha*op(A)*op(B) (tri 1/2: only the lower/upper triangle of a
+// square C) through residues.  kErrUnsupported when the route does not apply
+// (a stream under capture, no scratch memory, or the FP64 route is faster):
+// nothing has been launched then and the caller takes the FP64 kernel.
+int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
+                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s) {
+    if (!mod_gemm_wins(m, n, k, tri)) return kErrUnsupported;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return kErrUnsupported;
+    }
+    // its scratch would be freed while the graph still names it
+    if (cap != cudaStreamCaptureStatusNone) return kErrUnsupported;
+    const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
+    // block product sizes: equal parts of at most kBlkMN x kBlkMN x kBlkK
+    auto part = [](int x, int cap_, int unit) {
+        const int parts = ceil_div(x, cap_);
+        return ceil_div(ceil_div(x, parts), unit) * unit;
+    };
+    const int kb = part(k, kBlkK, KBLK);
+    // a shallow product may take larger blocks of C for the same scratch
+    const int capMN = kb <= 1024 ? 2 * kBlkMN : kBlkMN;
+    const int mb = part(m, capMN, NT), nb = part(n, capMN, NT);
+    const int mm = mb < m ? mb : m, nn = nb < n ? nb : n, kk = kb < k ? kb : k;
+    const Layout l = layout_for(mm, nn, ceil_div(kk, KBLK) * KBLK,
+                                make_tiles(mm, nn, tri && mb >= m && nb >= n ? tri : 0));
+    int *status = nullptr;
+    char *ws = (char *)scratch_acquire(l.total, s, &status);
+    if (!ws) return kErrUnsupported;
+    trace("dgemm: m=%d n=%d k=%d engine=residues blocks of %d x %d x %d", m, n, k, mm, nn, kk);
+    int rc = kOk;
+    for (int k0 = 0; k0 < k && rc == kOk; k0 += kb)
+        for (int i0 = 0; i0 < m && rc == kOk; i0 += mb)
+            for (int j0 = 0; j0 < n && rc == kOk; j0 += nb) {
+                int bt = tri;
+                const int bm = m - i0 < mb ? m - i0 : mb, bn = n - j0 < nb ? n - j0 : nb;
+                if (tri && i0 != j0) {
+                    if ((tri == 1) != (i0 > j0)) continue;     // the other triangle
+                    bt = 0;
+                }
+                const int bk = k - k0 < kb ? k - k0 : kb;
+                rc = mod_block(ta, tb, bm, bn, bk, alpha, A + (ta ? k0 + (size_t)i0 * ldA : i0 + (size_t)k0 * ldA),
+                               ldA, B + (tb ? j0 + (size_t)k0 * ldB : k0 + (size_t)j0 * ldB), ldB,
+                               k0 == 0 ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, ws, status, s);
+            }
+    scratch_release(ws, s);
+    return rc;
+}
+
+}  // namespace fg

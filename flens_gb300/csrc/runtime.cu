@@ -94,7 +94,10 @@ namespace {
 struct Registry {
     std::mutex mu;
     std::map<std::pair<int, cudaStream_t>, Workspace *> map;
+    std::map<int, cudaMemPool_t> pools;
     ~Registry() {
+        for (auto &kv : pools)
+            if (kv.second) cudaMemPoolDestroy(kv.second);
         // Library unload: free what is still allocated.  Errors are ignored
         // (the CUDA runtime may already be shutting down).
         for (auto &kv : map) {
@@ -235,6 +238,50 @@ void *workspace_slot(cudaStream_t stream, int slot, size_t bytes) {
         w->slot_bytes[slot] = want;
     }
     return w->slot_buf[slot];
+}
+
+void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status) {
+    Workspace *w = workspace_for(stream, 0);
+    if (!w) return nullptr;
+    *status = w->status;
+    int k = g_fail_allocs.load();
+    while (k > 0)
+        if (g_fail_allocs.compare_exchange_weak(k, k - 1)) return nullptr;
+    cudaMemPool_t pool = nullptr;
+    {
+        Registry &r = registry();
+        std::lock_guard<std::mutex> lock(r.mu);
+        auto it = r.pools.find(w->device);
+        if (it != r.pools.end()) {
+            pool = it->second;
+        } else {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof props);
+            props.allocType = cudaMemAllocationTypePinned;
+            props.handleTypes = cudaMemHandleTypeNone;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = w->device;
+            unsigned long long keep = kScratchKeep;
+            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+                cudaGetLastError();
+                pool = nullptr;
+            } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+                cudaGetLastError();
+            }
+            r.pools[w->device] = pool;
+        }
+    }
+    void *p = nullptr;
+    if (!pool || cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    g_dev_allocs.fetch_add(1);
+    return p;
+}
+
+void scratch_release(void *p, cudaStream_t stream) {
+    if (p && cudaFreeAsync(p, stream) != cudaSuccess) cudaGetLastError();
 }
 
 int set_smem_once(DeviceOnce &once, const void *fn, int bytes) {

@@ -411,15 +411,17 @@ int launch_diag(int kb, const T *M0, long long mi, long long mp, bool lowerM, bo
 
 template <typename T>
 int gemm_t(char ta, char tb, int m, int n, int k, T alpha, const T *A, int ldA, const T *B,
-           int ldB, T beta, T *C, int ldC, cudaStream_t s);
+           int ldB, T beta, T *C, int ldC, bool fixed, cudaStream_t s);
 template <>
 int gemm_t<double>(char ta, char tb, int m, int n, int k, double alpha, const double *A, int ldA,
-                   const double *B, int ldB, double beta, double *C, int ldC, cudaStream_t s) {
-    return dgemm_launch(ta, tb, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, s);
+                   const double *B, int ldB, double beta, double *C, int ldC, bool fixed,
+                   cudaStream_t s) {
+    // caller-supplied scratch (fixed): no product that allocates its own
+    return (fixed ? dgemm_fp64_launch : dgemm_launch)(ta, tb, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, s);
 }
 template <>
 int gemm_t<float>(char ta, char tb, int m, int n, int k, float alpha, const float *A, int ldA,
-                  const float *B, int ldB, float beta, float *C, int ldC, cudaStream_t s) {
+                  const float *B, int ldB, float beta, float *C, int ldC, bool, cudaStream_t s) {
     return sgemm_launch(ta, tb, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, s);
 }
 
@@ -476,13 +478,13 @@ int trsm_launch_t(char side, char upLo, char transA, char diag, int m, int n,
             const char opA = (mi == 1) ? 'N' : 'T';
             const T *Ap = (mi == 1) ? A + r0 + (size_t)k0 * ldA : A + k0 + (size_t)r0 * ldA;
             st = gemm_t<T>(opA, 'N', rn, n, kb, T(-1), Ap, ldA, B + k0, ldB, T(1), B + r0, ldB,
-                           stream);
+                           fx != nullptr, stream);
         } else {
             // B[:,R] -= B[:,blk] * M[R,blk]^T;  M[R,blk]^T(p,r) = A[r*mi + p*mp]
             const char opA = (mp == 1) ? 'N' : 'T';
             const T *Ap = (mp == 1) ? A + k0 + (size_t)r0 * ldA : A + r0 + (size_t)k0 * ldA;
             st = gemm_t<T>('N', opA, m, rn, kb, T(-1), B + (size_t)k0 * ldB, ldB, Ap, ldA, T(1),
-                           B + (size_t)r0 * ldB, ldB, stream);
+                           B + (size_t)r0 * ldB, ldB, fx != nullptr, stream);
         }
         if (st != kOk) return st;
     }

@@ -1,0 +1,200 @@
+"""The FP64 product by exact residues on the tensor cores (mod_gemm.cu), as
+dgemm and dsyrk take it for large products.
+
+Exactness: integer operands give the integer product itself.  Accuracy: sampled
+elements against rational arithmetic, with the route's own bound (rounding of
+the operands below 4 * 2^-53 * |A||B|, one rounding of the sum, one or two of C).
+Tiles the data check refuses (graded rows, non-finite entries, extreme
+exponents) come from the FP64 kernel and meet its bound k * 2^-53 * |A||B|.
+"""
+from __future__ import annotations
+
+import ctypes
+from fractions import Fraction
+
+import numpy as np
+import pytest
+
+import flens_gb300 as fg
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _dev(cuda, X, pad=0):
+    import torch
+    r, c = X.shape
+    t = torch.zeros((c, r + pad), dtype=torch.float64, device=cuda).t()[:r]
+    t.copy_(torch.from_numpy(np.ascontiguousarray(X)))
+    return t
+
+
+def _gemm(cuda, ta, tb, alpha, A, B, beta, C, pad=0):
+    """The product and the number of kernels it took (1: the FP64 kernel alone)."""
+    dA, dB, dC = _dev(cuda, A, pad), _dev(cuda, B, pad), _dev(cuda, C, pad)
+    before = fg.lib().flens_gb300_launch_count()
+    fg.dgemm_dev(ta, tb, alpha, dA, dB, beta, dC)
+    used = fg.lib().flens_gb300_launch_count() - before
+    fg.sync()
+    return dC.cpu().numpy(), used
+
+
+def _op(X, t):
+    return X if t == "N" else X.T
+
+
+# tile edges (128 x 256), one and several 1024-deep chunks, two k blocks (4097)
+SHAPES = [(300, 300, 300), (128, 256, 1024), (129, 257, 1025), (513, 255, 640), (257, 1100, 100),
+          (200, 100, 4097), (2000, 40, 2050)]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+@pytest.mark.parametrize("ta,tb", ["NN", "NT", "TN", "TT"])
+def test_integer_products_exact(cuda, m, n, k, ta, tb):
+    r = np.random.default_rng(m + n + k)
+    lim = 1 << 19
+    A = r.integers(-lim, lim + 1, (m, k) if ta == "N" else (k, m)).astype(np.float64)
+    B = r.integers(-lim, lim + 1, (k, n) if tb == "N" else (n, k)).astype(np.float64)
+    C = r.integers(-lim, lim + 1, (m, n)).astype(np.float64)
+    got, used = _gemm(cuda, ta, tb, -1.0, A, B, 2.0, C, pad=3)
+    assert used >= 5, "the FP64 kernel alone"
+    want = 2 * C.astype(np.int64) - _op(A, ta).astype(np.int64) @ _op(B, tb).astype(np.int64)
+    assert np.array_equal(got.astype(np.int64), want)
+
+
+@pytest.mark.parametrize("m,n,k,spread", [(400, 500, 300, 0), (300, 300, 3000, 2), (1500, 600, 64, 1)])
+def test_accuracy_sampled(cuda, m, n, k, spread):
+    r = np.random.default_rng(k)
+    A = r.uniform(-1, 1, (m, k)) * 2.0 ** r.integers(-40, 41, (m, 1)) * 2.0 ** r.integers(-spread, spread + 1, (m, k))
+    B = r.uniform(-1, 1, (k, n)) * 2.0 ** r.integers(-40, 41, (1, n))
+    C = np.zeros((m, n))
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, C)
+    assert used >= 5
+    for i, j in zip(r.integers(0, m, 60), r.integers(0, n, 60)):
+        ex = sum(Fraction(a) * Fraction(b) for a, b in zip(A[i].tolist(), B[:, j].tolist()))
+        mag = float(np.abs(A[i]) @ np.abs(B[:, j]))
+        assert abs(Fraction(got[i, j]) - ex) <= Fraction(4 * U * mag + U * abs(float(ex)))
+
+
+def _refused(cuda, A, B, C, alpha=1.0, beta=1.0):
+    k = A.shape[1]
+    got, used = _gemm(cuda, "N", "N", alpha, A, B, beta, C)
+    assert used >= 5
+    with np.errstate(all="ignore"):
+        want = beta * C + alpha * (A @ B)
+        mag = abs(beta) * np.abs(C) + np.abs(alpha) * (np.abs(A) @ np.abs(B))
+    fin = np.isfinite(want)
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    assert np.array_equal(got[~fin & ~np.isnan(want)], want[~fin & ~np.isnan(want)])
+    with np.errstate(all="ignore"):
+        assert np.all(np.abs(got - want)[fin] <= (2 * (k + 2) * U * mag)[fin])
+
+
+def test_graded_rows_keep_fp64_accuracy(cuda):
+    """One large entry per row where B is tiny: fixed point would lose the rest."""
+    r = np.random.default_rng(5)
+    A, B, C = r.uniform(-1, 1, (400, 300)), r.uniform(-1, 1, (300, 600)), np.zeros((400, 600))
+    A[:200, 0] *= 1e25
+    B[0, :300] *= 1e-25
+    _refused(cuda, A, B, C)
+
+
+def test_special_values(cuda):
+    r = np.random.default_rng(6)
+    A, B, C = r.uniform(-1, 1, (400, 300)), r.uniform(-1, 1, (300, 600)), r.uniform(-1, 1, (400, 600))
+    A[3, 7], A[200, 5], B[11, 400], C[390, 590] = np.nan, np.inf, -np.inf, np.nan
+    A[250], B[:, 20] = 0.0, 0.0                       # exact zeros, and 0 * Inf
+    _refused(cuda, A, B, C, alpha=1.5, beta=0.0)
+
+
+@pytest.mark.parametrize("ea,eb", [(900, -900), (-1000, 40), (500, 300), (-1060, 1000)])
+def test_extreme_exponents(cuda, ea, eb):
+    r = np.random.default_rng(7)
+    A, B = np.ldexp(r.uniform(-1, 1, (300, 300)), ea), np.ldexp(r.uniform(-1, 1, (300, 300)), eb)
+    _refused(cuda, A, B, np.zeros((300, 300)))
+
+
+def test_zero_and_sparse_operands(cuda):
+    """Columns that meet no nonzero give exact zeros; sparse rows stay accurate."""
+    r = np.random.default_rng(8)
+    A, B = r.uniform(-1, 1, (400, 512)), r.uniform(-1, 1, (512, 600))
+    A[:, 256:] = 0.0
+    B[:256, 300:] = 0.0
+    A[5] = 0.0
+    A[7, :] = 0.0
+    A[7, 9] = 0.3
+    _refused(cuda, A, B, np.zeros((400, 600)))
+    got, _ = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, np.zeros((400, 600)))
+    assert np.all(got[:, 300:] == 0.0) and np.all(got[5] == 0.0)
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("trans", "NT")
+@pytest.mark.parametrize("n,k", [(700, 200), (257, 1100), (4400, 70)])
+def test_triangle_products(cuda, uplo, trans, n, k):
+    import torch
+    r = np.random.default_rng(n)
+    A = r.integers(-9, 10, (n, k) if trans == "N" else (k, n)).astype(np.float64)
+    C = r.integers(-9, 10, (n, n)).astype(np.float64)
+    dA, dC = _dev(cuda, A), _dev(cuda, C, 1)
+    before = fg.lib().flens_gb300_launch_count()
+    fg.dsyrk_dev(uplo, trans, -1.0, dA, 1.0, dC)
+    assert fg.lib().flens_gb300_launch_count() - before >= 5
+    fg.sync()
+    X = torch.from_numpy(_op(A, trans)).to(cuda)
+    want = C - (X @ X.t()).cpu().numpy()
+    keep = np.tril(np.ones((n, n)), -1) if uplo == "U" else np.triu(np.ones((n, n)), 1)
+    assert np.array_equal(dC.cpu().numpy(), np.where(keep > 0, C, want))
+
+
+def test_capture_and_no_memory_take_the_fp64_kernel(cuda):
+    import torch
+    r = np.random.default_rng(9)
+    A, B = (_dev(cuda, r.uniform(-1, 1, (500, 500))) for _ in range(2))
+    C = [_dev(cuda, np.zeros((500, 500))) for _ in range(3)]
+    fg.dgemm_dev("N", "N", 1.0, A, B, 0.0, C[0])
+    fg.sync()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        fg.dgemm_dev("N", "N", 1.0, A, B, 0.0, C[1])
+    g.replay()
+    fail = fg.lib().flens_gb300_test_fail_device_allocs
+    fail.argtypes = [ctypes.c_int]
+    fail(1)
+    try:
+        before = fg.lib().flens_gb300_launch_count()
+        fg.dgemm_dev("N", "N", 1.0, A, B, 0.0, C[2])
+        assert fg.lib().flens_gb300_launch_count() - before == 1
+    finally:
+        fail(0)
+    fg.sync()
+    c = [x.cpu().numpy() for x in C]
+    assert np.array_equal(c[1], c[2])
+    assert np.abs(c[0] - c[1]).max() <= 500 * U * 500
+
+
+def test_threads_on_one_stream(cuda):
+    """Calls of several threads on one stream have their own scratch."""
+    import threading
+
+    import torch
+    r = np.random.default_rng(10)
+    ops = [(r.integers(-99, 100, (400, 300)).astype(float), r.integers(-99, 100, (300, 500)).astype(float))
+           for _ in range(8)]
+    dev = [(_dev(cuda, a), _dev(cuda, b), _dev(cuda, np.zeros((400, 500)))) for a, b in ops]
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+
+    def work(i):
+        with torch.cuda.stream(s):
+            for _ in range(10):
+                fg.dgemm_dev("N", "N", 1.0, dev[i][0], dev[i][1], 0.0, dev[i][2])
+
+    ts = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    s.synchronize()
+    for (a, b), (_, _, c) in zip(ops, dev):
+        assert np.array_equal(c.cpu().numpy(), a @ b)
