@@ -946,6 +946,23 @@ int panel_ctas(int sms) {
     return cap;
 }
 
+// Whether the FP64 LU takes the recursive order: its products then go to the
+// tensor cores.  From 2048 columns on: n = 1000, 2000, 4096, 8192 measured
+// 5.4, 11.8, 28, 71 ms against 4.9, 11.9, 49, 320 ms in the right-looking order
+// with look-ahead (the factorisation alone).  Not for a stream under capture, whose products run on the FP64
+// pipe: there the right-looking order with look-ahead is faster (n = 8192: 320
+// against 355 ms).
+bool recursive_lu(int m, int n, cudaStream_t stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const int h = (m < n ? m : n) / 2;
+    if (h < 1024) return false;
+    return cap == cudaStreamCaptureStatusNone && mod_gemm_wins(m - h, n - h, h, 0);
+}
+
 // Outer block of the split-update LU: FLENS_GB300_SPLIT_NB (a multiple of 64),
 // else 512.
 int split_outer_nb() {
@@ -1050,9 +1067,14 @@ size_t getrf_workspace_bytes(int m, int n, int tc_kind, int depth) {
 // and on the tensor cores in `tc_kind` for T = float.  This is the order of
 // LAPACK's dgetrf with a recursive panel; in exact arithmetic the factors
 // and pivots are those of the right-looking loop.
+//
+// recursive: the columns are halved down to panels (left half, U12 by trsm,
+// one product, right half), so that the products are as deep as they are
+// wide and run on the tensor cores by residues (mod_gemm.cu), where a 64-deep
+// update would only move C.
 template <typename T>
 int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int split_nb,
-            cudaStream_t stream) {
+            cudaStream_t stream, bool recursive = false) {
     FG_CUDA(cudaMemsetAsync(info, 0, sizeof(int), stream));
     if (m == 0 || n == 0) return kOk;
     const int mn = m < n ? m : n;
@@ -1090,7 +1112,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
     // n = 16384 FP32 LU spent 114 ms in its updates instead of 49 and the
     // panels did not shorten)
     Workspace *wl = nullptr;
-    if (tc_kind < 0 && lookahead_enabled()) {
+    if (tc_kind < 0 && !recursive && lookahead_enabled()) {
         wl = workspace_side(stream);
         if (!wl) return kErrCuda;
     }
@@ -1151,6 +1173,42 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
                           stream);
     };
 
+    // interchanges of the panel (j, jb) on the columns outside it
+    auto interchange = [&](int j, int jb) -> int {
+        const int ncols = n - jb;
+        if (ncols <= 0) return kOk;
+        const int blocks = ceil_div(ncols, 256 / 32);
+        KTimer ktl(kFamLaswp, stream, 0.0, 0.0);
+        laswp_pairs_kernel<T><<<blocks, 256, 0, stream>>>(A, ldA, ncols, j, jb, ps.swap_cnt, ps.swap_dst,
+                                                          ps.swap_src);
+        FG_CUDA(cudaGetLastError());
+        return kOk;
+    };
+    auto factor = [&](auto &&self, int j, int w) -> int {
+        int st, jb = 0;
+        if (w <= PANEL_NB) {
+            // (a panel of a very tall matrix comes out narrower)
+            ob_end = j + w;
+            if ((st = panel_at(j, stream, &jb, true)) != kOk) return st;
+            if ((st = interchange(j, jb)) != kOk) return st;
+        } else {
+            jb = ceil_div(ceil_div(w, 2), PANEL_NB) * PANEL_NB;
+            if ((st = self(self, j, jb)) != kOk) return st;
+        }
+        const int c = j + jb, r = w - jb;
+        if (r <= 0) return kOk;
+        if ((st = trsm_t<T>('L', 'L', 'N', 'U', jb, r, T(1), A + j + (size_t)j * ldA, ldA,
+                            A + j + (size_t)c * ldA, ldA, stream)) != kOk)
+            return st;
+        if (c < m && (st = update(j, jb, c, r)) != kOk) return st;
+        return self(self, c, r);
+    };
+    if (recursive) {
+        const int st = factor(factor, 0, mn);
+        if (st != kOk || n == mn) return st;
+        return trsm_t<T>('L', 'L', 'N', 'U', mn, n - mn, T(1), A, ldA, A + (size_t)mn * ldA, ldA, stream);
+    }
+
     bool ahead = false;     // the panel at j was launched on the side stream
     auto body = [&]() -> int {
         int jb = 0, st;
@@ -1161,15 +1219,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
             } else if ((st = panel_at(j, stream, &jb, true)) != kOk) {
                 return st;
             }
-            // interchanges on the columns outside the panel
-            const int ncols = n - jb;
-            if (ncols > 0) {
-                const int blocks = ceil_div(ncols, 256 / 32);
-                KTimer ktl(kFamLaswp, stream, 0.0, 0.0);
-                laswp_pairs_kernel<T><<<blocks, 256, 0, stream>>>(A, ldA, ncols, j, jb, ps.swap_cnt,
-                                                                  ps.swap_dst, ps.swap_src);
-                FG_CUDA(cudaGetLastError());
-            }
+            if ((st = interchange(j, jb)) != kOk) return st;
             int next_jb = 0;
             if (j + jb < ob_end) {
                 const int nr = ob_end - j - jb;
@@ -1231,7 +1281,8 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
 }
 
 int dgetrf_launch(int m, int n, double *A, int ldA, int *ipiv, int *info, cudaStream_t stream) {
-    return getrf_t<double>(m, n, A, ldA, ipiv, info, -1, 0, stream);
+    return getrf_t<double>(m, n, A, ldA, ipiv, info, -1, 0, stream,
+                           recursive_lu(m, n, stream));
 }
 
 int dgetrf_split_launch(int m, int n, double *A, int ldA, int *ipiv, int *info, int outer_nb,

@@ -461,6 +461,38 @@ int trsm_launch_t(char side, char upLo, char transA, char diag, int m, int n,
         if (st == kOk) done = true;
         else if (st != kErrUnsupported) return st;
     }
+    // Large FP64 solves by halves: T11 X1 = B1, B2 -= T21 X1, T22 X2 = B2.  The
+    // products are as deep as the halves and go to the tensor cores
+    // (mod_gemm.cu); 64-deep updates would read and write all of B for each.
+    if (!done && sizeof(T) == 8 && !fx && nblk >= 4) {
+        const int h = (nblk / 2) * TRSM_NB;            // first half in storage order
+        if (mod_gemm_wins(left ? ka - h : m, left ? n : ka - h, h, 0)) {
+            const T *A22 = A + h + (size_t)h * ldA;
+            T *B2 = left ? B + h : B + (size_t)h * ldB;
+            const int h2 = ka - h;
+            auto solve = [&](bool second) -> int {
+                return trsm_launch_t<T>(side, upLo, transA, diag, left ? (second ? h2 : h) : m,
+                                        left ? n : (second ? h2 : h), T(1), second ? A22 : A, ldA, second ? B2 : B,
+                                        ldB, stream);
+            };
+            // the stored off-diagonal block of the triangle; op() of it is
+            // transposed exactly when op(A) is
+            const T *Ao = lowerA ? A + h : A + (size_t)h * ldA;
+            const char op = nT ? 'N' : 'T';
+            // solved first: the first half for an effective lower triangle
+            int st = solve(!lowerM);
+            if (st != kOk) return st;
+            if (left)
+                st = lowerM ? gemm_t<T>(op, 'N', h2, n, h, T(-1), Ao, ldA, B, ldB, T(1), B2, ldB, false, stream)
+                            : gemm_t<T>(op, 'N', h, n, h2, T(-1), Ao, ldA, B2, ldB, T(1), B, ldB, false, stream);
+            else
+                st = lowerM ? gemm_t<T>('N', op, m, h2, h, T(-1), B, ldB, Ao, ldA, T(1), B2, ldB, false, stream)
+                            : gemm_t<T>('N', op, m, h, h2, T(-1), B2, ldB, Ao, ldA, T(1), B, ldB, false, stream);
+            if (st == kOk) st = solve(lowerM);
+            if (st != kOk) return st;
+            done = true;
+        }
+    }
     for (int s = 0; !done && s < nblk; ++s) {
         const int bi = lowerM ? s : nblk - 1 - s;
         const int k0 = bi * TRSM_NB;
