@@ -779,6 +779,368 @@ panel32_kernel(float *__restrict__ A, int lda, int mp, int jb, int j0,
     if (b == 0 && tid < 32) panel_moves(jb, j0, ipiv, ps, s_list_row, s_list_src, lane);
 }
 
+// ---- the panel of one thread-block cluster ----------------------------------
+// The same factorisation for panels whose rows fit the shared memory of one
+// cluster of 16 CTAs (16 SMs).  A column costs a search, an exchange of the
+// candidates and an update; across the whole grid the exchange goes through L2
+// (about 3 us a column with its polls and fences), inside a cluster it is one
+// st.async into every CTA's shared memory, which counts its bytes on the
+// receiver's mbarrier: no flags, fences or polls of memory.  Per column:
+//   - every CTA's candidate (largest key, first row) by redux and one block
+//     barrier; the pending update of the candidate row applied on the fly;
+//   - warp w sends candidate row, key and row number to CTA w (and row jj from
+//     its owner); warp 0 sends the candidate's reciprocal after it, so that the
+//     division runs while the rows travel;
+//   - the rest of the previous column's update, a warp per 32 rows and group of
+//     4-column quads, while the exchange is under way;
+//   - every warp settles the pivot from the 16 headers; a thread per row scales
+//     its entry, updates column jj+1 and takes its key for the next search.
+// The interchange of a row is applied where its entries are next read and
+// written by one warp after the next candidate is out.  Three exchange buffers: a
+// CTA can send column jj+3 only after all have sent jj+2, which they do after
+// their last read of column jj's buffer.
+// Bound: the chain search - exchange - settle (about 2200 clocks a column), from
+// about m = 2000 on the 16 SMs' FP64 pipes (m * 32 FMAs a column at 32 per
+// clock); in FP32 shared memory from about m = 6000 on.  Measured per column
+// against the grid panel: FP64 2.2 against 3.8 us at n = 500, 2.5 against 4.0 at
+// 2000, 3.1 against 4.1 at 4096 (whole LU); FP32 n = 16384, panels of the LU 45.9
+// against 59.8 ms.
+constexpr int CP_CS = 16;                       // CTAs of the cluster
+constexpr int CP_T = 512;                       // threads per CTA
+constexpr int CP_NW = CP_T / 32;
+static_assert(CP_NW == CP_CS, "warp w sends to CTA w");
+
+template <typename T>
+struct ClusterBuf {                             // one exchange buffer
+    T row[CP_CS][PANEL_NB];                     // candidate rows
+    T rowjj[PANEL_NB];
+    ulonglong2 head[CP_CS];                     // key, row
+    double rinv[CP_CS];                         // 1 / candidate (0: divide)
+};
+
+template <typename T>
+constexpr uint32_t cluster_bytes() {            // received per column
+    return CP_CS * (PANEL_NB * sizeof(T) + 16 + 8) + PANEL_NB * sizeof(T);
+}
+
+// Shared memory of a CTA: the buffers are static, R rows x 64 columns dynamic.
+template <typename T>
+constexpr size_t cluster_rows_max() {
+    return ((227 * 1024 - 2048 - 3 * sizeof(ClusterBuf<T>)) / (PANEL_NB * sizeof(T))) * CP_CS;
+}
+
+__device__ __forceinline__ uint32_t cp_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cp_map(uint32_t a, uint32_t rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cp_send16(uint32_t dst, uint32_t bar, unsigned long long a, unsigned long long b) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "l"(a), "l"(b), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_send8(uint32_t dst, uint32_t bar, unsigned long long a) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(dst), "l"(a),
+                 "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_send_pair(uint32_t dst, uint32_t bar, double a, double b) {
+    cp_send16(dst, bar, (unsigned long long)__double_as_longlong(a), (unsigned long long)__double_as_longlong(b));
+}
+__device__ __forceinline__ void cp_send_pair(uint32_t dst, uint32_t bar, float a, float b) {
+    cp_send8(dst, bar, (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32));
+}
+__device__ __forceinline__ unsigned long long cp_key(double x) { return pivot_key(x); }
+__device__ __forceinline__ unsigned long long cp_key(float x) { return pivot_key32(x); }
+__device__ __forceinline__ double cp_rinv(double p) { return (p != 0.0 && fabs(p) >= DBL_MIN) ? 1.0 / p : 0.0; }
+__device__ __forceinline__ float cp_rinv(float p) { return (p != 0.0f && fabsf(p) >= FLT_MIN) ? 1.0f / p : 0.0f; }
+__device__ __forceinline__ double cp_fma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float cp_fma(float a, float b, float c) { return fmaf(a, b, c); }
+
+// Bounded wait of the whole block's threads on one phase of an mbarrier.
+__device__ __forceinline__ bool cp_wait(uint32_t bar, uint32_t parity) {
+    for (unsigned i = 0; i < (1u << 20); ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+template <typename T>
+__global__ void __launch_bounds__(CP_T, 1)
+panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__restrict__ ipiv,
+                     int *__restrict__ info, int *__restrict__ status, PanelScratch ps, int R) {
+    extern __shared__ double S_raw[];
+    T *S = reinterpret_cast<T *>(S_raw);
+    __shared__ __align__(16) ClusterBuf<T> buf[3];
+    __shared__ __align__(16) T s_row[PANEL_NB], s_rowjj[PANEL_NB];
+    __shared__ unsigned long long bars[3];
+    __shared__ unsigned long long red_k[2][CP_NW];
+    __shared__ int red_i[2][CP_NW];
+    __shared__ int s_abort;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int b = blockIdx.x;                    // one cluster: the block index is the rank
+    const int rb = b * R, nr = max(0, min(mp, rb + R) - rb);
+
+    if (tid == 0) {
+        for (int i = 0; i < 3; ++i)
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(cp_smem(&bars[i])) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        s_abort = 0;
+    }
+    // columns beyond jb are sent as they are in the exchange: keep them defined
+    {
+        const int nrb = (nr + 31) / 32;
+        for (int u = warp; u < nrb * 4; u += CP_NW) {
+            const int r = (u % nrb) * 32 + lane, c0 = u / nrb;
+            if (r < nr)
+#pragma unroll
+                for (int h = 0; h < 16; ++h) {
+                    const int c = c0 + 4 * h;
+                    S[c * R + r] = c < jb ? A[(size_t)(rb + r) + (size_t)c * lda] : T(0);
+                }
+        }
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+
+    // pivot keys of column 0: thread per row (rows tid, tid + 512)
+    unsigned long long nbk = kKeyNone;
+    int nbi = INT_MAX;
+    for (int r = tid; r < nr; r += CP_T) {
+        const unsigned long long key = cp_key(S[r]);
+        if (better(key, rb + r, nbk, nbi)) { nbk = key; nbi = rb + r; }
+    }
+
+    // row moves of the interchanges, kept by CTA 0's last warp: entry e =
+    // lane + 32 h is (row, source); the first jb rows are the panel's top
+    int mv_row[4], mv_src[4], mv_cnt = jb;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) mv_row[h] = mv_src[h] = (lane + 32 * h < jb) ? j0 + lane + 32 * h : -1;
+
+    // the column whose update is pending (-1: none), its pivot row and buffers
+    int d_jj = -1, d_gs = -1;
+    bool d_swap = false;
+    const T *dP = nullptr, *dO = nullptr;
+    // deferred writes of the interchange of column d_jj: row d_jj <- dP, row
+    // d_gs <- dO (but its columns d_jj and d_jj + 1, which hold newer values)
+    auto write_swap = [&]() {
+        if (!d_swap) return;
+        const int rj = d_jj - rb, rg = d_gs - rb;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c = lane + 32 * h;
+            if (c < jb) {
+                if (rj >= 0 && rj < nr) S[c * R + rj] = dP[c];
+                // columns beyond d_jj + 1 are written by the pending update
+                if (rg >= 0 && rg < nr && c < d_jj) S[c * R + rg] = dO[c];
+            }
+        }
+    };
+
+    int bi = 0;                                  // buffer of this column
+    uint32_t phase = 0;                          // its parity
+    for (int jj = 0; jj < jb; ++jj) {
+        // -- this CTA's candidate among its rows g >= jj
+        unsigned long long k = nbk;
+        int i = nbi;
+        warp_argmax(k, i);
+        if (lane == 0) { red_k[jj & 1][warp] = k; red_i[jj & 1][warp] = i; }
+        const uint32_t bar = cp_smem(&bars[bi]);
+        if (tid == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                         "r"(cluster_bytes<T>())
+                         : "memory");
+        if (__syncthreads_or(s_abort)) break;                        // B1
+        k = lane < CP_NW ? red_k[jj & 1][lane] : kKeyNone;
+        i = lane < CP_NW ? red_i[jj & 1][lane] : INT_MAX;
+        warp_argmax(k, i);
+        // entry c of local row x with the pending interchange and update
+        auto fin = [&](int x, int c) -> T {
+            const bool sw = d_swap && rb + x == d_gs && c != d_jj && c != d_jj + 1;
+            const T v = sw ? dO[c] : S[c * R + x];
+            return (d_jj < 0 || c < d_jj + 2) ? v : cp_fma(-dP[c], S[d_jj * R + x], v);
+        };
+        // candidate row by warps 0 and 1, row jj by warps 2 and 3 (once per CTA:
+        // an FP64 instruction holds its scheduler's pipe for 64 clocks)
+        const bool has_i = i != INT_MAX, has_jj = jj >= rb && jj < rb + nr;
+        if (warp < 4) {
+            const int c = (warp & 1) * 32 + lane;
+            if (warp < 2) s_row[c] = has_i ? fin(i - rb, c) : T(0);
+            else if (has_jj) s_rowjj[c] = fin(jj - rb, c);
+        }
+        __syncthreads();                                             // B1b
+        // -- the candidate to CTA `warp`
+        ClusterBuf<T> &cur = buf[bi];
+        {
+            const uint32_t rbar = cp_map(bar, warp);
+            cp_send_pair(cp_map(cp_smem(&cur.row[b][2 * lane]), warp), rbar, s_row[2 * lane], s_row[2 * lane + 1]);
+            if (has_jj)
+                cp_send_pair(cp_map(cp_smem(&cur.rowjj[2 * lane]), warp), rbar, s_rowjj[2 * lane],
+                             s_rowjj[2 * lane + 1]);
+            if (lane == 0) cp_send16(cp_map(cp_smem(&cur.head[b]), warp), rbar, k, (unsigned long long)(unsigned)i);
+        }
+        if (warp == 0) {
+            const double r = (double)cp_rinv(s_row[jj]);
+            if (lane < CP_CS)
+                cp_send8(cp_map(cp_smem(&cur.rinv[b]), lane), cp_map(bar, lane),
+                         (unsigned long long)__double_as_longlong(r));
+        }
+        // -- the pending update of column d_jj: columns >= d_jj + 2
+        if (d_jj >= 0) {
+            const int nrb = (nr + 31) / 32;
+            const int ncg = nrb >= CP_NW ? 1 : CP_NW / max(nrb, 1);
+            const int q0 = (d_jj + 2) >> 2, q1 = (jb + 3) >> 2;
+            for (int u = warp; u < nrb * ncg; u += CP_NW) {
+                const int cg = u / nrb, r = (u - cg * nrb) * 32 + lane, g = rb + r;
+                if (r < nr && g > d_jj) {
+                    const T l = S[d_jj * R + r];
+                    const bool sw = d_swap && g == d_gs;
+                    for (int q = q0 + cg; q < q1; q += ncg) {
+                        T p[4], v[4];
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) p[h] = dP[4 * q + h];
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) v[h] = sw ? dO[4 * q + h] : S[(4 * q + h) * R + r];
+#pragma unroll
+                        for (int h = 0; h < 4; ++h)
+                            if (4 * q + h >= d_jj + 2) S[(4 * q + h) * R + r] = cp_fma(-p[h], l, v[h]);
+                    }
+                }
+            }
+            if (warp == CP_NW - 2) write_swap();
+        }
+        // -- the 16 candidates
+        if (!cp_wait(bar, phase)) {
+            atomicOr(status, kDevBarrierTimeout);
+            s_abort = 1;
+        }
+        unsigned long long gk = kKeyNone;
+        int gi = INT_MAX;
+        if (lane < CP_CS) {
+            const ulonglong2 h = cur.head[lane];
+            gk = h.x;
+            gi = (int)(unsigned)h.y;
+        }
+        warp_argmax(gk, gi);
+        const T ajj = cur.rowjj[jj];
+        const bool jnan = cp_key(ajj) == 1ull;    // integer tests: no FP64 compares
+        const int gs = (jnan || gi < 0 || gi >= mp) ? jj : gi;  // (out of range: a wait gave up)
+        const int src = gs / R;
+        const T *P = cur.row[src], *O = cur.rowjj;
+        if (jnan) P = O;
+        const T pv = P[jj];
+        const T rinv = jnan ? T(0) : (T)cur.rinv[src];
+        const bool pnz = cp_key(pv) != 2ull, rnz = cp_key(rinv) != 2ull;
+        const bool swap = pnz && gs != jj;
+        // -- thread per row: scale, column jj + 1, next key
+        nbk = kKeyNone;
+        nbi = INT_MAX;
+        for (int r = tid; r < nr; r += CP_T) {
+            const int g = rb + r;
+            if (g <= jj) continue;
+            const bool sw = swap && g == gs;
+            T l = sw ? O[jj] : S[jj * R + r];
+            if (pnz) l = rnz ? l * rinv : l / pv;
+            S[jj * R + r] = l;
+            if (jj + 1 < jb) {
+                const T v = cp_fma(-P[jj + 1], l, sw ? O[jj + 1] : S[(jj + 1) * R + r]);
+                S[(jj + 1) * R + r] = v;
+                const unsigned long long key = cp_key(v);
+                if (better(key, g, nbk, nbi)) { nbk = key; nbi = g; }
+            }
+        }
+        d_jj = jj;
+        d_gs = gs;
+        d_swap = swap;
+        dP = P;
+        dO = O;
+        if (b == 0 && warp == CP_NW - 1) {
+            if (lane == 0) {
+                ipiv[j0 + jj] = j0 + gs + 1;
+                if (!pnz && *info == 0) *info = j0 + jj + 1;
+            }
+            // the interchange jj <-> gs in the list of moves
+            const int p = j0 + gs;
+            int pos = gs;
+            if (gs >= jb) {
+                pos = -1;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const unsigned hit = __ballot_sync(0xffffffffu, mv_row[h] == p);
+                    if (hit) pos = 32 * h + __ffs(hit) - 1;
+                }
+                if (pos < 0) {
+                    pos = mv_cnt++;
+#pragma unroll
+                    for (int h = 0; h < 4; ++h)
+                        if (lane + 32 * h == pos) mv_row[h] = mv_src[h] = p;
+                }
+            }
+            int a = 0, c = 0;
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const int x = __shfl_sync(0xffffffffu, mv_src[h], jj & 31);
+                const int y = __shfl_sync(0xffffffffu, mv_src[h], pos & 31);
+                if (jj >> 5 == h) a = x;
+                if (pos >> 5 == h) c = y;
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (lane + 32 * h == jj) mv_src[h] = c;
+                if (lane + 32 * h == pos) mv_src[h] = a;
+            }
+        }
+        if (++bi == 3) {
+            bi = 0;
+            phase ^= 1u;
+        }
+    }
+    // the last interchange
+    if (warp == CP_NW - 2 && d_jj >= 0) write_swap();
+    __syncthreads();
+    // no CTA leaves while others may still send to it
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+    if (s_abort) return;
+    {
+        const int nrb = (nr + 31) / 32;
+        for (int u = warp; u < nrb * 4; u += CP_NW) {
+            const int r = (u % nrb) * 32 + lane, c0 = u / nrb;
+            if (r < nr)
+#pragma unroll
+                for (int h = 0; h < 16; ++h) {
+                    const int c = c0 + 4 * h;
+                    if (c < jb) A[(size_t)(rb + r) + (size_t)c * lda] = S[c * R + r];
+                }
+        }
+    }
+    if (b == 0 && warp == CP_NW - 1) {
+        int base = 0;
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const bool mv = lane + 32 * h < mv_cnt && mv_row[h] != mv_src[h];
+            const unsigned m = __ballot_sync(0xffffffffu, mv);
+            if (mv) {
+                const int e = base + __popc(m & ((1u << lane) - 1u));
+                ps.swap_dst[e] = mv_row[h];
+                ps.swap_src[e] = mv_src[h];
+            }
+            base += __popc(m);
+        }
+        if (lane == 0) *ps.swap_cnt = base;
+    }
+}
+
+
 // Apply the panel's row moves to columns [0, cSplit) and [cSplit+skip, ...),
 // ncols columns in total; one warp per column.
 template <typename T>
@@ -932,6 +1294,62 @@ bool lookahead_enabled() {
         return !(e && atoi(e) == 0);
     }();
     return on;
+}
+
+// Rows up to which a panel takes the cluster kernel: FLENS_GB300_PANEL_CLUSTER
+// (0: never), else as many as fit one cluster's shared memory in FP32 (13,600; per
+// column 1.7 us at 4096 rows, 3.0 at 13,000, the grid panel 3.5), and 6000 in
+// FP64, where the 16 SMs' FP64 pipes come level with the grid panel's 4.1 us.
+template <typename T>
+int cluster_rows() {
+    static int rows = [] {
+        const char *e = getenv("FLENS_GB300_PANEL_CLUSTER");
+        const int cap = (int)cluster_rows_max<T>(), want = sizeof(T) == 8 ? 6000 : cap;
+        const int v = e && *e ? atoi(e) : want;
+        return v < cap ? v : cap;
+    }();
+    return rows;
+}
+
+cudaLaunchConfig_t cluster_config(cudaLaunchAttribute *attr, size_t smem, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CP_CS);
+    cfg.blockDim = dim3(CP_T);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = CP_CS;
+    attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+// Whether a cluster of 16 full-size CTAs can be resident on the device
+// (16 SMs of one GPC); asked once per device.
+template <typename T>
+bool cluster_fits() {
+    static int known[64];                         // 0: not asked, 1: yes, 2: no
+    const int d = device_id();
+    if (d < 0 || d >= 64) return false;
+    int v = __atomic_load_n(&known[d], __ATOMIC_ACQUIRE);
+    if (v == 0) {
+        const size_t smem = cluster_rows_max<T>() / CP_CS * PANEL_NB * sizeof(T);
+        const void *fn = (const void *)panel_cluster_kernel<T>;
+        cudaLaunchAttribute attr;
+        cudaLaunchConfig_t cfg = cluster_config(&attr, smem, nullptr);
+        int n = 0;
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        v = n >= 1 ? 1 : 2;
+        __atomic_store_n(&known[d], v, __ATOMIC_RELEASE);
+        trace("getrf<%d>: clusters of %d CTAs resident: %d", (int)sizeof(T), CP_CS, n);
+    }
+    return v == 1;
 }
 
 // CTAs of a panel grid: at most one per SM and PANEL_GMAX, or
@@ -1130,8 +1548,22 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
     // against 322.8 ms per solve; the GEMM took 3 ms longer, the hidden
     // panels 6 ms less), since the panel's FP64 work then competes with the
     // GEMM's on the shared SMs.
+    // (FP32 storage with the FP64-arithmetic panel keeps the grid kernel)
+    const int cluster_mp = (std::is_same<T, float>::value && !f32) || !cluster_fits<T>() ? 0 : cluster_rows<T>();
     auto panel_at = [&](int j, cudaStream_t s, int *jb_out, bool defer) -> int {
         int mp = m - j;
+        if (mp <= cluster_mp) {
+            int jb = std::min(std::min(mn - j, PANEL_NB), ob_end - j);
+            const int R = ceil_div(mp, CP_CS);
+            cudaLaunchAttribute attr;
+            const cudaLaunchConfig_t cfg = cluster_config(&attr, (size_t)R * PANEL_NB * sizeof(T), s);
+            KTimer ktp(kFamPanel, s, (double)mp * jb * jb - (double)jb * jb * jb / 3.0,
+                       2.0 * sizeof(T) * (double)mp * jb);
+            FG_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T>, A + j + (size_t)j * ldA, ldA, mp, jb, j,
+                                       ipiv, info, w->status, ps, R));
+            *jb_out = jb;
+            return kOk;
+        }
         int R = ceil_div(mp, gcap);
         if (R < PANEL_RMIN) R = PANEL_RMIN;
         // panel width: the reference's 64, narrowed only if a CTA's rows
