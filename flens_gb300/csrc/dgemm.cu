@@ -68,10 +68,10 @@ struct SlabLoader {
 };
 
 // ---------------------------------------------------------------- DFMA ----
-// TM x TN CTA tile (64x64, or 32x32 for launches of few tiles), 256 threads as
-// 16x16, each thread a (TM/16)x(TN/16) sub-tile strided by 16 so shared-memory
+// TM x TN CTA tile (64x64, or 32x32, 16x16, 8x8 for launches of few tiles), 256
+// threads as 16x16 (64 as 8x8 for the smallest), each thread a (TM/16)x(TN/16) sub-tile strided by 16 so shared-memory
 // reads are conflict-free broadcasts.  Every element is summed over k in the
-// same order whatever the tile, so both tiles give the same bits.  TRI restricts the
+// same order whatever the tile, so all tiles give the same bits.  TRI restricts the
 // update to one triangle of a square C (syrk): 1 = lower (i >= j), 2 = upper
 // (i <= j); tiles wholly outside it exit at once and diagonal tiles store only
 // their part, so the other triangle of C is never written.
@@ -83,23 +83,24 @@ struct SlabLoader {
 // (column-major, flag_ld block rows) is set: what the residue product
 // (mod_gemm.cu) left to FP64.
 template <typename T, bool TA, bool TB, int TRI = 0, int KR = 0, int TM = BM, int TN = BN, bool FLAG = false>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(TM < 16 ? 64 : 256)
 dgemm_fma_kernel(int m, int n, int k, T alpha,
                  const T *__restrict__ A, int ldA,
                  const T *__restrict__ B, int ldB,
                  T beta, T *__restrict__ C, int ldC, const uint8_t *__restrict__ flag = nullptr,
                  int flag_ld = 0) {
-    constexpr int RI = TM / 16, RJ = TN / 16;
+    constexpr int TX = TM < 16 ? TM : 16, TY = TN < 16 ? TN : 16, NT = TX * TY;   // threads
+    constexpr int RI = TM / TX, RJ = TN / TY;
     __shared__ T As[2][BK][TM + PAD];
     __shared__ T Bs[2][BK][TN + PAD];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
     if (TRI == 1 && m0 + TM <= n0) return;       // tile strictly above the diagonal
     if (TRI == 2 && n0 + TN <= m0) return;       // tile strictly below the diagonal
     if (FLAG && !flag[m0 / 128 + flag_ld * (n0 / 256)]) return;
 
-    SlabLoader<T, !TA, TM, 256> la;
-    SlabLoader<T, TB, TN, 256> lb;
+    SlabLoader<T, !TA, TM, NT> la;
+    SlabLoader<T, TB, TN, NT> lb;
     T acc[RI][RJ];
 #pragma unroll
     for (int i = 0; i < RI; ++i)
@@ -128,9 +129,9 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
         for (int kk = 0; kk < BK; ++kk) {
             T a[RI], b[RJ];
 #pragma unroll
-            for (int i = 0; i < RI; ++i) a[i] = As[cur][kk][tx + 16 * i];
+            for (int i = 0; i < RI; ++i) a[i] = As[cur][kk][tx + TX * i];
 #pragma unroll
-            for (int j = 0; j < RJ; ++j) b[j] = Bs[cur][kk][ty + 16 * j];
+            for (int j = 0; j < RJ; ++j) b[j] = Bs[cur][kk][ty + TY * j];
 #pragma unroll
             for (int i = 0; i < RI; ++i)
 #pragma unroll
@@ -148,11 +149,11 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     const bool beta1 = beta == T(1);
 #pragma unroll
     for (int j = 0; j < RJ; ++j) {
-        const int gj = n0 + ty + 16 * j;
+        const int gj = n0 + ty + TY * j;
         if (gj >= n) continue;
 #pragma unroll
         for (int i = 0; i < RI; ++i) {
-            const int gi = m0 + tx + 16 * i;
+            const int gi = m0 + tx + TX * i;
             if (gi >= m) continue;
             if (TRI == 1 && gi < gj) continue;
             if (TRI == 2 && gi > gj) continue;
@@ -621,7 +622,15 @@ int gemm_launch_t(char transA, char transB, int m, int n, int k, T alpha, const 
         FG_CUDA(cudaGetLastError());
         return kOk;
     }
-    if (n <= 16) {
+    // A skinny NN launch has a CTA per 256 rows, whose pipe it fills for 128 NC
+    // clocks per unit of k; below about 256 rows per SM the tiled kernel uses more
+    // SMs: m = 936, n = 16, k = 64 took 69 us on 4 SMs, 8 us in tiles.
+    auto fp64_waves = [&](int t, int cols) { return ceil_div(ceil_div(m, t) * ceil_div(n, cols), num_sms()) * (t * cols / 2); };
+    const int nc = n <= 1 ? 1 : n <= 2 ? 2 : n <= 4 ? 4 : n <= 8 ? 8 : 16;
+    const bool tiled = sizeof(T) == 8 && !ta && pick_engine() == Engine::Fma &&
+                       (long long)grid.x * grid.y < 4LL * num_sms() &&   // (tiles below 64 x 64)
+                       2 * fp64_waves(8, 8) <= fp64_waves(256, nc);
+    if (n <= 16 && !tiled) {
         trace("gemm<%d> %c%c m=%d n=%d k=%d engine=skinny", (int)sizeof(T), transA, transB, m, n, k);
         if (n <= 1) launch_skinny<T, 1>(ta, tb, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream);
         else if (n <= 2) launch_skinny<T, 2>(ta, tb, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, stream);
@@ -647,13 +656,24 @@ int gemm_launch_t(char transA, char transB, int m, int n, int k, T alpha, const 
         // the last trailing updates): a 64x64x64 tile alone on an SM takes
         // 131k clocks of its FP64 pipe, so 32x32 tiles spread the same work
         // over four times as many SMs
-        const dim3 g32(ceil_div(m, 32), ceil_div(n, 32));
-#define FG_F32T(TA_, TB_) dgemm_fma_kernel<T, TA_, TB_, 0, 0, 32, 32><<<g32, 256, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC)
-        if (!ta && !tb) FG_F32T(false, false);
-        else if (ta && !tb) FG_F32T(true, false);
-        else if (!ta && tb) FG_F32T(false, true);
-        else FG_F32T(true, true);
-#undef FG_F32T
+        // and smaller ones on until every SM has a tile: the waves of tiles over
+        // the SMs times a tile's pipe time (16, 4, 1) decide.  64 x 48 x 80 took
+        // 21 us of one SM's pipe per 32x32 tile, 1.3 us per 8x8 tile.
+        auto cost = [&](int t) { return ceil_div(ceil_div(m, t) * ceil_div(n, t), num_sms()) * (t * t / 64); };
+        const int c32 = cost(32), c16 = cost(16), c8 = cost(8);
+        const int tile = c8 * 2 <= c16 && c8 * 4 <= c32 ? 8 : c16 * 4 <= c32 * 3 ? 16 : 32;
+        const dim3 gt(ceil_div(m, tile), ceil_div(n, tile));
+#define FG_FT(TA_, TB_)                                                                                        \
+    do {                                                                                                       \
+        if (tile == 8) dgemm_fma_kernel<T, TA_, TB_, 0, 0, 8, 8><<<gt, 64, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC); \
+        else if (tile == 16) dgemm_fma_kernel<T, TA_, TB_, 0, 0, 16, 16><<<gt, 256, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC); \
+        else dgemm_fma_kernel<T, TA_, TB_, 0, 0, 32, 32><<<gt, 256, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC); \
+    } while (0)
+        if (!ta && !tb) FG_FT(false, false);
+        else if (ta && !tb) FG_FT(true, false);
+        else if (!ta && tb) FG_FT(false, true);
+        else FG_FT(true, true);
+#undef FG_FT
     } else {
         if (!ta && !tb) dgemm_fma_kernel<T, false, false><<<grid, 256, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC);
         else if (ta && !tb) dgemm_fma_kernel<T, true, false><<<grid, 256, 0, stream>>>(m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC);

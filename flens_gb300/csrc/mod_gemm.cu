@@ -146,9 +146,9 @@ __device__ __forceinline__ unsigned mag_key(double v) {
 
 // ------------------------------------------------------------ exponents --
 // Row maxima of |x| (as high words) by integer atomicMax into zeroed keys.
-// A block takes 64 rows x 128 k (rows contiguous) or 8 rows x 1024 k.
-// Bound: HBM, one read of each operand.
-constexpr int EX_K0 = 128, EX_K1 = 1024;
+// A block takes 64 rows x 32 k (rows contiguous; 8 loads in flight per thread)
+// or 8 rows x 512 k.  Bound: HBM, one read of each operand; latency when small.
+constexpr int EX_K0 = 32, EX_K1 = 512;
 __host__ __device__ inline int exp_blocks(int R, int K, int rcontig) {
     return rcontig ? ((R + 63) / 64) * ((K + EX_K0 - 1) / EX_K0) : ((R + 7) / 8) * ((K + EX_K1 - 1) / EX_K1);
 }
@@ -167,8 +167,9 @@ mod_exp_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Opera
         if (r < o.R) {
             const double *p = o.X + (size_t)r + (size_t)k0 * o.ld;
             const int kn = min(EX_K0, K - k0);
-#pragma unroll 8
-            for (int k = y; k < kn; k += 4) m = max(m, mag_key(p[(size_t)k * o.ld]));
+#pragma unroll
+            for (int i = 0; i < EX_K0 / 4; ++i)
+                if (y + 4 * i < kn) m = max(m, mag_key(p[(size_t)(y + 4 * i) * o.ld]));
         }
         sm[y][x] = m;
         __syncthreads();
@@ -184,8 +185,9 @@ mod_exp_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Opera
         const double *p = o.X + (size_t)k0 + (size_t)r * o.ld;
         const int kn = min(EX_K1, K - k0);
         unsigned m = 0u;
-#pragma unroll 8
-        for (int k = lane; k < kn; k += 32) m = max(m, mag_key(p[k]));
+#pragma unroll
+        for (int i = 0; i < EX_K1 / 32; ++i)
+            if (lane + 32 * i < kn) m = max(m, mag_key(p[lane + 32 * i]));
         m = __reduce_max_sync(0xffffffffu, m);
         if (lane == 0 && m) atomicMax(&o.key[r], m);
     }
@@ -332,7 +334,7 @@ struct ModArgs {
     TileMap tiles;
     int nkb;                                  // 64-deep k blocks
     float qmin;                               // smallest accepted Q
-    uint8_t *res;                             // residues [modulus][tile][16-column group][row][16]
+    uint8_t *res;                             // residues [modulus][tile][4-column group][row][4]
     uint8_t *flag;                            // per tile (row tile + tm * column tile): 1 = left to FP64
     const unsigned *keyA, *keyB;
     float p[NM], ip[NM];
@@ -347,7 +349,7 @@ constexpr size_t MOD_SMEM = 1024 + (size_t)STAGES * (A_BYTES + B_BYTES) + 256;
 // epilogue warps over two TMEM accumulators); a residue plane runs one
 // accumulator per 1024 of k.  Epilogue: 6 FP32 operations per element reduce
 // the integer sum to a centred residue, 4 are packed per word, and a warp
-// stores 512 contiguous bytes per 16 columns.  MULTI (more than one chunk)
+// stores 128 contiguous bytes per 4 columns.  MULTI (more than one chunk)
 // keeps the running residue sums of the thread's 128 elements packed in 64
 // registers.  Bound: the BF16 tensor pipe (0.65 us of epilogue against 2.6 us of
 // MMAs per item at k = 512).
@@ -480,7 +482,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             const int chunks = mag ? 1 : nch;
             const float p = mag ? 1.0f : a.p[mag ? 0 : pl - 1], ip = mag ? 1.0f : a.ip[mag ? 0 : pl - 1];
             uint8_t *out = mag ? nullptr
-                               : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 16;
+                               : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 4;
             uint32_t st[MULTI ? 64 : 1];
             bool bad = false;
             for (int c = 0; c < chunks; ++c, ++i) {
@@ -542,16 +544,11 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                         }
                         if (lastc) {
 #pragma unroll
-                            for (int g = 0; g < 2; ++g) {
-                                uint4 w;
-                                uint32_t *wp = (uint32_t *)&w;
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    const uint32_t *s4 = &r[g * 16 + u * 4];
-                                    wp[u] = __byte_perm(__byte_perm(s4[0], s4[1], 0x0040),
-                                                        __byte_perm(s4[2], s4[3], 0x0040), 0x5410);
-                                }
-                                *(uint4 *)(out + (size_t)(c0 / 16 + g) * (MT * 16)) = w;
+                            for (int g = 0; g < 8; ++g) {
+                                const uint32_t *s4 = &r[g * 4];
+                                *(uint32_t *)(out + (size_t)(c0 / 4 + g) * (MT * 4)) =
+                                    __byte_perm(__byte_perm(s4[0], s4[1], 0x0040), __byte_perm(s4[2], s4[3], 0x0040),
+                                                0x5410);
                             }
                         }
                     }
@@ -649,57 +646,56 @@ __device__ __forceinline__ double crt_value(const uint32_t (&g)[NG], const CrtCo
     return __longlong_as_double((long long)bits);
 }
 
-// C from the residues.  A block takes 32 columns of a tile (8 blocks per tile), a
-// thread one row x 16 columns: its 17 residue loads are 16 bytes each,
-// contiguous over the warp, and C is read and written along columns, a warp
-// per 256 bytes.  About 230 integer operations per element; 17 bytes of residues and
-// 16 of C move.
+// C from the residues.  A thread takes one row x 4 columns: its 17 residue words
+// are contiguous over the warp, and C is read and written along columns, a warp
+// per 256 bytes.  A block takes 8 columns of a tile (32 blocks per tile).  Bound:
+// the integer pipes (about 230 operations per element, 90 of them dp4a); 17 bytes
+// of residues and 16 of C move.
+constexpr int CRT_PARTS = NT / 8;
 __global__ void __launch_bounds__(256)
 mod_crt_kernel(const __grid_constant__ TileMap tiles, const uint8_t *__restrict__ res,
                const uint8_t *__restrict__ flag, const unsigned *__restrict__ keyA,
                const unsigned *__restrict__ keyB, int bits2, double alpha, double beta,
                double *__restrict__ C, int ldC, const __grid_constant__ CrtConst k) {
-    const int t = blockIdx.x >> 3, part = blockIdx.x & 7;
+    const int t = blockIdx.x / CRT_PARTS, part = blockIdx.x % CRT_PARTS;
     int m0, n0;
     tile_at(tiles, t, m0, n0);
-    if (flag[m0 / MT + tiles.tm * (n0 / NT)]) return;     // left to the FP64 kernel
     const int rl = threadIdx.x & 127, cg = part * 2 + (threadIdx.x >> 7);
-    const int row = m0 + rl, col0 = n0 + cg * 16;
+    const int row = m0 + rl, col0 = n0 + cg * 4;
     if (row >= tiles.M || col0 >= tiles.N) return;
     if (tiles.tri == 1 && row < col0) return;
-    if (tiles.tri == 2 && row > col0 + 15) return;
+    if (tiles.tri == 2 && row > col0 + 3) return;
     const size_t tile_bytes = (size_t)MT * NT;
-    const uint8_t *src = res + (size_t)t * tile_bytes + (size_t)cg * (MT * 16) + (size_t)rl * 16;
+    const uint8_t *src = res + (size_t)t * tile_bytes + (size_t)cg * (MT * 4) + (size_t)rl * 4;
+    uint32_t x[NM];
+#pragma unroll
+    for (int i = 0; i < NM; ++i) x[i] = __ldcs((const unsigned *)(src + (size_t)i * tiles.ntiles * tile_bytes));
+    if (flag[m0 / MT + tiles.tm * (n0 / NT)]) return;     // left to the FP64 kernel
     bool ok;
     const int ea = key_exp(keyA[row], ok) - bits2;
     const bool beta1 = beta == 1.0;
-    uint4 w[NM];
+    double cv[4];
+    int eb[4];
+    bool in[4];
 #pragma unroll
-    for (int i = 0; i < NM; ++i) w[i] = __ldcs((const uint4 *)(src + (size_t)i * tiles.ntiles * tile_bytes));
+    for (int v = 0; v < 4; ++v) {
+        const int col = col0 + v;
+        in[v] = col < tiles.N && !(tiles.tri == 1 && row < col) && !(tiles.tri == 2 && row > col);
+        cv[v] = in[v] ? C[(size_t)row + (size_t)col * ldC] : 0.0;
+        eb[v] = in[v] ? key_exp(keyB[col], ok) : 0;
+    }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-        uint32_t x[NM];
+    for (int v = 0; v < 4; ++v) {
+        uint32_t g[NG];
 #pragma unroll
-        for (int i = 0; i < NM; ++i) x[i] = u == 0 ? w[i].x : u == 1 ? w[i].y : u == 2 ? w[i].z : w[i].w;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int col = col0 + u * 4 + v;
-            if (col >= tiles.N) continue;
-            if (tiles.tri == 1 && row < col) continue;
-            if (tiles.tri == 2 && row > col) continue;
-            uint32_t g[NG];
-#pragma unroll
-            for (int i = 0; i + 3 < NM; i += 4) {
-                const uint32_t lo = __byte_perm(x[i], x[i + 1], v | ((4 + v) << 4));
-                const uint32_t hi = __byte_perm(x[i + 2], x[i + 3], v | ((4 + v) << 4));
-                g[i / 4] = __byte_perm(lo, hi, 0x5410);
-            }
-            g[NG - 1] = (x[NM - 1] >> (8 * v)) & 0xFFu;
-            const double s = crt_value(g, k, ea + key_exp(keyB[col], ok));
-            double *c = C + (size_t)row + (size_t)col * ldC;
-            const double cv = *c;
-            *c = fma(alpha, s, beta1 ? cv : beta * cv);
+        for (int i = 0; i + 3 < NM; i += 4) {
+            const uint32_t lo = __byte_perm(x[i], x[i + 1], v | ((4 + v) << 4));
+            const uint32_t hi = __byte_perm(x[i + 2], x[i + 3], v | ((4 + v) << 4));
+            g[i / 4] = __byte_perm(lo, hi, 0x5410);
         }
+        g[NG - 1] = (x[NM - 1] >> (8 * v)) & 0xFFu;
+        const double s = crt_value(g, k, ea + eb[v]);
+        if (in[v]) C[(size_t)row + (size_t)(col0 + v) * ldC] = fma(alpha, s, beta1 ? cv[v] : beta * cv[v]);
     }
 }
 static_assert(NM % 4 == 1, "the last residue group holds one modulus");
@@ -784,7 +780,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     }
     {
         KTimer kt(kFamAux, s, 0.0, (NM + 16.0) * m * (double)n);
-        mod_crt_kernel<<<tiles.ntiles * 8, 256, 0, s>>>(tiles, a.res, a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta,
+        mod_crt_kernel<<<tiles.ntiles * CRT_PARTS, 256, 0, s>>>(tiles, a.res, a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta,
                                                         C, ldC, cs.crt);
         FG_CUDA(cudaGetLastError());
     }
@@ -805,19 +801,19 @@ bool mod_enabled() {
 
 }  // namespace
 
-// Estimated microseconds of the two routes, from measurements at the sizes
-// named: the FP64 kernel runs at 1.1 TFLOP/s; a residue product costs its
-// launches, its work items in waves over the SMs (5.2 ns per unit of k and
-// tile), 50 bytes of operand traffic per element and 40 per element of C.
+// Estimated microseconds of the two routes, fitted to measurements from 256^3 to
+// 4096^3 and 1000 x 100 x 1000 to 8192 x 256 x 256 (all within 12%).  FP64: an SM
+// takes 0.265 us of its pipe per unit of k and 32 x 32 tile, in waves over the
+// SMs.  Residues: the launches, the work items in waves (1.2 us + 5.5 ns per unit
+// of k), the operands and C.  Both at, say, 300^3: 85 and 35 us; 4032 x 64 x 64: 39 and 41;
+// 4096 x 128 x 128: 134 and 46.
 bool mod_gemm_wins(int m, int n, int k, int tri) {
     if (n <= 16 || m <= 16 || k < 32 || !mod_enabled()) return false;
-    const double half = tri ? 0.5 : 1.0;
-    const double fp64 = half * 2.0 * m * (double)n * k / 1.1e6;
-    if (fp64 < 40.0) return false;
+    const double half = tri ? 0.5 : 1.0, mn = half * m * (double)n;
     const int sms = num_sms() > 0 ? num_sms() : 1;
-    const double items = ceil(half * ceil_div(m, MT) * ceil_div(n, NT) * (double)NP / sms);
-    const double mod = 30.0 + items * (1.0 + 0.0052 * k) + 50.0e-6 / 3.0 * k * ((double)m + n) +
-                       half * 40.0e-6 / 3.0 * m * (double)n;
+    const double fp64 = 5.0 + ceil(half * ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 0.265 * k;
+    const double items = ceil(half * ceil_div(m, MT) * (double)ceil_div(n, NT) * NP / sms);
+    const double mod = 28.0 + items * (1.2 + 0.0055 * k) + 1.0e-5 * k * ((double)m + n) + 1.5e-5 * mn;
     return mod < 0.9 * fp64;
 }
 

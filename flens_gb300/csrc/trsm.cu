@@ -10,7 +10,7 @@
 // M(i,p) = A[i*mi + p*mp], and a set of vectors (columns of B for Left, rows
 // of B for Right).  The blocked, right-looking driver solves 64x64 diagonal
 // blocks (trsm_diag_tile_kernel: 32 vectors per CTA, 8 rows per thread;
-// trsm_diag_warp_kernel: a warp per vector for up to 32 vectors) and applies
+// trsm_diag_warp_kernel: a warp per vector for up to 2560 vectors) and applies
 // each solved block to the rest of B with the FP64 GEMM.  The
 // diagonal solve uses the column-sweep (axpy) form rather than the
 // reference's dot form, and multiplies by the reciprocal of the diagonal
@@ -28,6 +28,106 @@ constexpr int TRSM_NB = 64;      // diagonal block size
 constexpr int TRSM_VPC = 32;     // vectors per CTA
 constexpr int TRSM_THREADS = 256;
 constexpr int TRSM_RPT = TRSM_NB * TRSM_VPC / TRSM_THREADS;   // rows per thread (8)
+
+// D[p][r] = M(r, p) of an nr x np block (zeros up to 64 x 64), 8 loads in flight
+// per thread, along whichever index is contiguous.
+template <int NT, typename T>
+__device__ __forceinline__ void stage_block(T (*D)[TRSM_NB + 1], const T *__restrict__ M, long long mi, long long mp,
+                                            int nr, int np) {
+    const int t = threadIdx.x;
+#pragma unroll 1
+    for (int e0 = 0; e0 < TRSM_NB * TRSM_NB; e0 += 8 * NT) {
+        T v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = e0 + j * NT + t, lo = e % TRSM_NB, hi = e / TRSM_NB;
+            const int r = mi == 1 ? lo : hi, p = mi == 1 ? hi : lo;
+            v[j] = r < nr && p < np ? M[r * mi + p * mp] : T(0);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int e = e0 + j * NT + t, lo = e % TRSM_NB, hi = e / TRSM_NB;
+            if (mi == 1) D[hi][lo] = v[j];
+            else D[lo][hi] = v[j];
+        }
+    }
+}
+
+// Row scaling of a staged FP64 diagonal block by the reciprocals of its diagonal:
+// the substitution then has one FP64 instruction per step on its chain instead
+// of two (a multiply by rinv_i after the sum).  M' = diag(rinv) M has each entry
+// rounded once and b' = rinv b too, the same componentwise backward error as
+// the multiply at the end.  Only where no scaled entry leaves [2^-900, 2^900]
+// (or is zero already): `scaled` is false otherwise and the block stays as it was.
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
+__device__ __forceinline__ bool mid_range(double x) {
+    const int e = exp_field(x);
+    return e >= 1023 - 900 && e <= 1023 + 900;
+}
+template <int NT, typename T>
+__device__ __forceinline__ bool scale_rows(T (*D)[TRSM_NB + 1], const T *rinv) {
+    if (sizeof(T) != 8) return false;
+    constexpr int PER = TRSM_NB * TRSM_NB / NT;
+    T v[PER];
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = j * NT + threadIdx.x, r = e % TRSM_NB, p = e / TRSM_NB;
+        v[j] = D[p][r] * rinv[r];
+        ok &= mid_range((double)rinv[r]);
+        if (p != r) ok &= mid_range((double)v[j]) || (__double_as_longlong((double)D[p][r]) << 1) == 0;
+    }
+    if (!__syncthreads_and(ok)) return false;
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+        const int e = j * NT + threadIdx.x;
+        D[e / TRSM_NB][e % TRSM_NB] = v[j];
+    }
+    __syncthreads();
+    return true;
+}
+
+// Substitution in the 32 x 32 diagonal sub-block at row o, one warp, lane = row
+// (x: its entry).  A step is a shuffle of the finished entry and one FMA; an FP64
+// warp instruction holds the scheduler's pipe for 64 clocks, so the chain is
+// about 100 clocks a step.  MUL: times rinv[i] first (unscaled, not unit).
+template <bool LOWER, bool MUL, typename T>
+__device__ __forceinline__ void solve32(T &x, const T (*D)[TRSM_NB + 1], int o, const T *rinv) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int s = 0; s < 32; ++s) {
+        const int i = LOWER ? s : 31 - s;
+        T xi = __shfl_sync(0xffffffffu, x, i);
+        if (MUL) {
+            xi *= rinv[o + i];
+            if (lane == i) x = xi;
+        }
+        if (LOWER ? lane > i : lane < i) x = fma(-D[o + i][o + lane], xi, x);
+    }
+}
+template <bool LOWER, bool UNIT, typename T>
+__device__ __forceinline__ void solve32_any(T &x, const T (*D)[TRSM_NB + 1], int o, const T *rinv, bool scaled) {
+    if (UNIT || scaled) solve32<LOWER, false>(x, D, o, rinv);
+    else solve32<LOWER, true>(x, D, o, rinv);
+}
+
+// Right-hand sides of a warp's vector for the scaled block: b' = rinv b.  Where
+// that could overflow although x does not (|b'| >= 2^1000), the vector is solved
+// times 2^-200; returns what x is to be multiplied by.
+template <typename T>
+__device__ __forceinline__ T scale_rhs(T &x0, T &x1, T r0, T r1) {
+    const T y0 = x0 * r0, y1 = x1 * r1;
+    const bool ok = exp_field((double)y0) <= 1023 + 1000 && exp_field((double)y1) <= 1023 + 1000;
+    if (__all_sync(0xffffffffu, ok)) {
+        x0 = y0;
+        x1 = y1;
+        return T(1);
+    }
+    const double sc = 6.223015277861142e-61;      // 2^-200
+    x0 = (T)(((double)x0 * sc) * (double)r0);
+    x1 = (T)(((double)x1 * sc) * (double)r1);
+    return (T)1.6069380442589903e60;              // 2^200
+}
 
 // Solves the kb x kb (kb <= 64) diagonal block M for 32 vectors per CTA.
 // Lane l of every warp holds vector l; warp w holds the 8 consecutive rows
@@ -53,12 +153,7 @@ trsm_diag_tile_kernel(int nb, const T *__restrict__ M0, long long mi, long long 
     const int t = threadIdx.x;
     const long long v0 = (long long)blockIdx.x * TRSM_VPC;
     const int nv = (int)((nvec - v0) < TRSM_VPC ? (nvec - v0) : TRSM_VPC);
-    for (int e = t; e < nb * nb; e += TRSM_THREADS) {
-        int r, i;
-        if (mi == 1) { r = e % nb; i = e / nb; }
-        else { i = e % nb; r = e / nb; }
-        Ms[i][r] = M0[r * mi + i * mp];
-    }
+    stage_block<TRSM_THREADS>(Ms, M0, mi, mp, nb, nb);
     // X tile: lanes run along whichever index is contiguous in memory
     for (int e = t; e < TRSM_NB * TRSM_VPC; e += TRSM_THREADS) {
         int r, v;
@@ -108,11 +203,11 @@ trsm_diag_tile_kernel(int nb, const T *__restrict__ M0, long long mi, long long 
     }
 }
 
-// Few vectors (the solves with one or a handful of right-hand sides): one warp
-// per vector, lane l holding rows l and l + 32.  A step is a shuffle of the
-// finished x_i, one multiply by the precomputed 1/M(i,i) and the FMAs of the
-// rows still open -- no block barrier on the dependency chain.
-constexpr int TRSM_WARP_VECS = 8;      // warps (vectors) per CTA
+// Fewer vectors: one warp per vector, lane l holding rows l and l + 32.  The two
+// 32 x 32 diagonal sub-blocks are substituted (solve32), the block between them
+// is 32 independent FMAs.  Four warps per CTA, one per scheduler: with eight, two
+// shared an FP64 pipe and the launch took 20 us instead of about 8.
+constexpr int TRSM_WARP_VECS = 4;      // warps (vectors) per CTA
 
 // The warp kernel is the lower-latency choice while the tile kernel would
 // run at most one CTA per SM (each tile CTA is ~17 us of FP64 pipe time):
@@ -132,37 +227,35 @@ trsm_diag_warp_kernel(int nb, const T *__restrict__ M0, long long mi, long long 
                       T *__restrict__ X0, long long xs, long long vs, int nvec) {
     __shared__ T Ms[TRSM_NB][TRSM_NB + 1];     // Ms[i][r] = M(r, i)
     __shared__ T rinv[TRSM_NB];
-    for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-        int r, i;
-        if (mi == 1) { r = e % nb; i = e / nb; }
-        else { i = e % nb; r = e / nb; }
-        Ms[i][r] = M0[r * mi + i * mp];
-    }
-    __syncthreads();
-    if (!UNIT && threadIdx.x < nb) rinv[threadIdx.x] = T(1) / Ms[threadIdx.x][threadIdx.x];
-    __syncthreads();
     const int lane = threadIdx.x & 31;
     const long long v = (long long)blockIdx.x * TRSM_WARP_VECS + (threadIdx.x >> 5);
-    if (v >= nvec) return;
     T *x = X0 + v * vs;
     const int r0 = lane, r1 = lane + 32;
-    T x0 = r0 < nb ? x[r0 * xs] : T(0);
-    T x1 = r1 < nb ? x[r1 * xs] : T(0);
-    for (int s = 0; s < nb; ++s) {
-        const int i = LOWER ? s : nb - 1 - s;
-        T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31);
-        if (!UNIT) xi *= rinv[i];
-        if (lane == (i & 31)) {
-            if (i < 32) x0 = xi;
-            else x1 = xi;
-        }
-        if (LOWER) {
-            if (r0 > i && r0 < nb) x0 = fma(-Ms[i][r0], xi, x0);
-            if (r1 > i && r1 < nb) x1 = fma(-Ms[i][r1], xi, x1);
-        } else {
-            if (r0 < i) x0 = fma(-Ms[i][r0], xi, x0);
-            if (r1 < i) x1 = fma(-Ms[i][r1], xi, x1);
-        }
+    T x0 = v < nvec && r0 < nb ? x[r0 * xs] : T(0);
+    T x1 = v < nvec && r1 < nb ? x[r1 * xs] : T(0);
+    stage_block<32 * TRSM_WARP_VECS>(Ms, M0, mi, mp, nb, nb);
+    __syncthreads();
+    bool scaled = false;
+    if (!UNIT) {
+        if (threadIdx.x < TRSM_NB) rinv[threadIdx.x] = threadIdx.x < nb ? T(1) / Ms[threadIdx.x][threadIdx.x] : T(1);
+        __syncthreads();
+        scaled = scale_rows<32 * TRSM_WARP_VECS>(Ms, rinv);
+    }
+    if (v >= nvec) return;
+    T back = T(1);
+    if (scaled) back = scale_rhs(x0, x1, rinv[r0], rinv[r1]);
+    T &xa = LOWER ? x0 : x1, &xb = LOWER ? x1 : x0;        // solved first, second
+    const int oa = LOWER ? 0 : 32, ob = 32 - oa;
+    solve32_any<LOWER, UNIT>(xa, Ms, oa, rinv, scaled);
+#pragma unroll
+    for (int s = 0; s < 32; ++s) {
+        const int i = LOWER ? s : 31 - s;
+        xb = fma(-Ms[oa + i][ob + lane], __shfl_sync(0xffffffffu, xa, i), xb);
+    }
+    solve32_any<LOWER, UNIT>(xb, Ms, ob, rinv, scaled);
+    if (back != T(1)) {
+        x0 *= back;
+        x1 *= back;
     }
     if (r0 < nb) x[r0 * xs] = x0;
     if (r1 < nb) x[r1 * xs] = x1;
@@ -235,19 +328,19 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
     for (int v = 0; v < CH_MAXV; ++v) acc[v] = T(0);
 
     auto stage = [&](T (*D)[CH_NB + 1], int K0, int kk) {
-        for (int e = tid; e < CH_NB * CH_NB; e += CH_THREADS) {
-            int rr, pp;
-            if (mi == 1) { rr = e % CH_NB; pp = e / CH_NB; }
-            else { pp = e % CH_NB; rr = e / CH_NB; }
-            D[pp][rr] = (rr < kb && pp < kk) ? M0[(R0 + rr) * mi + (K0 + pp) * mp] : T(0);
-        }
+        stage_block<CH_THREADS>(D, M0 + R0 * mi + K0 * mp, mi, mp, kb, kk);
     };
-    // the diagonal block and its reciprocals do not depend on other blocks:
-    // off the critical path, before any wait
+    // the diagonal block, its reciprocals and the scaling of its rows do not
+    // depend on other blocks: off the critical path, before any wait
     stage(Md, R0, kb);
     __syncthreads();
     if (s_abort) return;
-    if (!UNIT && tid < kb) rinv[tid] = T(1) / Md[tid][tid];
+    bool scaled = false;
+    if (!UNIT) {
+        if (tid < CH_NB) rinv[tid] = tid < kb ? T(1) / Md[tid][tid] : T(1);
+        __syncthreads();
+        scaled = scale_rows<CH_THREADS>(Md, rinv);
+    }
 
     for (int s2 = 0; s2 < s; ++s2) {
         const int k = LOWER ? s2 : nblk - 1 - s2;
@@ -261,7 +354,7 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
                     s_abort = 1;
                     break;
                 }
-                if (spins > 32) __nanosleep(64);
+                if (spins > 256) __nanosleep(32);
             }
         }
         __syncthreads();
@@ -289,34 +382,41 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
 #pragma unroll
     for (int v = 0; v < CH_MAXV; ++v) part[q][v][r] = acc[v];
     __syncthreads();
+    // The block itself: warp v substitutes the first 32 rows of vector v (in solve
+    // order), four warps form the 32 x 32 product with them, warp v substitutes
+    // the other 32.  (One warp doing all 64 rows issued two to three FP64
+    // instructions per step on one scheduler's pipe: 11.5 us a block, now about 6.)
     const int warp = tid >> 5, lane = tid & 31;
+    const int oa = LOWER ? 0 : 32, ob = 32 - oa;
+    T xa = T(0), xb = T(0), back = T(1);
     if (warp < nvec) {
-        const int v = warp;
-        T *x = X0 + v * vs + (long long)R0 * xs;
+        const T *x = X0 + warp * vs + (long long)R0 * xs;
         auto rhs = [&](int rr) -> T {
             if (rr >= kb) return T(0);
-            return x[rr * xs] - ((part[0][v][rr] + part[1][v][rr]) + (part[2][v][rr] + part[3][v][rr]));
+            return x[rr * xs] - ((part[0][warp][rr] + part[1][warp][rr]) + (part[2][warp][rr] + part[3][warp][rr]));
         };
-        T x0 = rhs(lane), x1 = rhs(lane + 32);
-        for (int st = 0; st < kb; ++st) {
-            const int i = LOWER ? st : kb - 1 - st;
-            T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31);
-            if (!UNIT) xi *= rinv[i];
-            if (lane == (i & 31)) {
-                if (i < 32) x0 = xi;
-                else x1 = xi;
-            }
-            const int r1 = lane + 32;
-            if (LOWER) {
-                if (lane > i && lane < kb) x0 = fma(-Md[i][lane], xi, x0);
-                if (r1 > i && r1 < kb) x1 = fma(-Md[i][r1], xi, x1);
-            } else {
-                if (lane < i) x0 = fma(-Md[i][lane], xi, x0);
-                if (r1 < i) x1 = fma(-Md[i][r1], xi, x1);
-            }
-        }
-        if (lane < kb) x[lane * xs] = x0;
-        if (lane + 32 < kb) x[(lane + 32) * xs] = x1;
+        xa = rhs(oa + lane);
+        xb = rhs(ob + lane);
+        if (scaled) back = scale_rhs(xa, xb, rinv[oa + lane], rinv[ob + lane]);
+        solve32_any<LOWER, UNIT>(xa, Md, oa, rinv, scaled);
+        xk[warp][oa + lane] = xa;
+    }
+    __syncthreads();
+    // (part is free: its first 32 rows take the product's four partial sums)
+    for (int v = warp >> 2; v < nvec; v += CH_THREADS / 128) {
+        const int g = warp & 3;
+        T sum = T(0);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum = fma(Md[oa + 8 * g + j][ob + lane], xk[v][oa + 8 * g + j], sum);
+        part[g][v][lane] = sum;
+    }
+    __syncthreads();
+    if (warp < nvec) {
+        xb -= (part[0][warp][lane] + part[1][warp][lane]) + (part[2][warp][lane] + part[3][warp][lane]);
+        solve32_any<LOWER, UNIT>(xb, Md, ob, rinv, scaled);
+        T *x = X0 + warp * vs + (long long)R0 * xs;
+        if (oa + lane < kb) x[(oa + lane) * xs] = back != T(1) ? xa * back : xa;
+        if (ob + lane < kb) x[(ob + lane) * xs] = back != T(1) ? xb * back : xb;
     }
     __syncthreads();
     if (tid == 0) ch_release(&flags[s], epoch);

@@ -1,0 +1,99 @@
+"""Triangular solves with few right-hand sides (scaled diagonal blocks, the
+chained solve), and the row permutation of the LU solves, at block edges and
+for scalings where the scaled form must step aside.  Bound: the componentwise
+backward error of substitution, c * n * 2^-53 * |M||x| (c = 4: prescaled rows,
+the reciprocal, and the residual is taken in extended precision)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import flens_gb300 as fg
+import oracle
+
+pytestmark = pytest.mark.gpu
+U = 2.0 ** -53
+
+
+def _residual_ok(M, X, B):
+    L = np.longdouble
+    n = M.shape[0]
+    with np.errstate(all="ignore"):
+        R = np.abs(M.astype(L) @ X.astype(L) - B.astype(L))
+        bound = 4 * n * U * (np.abs(M).astype(L) @ np.abs(X).astype(L)) + L(1e-300)
+    assert np.all(R <= bound)
+
+
+def _tri(n, uplo, kind, seed):
+    A = oracle.uniform(seed, n, n) / n
+    A[np.arange(n), np.arange(n)] = 1.0 + oracle.uniform(seed + 1, n, 1)[:, 0] / 4
+    if kind == "rows":                       # rows over 2^+-400: still scaled
+        A = A * 2.0 ** np.random.default_rng(seed).integers(-400, 401, (n, 1))
+    elif kind == "wide":                     # reciprocals beyond 2^900: unscaled
+        A = A * 2.0 ** np.where(np.arange(n) % 5 == 0, -930, 0)[:, None]
+    return np.asfortranarray(np.tril(A) if uplo == "L" else np.triu(A))
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 65, 130, 200])
+@pytest.mark.parametrize("nvec", [1, 3, 4, 5, 33])
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("kind", ["plain", "rows", "wide"])
+def test_trsm_few(cuda, n, nvec, uplo, kind):
+    for trans in "NT":
+        A = _tri(n, uplo, kind, n)
+        B = oracle.uniform(n + 9, n, nvec)
+        X = fg.dtrsm("L", uplo, trans, "N", 1.0, A, B.copy(order="F"))
+        _residual_ok(A if trans == "N" else A.T, X, B)
+
+
+def test_large_right_hand_side_that_cancels(cuda):
+    """b / diagonal overflows, the solution does not."""
+    n = 100
+    A = _tri(n, "L", "plain", 4)
+    A[:, 0] = 1e-5
+    A[0, 0] = 1.0
+    A[50, :] *= 2.0 ** -60
+    A[50, 0] = 1.0
+    A = np.asfortranarray(A)
+    B = np.zeros((n, 2))
+    B[0, 0] = 2.0 ** 1000
+    B[:, 0] = A[:, 0] * B[0, 0]
+    B[0, 1] = 1.0
+    X = fg.dtrsm("L", "L", "N", "N", 1.0, A, B.copy(order="F"))
+    assert np.all(np.isfinite(X))
+    _residual_ok(A, X, B)
+
+
+def test_infinite_right_hand_side(cuda):
+    n = 96
+    A = _tri(n, "L", "plain", 5)
+    B = np.zeros((n, 1))
+    B[40] = np.inf
+    X = fg.dtrsm("L", "L", "N", "N", 1.0, A, B.copy(order="F"))
+    assert np.all(X[:40] == 0) and np.isinf(X[40, 0]) and not np.any(np.isfinite(X[41:]))
+
+
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 129, 700, 2111])
+@pytest.mark.parametrize("trans", "NT")
+@pytest.mark.parametrize("nrhs", [1, 4, 16, 40])
+def test_solve_with_interchanges(cuda, n, trans, nrhs):
+    import torch
+    A0 = fg.to_colmajor(torch.from_numpy(oracle.uniform(n, n, n)).to(cuda))
+    B0 = fg.to_colmajor(torch.from_numpy(oracle.uniform(n + 1, n, nrhs)).to(cuda))
+    A, X = fg.to_colmajor(A0.clone()), fg.to_colmajor(B0.clone())
+    piv = torch.zeros(n, dtype=torch.int32, device=cuda)
+    info = torch.zeros(1, dtype=torch.int32, device=cuda)
+    fg.dgetrf_dev(A, piv, info)
+    fg.dgetrs_dev(trans, A, piv, X)
+    fg.sync()
+    L = torch.tril(A, -1).abs()
+    L.diagonal().add_(1.0)
+    LU = L @ torch.triu(A).abs()
+    p = piv.cpu().numpy() - 1
+    perm = np.arange(n)
+    for i in range(n):
+        perm[[i, p[i]]] = perm[[p[i], i]]
+    LU = LU[torch.from_numpy(np.argsort(perm)).to(cuda)]          # |P^T| |L| |U|
+    op = (lambda M: M) if trans == "N" else (lambda M: M.t())  # noqa: E731
+    R = (op(A0) @ X - B0).abs()
+    assert bool((R <= 12 * n * U * (op(LU) @ X.abs()) + 4 * n * U * (op(A0).abs() @ X.abs())).all())
