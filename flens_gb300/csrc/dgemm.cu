@@ -600,6 +600,21 @@ int sscal_matrix_launch(int m, int n, float alpha, float *X, int ld, cudaStream_
     return scal_matrix_launch_t<float>(m, n, alpha, X, ld, stream);
 }
 
+// Tile of dgemm_fma_kernel for an m x n product (`part` of whose tiles are
+// computed).  Few 64x64 tiles (the look-ahead update of the next panel's columns,
+// the last trailing updates): a 64x64x64 tile alone on an SM takes 131k clocks of
+// its FP64 pipe, so 32x32 tiles spread the same work over four times as many
+// SMs, and smaller ones on until every SM has a tile: the waves of tiles over the
+// SMs times a tile's pipe time (16, 4, 1) decide.  64 x 48 x 80 took 21 us of one
+// SM's pipe per 32x32 tile, 1.3 us per 8x8 tile.
+static int fp64_tile(int m, int n, double part = 1.0) {
+    const int sms = num_sms() > 0 ? num_sms() : 1;
+    if ((double)ceil_div(m, BM) * ceil_div(n, BN) * part >= 4.0 * sms) return 64;
+    auto cost = [&](int t) { return (int)(ceil_div(m, t) * (double)ceil_div(n, t) * part / sms + 0.999) * (t * t / 64); };
+    const int c32 = cost(32), c16 = cost(16), c8 = cost(8);
+    return c8 * 2 <= c16 && c8 * 4 <= c32 ? 8 : c16 * 4 <= c32 * 3 ? 16 : 32;
+}
+
 template <typename T>
 int gemm_launch_t(char transA, char transB, int m, int n, int k, T alpha, const T *A, int ldA,
                   const T *B, int ldB, T beta, T *C, int ldC, cudaStream_t stream) {
@@ -651,17 +666,7 @@ int gemm_launch_t(char transA, char transB, int m, int n, int k, T alpha, const 
         else if (ta && !tb) dgemm_dmma_kernel<true, false><<<grid, 128, 0, stream>>>(m, n, k, al, Ad, ldA, Bd, ldB, be, Cd, ldC);
         else if (!ta && tb) dgemm_dmma_kernel<false, true><<<grid, 128, 0, stream>>>(m, n, k, al, Ad, ldA, Bd, ldB, be, Cd, ldC);
         else dgemm_dmma_kernel<true, true><<<grid, 128, 0, stream>>>(m, n, k, al, Ad, ldA, Bd, ldB, be, Cd, ldC);
-    } else if ((long long)grid.x * grid.y < 4LL * num_sms()) {
-        // few 64x64 tiles (the look-ahead update of the next panel's columns,
-        // the last trailing updates): a 64x64x64 tile alone on an SM takes
-        // 131k clocks of its FP64 pipe, so 32x32 tiles spread the same work
-        // over four times as many SMs
-        // and smaller ones on until every SM has a tile: the waves of tiles over
-        // the SMs times a tile's pipe time (16, 4, 1) decide.  64 x 48 x 80 took
-        // 21 us of one SM's pipe per 32x32 tile, 1.3 us per 8x8 tile.
-        auto cost = [&](int t) { return ceil_div(ceil_div(m, t) * ceil_div(n, t), num_sms()) * (t * t / 64); };
-        const int c32 = cost(32), c16 = cost(16), c8 = cost(8);
-        const int tile = c8 * 2 <= c16 && c8 * 4 <= c32 ? 8 : c16 * 4 <= c32 * 3 ? 16 : 32;
+    } else if (const int tile = fp64_tile(m, n); tile < 64) {
         const dim3 gt(ceil_div(m, tile), ceil_div(n, tile));
 #define FG_FT(TA_, TB_)                                                                                        \
     do {                                                                                                       \
@@ -746,14 +751,26 @@ int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const dou
               8.0 * ((double)n * k * 2.0 + (double)n * (n + 1)));
     const double *Ak = k > 0 ? A : nullptr, *Bk = k > 0 ? B : nullptr;
     const int lda = k > 0 ? ldA : 1, ldb = k > 0 ? ldB : 1;
-    // op(A) op(B)^T as gemm(op, op^T)
+    // op(A) op(B)^T as gemm(op, op^T); tiles by the rule of gemm_launch_t, half of
+    // them outside the triangle (192 x 192 x 64, the update inside a 256-column
+    // Cholesky block: 70 us in 64x64 tiles, 9 in 16x16)
+    const int tile = fp64_tile(n, n, 0.5);
+    const dim3 gt(ceil_div(n, tile), ceil_div(n, tile));
+#define FG_TRI(TA_, TB_, TRI_)                                                                                 \
+    do {                                                                                                       \
+        if (tile == 8) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 8, 8><<<gt, 64, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
+        else if (tile == 16) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 16, 16><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
+        else if (tile == 32) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
+        else dgemm_fma_kernel<double, TA_, TB_, TRI_><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
+    } while (0)
     if (lower) {
-        if (nt) dgemm_fma_kernel<double, false, true, 1><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC);
-        else dgemm_fma_kernel<double, true, false, 1><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC);
+        if (nt) FG_TRI(false, true, 1);
+        else FG_TRI(true, false, 1);
     } else {
-        if (nt) dgemm_fma_kernel<double, false, true, 2><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC);
-        else dgemm_fma_kernel<double, true, false, 2><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC);
+        if (nt) FG_TRI(false, true, 2);
+        else FG_TRI(true, false, 2);
     }
+#undef FG_TRI
     FG_CUDA(cudaGetLastError());
     return kOk;
 }
