@@ -845,9 +845,9 @@ __device__ __forceinline__ int move_store(const int (&mv_row)[4], const int (&mv
 // receiver's mbarrier: no flags, fences or polls of memory.  Per column:
 //   - every CTA's candidate (largest key, first row) by redux and one block
 //     barrier; the pending update of the candidate row applied on the fly;
-//   - warp w sends candidate row, key and row number to CTA w (and row jj from
-//     its owner); warp 0 sends the candidate's reciprocal after it, so that the
-//     division runs while the rows travel;
+//   - three warps send the candidate row, row jj (its owner) and key and row number
+//     to every CTA; in FP64 a fourth sends the candidate's reciprocal after them,
+//     so that the division runs while the rows travel;
 //   - the rest of the previous column's update, a warp per 32 rows and group of
 //     4-column quads, while the exchange is under way;
 //   - every warp settles the pivot from the 16 headers; a thread per row scales
@@ -859,25 +859,24 @@ __device__ __forceinline__ int move_store(const int (&mv_row)[4], const int (&mv
 // Bound: the chain search - exchange - settle (about 2200 clocks a column), from
 // about m = 2000 on the 16 SMs' FP64 pipes (m * 32 FMAs a column at 32 per
 // clock); in FP32 shared memory from about m = 6000 on.  Measured per column
-// against the grid panel: FP64 2.2 against 3.8 us at n = 500, 2.5 against 4.0 at
-// 2000, 3.1 against 4.1 at 4096 (whole LU); FP32 n = 16384, panels of the LU 45.9
+// against the grid panel: FP64 2.0 against 3.8 us at n = 500, 2.4 against 4.0 at
+// 2000, 3.0 against 4.1 at 4096 (whole LU); FP32 n = 16384, panels of the LU 42.7
 // against 59.8 ms.
 constexpr int CP_CS = 16;                       // CTAs of the cluster
 constexpr int CP_T = 512;                       // threads per CTA
 constexpr int CP_NW = CP_T / 32;
-static_assert(CP_NW == CP_CS, "warp w sends to CTA w");
 
 template <typename T>
 struct ClusterBuf {                             // one exchange buffer
     T row[CP_CS][PANEL_NB];                     // candidate rows
     T rowjj[PANEL_NB];
     ulonglong2 head[CP_CS];                     // key, row
-    double rinv[CP_CS];                         // 1 / candidate (0: divide)
+    double rinv[CP_CS];                         // FP64: 1 / candidate (0: divide)
 };
 
 template <typename T>
 constexpr uint32_t cluster_bytes() {            // received per column
-    return CP_CS * (PANEL_NB * sizeof(T) + 16 + 8) + PANEL_NB * sizeof(T);
+    return CP_CS * (PANEL_NB * sizeof(T) + 16 + (sizeof(T) == 8 ? 8 : 0)) + PANEL_NB * sizeof(T);
 }
 
 // Shared memory of a CTA: the buffers are static, R rows x 64 columns dynamic.
@@ -915,6 +914,18 @@ __device__ __forceinline__ float cp_rinv(float p) { return (p != 0.0f && fabsf(p
 __device__ __forceinline__ double cp_fma(double a, double b, double c) { return fma(a, b, c); }
 __device__ __forceinline__ float cp_fma(float a, float b, float c) { return fmaf(a, b, c); }
 
+// The lane holding the warp's largest key, the first on equal keys.
+__device__ __forceinline__ int cp_best(unsigned long long k, double) {
+    const unsigned hi = (unsigned)(k >> 32), lo = (unsigned)k;
+    const unsigned mhi = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+    return __ffs(__ballot_sync(0xffffffffu, hi == mhi && lo == mlo)) - 1;
+}
+__device__ __forceinline__ int cp_best(unsigned long long k, float) {      // keys below 2^32
+    const unsigned lo = (unsigned)k, m = __reduce_max_sync(0xffffffffu, lo);
+    return __ffs(__ballot_sync(0xffffffffu, lo == m)) - 1;
+}
+
 // Bounded wait of the whole block's threads on one phase of an mbarrier.
 __device__ __forceinline__ bool cp_wait(uint32_t bar, uint32_t parity) {
     for (unsigned i = 0; i < (1u << 20); ++i) {
@@ -938,7 +949,6 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
     extern __shared__ double S_raw[];
     T *S = reinterpret_cast<T *>(S_raw);
     __shared__ __align__(16) ClusterBuf<T> buf[3];
-    __shared__ __align__(16) T s_row[PANEL_NB], s_rowjj[PANEL_NB];
     __shared__ unsigned long long bars[3];
     __shared__ unsigned long long red_k[2][CP_NW];
     __shared__ int red_i[2][CP_NW];
@@ -1005,52 +1015,80 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
 
     int bi = 0;                                  // buffer of this column
     uint32_t phase = 0;                          // its parity
+    // rows are in the order of lanes, warps and CTAs: on equal keys the first lane
+    // (warp, CTA) wins.  Not with two rows per thread.
+    const bool ordered = nr <= CP_T;
     for (int jj = 0; jj < jb; ++jj) {
         // -- this CTA's candidate among its rows g >= jj
         unsigned long long k = nbk;
         int i = nbi;
-        warp_argmax(k, i);
-        if (lane == 0) { red_k[jj & 1][warp] = k; red_i[jj & 1][warp] = i; }
+        if (ordered) {
+            const int w = cp_best(k, T(0));
+            if (lane == w) { red_k[jj & 1][warp] = k; red_i[jj & 1][warp] = i; }
+        } else {
+            warp_argmax(k, i);
+            if (lane == 0) { red_k[jj & 1][warp] = k; red_i[jj & 1][warp] = i; }
+        }
         const uint32_t bar = cp_smem(&bars[bi]);
         if (tid == 0)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                          "r"(cluster_bytes<T>())
                          : "memory");
         if (__syncthreads_or(s_abort)) break;                        // B1
-        k = lane < CP_NW ? red_k[jj & 1][lane] : kKeyNone;
-        i = lane < CP_NW ? red_i[jj & 1][lane] : INT_MAX;
-        warp_argmax(k, i);
-        // entry c of local row x with the pending interchange and update
-        auto fin = [&](int x, int c) -> T {
-            const bool sw = d_swap && rb + x == d_gs && c != d_jj && c != d_jj + 1;
-            const T v = sw ? dO[c] : S[c * R + x];
-            return (d_jj < 0 || c < d_jj + 2) ? v : cp_fma(-dP[c], S[d_jj * R + x], v);
-        };
-        // candidate row by warps 0 and 1, row jj by warps 2 and 3 (once per CTA:
-        // an FP64 instruction holds its scheduler's pipe for 64 clocks)
-        const bool has_i = i != INT_MAX, has_jj = jj >= rb && jj < rb + nr;
-        if (warp < 4) {
-            const int c = (warp & 1) * 32 + lane;
-            if (warp < 2) s_row[c] = has_i ? fin(i - rb, c) : T(0);
-            else if (has_jj) s_rowjj[c] = fin(jj - rb, c);
-        }
-        __syncthreads();                                             // B1b
-        // -- the candidate to CTA `warp`
         ClusterBuf<T> &cur = buf[bi];
-        {
-            const uint32_t rbar = cp_map(bar, warp);
-            cp_send_pair(cp_map(cp_smem(&cur.row[b][2 * lane]), warp), rbar, s_row[2 * lane], s_row[2 * lane + 1]);
-            if (has_jj)
-                cp_send_pair(cp_map(cp_smem(&cur.rowjj[2 * lane]), warp), rbar, s_rowjj[2 * lane],
-                             s_rowjj[2 * lane + 1]);
-            if (lane == 0) cp_send16(cp_map(cp_smem(&cur.head[b]), warp), rbar, k, (unsigned long long)(unsigned)i);
+        // Warps 0 and 1 send the candidate row and row jj, each lane two columns of
+        // it to all CTAs; warp 2 the key and row number, a lane per CTA; warp 3 (FP64)
+        // the reciprocal.  The others wait only until the rows are read.
+        constexpr int NSEND = sizeof(T) == 8 ? 4 : 3;
+        bool sent = false;
+        if (warp < NSEND) {
+            k = lane < CP_NW ? red_k[jj & 1][lane] : kKeyNone;
+            i = lane < CP_NW ? red_i[jj & 1][lane] : INT_MAX;
+            if (ordered) {
+                const int w = cp_best(k, T(0));
+                k = __shfl_sync(0xffffffffu, k, w);
+                i = __shfl_sync(0xffffffffu, i, w);
+            } else {
+                warp_argmax(k, i);
+            }
+            // entry c of local row x with the pending interchange and update
+            auto fin = [&](int x, int c) -> T {
+                const bool sw = d_swap && rb + x == d_gs && c != d_jj && c != d_jj + 1;
+                const T v = sw ? dO[c] : S[c * R + x];
+                return (d_jj < 0 || c < d_jj + 2) ? v : cp_fma(-dP[c], S[d_jj * R + x], v);
+            };
+            const bool has = warp == 0 ? i != INT_MAX : (jj >= rb && jj < rb + nr);
+            if (warp < 2) {
+                const int x = (warp == 0 ? i : jj) - rb;
+                T v0 = T(0), v1 = T(0);
+                if (has) {
+                    v0 = fin(x, 2 * lane);
+                    v1 = fin(x, 2 * lane + 1);
+                }
+                __syncwarp();
+                named_bar_arrive(1, CP_T);
+                sent = true;
+                if (warp == 0 || has) {
+                    const uint32_t dst = cp_smem(warp == 0 ? &cur.row[b][2 * lane] : &cur.rowjj[2 * lane]);
+#pragma unroll
+                    for (int t = 0; t < CP_CS; ++t) cp_send_pair(cp_map(dst, t), cp_map(bar, t), v0, v1);
+                }
+                named_bar_sync(2, 64);           // both rows are read
+            } else if (warp == 2) {
+                if (lane < CP_CS)
+                    cp_send16(cp_map(cp_smem(&cur.head[b]), lane), cp_map(bar, lane), k, (unsigned long long)(unsigned)i);
+            } else {
+                // (column jj is final; 0 where the CTA has no row left)
+                const T pc = i != INT_MAX ? S[jj * R + i - rb] : T(0);
+                named_bar_sync(1, CP_T);
+                sent = true;
+                const double r = (double)cp_rinv(pc);
+                if (lane < CP_CS)
+                    cp_send8(cp_map(cp_smem(&cur.rinv[b]), lane), cp_map(bar, lane),
+                             (unsigned long long)__double_as_longlong(r));
+            }
         }
-        if (warp == 0) {
-            const double r = (double)cp_rinv(s_row[jj]);
-            if (lane < CP_CS)
-                cp_send8(cp_map(cp_smem(&cur.rinv[b]), lane), cp_map(bar, lane),
-                         (unsigned long long)__double_as_longlong(r));
-        }
+        if (!sent) named_bar_sync(1, CP_T);
         // -- the pending update of column d_jj: columns >= d_jj + 2
         if (d_jj >= 0) {
             const int nrb = (nr + 31) / 32;
@@ -1061,55 +1099,71 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
                 if (r < nr && g > d_jj) {
                     const T l = S[d_jj * R + r];
                     const bool sw = d_swap && g == d_gs;
-                    for (int q = q0 + cg; q < q1; q += ncg) {
-                        T p[4], v[4];
+                    // two quads at a time: eight loads before the first store
+                    for (int q = q0 + cg; q < q1; q += 2 * ncg) {
+                        const int qb = q + ncg < q1 ? q + ncg : q;
+                        T p[8], v[8];
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) p[h] = dP[4 * q + h];
+                        for (int h = 0; h < 4; ++h) {
+                            p[h] = dP[4 * q + h];
+                            p[4 + h] = dP[4 * qb + h];
+                        }
 #pragma unroll
-                        for (int h = 0; h < 4; ++h) v[h] = sw ? dO[4 * q + h] : S[(4 * q + h) * R + r];
+                        for (int h = 0; h < 4; ++h) {
+                            v[h] = sw ? dO[4 * q + h] : S[(4 * q + h) * R + r];
+                            v[4 + h] = sw ? dO[4 * qb + h] : S[(4 * qb + h) * R + r];
+                        }
 #pragma unroll
                         for (int h = 0; h < 4; ++h)
                             if (4 * q + h >= d_jj + 2) S[(4 * q + h) * R + r] = cp_fma(-p[h], l, v[h]);
+                        if (qb != q)
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) S[(4 * qb + h) * R + r] = cp_fma(-p[4 + h], l, v[4 + h]);
                     }
                 }
             }
             if (warp == CP_NW - 2) write_swap();
         }
+        // -- this thread's entries of columns jj and jj + 1 (its own writes)
+        constexpr int RPT = sizeof(T) == 8 ? 1 : 2;              // rows per thread at most
+        T c0[RPT], c1[RPT];
+#pragma unroll
+        for (int h = 0; h < RPT; ++h) {
+            const int r = tid + h * CP_T;
+            c0[h] = r < nr ? S[jj * R + r] : T(0);
+            c1[h] = r < nr && jj + 1 < jb ? S[(jj + 1) * R + r] : T(0);
+        }
         // -- the 16 candidates
-        if (!cp_wait(bar, phase)) {
+        const bool arrived = cp_wait(bar, phase);
+        if (!arrived) {
             atomicOr(status, kDevBarrierTimeout);
             s_abort = 1;
         }
-        unsigned long long gk = kKeyNone;
-        int gi = INT_MAX;
-        if (lane < CP_CS) {
-            const ulonglong2 h = cur.head[lane];
-            gk = h.x;
-            gi = (int)(unsigned)h.y;
-        }
-        warp_argmax(gk, gi);
+        const ulonglong2 head = cur.head[lane & (CP_CS - 1)];
         const T ajj = cur.rowjj[jj];
+        int src = cp_best(head.x, T(0)) & (CP_CS - 1);
+        const int gi = (int)(unsigned)__shfl_sync(0xffffffffu, (unsigned)head.y, src);
         const bool jnan = cp_key(ajj) == 1ull;    // integer tests: no FP64 compares
-        const int gs = (jnan || gi < 0 || gi >= mp) ? jj : gi;  // (out of range: a wait gave up)
-        const int src = gs / R;
-        const T *P = cur.row[src], *O = cur.rowjj;
-        if (jnan) P = O;
+        const bool own = jnan || gi < 0 || gi >= mp;              // (out of range: a wait gave up)
+        const int gs = own ? jj : gi;
+        const T *P = own ? cur.rowjj : cur.row[src], *O = cur.rowjj;
         const T pv = P[jj];
-        const T rinv = jnan ? T(0) : (T)cur.rinv[src];
+        const T rinv = jnan ? T(0) : sizeof(T) == 8 ? (T)cur.rinv[src] : cp_rinv(pv);
         const bool pnz = cp_key(pv) != 2ull, rnz = cp_key(rinv) != 2ull;
         const bool swap = pnz && gs != jj;
         // -- thread per row: scale, column jj + 1, next key
         nbk = kKeyNone;
         nbi = INT_MAX;
-        for (int r = tid; r < nr; r += CP_T) {
-            const int g = rb + r;
-            if (g <= jj) continue;
+#pragma unroll
+        for (int h = 0; h < RPT; ++h) {
+            const int r = tid + h * CP_T, g = rb + r;
+            if (r >= nr || g <= jj) continue;
             const bool sw = swap && g == gs;
-            T l = sw ? O[jj] : S[jj * R + r];
+            T l = sw ? O[jj] : c0[h];
             if (pnz) l = rnz ? l * rinv : l / pv;
             S[jj * R + r] = l;
             if (jj + 1 < jb) {
-                const T v = cp_fma(-P[jj + 1], l, sw ? O[jj + 1] : S[(jj + 1) * R + r]);
+                const T v = cp_fma(-P[jj + 1], l, sw ? O[jj + 1] : c1[h]);
                 S[(jj + 1) * R + r] = v;
                 const unsigned long long key = cp_key(v);
                 if (better(key, g, nbk, nbi)) { nbk = key; nbi = g; }
