@@ -849,9 +849,14 @@ __device__ __forceinline__ int move_store(const int (&mv_row)[4], const int (&mv
 //     to every CTA; in FP64 a fourth sends the candidate's reciprocal after them,
 //     so that the division runs while the rows travel;
 //   - the rest of the previous column's update, a warp per 32 rows and group of
-//     4-column quads, while the exchange is under way;
+//     4-column quads, while the exchange is under way; it reaches only to the end of
+//     the sub-panel of 16 columns (FP32);
 //   - every warp settles the pivot from the 16 headers; a thread per row scales
 //     its entry, updates column jj+1 and takes its key for the next search.
+// After the last column of a sub-panel all columns beyond it take its 16 updates at
+// once, from registers (their U rows are solved column by column meanwhile): in
+// shared memory every entry is then read and written 1/16 as often.  Per element the
+// operations and their order stay those of the column-by-column update.
 // The interchange of a row is applied where its entries are next read and
 // written by one warp after the next candidate is out.  Three exchange buffers: a
 // CTA can send column jj+3 only after all have sent jj+2, which they do after
@@ -865,6 +870,10 @@ __device__ __forceinline__ int move_store(const int (&mv_row)[4], const int (&mv
 constexpr int CP_CS = 16;                       // CTAs of the cluster
 constexpr int CP_T = 512;                       // threads per CTA
 constexpr int CP_NW = CP_T / 32;
+// Columns of a sub-panel.  FP64 has none: its bound is the FP64 pipe, not shared
+// memory, and the U rows, 15 dependent FP64 FMAs, made a column 12% slower.
+template <typename T>
+constexpr int CP_SB = sizeof(T) == 8 ? PANEL_NB : 16;
 
 template <typename T>
 struct ClusterBuf {                             // one exchange buffer
@@ -882,7 +891,8 @@ constexpr uint32_t cluster_bytes() {            // received per column
 // Shared memory of a CTA: the buffers are static, R rows x 64 columns dynamic.
 template <typename T>
 constexpr size_t cluster_rows_max() {
-    return ((227 * 1024 - 2048 - 3 * sizeof(ClusterBuf<T>)) / (PANEL_NB * sizeof(T))) * CP_CS;
+    return ((227 * 1024 - 2048 - 3 * sizeof(ClusterBuf<T>) - (CP_SB<T> % PANEL_NB) * PANEL_NB * sizeof(T)) / (PANEL_NB * sizeof(T))) *
+           CP_CS;
 }
 
 __device__ __forceinline__ uint32_t cp_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -949,6 +959,8 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
     extern __shared__ double S_raw[];
     T *S = reinterpret_cast<T *>(S_raw);
     __shared__ __align__(16) ClusterBuf<T> buf[3];
+    constexpr int SB = CP_SB<T>;
+    __shared__ __align__(16) T Us[SB < PANEL_NB ? SB : 1][PANEL_NB];   // U rows of the sub-panel, columns beyond it
     __shared__ unsigned long long bars[3];
     __shared__ unsigned long long red_k[2][CP_NW];
     __shared__ int red_i[2][CP_NW];
@@ -994,11 +1006,13 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
     move_init(mv_row, mv_src, lane, j0, jb);
 
     // the column whose update is pending (-1: none), its pivot row and buffers
-    int d_jj = -1, d_gs = -1;
+    // (d_end: end of the columns it covers, 0 after a bulk update; d_done: the
+    // columns d_jj .. d_done of row d_gs hold newer values than dO)
+    int d_jj = -1, d_gs = -1, d_end = 0, d_done = 0;
     bool d_swap = false;
     const T *dP = nullptr, *dO = nullptr;
     // deferred writes of the interchange of column d_jj: row d_jj <- dP, row
-    // d_gs <- dO (but its columns d_jj and d_jj + 1, which hold newer values)
+    // d_gs <- dO (its columns d_jj + 2 .. d_end - 1: by the pending update)
     auto write_swap = [&]() {
         if (!d_swap) return;
         const int rj = d_jj - rb, rg = d_gs - rb;
@@ -1006,10 +1020,21 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
         for (int h = 0; h < 2; ++h) {
             const int c = lane + 32 * h;
             if (c < jb) {
-                if (rj >= 0 && rj < nr) S[c * R + rj] = dP[c];
-                // columns beyond d_jj + 1 are written by the pending update
-                if (rg >= 0 && rg < nr && c < d_jj) S[c * R + rg] = dO[c];
+                if (rj >= 0 && rj < nr && (c <= d_jj || d_end)) S[c * R + rj] = dP[c];
+                if (rg >= 0 && rg < nr && (c < d_jj || (d_end && c >= d_end))) S[c * R + rg] = dO[c];
             }
+        }
+    };
+
+    // U row jj of the sub-panel at s0 beyond it, from the pivot row P as exchanged (whose
+    // entries there are not updated yet): warp half `w` takes 32 of the columns
+    auto u_row = [&](int jj, int s0, int w, const T *P) {
+        if constexpr (SB < PANEL_NB) {
+        const int c = s0 + SB + 32 * w + lane;
+        if (c >= PANEL_NB) return;
+        T v = P[c];
+        for (int t = s0; t < jj; ++t) v = cp_fma(-Us[t - s0][c], P[t], v);
+        Us[jj - s0][c] = v;
         }
     };
 
@@ -1019,6 +1044,8 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
     // (warp, CTA) wins.  Not with two rows per thread.
     const bool ordered = nr <= CP_T;
     for (int jj = 0; jj < jb; ++jj) {
+        const int s0 = jj & ~(SB - 1), s1 = s0 + SB;
+        const bool bulk = SB < PANEL_NB && jj == s1 - 1 && s1 < jb;           // last column of a sub-panel
         // -- this CTA's candidate among its rows g >= jj
         unsigned long long k = nbk;
         int i = nbi;
@@ -1053,9 +1080,9 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
             }
             // entry c of local row x with the pending interchange and update
             auto fin = [&](int x, int c) -> T {
-                const bool sw = d_swap && rb + x == d_gs && c != d_jj && c != d_jj + 1;
+                const bool sw = d_swap && rb + x == d_gs && (c < d_jj || c > d_done);
                 const T v = sw ? dO[c] : S[c * R + x];
-                return (d_jj < 0 || c < d_jj + 2) ? v : cp_fma(-dP[c], S[d_jj * R + x], v);
+                return (c >= d_jj + 2 && c < d_end) ? cp_fma(-dP[c], S[d_jj * R + x], v) : v;
             };
             const bool has = warp == 0 ? i != INT_MAX : (jj >= rb && jj < rb + nr);
             if (warp < 2) {
@@ -1089,11 +1116,11 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
             }
         }
         if (!sent) named_bar_sync(1, CP_T);
-        // -- the pending update of column d_jj: columns >= d_jj + 2
-        if (d_jj >= 0) {
+        // -- the pending update of column d_jj: columns d_jj + 2 .. d_end - 1
+        if (d_end) {
             const int nrb = (nr + 31) / 32;
             const int ncg = nrb >= CP_NW ? 1 : CP_NW / max(nrb, 1);
-            const int q0 = (d_jj + 2) >> 2, q1 = (jb + 3) >> 2;
+            const int q0 = (d_jj + 2) >> 2, q1 = d_end >> 2;
             for (int u = warp; u < nrb * ncg; u += CP_NW) {
                 const int cg = u / nrb, r = (u - cg * nrb) * 32 + lane, g = rb + r;
                 if (r < nr && g > d_jj) {
@@ -1122,8 +1149,9 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
                     }
                 }
             }
-            if (warp == CP_NW - 2) write_swap();
+            if (SB < PANEL_NB && s1 < jb && (warp == CP_NW - 4 || warp == CP_NW - 3)) u_row(d_jj, s0, warp - (CP_NW - 4), dP);
         }
+        if (warp == CP_NW - 2) write_swap();
         // -- this thread's entries of columns jj and jj + 1 (its own writes)
         constexpr int RPT = sizeof(T) == 8 ? 1 : 2;              // rows per thread at most
         T c0[RPT], c1[RPT];
@@ -1162,16 +1190,59 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
             T l = sw ? O[jj] : c0[h];
             if (pnz) l = rnz ? l * rinv : l / pv;
             S[jj * R + r] = l;
-            if (jj + 1 < jb) {
+            if (jj + 1 < jb && !bulk) {
                 const T v = cp_fma(-P[jj + 1], l, sw ? O[jj + 1] : c1[h]);
                 S[(jj + 1) * R + r] = v;
                 const unsigned long long key = cp_key(v);
                 if (better(key, g, nbk, nbi)) { nbk = key; nbi = g; }
             }
         }
+        if constexpr (SB < PANEL_NB) if (bulk) {
+            // -- the columns beyond the sub-panel, all its updates at once
+            if (warp == CP_NW - 4 || warp == CP_NW - 3) u_row(jj, s0, warp - (CP_NW - 4), P);
+            __syncthreads();
+            const int nrb = (nr + 31) / 32;
+            const int ncg = nrb >= CP_NW ? 1 : CP_NW / max(nrb, 1);
+            const int q1 = (jb + 3) >> 2;
+            for (int u = warp; u < nrb * ncg; u += CP_NW) {
+                const int cg = u / nrb, r = (u - cg * nrb) * 32 + lane, g = rb + r;
+                if (r >= nr || g < s0) continue;
+                const bool sw = swap && g == gs;
+                T l[SB];
+#pragma unroll
+                for (int t = 0; t < SB; ++t)
+                    l[t] = g < s1 ? T(0) : (sw && t < SB - 1) ? O[s0 + t] : S[(s0 + t) * R + r];
+                for (int q = (s1 >> 2) + cg; q < q1; q += ncg) {
+                    T v[4];
+                    if (g < s1) {                        // a pivot row: final
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) v[h] = Us[g - s0][4 * q + h];
+                    } else {
+#pragma unroll
+                        for (int h = 0; h < 4; ++h) v[h] = sw ? O[4 * q + h] : S[(4 * q + h) * R + r];
+#pragma unroll
+                        for (int t = 0; t < SB; ++t) {
+                            T p[4];
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) p[h] = Us[t][4 * q + h];
+#pragma unroll
+                            for (int h = 0; h < 4; ++h) v[h] = cp_fma(-p[h], l[t], v[h]);
+                        }
+                        if (q == (s1 >> 2)) {            // column s1, by the thread of this row
+                            const unsigned long long key = cp_key(v[0]);
+                            if (better(key, g, nbk, nbi)) { nbk = key; nbi = g; }
+                        }
+                    }
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) S[(4 * q + h) * R + r] = v[h];
+                }
+            }
+        }
         d_jj = jj;
         d_gs = gs;
         d_swap = swap;
+        d_end = bulk ? 0 : s1;
+        d_done = bulk ? PANEL_NB : jj + 1;
         dP = P;
         dO = O;
         if (b == 0 && warp == CP_NW - 1) {
