@@ -41,7 +41,7 @@ struct EpiF32 {
     // column j of the next tile's C into L2 (a contiguous run of its rows),
     // so that the epilogue's loads of it hit L2 instead of HBM
     __device__ void prefetch(int m0, int n0, int M, int N, int j) const {
-        if (!pf || beta == 0.0f || j >= min(kBN, N - n0)) return;
+        if (!pf || j >= min(kBN, N - n0)) return;      // (C is read for every beta: 0 * NaN)
         const int bytes = (min(BM, M - m0) * 4) & ~15;
         if (bytes <= 0) return;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(
@@ -80,29 +80,29 @@ struct EpiF32 {
 // in[k + r*ld] (TRANS = true).  out is K-major: out[r*ldo + k].  Columns
 // k >= K up to ldo are zero-filled.
 template <int KIND>
-__device__ __forceinline__ void store_lp(void *out, size_t idx, float v);
+__device__ __forceinline__ uint32_t to_lp(float v);
 
 template <>
-__device__ __forceinline__ void store_lp<kTcBF16>(void *out, size_t idx, float v) {
-    ((__nv_bfloat16 *)out)[idx] = __float2bfloat16_rn(v);
+__device__ __forceinline__ uint32_t to_lp<kTcBF16>(float v) {
+    return __bfloat16_as_ushort(__float2bfloat16_rn(v));
 }
 template <>
-__device__ __forceinline__ void store_lp<kTcTF32>(void *out, size_t idx, float v) {
+__device__ __forceinline__ uint32_t to_lp<kTcTF32>(float v) {
     uint32_t t;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(t) : "f"(v));
-    ((uint32_t *)out)[idx] = t;
+    return t;
 }
 template <>
-__device__ __forceinline__ void store_lp<kTcTF32Lo>(void *out, size_t idx, float v) {
+__device__ __forceinline__ uint32_t to_lp<kTcTF32Lo>(float v) {
     uint32_t h, t;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
     const float lo = v - __uint_as_float(h);
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(t) : "f"(lo));
-    ((uint32_t *)out)[idx] = t;
+    return t;
 }
 template <>
-__device__ __forceinline__ void store_lp<kTcFP8>(void *out, size_t idx, float v) {
-    ((__nv_fp8_storage_t *)out)[idx] = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
+__device__ __forceinline__ uint32_t to_lp<kTcFP8>(float v) {
+    return __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
 // the terms of the e4m3 splits: t0 = e4m3(v), t1 = e4m3(v - t0),
 // t2 = e4m3(v - t0 - t1).  Each difference is exact in FP32: a term has 4
@@ -112,71 +112,111 @@ __device__ __forceinline__ float fp8_round(float v, __nv_fp8_storage_t *q) {
     return __half2float(__half(__nv_cvt_fp8_to_halfraw(*q, __NV_E4M3)));
 }
 template <>
-__device__ __forceinline__ void store_lp<kTcFP8Lo>(void *out, size_t idx, float v) {
+__device__ __forceinline__ uint32_t to_lp<kTcFP8Lo>(float v) {
     __nv_fp8_storage_t q;
     const float t0 = fp8_round(v, &q);
     fp8_round(v - t0, &q);
-    ((__nv_fp8_storage_t *)out)[idx] = q;
+    return q;
 }
 template <>
-__device__ __forceinline__ void store_lp<kTcFP8Lo2>(void *out, size_t idx, float v) {
+__device__ __forceinline__ uint32_t to_lp<kTcFP8Lo2>(float v) {
     __nv_fp8_storage_t q;
     const float t0 = fp8_round(v, &q);
     const float t1 = fp8_round(v - t0, &q);
     fp8_round(v - t0 - t1, &q);
-    ((__nv_fp8_storage_t *)out)[idx] = q;
+    return q;
+}
+
+// A block takes 32 rows x 64 k through shared memory: 8 loads in flight per
+// thread along whichever index is contiguous, then a thread stores 4 consecutive
+// k at once (16 lanes: 64 to 256 bytes of a row).  Bound: HBM.  4100 x 3000 to
+// BF16: 29 us with one 4-byte load and one 2-byte store at a time.
+constexpr int CONV_R = 32, CONV_K = 64;
+template <bool RCONTIG>
+__device__ __forceinline__ void conv_load(float (*tile)[CONV_K + 2], int r0, int k0, int R, int K,
+                                          const float *__restrict__ in, int ld) {
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = RCONTIG ? r0 + lane : r0 + wy + 8 * (i >> 1);
+        const int k = RCONTIG ? k0 + wy + 8 * i : k0 + lane + 32 * (i & 1);
+        v[i] = (r < R && k < K) ? in[RCONTIG ? (size_t)r + (size_t)k * ld : (size_t)k + (size_t)r * ld] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        tile[RCONTIG ? lane : wy + 8 * (i >> 1)][RCONTIG ? wy + 8 * i : lane + 32 * (i & 1)] = v[i];
+    __syncthreads();
+}
+
+// Four consecutive entries at out[idx]: one store where the row has them all
+// (idx is a multiple of 4 and the rows start on 16 bytes).
+template <int BYTES>
+__device__ __forceinline__ void store4(void *out, size_t idx, const uint32_t (&w)[4], int n) {
+    if (n >= 4) {
+        if (BYTES == 4) ((uint4 *)out)[idx / 4] = make_uint4(w[0], w[1], w[2], w[3]);
+        else if (BYTES == 2) ((uint2 *)out)[idx / 4] = make_uint2(w[0] | (w[1] << 16), w[2] | (w[3] << 16));
+        else ((uint32_t *)out)[idx / 4] = w[0] | (w[1] << 8) | (w[2] << 16) | (w[3] << 24);
+        return;
+    }
+    for (int i = 0; i < n; ++i) {
+        if (BYTES == 4) ((uint32_t *)out)[idx + i] = w[i];
+        else if (BYTES == 2) ((uint16_t *)out)[idx + i] = (uint16_t)w[i];
+        else ((uint8_t *)out)[idx + i] = (uint8_t)w[i];
+    }
 }
 
 template <int KIND, bool RCONTIG>
 __global__ void __launch_bounds__(256)
 to_kmajor_kernel(int R, int K, const float *__restrict__ in, int ld, void *__restrict__ out,
                  int ldo, int width, const float *__restrict__ inv_scale) {
-    __shared__ float tile[32][33];
-    const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
-    if (RCONTIG) {
-        for (int kk = ty; kk < 32; kk += 8) {
-            const int r = r0 + tx, k = k0 + kk;
-            tile[kk][tx] = (r < R && k < K) ? in[(size_t)r + (size_t)k * ld] : 0.0f;
-        }
-        __syncthreads();
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            if (r < R && k < width) {
-                float v = tile[tx][rr];
-                if (inv_scale) v *= inv_scale[r];
-                store_lp<KIND>(out, (size_t)r * ldo + k, v);
-            }
-        }
-    } else {
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            if (r < R && k < width) {
-                float v = (k < K) ? in[(size_t)k + (size_t)r * ld] : 0.0f;
-                if (inv_scale) v *= inv_scale[r];
-                store_lp<KIND>(out, (size_t)r * ldo + k, v);
-            }
-        }
+    __shared__ float tile[CONV_R][CONV_K + 2];
+    const int r0 = blockIdx.x * CONV_R, k0 = blockIdx.y * CONV_K;
+    conv_load<RCONTIG>(tile, r0, k0, R, K, in, ld);
+    constexpr int BYTES = KIND == kTcBF16 ? 2 : (KIND == kTcTF32 || KIND == kTcTF32Lo) ? 4 : 1;
+    const int kq = (threadIdx.x & 15) * 4, k = k0 + kq;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int rr = (threadIdx.x >> 4) + 16 * h, r = r0 + rr;
+        if (r >= R || k >= width) continue;
+        const float sc = inv_scale ? inv_scale[r] : 1.0f;
+        uint32_t w[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = to_lp<KIND>(inv_scale ? tile[rr][kq + i] * sc : tile[rr][kq + i]);
+        store4<BYTES>(out, (size_t)r * ldo + k, w, width - k);
     }
 }
 
 // Per-row amax of op(X) (R rows, K columns) -> scale = amax/448 and 1/scale
 // (FP8 e4m3 per-row scaling; a zero row keeps scale 1).
+// Rows contiguous: 32 rows x 32 k-lanes per block (a warp per row would touch a
+// sector per entry); else a warp per row.
+constexpr int RS_THREADS = 1024;
 template <bool RCONTIG>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(RS_THREADS)
 row_scale_kernel(int R, int K, const float *__restrict__ in, int ld, float *__restrict__ scale,
                  float *__restrict__ inv_scale) {
+    __shared__ float sm[32][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r = blockIdx.x * 8 + warp;
-    if (r >= R) return;
     float m = 0.0f;
-    for (int k = lane; k < K; k += 32) {
-        const float v = RCONTIG ? in[(size_t)r + (size_t)k * ld] : in[(size_t)k + (size_t)r * ld];
-        m = fmaxf(m, fabsf(v));
+    if (RCONTIG) {
+        const int r = blockIdx.x * 32 + lane;
+        if (r < R)
+#pragma unroll 8
+            for (int k = warp; k < K; k += 32) m = fmaxf(m, fabsf(in[(size_t)r + (size_t)k * ld]));
+        sm[lane][warp] = m;
+        __syncthreads();
+        m = sm[warp][lane];
+    } else {
+        const int r = blockIdx.x * 32 + warp;
+        if (r < R)
+#pragma unroll 8
+            for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(in[(size_t)k + (size_t)r * ld]));
     }
+    const int r = blockIdx.x * 32 + warp;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    if (lane == 0) {
+    if (lane == 0 && r < R) {
         const float s = (m > 0.0f && isfinite(m)) ? m / 448.0f : 1.0f;
         scale[r] = s;
         inv_scale[r] = 1.0f / s;
@@ -185,7 +225,7 @@ row_scale_kernel(int R, int K, const float *__restrict__ in, int ld, float *__re
 
 // The split forms' operands in one pass: each entry of op(X) (R x K) is read
 // once, split into its terms -- TF32: t0 = tf32(v), t1 = tf32(v - t0); e4m3
-// (after the row scale): t0, t1, t2 as store_lp -- and segment q of the
+// (after the row scale): t0, t1, t2 as to_lp -- and segment q of the
 // K-major output row (columns q*kp .. q*kp + kp - 1, zero beyond K) gets term
 // seg[q].  Bitwise the terms of one tc_convert call per segment.
 struct SegTerms {
@@ -197,48 +237,41 @@ template <bool FP8, bool RCONTIG>
 __global__ void __launch_bounds__(256)
 to_kmajor_terms_kernel(int R, int K, const float *__restrict__ in, int ld, void *__restrict__ out,
                        int ldo, int kp, SegTerms st, const float *__restrict__ inv_scale) {
-    __shared__ float tile[32][33];
-    const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
-    auto emit = [&](int r, int k, float v) {
-        if (FP8 && inv_scale) v *= inv_scale[r];
-        uint32_t w0, w1, w2 = 0u;
-        if (FP8) {
-            __nv_fp8_storage_t q;
-            const float t0 = fp8_round(v, &q);
-            w0 = q;
-            const float t1 = fp8_round(v - t0, &q);
-            w1 = q;
-            fp8_round(v - t0 - t1, &q);
-            w2 = q;
-        } else {
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(w0) : "f"(v));
-            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(w1) : "f"(v - __uint_as_float(w0)));
+    __shared__ float tile[CONV_R][CONV_K + 2];
+    const int r0 = blockIdx.x * CONV_R, k0 = blockIdx.y * CONV_K;
+    conv_load<RCONTIG>(tile, r0, k0, R, K, in, ld);
+    const int kq = (threadIdx.x & 15) * 4, k = k0 + kq;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int rr = (threadIdx.x >> 4) + 16 * h, r = r0 + rr;
+        if (r >= R || k >= kp) continue;
+        const float sc = FP8 && inv_scale ? inv_scale[r] : 1.0f;
+        uint32_t w[3][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float v = FP8 && inv_scale ? tile[rr][kq + i] * sc : tile[rr][kq + i];
+            if (FP8) {
+                __nv_fp8_storage_t q;
+                const float t0 = fp8_round(v, &q);
+                w[0][i] = q;
+                const float t1 = fp8_round(v - t0, &q);
+                w[1][i] = q;
+                fp8_round(v - t0 - t1, &q);
+                w[2][i] = q;
+            } else {
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(w[0][i]) : "f"(v));
+                asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(w[1][i]) : "f"(v - __uint_as_float(w[0][i])));
+                w[2][i] = 0u;
+            }
         }
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
             if (q >= st.nseg) break;
             const int tq = st.term[q];
-            const uint32_t val = tq == 0 ? w0 : tq == 1 ? w1 : w2;
-            const size_t idx = (size_t)r * ldo + (size_t)q * kp + k;
-            if (FP8) ((__nv_fp8_storage_t *)out)[idx] = (__nv_fp8_storage_t)val;
-            else ((uint32_t *)out)[idx] = val;
-        }
-    };
-    if (RCONTIG) {
-        for (int kk = ty; kk < 32; kk += 8) {
-            const int r = r0 + tx, k = k0 + kk;
-            tile[kk][tx] = (r < R && k < K) ? in[(size_t)r + (size_t)k * ld] : 0.0f;
-        }
-        __syncthreads();
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            if (r < R && k < kp) emit(r, k, tile[tx][rr]);
-        }
-    } else {
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            if (r < R && k < kp) emit(r, k, (k < K) ? in[(size_t)k + (size_t)r * ld] : 0.0f);
+            uint32_t x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = tq == 0 ? w[0][i] : tq == 1 ? w[1][i] : w[2][i];
+            store4<FP8 ? 1 : 4>(out, (size_t)r * ldo + (size_t)q * kp + k, x, kp - k);
         }
     }
 }
@@ -309,6 +342,16 @@ int tc_kmajor_ld(int kind, int K) {
     return (K + per16 - 1) / per16 * per16;
 }
 
+size_t tc_elem_bytes(int kind);
+
+// Row pitch (elements) of a K-major operand of `cols` columns: whole 128-byte
+// lines, so that the 128-byte rows of a TMA box lie in one line each (4100 x 4000
+// x 3000 in BF16: 127 us on rows of 6000 bytes, 95 on 6016).
+int tc_row_pitch(int kind, int cols) {
+    const int line = 128 / (int)tc_elem_bytes(kind);
+    return (cols + line - 1) / line * line;
+}
+
 size_t tc_elem_bytes(int kind) {
     kind = gemm_kind(kind);
     return kind == kTcTF32 ? 4 : kind == kTcBF16 ? 2 : 1;
@@ -327,12 +370,12 @@ int tc_convert(int kind, bool trans, int R, int K, const float *X, int ldx, void
     const bool rcontig = !trans;
     const bool fp8 = kind == kTcFP8 || kind == kTcFP8Lo || kind == kTcFP8Lo2;
     if (fp8 && scale != nullptr) {
-        const dim3 g(ceil_div(R, 8));
-        if (rcontig) row_scale_kernel<true><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        const dim3 g(ceil_div(R, 32));
+        if (rcontig) row_scale_kernel<true><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        else row_scale_kernel<false><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
         FG_CUDA(cudaGetLastError());
     }
-    const dim3 grid(ceil_div(R, 32), ceil_div(width, 32));
+    const dim3 grid(ceil_div(R, CONV_R), ceil_div(width, CONV_K));
     const float *inv = fp8 ? inv_scale : nullptr;
 #define FG_CONV(KD)                                                                          \
     do {                                                                                     \
@@ -360,11 +403,11 @@ int tc_convert_terms(bool fp8, bool trans, int R, int K, const float *X, int ldx
     KTimer kt(kFamAux, stream, 0.0, (4.0 + (fp8 ? 1.0 : 4.0) * st.nseg) * R * (double)K);
     const bool rcontig = !trans;
     if (fp8) {
-        const dim3 g(ceil_div(R, 8));
-        if (rcontig) row_scale_kernel<true><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        const dim3 g(ceil_div(R, 32));
+        if (rcontig) row_scale_kernel<true><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        else row_scale_kernel<false><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
     }
-    const dim3 grid(ceil_div(R, 32), ceil_div(kp, 32));
+    const dim3 grid(ceil_div(R, CONV_R), ceil_div(kp, CONV_K));
     const float *inv = fp8 ? inv_scale : nullptr;
     if (fp8) {
         if (rcontig) to_kmajor_terms_kernel<true, true><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, kp, st, inv);
@@ -423,6 +466,7 @@ size_t tc_update_workspace_bytes(int kind, int m, int n, int k) {
     int ld = tc_kmajor_ld(kind, k);
     if (kind == kTcF32x3 || kind == kTcFP8x2) ld *= 3;   // three K segments, see f32x3_gemm
     if (kind == kTcFP8x3) ld *= 6;                       // six, see fp8_terms_gemm
+    ld = tc_row_pitch(kind, ld);
     const size_t eb = tc_elem_bytes(kind);
     const size_t a = round256((size_t)m * ld * eb), b = round256((size_t)n * ld * eb);
     size_t total = a + b;
@@ -439,14 +483,14 @@ namespace {
 // written once (three separate products each read and wrote C).
 int f32x3_gemm(bool ta_rows, bool tb_rows, int m, int n, int k, float alpha, const float *A, int ldA,
                const float *B, int ldB, float beta, float *C, int ldC, void *buf, cudaStream_t s) {
-    const int kp = tc_kmajor_ld(kTcTF32, k), ld3 = 3 * kp;
+    const int kp = tc_kmajor_ld(kTcTF32, k), k3 = 3 * kp, ld3 = tc_row_pitch(kTcTF32, k3);
     float *Ak = (float *)buf;
     float *Bk = (float *)((char *)buf + round256((size_t)m * ld3 * sizeof(float)));
     const SegTerms sa{3, {1, 0, 0}}, sb{3, {0, 1, 0}};     // [lo | hi | hi], [hi | lo | hi]
     int st;
     if ((st = tc_convert_terms(false, ta_rows, m, k, A, ldA, Ak, ld3, kp, sa, nullptr, nullptr, s))) return st;
     if ((st = tc_convert_terms(false, tb_rows, n, k, B, ldB, Bk, ld3, kp, sb, nullptr, nullptr, s))) return st;
-    return tc_gemm_launch(kTcTF32, m, n, ld3, alpha, Ak, ld3, Bk, ld3, beta, C, ldC, nullptr, nullptr, s);
+    return tc_gemm_launch(kTcTF32, m, n, k3, alpha, Ak, ld3, Bk, ld3, beta, C, ldC, nullptr, nullptr, s);
 }
 
 // The same segmented product in e4m3: op(A) row i is scaled by 1/sa_i
@@ -464,14 +508,14 @@ int fp8_terms_gemm(int nterms, bool ta_rows, bool tb_rows, int m, int n, int k, 
     const SegTerms a3{6, {2, 0, 1, 1, 0, 0}}, b3{6, {0, 2, 1, 0, 1, 0}};
     const SegTerms &tA = nterms == 3 ? a3 : a2, &tB = nterms == 3 ? b3 : b2;
     const int nseg = tA.nseg;
-    const int kp = tc_kmajor_ld(kTcFP8, k), ldw = nseg * kp;
+    const int kp = tc_kmajor_ld(kTcFP8, k), kw = nseg * kp, ldw = tc_row_pitch(kTcFP8, kw);
     const size_t a = round256((size_t)m * ldw), b = round256((size_t)n * ldw);
     uint8_t *Ak = (uint8_t *)buf, *Bk = (uint8_t *)buf + a;
     float *sa = (float *)((char *)buf + a + b), *sia = sa + m, *sb = sia + m, *sib = sb + n;
     int st;
     if ((st = tc_convert_terms(true, ta_rows, m, k, A, ldA, Ak, ldw, kp, tA, sa, sia, s))) return st;
     if ((st = tc_convert_terms(true, tb_rows, n, k, B, ldB, Bk, ldw, kp, tB, sb, sib, s))) return st;
-    return tc_gemm_launch(kTcFP8, m, n, ldw, alpha, Ak, ldw, Bk, ldw, beta, C, ldC, sa, sb, s);
+    return tc_gemm_launch(kTcFP8, m, n, kw, alpha, Ak, ldw, Bk, ldw, beta, C, ldC, sa, sb, s);
 }
 
 }  // namespace
@@ -486,7 +530,7 @@ int tc_trailing_update(int kind, int m, int n, int k, const float *A21, int ldA2
                        const float *U12, int ldU12, float *A22, int ldA22, void *buf,
                        cudaStream_t stream) {
     if (m <= 0 || n <= 0 || k <= 0) return kOk;
-    const int ld = tc_kmajor_ld(kind, k);
+    const int ld = tc_row_pitch(kind, k);
     const size_t eb = tc_elem_bytes(kind);
     const size_t a = round256((size_t)m * ld * eb), b = round256((size_t)n * ld * eb);
     char *p = (char *)buf;
@@ -548,7 +592,7 @@ FG_API int flens_gb300_sgemm_tc(int precision, char transA, char transB, int m, 
     const size_t need = tc_update_workspace_bytes(precision, m, n, k);
     Workspace *w = workspace_for(s, need);
     if (!w) return kErrAlloc;
-    const int ld = tc_kmajor_ld(precision, k);
+    const int ld = tc_row_pitch(precision, k);
     const size_t eb = tc_elem_bytes(precision);
     const size_t a = round256((size_t)m * ld * eb), b = round256((size_t)n * ld * eb);
     char *p = (char *)w->buf;

@@ -211,8 +211,8 @@ __device__ __forceinline__ void tile_origin(int t, int tiles_m, int tiles_n, int
 //        the TMEM address of the policy's own kTmemExtra columns for this
 //        warp's lane quarter (tile-local column 0).
 //   void prefetch(int m0, int n0, int M, int N, int j) const
-//        called by epilogue thread j (0..255) when its warps start a tile,
-//        with the origin of the CTA's next tile: may bring column j of that
+//        called by epilogue thread j (0..255) before the first tile with its
+//        origin, and when its warps start a tile with the origin of the CTA's next: may bring column j of that
 //        tile's output into L2 (a no-op for policies that read none)
 //   static constexpr int kBN, kTmemExtra (see Shape)
 template <int KIND, class Epi>
@@ -344,6 +344,12 @@ tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
         const int half = ew >> 2;                // column half
         int i = 0;
         bool live = true;
+        if ((int)blockIdx.x < ntiles) {
+            // the first tile's output while its operands are loaded
+            int m1, n1;
+            tile_origin(blockIdx.x, tiles_m, tiles_n, BN, m1, n1);
+            epi.prefetch(m1, n1, M, N, ew * 32 + lane);
+        }
         for (int t = blockIdx.x; t < ntiles && live; t += gridDim.x) {
             int m0, n0;
             tile_origin(t, tiles_m, tiles_n, BN, m0, n0);
