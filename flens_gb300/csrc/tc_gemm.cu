@@ -190,13 +190,12 @@ to_kmajor_kernel(int R, int K, const float *__restrict__ in, int ld, void *__res
 // Per-row amax of op(X) (R rows, K columns) -> scale = amax/448 and 1/scale
 // (FP8 e4m3 per-row scaling; a zero row keeps scale 1).
 // Rows contiguous: 32 rows x 32 k-lanes per block (a warp per row would touch a
-// sector per entry); else a warp per row.
-constexpr int RS_THREADS = 1024;
+// sector per entry); else a warp per row, 8 rows per block.
 template <bool RCONTIG>
-__global__ void __launch_bounds__(RS_THREADS)
+__global__ void __launch_bounds__(RCONTIG ? 1024 : 256)
 row_scale_kernel(int R, int K, const float *__restrict__ in, int ld, float *__restrict__ scale,
                  float *__restrict__ inv_scale) {
-    __shared__ float sm[32][33];
+    __shared__ float sm[RCONTIG ? 32 : 1][33];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float m = 0.0f;
     if (RCONTIG) {
@@ -208,12 +207,12 @@ row_scale_kernel(int R, int K, const float *__restrict__ in, int ld, float *__re
         __syncthreads();
         m = sm[warp][lane];
     } else {
-        const int r = blockIdx.x * 32 + warp;
+        const int r = blockIdx.x * 8 + warp;
         if (r < R)
 #pragma unroll 8
             for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(in[(size_t)k + (size_t)r * ld]));
     }
-    const int r = blockIdx.x * 32 + warp;
+    const int r = blockIdx.x * (RCONTIG ? 32 : 8) + warp;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
     if (lane == 0 && r < R) {
@@ -370,9 +369,9 @@ int tc_convert(int kind, bool trans, int R, int K, const float *X, int ldx, void
     const bool rcontig = !trans;
     const bool fp8 = kind == kTcFP8 || kind == kTcFP8Lo || kind == kTcFP8Lo2;
     if (fp8 && scale != nullptr) {
-        const dim3 g(ceil_div(R, 32));
-        if (rcontig) row_scale_kernel<true><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        const dim3 g(ceil_div(R, rcontig ? 32 : 8));
+        if (rcontig) row_scale_kernel<true><<<g, 1024, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
         FG_CUDA(cudaGetLastError());
     }
     const dim3 grid(ceil_div(R, CONV_R), ceil_div(width, CONV_K));
@@ -403,9 +402,9 @@ int tc_convert_terms(bool fp8, bool trans, int R, int K, const float *X, int ldx
     KTimer kt(kFamAux, stream, 0.0, (4.0 + (fp8 ? 1.0 : 4.0) * st.nseg) * R * (double)K);
     const bool rcontig = !trans;
     if (fp8) {
-        const dim3 g(ceil_div(R, 32));
-        if (rcontig) row_scale_kernel<true><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, RS_THREADS, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        const dim3 g(ceil_div(R, rcontig ? 32 : 8));
+        if (rcontig) row_scale_kernel<true><<<g, 1024, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
     }
     const dim3 grid(ceil_div(R, CONV_R), ceil_div(kp, CONV_K));
     const float *inv = fp8 ? inv_scale : nullptr;
