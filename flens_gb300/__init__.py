@@ -396,18 +396,34 @@ def dposv(uplo: str, A: np.ndarray, B: np.ndarray) -> int:
 # -------------------------------------------------------- device (torch) ---
 def _colmajor(t):
     """(pointer, rows, cols, ld) of a column-major CUDA float64 tensor."""
-    if t.dim() == 2 and t.numel() == 0:
-        return t.data_ptr(), t.shape[0], t.shape[1], max(1, t.shape[0])
-    if t.dim() != 2 or (t.stride(0) != 1 and t.shape[0] != 1):   # a 1-row stride is free
-        raise ValueError("expected a 2-D column-major tensor (stride(0) == 1)")
-    return t.data_ptr(), t.shape[0], t.shape[1], max(1, t.stride(1), t.shape[0])
+    if t.dim() == 2:
+        r, c = t.shape
+        if r == 0 or c == 0:
+            return t.data_ptr(), r, c, max(1, r)
+        s0, s1 = t.stride()
+        if s0 == 1 or r == 1:                                    # a 1-row stride is free
+            return t.data_ptr(), r, c, max(s1, r)
+    raise ValueError("expected a 2-D column-major tensor (stride(0) == 1)")
+
+
+_raw_stream = None      # (device index -> stream handle, current device index), from torch
 
 
 def _stream(stream):
-    if stream is None:
+    # A stream object per call cost 3 to 6 us of a 64 x 48 x 80 product's 15; the
+    # handle alone is asked for where torch offers it.
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    global _raw_stream
+    if _raw_stream is None:
         import torch
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
+        torch.cuda.init()
+        raw, dev = (getattr(torch._C, f, None) for f in ("_cuda_getCurrentRawStream", "_cuda_getDevice"))
+        if raw is None or dev is None:
+            raw, dev = (lambda d: torch.cuda.current_stream(d).cuda_stream), torch.cuda.current_device
+        _raw_stream = (raw, dev)
+    raw, dev = _raw_stream
+    return ctypes.c_void_p(raw(dev()))
 
 
 def _check(code: int, where: str) -> None:
@@ -429,7 +445,7 @@ def dgemm_dev(transA, transB, alpha, A, B, beta, C, stream=None):
     pa, ra, ca, lda = _colmajor(A)
     pb, rb, cb, ldb = _colmajor(B)
     pc, m, n, ldc = _colmajor(C)
-    k = ca if transA.upper() == "N" else ra
+    k = ca if transA in ("N", "n") else ra
     _check(lib().flens_gb300_dgemm(transA.encode(), transB.encode(), m, n, k, alpha, pa, lda,
                                    pb, ldb, beta, pc, ldc, _stream(stream)), "flens_gb300_dgemm")
     return C
