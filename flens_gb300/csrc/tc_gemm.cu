@@ -93,14 +93,6 @@ __device__ __forceinline__ uint32_t to_lp<kTcTF32>(float v) {
     return t;
 }
 template <>
-__device__ __forceinline__ uint32_t to_lp<kTcTF32Lo>(float v) {
-    uint32_t h, t;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(h) : "f"(v));
-    const float lo = v - __uint_as_float(h);
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(t) : "f"(lo));
-    return t;
-}
-template <>
 __device__ __forceinline__ uint32_t to_lp<kTcFP8>(float v) {
     return __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
@@ -111,41 +103,40 @@ __device__ __forceinline__ float fp8_round(float v, __nv_fp8_storage_t *q) {
     *q = __nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
     return __half2float(__half(__nv_cvt_fp8_to_halfraw(*q, __NV_E4M3)));
 }
-template <>
-__device__ __forceinline__ uint32_t to_lp<kTcFP8Lo>(float v) {
-    __nv_fp8_storage_t q;
-    const float t0 = fp8_round(v, &q);
-    fp8_round(v - t0, &q);
-    return q;
-}
-template <>
-__device__ __forceinline__ uint32_t to_lp<kTcFP8Lo2>(float v) {
-    __nv_fp8_storage_t q;
-    const float t0 = fp8_round(v, &q);
-    const float t1 = fp8_round(v - t0, &q);
-    fp8_round(v - t0 - t1, &q);
-    return q;
-}
 
 // A block takes 32 rows x 64 k through shared memory: 8 loads in flight per
 // thread along whichever index is contiguous, then a thread stores 4 consecutive
 // k at once (16 lanes: 64 to 256 bytes of a row).  Bound: HBM.  4100 x 3000 to
 // BF16: 29 us with one 4-byte load and one 2-byte store at a time.
+// Both operands of a product share a launch (blocks below blocks_a: the first).
 constexpr int CONV_R = 32, CONV_K = 64;
-template <bool RCONTIG>
-__device__ __forceinline__ void conv_load(float (*tile)[CONV_K + 2], int r0, int k0, int R, int K,
-                                          const float *__restrict__ in, int ld) {
+struct ConvOp {
+    const float *X;
+    int ld, R;
+    int rcontig;                             // element (r, k) at X[r + k ld], else X[k + r ld]
+    void *out;
+    float *scale, *inv;                      // e4m3: per-row scale and its reciprocal
+};
+__device__ __forceinline__ void conv_load(float (*tile)[CONV_K + 2], const ConvOp &o, int r0, int k0, int K) {
     const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
     float v[8];
+    if (o.rcontig) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = RCONTIG ? r0 + lane : r0 + wy + 8 * (i >> 1);
-        const int k = RCONTIG ? k0 + wy + 8 * i : k0 + lane + 32 * (i & 1);
-        v[i] = (r < R && k < K) ? in[RCONTIG ? (size_t)r + (size_t)k * ld : (size_t)k + (size_t)r * ld] : 0.0f;
+        for (int i = 0; i < 8; ++i) {
+            const int r = r0 + lane, k = k0 + wy + 8 * i;
+            v[i] = (r < o.R && k < K) ? o.X[(size_t)r + (size_t)k * o.ld] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tile[lane][wy + 8 * i] = v[i];
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = r0 + wy + 8 * (i >> 1), k = k0 + lane + 32 * (i & 1);
+            v[i] = (r < o.R && k < K) ? o.X[(size_t)k + (size_t)r * o.ld] : 0.0f;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) tile[wy + 8 * (i >> 1)][lane + 32 * (i & 1)] = v[i];
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-        tile[RCONTIG ? lane : wy + 8 * (i >> 1)][RCONTIG ? wy + 8 * i : lane + 32 * (i & 1)] = v[i];
     __syncthreads();
 }
 
@@ -166,14 +157,19 @@ __device__ __forceinline__ void store4(void *out, size_t idx, const uint32_t (&w
     }
 }
 
-template <int KIND, bool RCONTIG>
+template <int KIND>
 __global__ void __launch_bounds__(256)
-to_kmajor_kernel(int R, int K, const float *__restrict__ in, int ld, void *__restrict__ out,
-                 int ldo, int width, const float *__restrict__ inv_scale) {
+to_kmajor_kernel(const __grid_constant__ ConvOp oa, const __grid_constant__ ConvOp ob, int blocks_a, int K,
+                 int ldo, int width) {
     __shared__ float tile[CONV_R][CONV_K + 2];
-    const int r0 = blockIdx.x * CONV_R, k0 = blockIdx.y * CONV_K;
-    conv_load<RCONTIG>(tile, r0, k0, R, K, in, ld);
-    constexpr int BYTES = KIND == kTcBF16 ? 2 : (KIND == kTcTF32 || KIND == kTcTF32Lo) ? 4 : 1;
+    const bool second = (int)blockIdx.x >= blocks_a;
+    const ConvOp &o = second ? ob : oa;
+    const int bx = second ? blockIdx.x - blocks_a : blockIdx.x, nr = (o.R + CONV_R - 1) / CONV_R;
+    const int r0 = (bx % nr) * CONV_R, k0 = (bx / nr) * CONV_K, R = o.R;
+    const float *inv_scale = o.inv;
+    void *out = o.out;
+    conv_load(tile, o, r0, k0, K);
+    constexpr int BYTES = KIND == kTcBF16 ? 2 : KIND == kTcTF32 ? 4 : 1;
     const int kq = (threadIdx.x & 15) * 4, k = k0 + kq;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -190,35 +186,34 @@ to_kmajor_kernel(int R, int K, const float *__restrict__ in, int ld, void *__res
 // Per-row amax of op(X) (R rows, K columns) -> scale = amax/448 and 1/scale
 // (FP8 e4m3 per-row scaling; a zero row keeps scale 1).
 // Rows contiguous: 32 rows x 32 k-lanes per block (a warp per row would touch a
-// sector per entry); else a warp per row, 8 rows per block.
-template <bool RCONTIG>
-__global__ void __launch_bounds__(RCONTIG ? 1024 : 256)
-row_scale_kernel(int R, int K, const float *__restrict__ in, int ld, float *__restrict__ scale,
-                 float *__restrict__ inv_scale) {
-    __shared__ float sm[RCONTIG ? 32 : 1][33];
+// sector per entry); else a warp per row, 32 rows per block.
+constexpr int RS_THREADS = 1024;
+__global__ void __launch_bounds__(RS_THREADS)
+row_scale_kernel(const __grid_constant__ ConvOp oa, const __grid_constant__ ConvOp ob, int blocks_a, int K) {
+    __shared__ float sm[32][33];
+    const bool second = (int)blockIdx.x >= blocks_a;
+    const ConvOp &o = second ? ob : oa;
+    const int r0 = (second ? blockIdx.x - blocks_a : blockIdx.x) * 32;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = r0 + warp;
     float m = 0.0f;
-    if (RCONTIG) {
-        const int r = blockIdx.x * 32 + lane;
-        if (r < R)
+    if (o.rcontig) {
+        if (r0 + lane < o.R)
 #pragma unroll 8
-            for (int k = warp; k < K; k += 32) m = fmaxf(m, fabsf(in[(size_t)r + (size_t)k * ld]));
+            for (int k = warp; k < K; k += 32) m = fmaxf(m, fabsf(o.X[(size_t)(r0 + lane) + (size_t)k * o.ld]));
         sm[lane][warp] = m;
         __syncthreads();
         m = sm[warp][lane];
-    } else {
-        const int r = blockIdx.x * 8 + warp;
-        if (r < R)
+    } else if (r < o.R) {
 #pragma unroll 8
-            for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(in[(size_t)k + (size_t)r * ld]));
+        for (int k = lane; k < K; k += 32) m = fmaxf(m, fabsf(o.X[(size_t)k + (size_t)r * o.ld]));
     }
-    const int r = blockIdx.x * (RCONTIG ? 32 : 8) + warp;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-    if (lane == 0 && r < R) {
+    if (lane == 0 && r < o.R) {
         const float s = (m > 0.0f && isfinite(m)) ? m / 448.0f : 1.0f;
-        scale[r] = s;
-        inv_scale[r] = 1.0f / s;
+        o.scale[r] = s;
+        o.inv[r] = 1.0f / s;
     }
 }
 
@@ -232,13 +227,19 @@ struct SegTerms {
     int term[6];
 };
 
-template <bool FP8, bool RCONTIG>
+template <bool FP8>
 __global__ void __launch_bounds__(256)
-to_kmajor_terms_kernel(int R, int K, const float *__restrict__ in, int ld, void *__restrict__ out,
-                       int ldo, int kp, SegTerms st, const float *__restrict__ inv_scale) {
+to_kmajor_terms_kernel(const __grid_constant__ ConvOp oa, const __grid_constant__ ConvOp ob, int blocks_a, int K,
+                       int ldo, int kp, SegTerms sa, SegTerms sb) {
     __shared__ float tile[CONV_R][CONV_K + 2];
-    const int r0 = blockIdx.x * CONV_R, k0 = blockIdx.y * CONV_K;
-    conv_load<RCONTIG>(tile, r0, k0, R, K, in, ld);
+    const bool second = (int)blockIdx.x >= blocks_a;
+    const ConvOp &o = second ? ob : oa;
+    const SegTerms &st = second ? sb : sa;
+    const int bx = second ? blockIdx.x - blocks_a : blockIdx.x, nr = (o.R + CONV_R - 1) / CONV_R;
+    const int r0 = (bx % nr) * CONV_R, k0 = (bx / nr) * CONV_K, R = o.R;
+    const float *inv_scale = o.inv;
+    void *out = o.out;
+    conv_load(tile, o, r0, k0, K);
     const int kq = (threadIdx.x & 15) * 4, k = k0 + kq;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
@@ -330,8 +331,8 @@ int make_kmajor_map(CUtensorMap *map, int kind, const void *base, int rows, int 
 
 // K-major leading dimension (elements) for `kind`: K rounded up to 16 bytes.
 static int gemm_kind(int kind) {
-    if (kind == kTcF32x3 || kind == kTcTF32Lo) return kTcTF32;
-    if (kind == kTcFP8x2 || kind == kTcFP8x3 || kind == kTcFP8Lo || kind == kTcFP8Lo2) return kTcFP8;
+    if (kind == kTcF32x3) return kTcTF32;
+    if (kind == kTcFP8x2 || kind == kTcFP8x3) return kTcFP8;
     return kind;
 }
 
@@ -356,65 +357,38 @@ size_t tc_elem_bytes(int kind) {
     return kind == kTcTF32 ? 4 : kind == kTcBF16 ? 2 : 1;
 }
 
-// Convert op(X) (R x K, FP32, column-major storage, transposed or not) to a
-// K-major low-precision operand: columns 0..width-1 of rows of stride ldo
-// (zero beyond K).  For FP8, scales each row by inv_scale; when `scale` is
-// given, first computes the per-row scales (else inv_scale holds them already).
-int tc_convert(int kind, bool trans, int R, int K, const float *X, int ldx, void *out, int ldo,
-               float *scale, float *inv_scale, cudaStream_t stream, int width = -1) {
-    if (width < 0) width = ldo;
-    if (R <= 0 || K <= 0) return kOk;
-    KTimer kt(kFamAux, stream, 0.0, (4.0 + tc_elem_bytes(kind)) * R * (double)K);
-    // op(X)(r, k): r-contiguous when X is stored R x K (no transpose)
-    const bool rcontig = !trans;
-    const bool fp8 = kind == kTcFP8 || kind == kTcFP8Lo || kind == kTcFP8Lo2;
-    if (fp8 && scale != nullptr) {
-        const dim3 g(ceil_div(R, rcontig ? 32 : 8));
-        if (rcontig) row_scale_kernel<true><<<g, 1024, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+// Convert op(A) and op(B)^T (a.R x K and b.R x K, FP32) to K-major
+// low-precision operands with rows of stride ldo; FP8 rows are scaled by
+// 448 / amax first (scale and inv receive the scales).
+int tc_convert(int kind, const ConvOp &a, const ConvOp &b, int K, int ldo, cudaStream_t stream) {
+    if (a.R <= 0 || b.R <= 0 || K <= 0) return kOk;
+    KTimer kt(kFamAux, stream, 0.0, (4.0 + tc_elem_bytes(kind)) * ((double)a.R + b.R) * (double)K);
+    if (kind == kTcFP8) {
+        row_scale_kernel<<<ceil_div(a.R, 32) + ceil_div(b.R, 32), RS_THREADS, 0, stream>>>(a, b, ceil_div(a.R, 32), K);
         FG_CUDA(cudaGetLastError());
     }
-    const dim3 grid(ceil_div(R, CONV_R), ceil_div(width, CONV_K));
-    const float *inv = fp8 ? inv_scale : nullptr;
-#define FG_CONV(KD)                                                                          \
-    do {                                                                                     \
-        if (rcontig) to_kmajor_kernel<KD, true><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, width, inv); \
-        else to_kmajor_kernel<KD, false><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, width, inv);        \
-    } while (0)
-    if (kind == kTcTF32) FG_CONV(kTcTF32);
-    else if (kind == kTcTF32Lo) FG_CONV(kTcTF32Lo);
-    else if (kind == kTcBF16) FG_CONV(kTcBF16);
-    else if (kind == kTcFP8Lo) FG_CONV(kTcFP8Lo);
-    else if (kind == kTcFP8Lo2) FG_CONV(kTcFP8Lo2);
-    else FG_CONV(kTcFP8);
-#undef FG_CONV
+    const int nk = ceil_div(ldo, CONV_K), ba = ceil_div(a.R, CONV_R) * nk, bb = ceil_div(b.R, CONV_R) * nk;
+    if (kind == kTcTF32) to_kmajor_kernel<kTcTF32><<<ba + bb, 256, 0, stream>>>(a, b, ba, K, ldo, ldo);
+    else if (kind == kTcBF16) to_kmajor_kernel<kTcBF16><<<ba + bb, 256, 0, stream>>>(a, b, ba, K, ldo, ldo);
+    else to_kmajor_kernel<kTcFP8><<<ba + bb, 256, 0, stream>>>(a, b, ba, K, ldo, ldo);
     FG_CUDA(cudaGetLastError());
     return kOk;
 }
 
-// The split operand of op(X) (R x K) in one pass: segments st.term[q] at
-// columns q*kp of the K-major rows (see to_kmajor_terms_kernel); for e4m3
-// the per-row scales first (scale, inv_scale).
-int tc_convert_terms(bool fp8, bool trans, int R, int K, const float *X, int ldx, void *out,
-                     int ldo, int kp, const SegTerms &st, float *scale, float *inv_scale,
-                     cudaStream_t stream) {
-    if (R <= 0 || K <= 0) return kOk;
-    KTimer kt(kFamAux, stream, 0.0, (4.0 + (fp8 ? 1.0 : 4.0) * st.nseg) * R * (double)K);
-    const bool rcontig = !trans;
+// The split operands in one pass: segments st.term[q] of each operand at
+// columns q*kp of its K-major rows (see to_kmajor_terms_kernel); for e4m3
+// the per-row scales first.
+int tc_convert_terms(bool fp8, const ConvOp &a, const ConvOp &b, const SegTerms &sa, const SegTerms &sb, int K,
+                     int ldo, int kp, cudaStream_t stream) {
+    if (a.R <= 0 || b.R <= 0 || K <= 0) return kOk;
+    KTimer kt(kFamAux, stream, 0.0, (4.0 + (fp8 ? 1.0 : 4.0) * sa.nseg) * ((double)a.R + b.R) * (double)K);
     if (fp8) {
-        const dim3 g(ceil_div(R, rcontig ? 32 : 8));
-        if (rcontig) row_scale_kernel<true><<<g, 1024, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
-        else row_scale_kernel<false><<<g, 256, 0, stream>>>(R, K, X, ldx, scale, inv_scale);
+        row_scale_kernel<<<ceil_div(a.R, 32) + ceil_div(b.R, 32), RS_THREADS, 0, stream>>>(a, b, ceil_div(a.R, 32), K);
+        FG_CUDA(cudaGetLastError());
     }
-    const dim3 grid(ceil_div(R, CONV_R), ceil_div(kp, CONV_K));
-    const float *inv = fp8 ? inv_scale : nullptr;
-    if (fp8) {
-        if (rcontig) to_kmajor_terms_kernel<true, true><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, kp, st, inv);
-        else to_kmajor_terms_kernel<true, false><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, kp, st, inv);
-    } else {
-        if (rcontig) to_kmajor_terms_kernel<false, true><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, kp, st, inv);
-        else to_kmajor_terms_kernel<false, false><<<grid, 256, 0, stream>>>(R, K, X, ldx, out, ldo, kp, st, inv);
-    }
+    const int nk = ceil_div(kp, CONV_K), ba = ceil_div(a.R, CONV_R) * nk, bb = ceil_div(b.R, CONV_R) * nk;
+    if (fp8) to_kmajor_terms_kernel<true><<<ba + bb, 256, 0, stream>>>(a, b, ba, K, ldo, kp, sa, sb);
+    else to_kmajor_terms_kernel<false><<<ba + bb, 256, 0, stream>>>(a, b, ba, K, ldo, kp, sa, sb);
     FG_CUDA(cudaGetLastError());
     return kOk;
 }
@@ -487,8 +461,8 @@ int f32x3_gemm(bool ta_rows, bool tb_rows, int m, int n, int k, float alpha, con
     float *Bk = (float *)((char *)buf + round256((size_t)m * ld3 * sizeof(float)));
     const SegTerms sa{3, {1, 0, 0}}, sb{3, {0, 1, 0}};     // [lo | hi | hi], [hi | lo | hi]
     int st;
-    if ((st = tc_convert_terms(false, ta_rows, m, k, A, ldA, Ak, ld3, kp, sa, nullptr, nullptr, s))) return st;
-    if ((st = tc_convert_terms(false, tb_rows, n, k, B, ldB, Bk, ld3, kp, sb, nullptr, nullptr, s))) return st;
+    const ConvOp oa{A, ldA, m, !ta_rows, Ak, nullptr, nullptr}, ob{B, ldB, n, !tb_rows, Bk, nullptr, nullptr};
+    if ((st = tc_convert_terms(false, oa, ob, sa, sb, k, ld3, kp, s))) return st;
     return tc_gemm_launch(kTcTF32, m, n, k3, alpha, Ak, ld3, Bk, ld3, beta, C, ldC, nullptr, nullptr, s);
 }
 
@@ -512,8 +486,8 @@ int fp8_terms_gemm(int nterms, bool ta_rows, bool tb_rows, int m, int n, int k, 
     uint8_t *Ak = (uint8_t *)buf, *Bk = (uint8_t *)buf + a;
     float *sa = (float *)((char *)buf + a + b), *sia = sa + m, *sb = sia + m, *sib = sb + n;
     int st;
-    if ((st = tc_convert_terms(true, ta_rows, m, k, A, ldA, Ak, ldw, kp, tA, sa, sia, s))) return st;
-    if ((st = tc_convert_terms(true, tb_rows, n, k, B, ldB, Bk, ldw, kp, tB, sb, sib, s))) return st;
+    const ConvOp oa{A, ldA, m, !ta_rows, Ak, sa, sia}, ob{B, ldB, n, !tb_rows, Bk, sb, sib};
+    if ((st = tc_convert_terms(true, oa, ob, tA, tB, k, ldw, kp, s))) return st;
     return tc_gemm_launch(kTcFP8, m, n, kw, alpha, Ak, ldw, Bk, ldw, beta, C, ldC, sa, sb, s);
 }
 
@@ -547,8 +521,8 @@ int tc_trailing_update(int kind, int m, int n, int k, const float *A21, int ldA2
         sb = sia + m;
         sib = sb + n;
     }
-    if ((st = tc_convert(kind, false, m, k, A21, ldA21, Ahi, ld, sa, sia, stream))) return st;
-    if ((st = tc_convert(kind, true, n, k, U12, ldU12, Bhi, ld, sb, sib, stream))) return st;
+    const ConvOp oa{A21, ldA21, m, 1, Ahi, sa, sia}, ob{U12, ldU12, n, 0, Bhi, sb, sib};
+    if ((st = tc_convert(kind, oa, ob, k, ld, stream))) return st;
     return tc_gemm_launch(kind, m, n, k, -1.0f, Ahi, ld, Bhi, ld, 1.0f, A22, ldA22, sa, sb, stream);
 }
 
@@ -609,8 +583,8 @@ FG_API int flens_gb300_sgemm_tc(int precision, char transA, char transB, int m, 
         sb = sia + m;
         sib = sb + n;
     }
-    if ((st = tc_convert(precision, ta, m, k, A, ldA, Alp, ld, sa, sia, s))) return st;
     // B^T(j, p) = op(B)(p, j): for op(B) = B (K x N col-major) row j of B^T is contiguous in p
-    if ((st = tc_convert(precision, !tb, n, k, B, ldB, Blp, ld, sb, sib, s))) return st;
+    const ConvOp oa{A, ldA, m, !ta, Alp, sa, sia}, ob{B, ldB, n, tb, Blp, sb, sib};
+    if ((st = tc_convert(precision, oa, ob, k, ld, s))) return st;
     return tc_gemm_launch(precision, m, n, k, alpha, Alp, ld, Blp, ld, beta, C, ldC, sa, sb, s);
 }

@@ -37,17 +37,13 @@ namespace fg {
 // t1 = e4m3(v - t0) (and t2 = e4m3(v - t0 - t1)), and the products t_i t_j
 // with i + j <= 1 (3 of them) or <= 2 (6 of them) are accumulated: about
 // 2^-8 or 2^-12 relative per operand entry instead of e4m3's 2^-4.
-// kTcTF32Lo, kTcFP8Lo (t1) and kTcFP8Lo2 (t2) are only conversion modes.
 enum TcKind : int {
     kTcTF32 = 0,
     kTcBF16 = 1,
     kTcFP8 = 2,
     kTcF32x3 = 3,
-    kTcTF32Lo = 4,
     kTcFP8x2 = 5,
-    kTcFP8x3 = 6,
-    kTcFP8Lo = 7,
-    kTcFP8Lo2 = 8
+    kTcFP8x3 = 6
 };
 
 namespace tc {
