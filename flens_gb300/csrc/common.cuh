@@ -102,6 +102,16 @@ constexpr size_t kScratchKeep = (size_t)2 << 30;
 void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status);
 void scratch_release(void *p, cudaStream_t stream);
 
+// SMs that the persistent tensor-core kernels launched by this thread leave free
+// while a SpareSms lives: for a kernel that runs beside them on another stream.
+int spare_sms();
+struct SpareSms {
+    explicit SpareSms(int n);
+    ~SpareSms();
+    SpareSms(const SpareSms &) = delete;
+    int before;
+};
+
 int num_sms();                 // SM count of the current device
 int device_id();               // current device ordinal
 

@@ -870,6 +870,11 @@ __device__ __forceinline__ int move_store(const int (&mv_row)[4], const int (&mv
 constexpr int CP_CS = 16;                       // CTAs of the cluster
 constexpr int CP_T = 512;                       // threads per CTA
 constexpr int CP_NW = CP_T / 32;
+// Rows per thread at most.  (A second one in FP64, for panels of 8192 to 12,700
+// rows, made every column 7% slower at n = 500.)
+template <typename T>
+constexpr int CP_RPT = sizeof(T) == 8 ? 1 : 2;
+constexpr int CP_NARROW = 32;                   // columns held for a panel of at most as many
 // Columns of a sub-panel.  FP64 has none: its bound is the FP64 pipe, not shared
 // memory, and the U rows, 15 dependent FP64 FMAs, made a column 12% slower.
 template <typename T>
@@ -888,11 +893,13 @@ constexpr uint32_t cluster_bytes() {            // received per column
     return CP_CS * (PANEL_NB * sizeof(T) + 16 + (sizeof(T) == 8 ? 8 : 0)) + PANEL_NB * sizeof(T);
 }
 
-// Shared memory of a CTA: the buffers are static, R rows x 64 columns dynamic.
+// Rows a cluster holds beside its static buffers, `cols` (64 or 32) columns wide (at
+// most CP_RPT per thread).
 template <typename T>
-constexpr size_t cluster_rows_max() {
-    return ((227 * 1024 - 2048 - 3 * sizeof(ClusterBuf<T>) - (CP_SB<T> % PANEL_NB) * PANEL_NB * sizeof(T)) / (PANEL_NB * sizeof(T))) *
-           CP_CS;
+constexpr size_t cluster_rows_max(int cols) {
+    const size_t bytes = 227 * 1024 - 2048 - 3 * sizeof(ClusterBuf<T>) - (CP_SB<T> % PANEL_NB) * PANEL_NB * sizeof(T);
+    const size_t rows = bytes / (cols * sizeof(T));
+    return (rows < CP_RPT<T> * CP_T ? rows : CP_RPT<T> * CP_T) * CP_CS;
 }
 
 __device__ __forceinline__ uint32_t cp_smem(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -976,7 +983,8 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
     }
-    // columns beyond jb are sent as they are in the exchange: keep them defined
+    // columns jb .. ncol - 1 take part in the updates: keep them defined
+    const int ncol = jb <= CP_NARROW ? CP_NARROW : PANEL_NB;
     {
         const int nrb = (nr + 31) / 32;
         for (int u = warp; u < nrb * 4; u += CP_NW) {
@@ -985,7 +993,7 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
 #pragma unroll
                 for (int h = 0; h < 16; ++h) {
                     const int c = c0 + 4 * h;
-                    S[c * R + r] = c < jb ? A[(size_t)(rb + r) + (size_t)c * lda] : T(0);
+                    if (c < ncol) S[c * R + r] = c < jb ? A[(size_t)(rb + r) + (size_t)c * lda] : T(0);
                 }
         }
     }
@@ -1088,7 +1096,7 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
             if (warp < 2) {
                 const int x = (warp == 0 ? i : jj) - rb;
                 T v0 = T(0), v1 = T(0);
-                if (has) {
+                if (has && 2 * lane < ncol) {
                     v0 = fin(x, 2 * lane);
                     v1 = fin(x, 2 * lane + 1);
                 }
@@ -1120,7 +1128,7 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
         if (d_end) {
             const int nrb = (nr + 31) / 32;
             const int ncg = nrb >= CP_NW ? 1 : CP_NW / max(nrb, 1);
-            const int q0 = (d_jj + 2) >> 2, q1 = d_end >> 2;
+            const int q0 = (d_jj + 2) >> 2, q1 = min(d_end, ncol) >> 2;
             for (int u = warp; u < nrb * ncg; u += CP_NW) {
                 const int cg = u / nrb, r = (u - cg * nrb) * 32 + lane, g = rb + r;
                 if (r < nr && g > d_jj) {
@@ -1153,10 +1161,9 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
         }
         if (warp == CP_NW - 2) write_swap();
         // -- this thread's entries of columns jj and jj + 1 (its own writes)
-        constexpr int RPT = sizeof(T) == 8 ? 1 : 2;              // rows per thread at most
-        T c0[RPT], c1[RPT];
+        T c0[CP_RPT<T>], c1[CP_RPT<T>];
 #pragma unroll
-        for (int h = 0; h < RPT; ++h) {
+        for (int h = 0; h < CP_RPT<T>; ++h) {
             const int r = tid + h * CP_T;
             c0[h] = r < nr ? S[jj * R + r] : T(0);
             c1[h] = r < nr && jj + 1 < jb ? S[(jj + 1) * R + r] : T(0);
@@ -1183,7 +1190,7 @@ panel_cluster_kernel(T *__restrict__ A, int lda, int mp, int jb, int j0, int *__
         nbk = kKeyNone;
         nbi = INT_MAX;
 #pragma unroll
-        for (int h = 0; h < RPT; ++h) {
+        for (int h = 0; h < CP_RPT<T>; ++h) {
             const int r = tid + h * CP_T, g = rb + r;
             if (r >= nr || g <= jj) continue;
             const bool sw = swap && g == gs;
@@ -1462,19 +1469,23 @@ bool lookahead_enabled() {
     return on;
 }
 
-// Rows up to which a panel takes the cluster kernel: FLENS_GB300_PANEL_CLUSTER
-// (0: never), else as many as fit one cluster's shared memory in FP32 (13,600; per
-// column 1.7 us at 4096 rows, 3.0 at 13,000, the grid panel 3.5), and 6000 in
-// FP64, where the 16 SMs' FP64 pipes come level with the grid panel's 4.1 us.
+// Width of the cluster panel at mp rows, 0: the grid panel.  64 as far as a
+// cluster holds 64 columns (FP32: 13,300 rows; per column 1.7 us at 4096 rows, 3.0
+// at 13,000, the grid panel 3.5), in FP64 up to 6000 rows, where its 16 SMs' FP64
+// pipes come level with the grid panel's 4.1 us.  Beyond, 32 columns up to twice
+// the rows where the panel runs beside an update (`beside`): the grid panel needs
+// all SMs.  (Alone, 32-wide panels were no faster: half the pipe time per column,
+// twice the launches.)  FLENS_GB300_PANEL_CLUSTER bounds the rows (0: never).
 template <typename T>
-int cluster_rows() {
-    static int rows = [] {
+int cluster_width(int mp, bool beside) {
+    static int cap = [] {
         const char *e = getenv("FLENS_GB300_PANEL_CLUSTER");
-        const int cap = (int)cluster_rows_max<T>(), want = sizeof(T) == 8 ? 6000 : cap;
-        const int v = e && *e ? atoi(e) : want;
-        return v < cap ? v : cap;
+        return e && *e ? atoi(e) : INT_MAX;
     }();
-    return rows;
+    const int wide = sizeof(T) == 8 ? 6000 : (int)cluster_rows_max<T>(PANEL_NB);
+    if (mp > cap) return 0;
+    if (mp <= wide) return PANEL_NB;
+    return beside && mp <= (int)cluster_rows_max<T>(CP_NARROW) ? CP_NARROW : 0;
 }
 
 cudaLaunchConfig_t cluster_config(cudaLaunchAttribute *attr, size_t smem, cudaStream_t s) {
@@ -1500,7 +1511,8 @@ bool cluster_fits() {
     if (d < 0 || d >= 64) return false;
     int v = __atomic_load_n(&known[d], __ATOMIC_ACQUIRE);
     if (v == 0) {
-        const size_t smem = cluster_rows_max<T>() / CP_CS * PANEL_NB * sizeof(T);
+        const size_t smem = std::max(cluster_rows_max<T>(PANEL_NB) / CP_CS * PANEL_NB,
+                                     cluster_rows_max<T>(CP_NARROW) / CP_CS * CP_NARROW) * sizeof(T);
         const void *fn = (const void *)panel_cluster_kernel<T>;
         cudaLaunchAttribute attr;
         cudaLaunchConfig_t cfg = cluster_config(&attr, smem, nullptr);
@@ -1530,12 +1542,28 @@ int panel_ctas(int sms) {
     return cap;
 }
 
-// Whether the FP64 LU takes the recursive order: its products then go to the
-// tensor cores.  From 2048 columns on: n = 1000, 2000, 4096, 8192 measured
-// 5.4, 11.8, 28, 71 ms against 4.9, 11.9, 49, 320 ms in the right-looking order
-// with look-ahead (the factorisation alone).  Not for a stream under capture, whose products run on the FP64
-// pipe: there the right-looking order with look-ahead is faster (n = 8192: 320
-// against 355 ms).
+// SMs left to the side stream's cluster panel.
+constexpr int kClusterSms = CP_CS;
+
+// Outer block of the FP64 order with look-ahead (FLENS_GB300_LOOKAHEAD_NB, a
+// multiple of 64).  A narrow block gets the next panel started sooner, a wide one
+// makes the updates deeper.  Factorisations of n = 2000, 4096, 5000, 8192 in ms: 64
+// columns 5.9, 16.9, 25.4, -; 128 columns 6.6, 17.2, 23.5, 55.5; 256 columns
+// -, 18.2, 24.3, 50.2; halved without look-ahead 7.7 (2048), 20.6, 28.5, 60.0.
+int lookahead_nb(int mn) {
+    static int nb = [] {
+        const char *e = getenv("FLENS_GB300_LOOKAHEAD_NB");
+        const int v = e ? atoi(e) : 0;
+        return (v >= 64 && v <= 1024 && v % 64 == 0) ? v : 0;
+    }();
+    return nb > 0 ? nb : mn < 4500 ? 64 : mn < 6500 ? 128 : 256;
+}
+
+// Whether the FP64 LU takes outer blocks with look-ahead, or halves the columns
+// (matrices too tall for cluster panels): its products then go to the tensor
+// cores.  From 1024 columns on (n = 1000: 2.59 ms both ways).  Not for a stream
+// under capture, whose products run on the FP64 pipe: there the right-looking
+// order of 64-column steps is faster (n = 8192: 320 against 355 ms).
 bool recursive_lu(int m, int n, cudaStream_t stream) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
@@ -1543,8 +1571,19 @@ bool recursive_lu(int m, int n, cudaStream_t stream) {
         return false;
     }
     const int h = (m < n ? m : n) / 2;
-    if (h < 1024) return false;
+    if (h < 512) return false;
     return cap == cudaStreamCaptureStatusNone && mod_gemm_wins(m - h, n - h, h, 0);
+}
+
+// Whether the FP32 LU with tensor-core updates takes its outer blocks with
+// look-ahead.
+bool sgetrf_lookahead(int m, int n, cudaStream_t stream) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return cap == cudaStreamCaptureStatusNone && (m < n ? m : n) >= 2048;
 }
 
 // Outer block of the split-update LU: FLENS_GB300_SPLIT_NB (a multiple of 64),
@@ -1667,14 +1706,27 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
     // update now so that slot 0 never moves under the panel scratch
     const size_t split_off = (ws0 + 255) / 256 * 256;
     const bool fp64_split = split_nb > 0 && tc_kind < 0;
-    Workspace *w = workspace_for(stream, fp64_split ? split_off + split_ws0_bytes(m, n) : ws0);
+    // look-ahead over outer blocks: its lists of row moves and the side stream's
+    // operands, after ours too.  The blocks of the tensor-core LU are split_nb wide:
+    // tc_buf is sized for updates of that depth.  (onb bounded: the lists have room
+    // for 32 panels of a block, 32 wide at least; m, because beyond 8192 rows, FP32
+    // 16,384, panels need the whole grid and nothing runs beside them.)
+    int onb = !recursive ? 0 : tc_kind >= 0 ? split_nb : lookahead_nb(mn);
+    if (m > 20000 || onb > 1024) onb = 0;
+    const bool f32 = std::is_same<T, float>::value && panel32_enabled();   // FP32 panels, else FP64 arithmetic
+    const bool cluster = !(std::is_same<T, float>::value && !f32) && cluster_fits<T>();
+    const bool ahead_blocks = onb > 0 && mn > 2 * onb && cluster && lookahead_enabled();
+    constexpr int kLists = 1024 / CP_NARROW, kListInts = 2 + 4 * PANEL_NB;
+    const size_t list_bytes = ((size_t)2 * kLists * kListInts * sizeof(int) + 255) / 256 * 256;
+    const size_t side_bytes = tc_kind >= 0 ? tc_update_workspace_bytes(tc_kind, m, onb, PANEL_NB) : 0;
+    Workspace *w = workspace_for(stream, fp64_split     ? split_off + split_ws0_bytes(m, n)
+                                         : ahead_blocks ? split_off + list_bytes + side_bytes
+                                                        : ws0);
     if (!w) return kErrAlloc;
     PanelScratch ps = carve_panel_scratch(w->buf);
     void *tc_buf = (char *)w->buf + (panel_scratch_bytes() + 255) / 256 * 256;
     FG_CUDA(cudaMemsetAsync(ps.slots, 0, kSlotBytes, stream));
     unsigned long long epoch = 0;
-    // FP32 storage: the FP32 panel (panel32_kernel); FP64: panel_kernel
-    const bool f32 = std::is_same<T, float>::value && panel32_enabled();
     const void *panel_fn[2] = {
         f32 ? (const void *)panel32_kernel<false> : (const void *)panel_kernel<T, false>,
         f32 ? (const void *)panel32_kernel<true> : (const void *)panel_kernel<T, true>};
@@ -1715,14 +1767,15 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
     // panels 6 ms less), since the panel's FP64 work then competes with the
     // GEMM's on the shared SMs.
     // (FP32 storage with the FP64-arithmetic panel keeps the grid kernel)
-    const int cluster_mp = (std::is_same<T, float>::value && !f32) || !cluster_fits<T>() ? 0 : cluster_rows<T>();
-    auto panel_at = [&](int j, cudaStream_t s, int *jb_out, bool defer) -> int {
+    auto panel_at = [&](int j, cudaStream_t s, int *jb_out, bool defer, PanelScratch ps, bool beside) -> int {
         int mp = m - j;
-        if (mp <= cluster_mp) {
-            int jb = std::min(std::min(mn - j, PANEL_NB), ob_end - j);
+        const int cw = cluster ? cluster_width<T>(mp, beside) : 0;
+        if (cw > 0) {
+            int jb = std::min(std::min(mn - j, cw), ob_end - j);
             const int R = ceil_div(mp, CP_CS);
             cudaLaunchAttribute attr;
-            const cudaLaunchConfig_t cfg = cluster_config(&attr, (size_t)R * PANEL_NB * sizeof(T), s);
+            const cudaLaunchConfig_t cfg =
+                cluster_config(&attr, (size_t)R * (jb <= CP_NARROW ? CP_NARROW : PANEL_NB) * sizeof(T), s);
             KTimer ktp(kFamPanel, s, (double)mp * jb * jb - (double)jb * jb * jb / 3.0,
                        2.0 * sizeof(T) * (double)mp * jb);
             FG_CUDA(cudaLaunchKernelEx(&cfg, panel_cluster_kernel<T>, A + j + (size_t)j * ldA, ldA, mp, jb, j,
@@ -1759,52 +1812,139 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
         *jb_out = jb;
         return kOk;
     };
-    auto update = [&](int j, int jb, int c0, int nc) -> int {
+    auto update_on = [&](int j, int jb, int c0, int nc, void *buf, cudaStream_t s) -> int {
         // A(j+jb:m, c0:c0+nc) -= A(j+jb:m, j:j+jb) * A(j:j+jb, c0:c0+nc)
         T *A21 = A + (j + jb) + (size_t)j * ldA;
         T *U12 = A + j + (size_t)c0 * ldA;
         T *A22 = A + (j + jb) + (size_t)c0 * ldA;
         if (tc_kind >= 0)
             return tc_trailing_update(tc_kind, m - j - jb, nc, jb, (const float *)A21, ldA,
-                                      (const float *)U12, ldA, (float *)A22, ldA, tc_buf, stream);
-        return gemm_tt<T>('N', 'N', m - j - jb, nc, jb, T(-1), A21, ldA, U12, ldA, T(1), A22, ldA,
-                          stream);
+                                      (const float *)U12, ldA, (float *)A22, ldA, buf, s);
+        return gemm_tt<T>('N', 'N', m - j - jb, nc, jb, T(-1), A21, ldA, U12, ldA, T(1), A22, ldA, s);
     };
+    auto update = [&](int j, int jb, int c0, int nc) -> int { return update_on(j, jb, c0, nc, tc_buf, stream); };
 
-    // interchanges of the panel (j, jb) on the columns outside it
-    auto interchange = [&](int j, int jb) -> int {
-        const int ncols = n - jb;
+    // interchanges of a panel (its moves in pl) on the columns c0 .. c1 - 1 but for
+    // the `skip` columns from j on
+    auto interchange_on = [&](const PanelScratch &pl, int c0, int c1, int j, int skip, cudaStream_t s) -> int {
+        const int ncols = c1 - c0 - skip;
         if (ncols <= 0) return kOk;
         const int blocks = ceil_div(ncols, 256 / 32);
-        KTimer ktl(kFamLaswp, stream, 0.0, 0.0);
-        laswp_pairs_kernel<T><<<blocks, 256, 0, stream>>>(A, ldA, ncols, j, jb, ps.swap_cnt, ps.swap_dst,
-                                                          ps.swap_src);
+        KTimer ktl(kFamLaswp, s, 0.0, 0.0);
+        laswp_pairs_kernel<T><<<blocks, 256, 0, s>>>(A + (size_t)c0 * ldA, ldA, ncols, j - c0, skip, pl.swap_cnt,
+                                                     pl.swap_dst, pl.swap_src);
         FG_CUDA(cudaGetLastError());
         return kOk;
     };
-    auto factor = [&](auto &&self, int j, int w) -> int {
+    auto interchange = [&](int j, int jb) -> int { return interchange_on(ps, 0, n, j, jb, stream); };
+    auto u12_on = [&](int j, int jb, int c0, int nc, cudaStream_t s) -> int {
+        return trsm_t<T>('L', 'L', 'N', 'U', jb, nc, T(1), A + j + (size_t)j * ldA, ldA, A + j + (size_t)c0 * ldA,
+                         ldA, s);
+    };
+    // Columns j .. j + w - 1 on stream s, interchanges within [c0, c1), the moves of
+    // its panels in lists[*nl], lists[*nl + 1], ...: halved, or (FP32 storage) in
+    // 64-column steps as the two-level order has them.
+    struct Block {
+        int c0, c1, nl;
+        bool beside;
+        const PanelScratch *lists;              // nullptr: ps for every panel
+        void *buf;
+        cudaStream_t s;
+    };
+    auto factor = [&](auto &&self, int j, int w, Block &k) -> int {
         int st, jb = 0;
-        if (w <= PANEL_NB) {
+        if (w <= PANEL_NB || std::is_same<T, float>::value) {
             // (a panel of a very tall matrix comes out narrower)
             ob_end = j + w;
-            if ((st = panel_at(j, stream, &jb, true)) != kOk) return st;
-            if ((st = interchange(j, jb)) != kOk) return st;
+            const PanelScratch &pl = k.lists ? k.lists[k.nl] : ps;
+            if ((st = panel_at(j, k.s, &jb, true, pl, k.beside)) != kOk) return st;
+            ++k.nl;
+            if ((st = interchange_on(pl, k.c0, k.c1, j, jb, k.s)) != kOk) return st;
         } else {
             jb = ceil_div(ceil_div(w, 2), PANEL_NB) * PANEL_NB;
-            if ((st = self(self, j, jb)) != kOk) return st;
+            if ((st = self(self, j, jb, k)) != kOk) return st;
         }
         const int c = j + jb, r = w - jb;
         if (r <= 0) return kOk;
-        if ((st = trsm_t<T>('L', 'L', 'N', 'U', jb, r, T(1), A + j + (size_t)j * ldA, ldA,
-                            A + j + (size_t)c * ldA, ldA, stream)) != kOk)
-            return st;
-        if (c < m && (st = update(j, jb, c, r)) != kOk) return st;
-        return self(self, c, r);
+        if ((st = u12_on(j, jb, c, r, k.s)) != kOk) return st;
+        if (c < m && (st = update_on(j, jb, c, r, k.buf, k.s)) != kOk) return st;
+        return self(self, c, r, k);
     };
-    if (recursive) {
-        const int st = factor(factor, 0, mn);
+    // Outer blocks with look-ahead: a block's panels run on 16 SMs (one cluster) and
+    // wait for each other column by column, so the next block is factored on the side
+    // stream while the rest of the trailing update runs beside it, on 16 SMs less
+    // (kClusterSms: its persistent products would take the cluster's SMs in the gaps
+    // between panels, and keep them).  Block k's interchanges on the columns outside
+    // it are taken from the lists its panels left.
+    if (ahead_blocks) {
+        int *mem = (int *)((char *)w->buf + split_off);
+        Workspace *wo = workspace_side(stream);
+        if (!wo) return kErrCuda;
+        {
+            PanelScratch lists[2][kLists];
+            for (int i = 0; i < 2 * kLists; ++i) {
+                PanelScratch &q = lists[i / kLists][i % kLists];
+                q = ps;
+                q.swap_cnt = mem + (size_t)i * kListInts;
+                q.swap_dst = q.swap_cnt + 2;
+                q.swap_src = q.swap_dst + 2 * PANEL_NB;
+            }
+            void *side_buf = (char *)mem + list_bytes;
+            cudaStream_t side = wo->side;
+            bool open = false;                  // side-stream work not yet joined
+            auto run = [&]() -> int {
+                int st;
+                Block blk[2];
+                auto start = [&](int i, int j) -> int {     // block i at column j on the side stream
+                    const int e = j + std::min(onb, mn - j);
+                    FG_CUDA(cudaEventRecord(wo->ev_fwd, stream));
+                    FG_CUDA(cudaStreamWaitEvent(side, wo->ev_fwd, 0));
+                    open = true;
+                    blk[i & 1] = Block{j, e, 0, true, lists[i & 1], side_buf, side};
+                    const int st1 = factor(factor, j, e - j, blk[i & 1]);
+                    FG_CUDA(cudaEventRecord(wo->ev_back, side));
+                    return st1;
+                };
+                if ((st = start(0, 0)) != kOk) return st;
+                for (int i = 0, j = 0; j < mn; ++i) {
+                    const Block b = blk[i & 1];
+                    const int e = b.c1, w = e - j;
+                    FG_CUDA(cudaStreamWaitEvent(stream, wo->ev_back, 0));
+                    open = false;
+                    // the next block's columns (all that is left when there is none)
+                    const int e2 = e < mn ? e + std::min(onb, mn - e) : n;
+                    for (int l = 0; l < b.nl && e2 > e; ++l)
+                        if ((st = interchange_on(b.lists[l], e, e2, e2, 0, stream)) != kOk) return st;
+                    if (e2 > e) {
+                        if ((st = u12_on(j, w, e, e2 - e, stream)) != kOk) return st;
+                        if (e < m && (st = update_on(j, w, e, e2 - e, tc_buf, stream)) != kOk) return st;
+                    }
+                    if (e < mn && (st = start(i + 1, e)) != kOk) return st;
+                    // the rest, beside that block's panels
+                    SpareSms spare(e < mn && cluster_width<T>(m - e, true) > 0 ? kClusterSms : 0);
+                    for (int l = 0; l < b.nl; ++l) {
+                        if ((st = interchange_on(b.lists[l], 0, j, j, 0, stream)) != kOk) return st;
+                        if ((st = interchange_on(b.lists[l], e2, n, n, 0, stream)) != kOk) return st;
+                    }
+                    if (n > e2) {
+                        if ((st = u12_on(j, w, e2, n - e2, stream)) != kOk) return st;
+                        if (e < m && (st = update_on(j, w, e2, n - e2, tc_buf, stream)) != kOk) return st;
+                    }
+                    j = e;
+                }
+                return kOk;
+            };
+            const int st = run();
+            // never leave side-stream work unjoined, also on an error path
+            if (open) cudaStreamWaitEvent(stream, wo->ev_back, 0);
+            return st;
+        }
+    }
+    if (recursive && !std::is_same<T, float>::value) {
+        Block all{0, n, 0, false, nullptr, tc_buf, stream};
+        const int st = factor(factor, 0, mn, all);
         if (st != kOk || n == mn) return st;
-        return trsm_t<T>('L', 'L', 'N', 'U', mn, n - mn, T(1), A, ldA, A + (size_t)mn * ldA, ldA, stream);
+        return u12_on(0, mn, mn, n - mn, stream);
     }
 
     bool ahead = false;     // the panel at j was launched on the side stream
@@ -1814,7 +1954,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
             if (ahead) {
                 FG_CUDA(cudaStreamWaitEvent(stream, wl->ev_back, 0));
                 ahead = false;
-            } else if ((st = panel_at(j, stream, &jb, true)) != kOk) {
+            } else if ((st = panel_at(j, stream, &jb, true, ps, false)) != kOk) {
                 return st;
             }
             if ((st = interchange(j, jb)) != kOk) return st;
@@ -1836,7 +1976,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
                         // defer when the update beside the panel is small
                         // (under ~4M elements: about the panel's own time)
                         const bool small = (double)(m - j - jb) * (double)(nr - w2) < 4.0e6;
-                        if ((st = panel_at(nx, wl->side, &next_jb, small)) != kOk) return st;
+                        if ((st = panel_at(nx, wl->side, &next_jb, small, ps, false)) != kOk) return st;
                         FG_CUDA(cudaEventRecord(wl->ev_back, wl->side));
                         ahead = true;
                         if (next_jb > w2) {
@@ -1896,7 +2036,8 @@ int dgetrf_split_launch(int m, int n, double *A, int ldA, int *ipiv, int *info, 
 int sgetrf_launch(int m, int n, float *A, int ldA, int *ipiv, int *info, int tc_kind,
                   cudaStream_t stream) {
     const int onb = tc_kind >= 0 ? tc_outer_nb() : 0;
-    return getrf_t<float>(m, n, A, ldA, ipiv, info, tc_kind, onb > PANEL_NB ? onb : 0, stream);
+    return getrf_t<float>(m, n, A, ldA, ipiv, info, tc_kind, onb > PANEL_NB ? onb : 0, stream,
+                          onb > PANEL_NB && sgetrf_lookahead(m, n, stream));
 }
 
 template <typename T>

@@ -763,7 +763,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
         a.p[i] = cs.res.p[i];
         a.ip[i] = cs.res.ip[i];
     }
-    const int items = tiles.ntiles * NP, sms = num_sms();
+    const int items = tiles.ntiles * NP, sms = num_sms() - spare_sms();
     const int grid = items < sms ? items : sms;
     {
         KTimer kt(kFamGemm, s, 2.0 * (tri ? 0.5 : 1.0) * m * (double)n * k,

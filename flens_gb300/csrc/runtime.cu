@@ -240,6 +240,11 @@ void *workspace_slot(cudaStream_t stream, int slot, size_t bytes) {
     return w->slot_buf[slot];
 }
 
+static thread_local int t_spare_sms = 0;
+int spare_sms() { return t_spare_sms; }
+SpareSms::SpareSms(int n) : before(t_spare_sms) { t_spare_sms = n; }
+SpareSms::~SpareSms() { t_spare_sms = before; }
+
 void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status) {
     Workspace *w = workspace_for(stream, 0);
     if (!w) return nullptr;
@@ -265,8 +270,13 @@ void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status) {
             if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
                 cudaGetLastError();
                 pool = nullptr;
-            } else if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-                cudaGetLastError();
+            } else {
+                // no reuse across streams by inserted waits: a panel's stream would
+                // wait for the update beside it
+                int off = 0;
+                if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
+                    cudaMemPoolSetAttribute(pool, cudaMemPoolReuseAllowInternalDependencies, &off) != cudaSuccess)
+                    cudaGetLastError();
             }
             r.pools[w->device] = pool;
         }
@@ -294,11 +304,17 @@ int set_smem_once(DeviceOnce &once, const void *fn, int bytes) {
 int check_device_status(cudaStream_t stream) {
     Workspace *w = workspace_for(stream, 0);
     if (!w) return kErrAlloc;
-    int h = 0;
+    // the side stream's products have a status word of their own; its work is
+    // joined to `stream`
+    Workspace *side = w->side ? workspace_for(w->side, 0) : nullptr;
+    int h = 0, hs = 0;
     FG_CUDA(cudaMemcpyAsync(&h, w->status, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    if (side) FG_CUDA(cudaMemcpyAsync(&hs, side->status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     FG_CUDA(cudaStreamSynchronize(stream));
+    h |= hs;
     if (h != kDevOk) {
         cudaMemsetAsync(w->status, 0, sizeof(int), stream);
+        if (side) cudaMemsetAsync(side->status, 0, sizeof(int), stream);
         cudaStreamSynchronize(stream);
         set_last_error("device-side wait timed out (status bits 0x%x)", h);
         return kErrTimeout;

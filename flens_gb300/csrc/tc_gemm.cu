@@ -411,7 +411,7 @@ int tc_gemm_launch(int kind, int M, int N, int K, float alpha, const void *A_lp,
     if (st != kOk) return st;
     if ((st = tc::make_kmajor_map(&mb, kind, B_lp, N, K, ldb, BN)) != kOk) return st;
     const int ntiles = ceil_div(M, BM) * ceil_div(N, BN);
-    const int sms = num_sms();
+    const int sms = num_sms() - spare_sms();
     const dim3 grid(ntiles < sms ? ntiles : sms);
     const int bk = 128 / (int)tc_elem_bytes(kind);
     const int pf = (((uintptr_t)C | ((uintptr_t)ldc * 4)) & 15) == 0 ? 1 : 0;
