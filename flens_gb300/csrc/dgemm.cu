@@ -95,9 +95,13 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     __shared__ T Bs[2][BK][TN + PAD];
     const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
     const int m0 = blockIdx.x * TM, n0 = blockIdx.y * TN;
+    if (FLAG) {
+        // (launched under the end of the kernel before it: nothing is read earlier)
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (!flag[m0 / 128 + flag_ld * (n0 / 256)]) return;
+    }
     if (TRI == 1 && m0 + TM <= n0) return;       // tile strictly above the diagonal
     if (TRI == 2 && n0 + TN <= m0) return;       // tile strictly below the diagonal
-    if (FLAG && !flag[m0 / 128 + flag_ld * (n0 / 256)]) return;
 
     SlabLoader<T, !TA, TM, NT> la;
     SlabLoader<T, TB, TN, NT> lb;
@@ -809,15 +813,20 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
     KTimer kt(kFamGemm, stream, 0.0, 0.0);
     const dim3 g64(ceil_div(m, BM), ceil_div(n, BN)), g32(ceil_div(m, 32), ceil_div(n, 32));
     const bool small = (long long)g64.x * g64.y < 4LL * num_sms();
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = small ? g32 : g64;
+    cfg.blockDim = dim3(256);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
 #define FG_FL(TA_, TB_, TRI_)                                                                              \
-    do {                                                                                                   \
-        if (small)                                                                                         \
-            dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32, true><<<g32, 256, 0, stream>>>(            \
-                m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld);                              \
-        else                                                                                               \
-            dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, BM, BN, true><<<g64, 256, 0, stream>>>(            \
-                m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld);                              \
-    } while (0)
+    FG_CUDA(cudaLaunchKernelEx(&cfg,                                                                       \
+                               small ? dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32, true>           \
+                                     : dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, BM, BN, true>,          \
+                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld))
 #define FG_FLT(TA_, TB_) do { if (tri == 1) FG_FL(TA_, TB_, 1); else if (tri == 2) FG_FL(TA_, TB_, 2); else FG_FL(TA_, TB_, 0); } while (0)
     if (!ta && !tb) FG_FL(false, false, 0);      // a triangle's product has one transposed operand
     else if (ta && !tb) FG_FLT(true, false);
@@ -825,7 +834,6 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
     else FG_FL(true, true, 0);
 #undef FG_FLT
 #undef FG_FL
-    FG_CUDA(cudaGetLastError());
     return kOk;
 }
 

@@ -56,9 +56,9 @@ constexpr int CHUNK = 1024;                  // 2^14 * 1024 = 2^24: exact FP32 s
 constexpr int kExpLimit = 450;
 constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23: adds round to integers
 
-struct ResConst {                            // operand side, per modulus
-    float p[NM], ip[NM];
-    float ca[NM][4], cb[NM][4];              // 2^(16 t) (times the CRT inverse for A) mod p
+struct ResConst {                            // operand side, per modulus, each value twice
+    float2 p[NM], ip[NM];
+    float2 ca[NM][4], cb[NM][4];             // 2^(16 t) (times the CRT inverse for A) mod p
 };
 struct CrtConst {
     uint32_t w[NG][NL];                      // byte l of P/p_i, four moduli per word
@@ -107,12 +107,13 @@ Consts make_consts() {
         while ((wmod * y) % p != 1) ++y;
         for (int l = 0; l < NL; ++l) c.crt.w[i / 4][l] |= (uint32_t)W[l] << (8 * (i % 4));
         c.crt.qw[i / 4] |= (uint32_t)((2 * 16384 + p) / (2 * p)) << (8 * (i % 4));
-        c.res.p[i] = (float)p;
-        c.res.ip[i] = 1.0f / (float)p;
+        c.res.p[i] = make_float2(-(float)p, -(float)p);      // (negated)
+        c.res.ip[i] = make_float2(1.0f / (float)p, 1.0f / (float)p);
         int b = 1;
         for (int t = 0; t < 4; ++t) {
-            c.res.cb[i][t] = (float)centred(b, p);
-            c.res.ca[i][t] = (float)centred(b * y, p);
+            const float fb = (float)centred(b, p), fa = (float)centred(b * y, p);
+            c.res.cb[i][t] = make_float2(fb, fb);
+            c.res.ca[i][t] = make_float2(fa, fa);
             b = b * (65536 % p) % p;
         }
     }
@@ -144,6 +145,26 @@ __device__ __forceinline__ unsigned mag_key(double v) {
     return hi ? hi : ((unsigned)b ? 1u : 0u);
 }
 
+// Every kernel here waits for the one before it before it reads or writes memory
+// (griddepcontrol), so that its launch and set-up run under that one's end.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... P, typename... Q>
+cudaError_t launch_early(void (*fn)(P...), int grid, int block, size_t smem, cudaStream_t s, Q... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, P(args)...);
+}
+
 // ------------------------------------------------------------ exponents --
 // Row maxima of |x| (as high words) by integer atomicMax into zeroed keys.
 // A block takes 64 rows x 32 k (rows contiguous; 8 loads in flight per thread)
@@ -155,6 +176,7 @@ __host__ __device__ inline int exp_blocks(int R, int K, int rcontig) {
 
 __global__ void __launch_bounds__(256)
 mod_exp_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Operand ob, int K, int blocksA) {
+    let_next_start();
     const bool isB = (int)blockIdx.x >= blocksA;
     const Operand &o = isB ? ob : oa;
     const int b = isB ? blockIdx.x - blocksA : blockIdx.x;
@@ -219,16 +241,42 @@ __device__ __forceinline__ float magnitude(double v, int e) {
     return __uint_as_float(((unsigned)(ex + 127) << 23) | (mant << 16));
 }
 
+// Two FP32 operations per instruction (each lane as the scalar one).
+__device__ __forceinline__ unsigned long long f2(float2 a) { return *(const unsigned long long *)&a; }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ unsigned bf16x2(unsigned long long a) {
+    unsigned d;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(d) : "f"(__uint_as_float((unsigned)(a >> 32))), "f"(__uint_as_float((unsigned)a)));
+    return d;
+}
+
 // A block turns 32 rows x 64 k of one operand into its NP planes.  The tile is
 // staged through shared memory so that both the FP64 reads and the BF16
 // writes (16 lanes x 8 bytes = one 128-byte line per row) are coalesced; a
 // thread holds 4 consecutive k, each as four signed 16-bit pieces in FP32, so
-// a residue is 4 FMAs (exact: |sum| < 2^24) and 3 operations of reduction.
-// Bound: 8 bytes read and 36 written per element, about 130 FP32 operations.
+// a residue is 4 FMAs (exact: |sum| < 2^24) and 3 operations of reduction, two
+// entries per instruction.  Bound: 8 bytes read and 36 written per element,
+// about 60 paired FP32 instructions.
 __global__ void __launch_bounds__(256)
 mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Operand ob, int K, int Kp,
                    int bits, int blocksA, const __grid_constant__ ResConst rc) {
     __shared__ __align__(16) double tile[32][66];
+    let_next_start();
+    wait_previous();
     const bool isB = (int)blockIdx.x >= blocksA;
     const Operand &o = isB ? ob : oa;
     const int b = isB ? blockIdx.x - blocksA : blockIdx.x;
@@ -258,7 +306,7 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
         if (r >= o.R) continue;
         bool ok;
         const int e = key_exp(o.key[r], ok);
-        float x[4][4], mg[4];
+        float x[4][4], mg[4];                     // [piece][entry]
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const double d = ok ? tile[rr][kq + i] : 0.0;
@@ -267,33 +315,35 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
                 const int piece = (int)(short)(v & 0xFFFF);
-                x[i][t] = (float)piece;
+                x[t][i] = (float)piece;
                 v = (v - piece) >> 16;
             }
         }
+        unsigned long long xl[4], xh[4];          // entries 0 and 1, 2 and 3
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            xl[t] = f2(make_float2(x[t][0], x[t][1]));
+            xh[t] = f2(make_float2(x[t][2], x[t][3]));
+        }
         __nv_bfloat16 *out = o.planes + (size_t)r * Kp + (k0 + kq);
-        auto put = [&](const float (&f)[4]) {
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
-            uint2 w;
-            w.x = *(const unsigned *)&lo;
-            w.y = *(const unsigned *)&hi;
-            *(uint2 *)out = w;
-            out += plane;
-        };
+        const unsigned long long magic = f2(make_float2(kMagic, kMagic)), unmagic = f2(make_float2(-kMagic, -kMagic));
 #pragma unroll
         for (int j = 0; j < NM; ++j) {
-            const float *c = isB ? rc.cb[j] : rc.ca[j];
-            const float c0 = c[0], c1 = c[1], c2 = c[2], c3 = c[3];
-            float f[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float s = fmaf(x[i][3], c3, fmaf(x[i][2], c2, fmaf(x[i][1], c1, x[i][0] * c0)));
-                const float q = fmaf(s, rc.ip[j], kMagic) - kMagic;
-                f[i] = fmaf(-q, rc.p[j], s);
-            }
-            put(f);
+            const float2 *c = isB ? rc.cb[j] : rc.ca[j];
+            const unsigned long long c0 = f2(c[0]), c1 = f2(c[1]), c2 = f2(c[2]), c3 = f2(c[3]);
+            const unsigned long long ip = f2(rc.ip[j]), mp = f2(rc.p[j]);
+            const unsigned long long sl = fma2(xl[3], c3, fma2(xl[2], c2, fma2(xl[1], c1, mul2(xl[0], c0))));
+            const unsigned long long sh = fma2(xh[3], c3, fma2(xh[2], c2, fma2(xh[1], c1, mul2(xh[0], c0))));
+            uint2 w;
+            w.x = bf16x2(fma2(add2(fma2(sl, ip, magic), unmagic), mp, sl));
+            w.y = bf16x2(fma2(add2(fma2(sh, ip, magic), unmagic), mp, sh));
+            *(uint2 *)out = w;
+            out += plane;
         }
-        put(mg);
+        uint2 w;
+        w.x = bf16x2(f2(make_float2(mg[0], mg[1])));
+        w.y = bf16x2(f2(make_float2(mg[2], mg[3])));
+        *(uint2 *)out = w;
     }
 }
 
@@ -398,6 +448,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     __syncthreads();
     fence_after();
     const uint32_t tmem = *tmem_slot;
+    wait_previous();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -567,6 +618,9 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 a.flag[m0 / MT + a.tiles.tm * (n0 / NT)] = 1;
         }
     }
+    // (not at the start: waiting reconstruction blocks would take the SMs left to a
+    // panel on another stream)
+    let_next_start();
     fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -657,6 +711,7 @@ mod_crt_kernel(const __grid_constant__ TileMap tiles, const uint8_t *__restrict_
                const uint8_t *__restrict__ flag, const unsigned *__restrict__ keyA,
                const unsigned *__restrict__ keyB, int bits2, double alpha, double beta,
                double *__restrict__ C, int ldC, const __grid_constant__ CrtConst k) {
+    wait_previous();
     const int t = blockIdx.x / CRT_PARTS, part = blockIdx.x % CRT_PARTS;
     int m0, n0;
     tile_at(tiles, t, m0, n0);
@@ -744,8 +799,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     {
         KTimer kt(kFamAux, s, 0.0, (8.0 + 2.0 * NP) * Kp * ((double)m + n));
         const int ba = ceil_div(m, 32) * (Kp / KBLK), bb = ceil_div(n, 32) * (Kp / KBLK);
-        mod_residue_kernel<<<ba + bb, 256, 0, s>>>(oa, ob, k, Kp, bits, ba, cs.res);
-        FG_CUDA(cudaGetLastError());
+        FG_CUDA(launch_early(mod_residue_kernel, ba + bb, 256, 0, s, oa, ob, k, Kp, bits, ba, cs.res));
     }
     CUtensorMap ma, mb;
     int rc = tc::make_kmajor_map(&ma, kTcBF16, oa.planes, NP * m, Kp, Kp, MT);
@@ -760,8 +814,8 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     a.keyA = oa.key;
     a.keyB = ob.key;
     for (int i = 0; i < NM; ++i) {
-        a.p[i] = cs.res.p[i];
-        a.ip[i] = cs.res.ip[i];
+        a.p[i] = -cs.res.p[i].x;
+        a.ip[i] = cs.res.ip[i].x;
     }
     const int items = tiles.ntiles * NP, sms = num_sms() - spare_sms();
     const int grid = items < sms ? items : sms;
@@ -771,18 +825,16 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
         static DeviceOnce once1, onceN;
         if (Kp <= CHUNK) {
             if ((rc = set_smem_once(once1, (const void *)mod_product_kernel<false>, (int)MOD_SMEM)) != kOk) return rc;
-            mod_product_kernel<false><<<grid, tc::THREADS, MOD_SMEM, s>>>(ma, mb, a, status);
+            FG_CUDA(launch_early(mod_product_kernel<false>, grid, tc::THREADS, MOD_SMEM, s, ma, mb, a, status));
         } else {
             if ((rc = set_smem_once(onceN, (const void *)mod_product_kernel<true>, (int)MOD_SMEM)) != kOk) return rc;
-            mod_product_kernel<true><<<grid, tc::THREADS, MOD_SMEM, s>>>(ma, mb, a, status);
+            FG_CUDA(launch_early(mod_product_kernel<true>, grid, tc::THREADS, MOD_SMEM, s, ma, mb, a, status));
         }
-        FG_CUDA(cudaGetLastError());
     }
     {
         KTimer kt(kFamAux, s, 0.0, (NM + 16.0) * m * (double)n);
-        mod_crt_kernel<<<tiles.ntiles * CRT_PARTS, 256, 0, s>>>(tiles, a.res, a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta,
-                                                        C, ldC, cs.crt);
-        FG_CUDA(cudaGetLastError());
+        FG_CUDA(launch_early(mod_crt_kernel, tiles.ntiles * CRT_PARTS, 256, 0, s, tiles, (const uint8_t *)a.res,
+                             (const uint8_t *)a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta, C, ldC, cs.crt));
     }
     // tiles the check refused
     return dgemm_flagged_launch(ta ? 'T' : 'N', tb ? 'T' : 'N', m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, tri,
@@ -802,18 +854,18 @@ bool mod_enabled() {
 }  // namespace
 
 // Estimated microseconds of the two routes, fitted to measurements from 256^3 to
-// 4096^3 and 1000 x 100 x 1000 to 8192 x 256 x 256 (all within 12%).  FP64: an SM
+// 4096^3 and 1000 x 100 x 1000 to 8192 x 256 x 256 (within 15%).  FP64: an SM
 // takes 0.265 us of its pipe per unit of k and 32 x 32 tile, in waves over the
 // SMs.  Residues: the launches, the work items in waves (1.2 us + 5.5 ns per unit
-// of k), the operands and C.  Both at, say, 300^3: 85 and 35 us; 4032 x 64 x 64: 39 and 41;
-// 4096 x 128 x 128: 134 and 46.
+// of k), the operands and C.  Both at, say, 300^3: 85 and 28 us; 4032 x 64 x 64: 38 and 37;
+// 4096 x 128 x 128: 134 and 44.
 bool mod_gemm_wins(int m, int n, int k, int tri) {
     if (n <= 16 || m <= 16 || k < 32 || !mod_enabled()) return false;
     const double half = tri ? 0.5 : 1.0, mn = half * m * (double)n;
     const int sms = num_sms() > 0 ? num_sms() : 1;
     const double fp64 = 5.0 + ceil(half * ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 0.265 * k;
     const double items = ceil(half * ceil_div(m, MT) * (double)ceil_div(n, NT) * NP / sms);
-    const double mod = 28.0 + items * (1.2 + 0.0055 * k) + 1.0e-5 * k * ((double)m + n) + 1.5e-5 * mn;
+    const double mod = 24.0 + items * (1.2 + 0.0055 * k) + 1.0e-5 * k * ((double)m + n) + 1.5e-5 * mn;
     return mod < 0.9 * fp64;
 }
 
