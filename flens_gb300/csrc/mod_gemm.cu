@@ -392,19 +392,23 @@ struct ModArgs {
 
 constexpr int STAGES = 4;
 constexpr uint32_t A_BYTES = MT * 128, B_BYTES = NT * 128;
+constexpr int EPI = 16;                       // epilogue warps
+constexpr int MOD_THREADS = 32 * (2 + EPI);
 constexpr size_t MOD_SMEM = 1024 + (size_t)STAGES * (A_BYTES + B_BYTES) + 256;
 
 // Persistent, one CTA per SM; a work item is (plane, tile), the magnitude
-// plane first.  Same roles as tc::tc_kernel (TMA producer, MMA issuer, eight
-// epilogue warps over two TMEM accumulators); a residue plane runs one
+// plane first.  Same roles as tc::tc_kernel (TMA producer, MMA issuer, epilogue
+// warps over two TMEM accumulators), with 16 epilogue warps; a residue plane runs one
 // accumulator per 1024 of k.  Epilogue: 6 FP32 operations per element reduce
 // the integer sum to a centred residue, 4 are packed per word, and a warp
 // stores 128 contiguous bytes per 4 columns.  MULTI (more than one chunk)
-// keeps the running residue sums of the thread's 128 elements packed in 64
-// registers.  Bound: the BF16 tensor pipe (0.65 us of epilogue against 2.6 us of
-// MMAs per item at k = 512).
+// keeps the running residue sums of the thread's 64 elements packed in 32
+// registers.  Bound: the BF16 tensor pipe plus, per item, about 1.25 us that the
+// accumulator's way out of TMEM adds (128 KB; 8 or 16 epilogue warps and
+// prefetching the next operands into L2 measured the same): 4096 x 4096 x k takes
+// 61 items of 1.25 us + 5.3 ns k per SM, 0.66 of the burst rate at k = 512, 0.89 at 4096.
 template <bool MULTI>
-__global__ void __launch_bounds__(tc::THREADS, 1)
+__global__ void __launch_bounds__(MOD_THREADS, 1)
 mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ ModArgs a, int *__restrict__ status) {
     using namespace tc;
@@ -432,7 +436,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&tfull[b], 1);
-            mbar_init(&tempty[b], EPI_WARPS);
+            mbar_init(&tempty[b], EPI);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         s_abort = 0;
@@ -520,7 +524,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
     } else {
         const int quarter = warp & 3;                // TMEM lane quarter this warp may access
-        const int half = (warp - 2) >> 2;            // column half
+        const int cq = (warp - 2) >> 2;              // column quarter
         const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
         const int rl = quarter * 32 + lane;          // tile row
         int i = 0;
@@ -534,7 +538,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             const float p = mag ? 1.0f : a.p[mag ? 0 : pl - 1], ip = mag ? 1.0f : a.ip[mag ? 0 : pl - 1];
             uint8_t *out = mag ? nullptr
                                : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 4;
-            uint32_t st[MULTI ? 64 : 1];
+            uint32_t st[MULTI ? 32 : 1];
             bool bad = false;
             for (int c = 0; c < chunks; ++c, ++i) {
                 const int b = i & 1;
@@ -547,8 +551,8 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                 const uint32_t base = tmem + (uint32_t)(b * NT) + lanes;
                 const bool lastc = c == chunks - 1;
 #pragma unroll
-                for (int cc = 0; cc < 4; ++cc) {
-                    const int c0 = half * 128 + cc * 32;
+                for (int cc = 0; cc < 2; ++cc) {
+                    const int c0 = cq * 64 + cc * 32;
                     if (n0 + c0 >= N) break;         // uniform across the warp
                     uint32_t r[32];
                     tmem_ld32(base + (uint32_t)c0, r);
@@ -825,10 +829,10 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
         static DeviceOnce once1, onceN;
         if (Kp <= CHUNK) {
             if ((rc = set_smem_once(once1, (const void *)mod_product_kernel<false>, (int)MOD_SMEM)) != kOk) return rc;
-            FG_CUDA(launch_early(mod_product_kernel<false>, grid, tc::THREADS, MOD_SMEM, s, ma, mb, a, status));
+            FG_CUDA(launch_early(mod_product_kernel<false>, grid, MOD_THREADS, MOD_SMEM, s, ma, mb, a, status));
         } else {
             if ((rc = set_smem_once(onceN, (const void *)mod_product_kernel<true>, (int)MOD_SMEM)) != kOk) return rc;
-            FG_CUDA(launch_early(mod_product_kernel<true>, grid, tc::THREADS, MOD_SMEM, s, ma, mb, a, status));
+            FG_CUDA(launch_early(mod_product_kernel<true>, grid, MOD_THREADS, MOD_SMEM, s, ma, mb, a, status));
         }
     }
     {
