@@ -10,16 +10,15 @@
 // the failing pivot stored in A(j,j), column scaled by the reciprocal 1/ajj)
 // and potrs (flens/lapack/po/potrs.tcc:54-100).  The reference updates
 // left-looking (syrk of the diagonal block, gemm of the block column, then
-// trsm); on the GPU the columns are halved down to 256,
+// trsm); on the GPU, by blocks of 256 columns,
 //
-//   factor(left half);  A21 <- A21 L11^-T  (trsm);  A22 -= A21 A21^T  (syrk, lower
-//   tiles only);  factor(right half)
+//   factor A11;  A21 <- A21 L11^-T  (trsm);  A22 -= A21 A21^T  (syrk, lower tiles only)
 //
-// so that the updates are deep products, and a block of 256 columns takes the
-// same three steps 64 columns at a time with potf2 of the 64 x 64 diagonal block
-// in one CTA.  n = 4000 with one right-hand side: 31.6 ms with right-looking
-// 64-column steps on the FP64 pipe, 17.5 with their products on the tensor cores,
-// 11.5 halved and with the diagonal block below.
+// with the 256-deep updates on the tensor cores (mod_gemm.cu), the next diagonal
+// block first, which is then factored beside the rest; a diagonal block takes the
+// same three steps 64 columns at a time with potf2 of the 64 x 64 block in one CTA.
+// n = 4000 with one right-hand side: 31.6 ms with right-looking 64-column steps on
+// the FP64 pipe, 11.1 one after the other, 8.9 in this order.
 //
 // Pivots, INFO and the factor agree with the reference to rounding; when
 // INFO > 0 the columns after the failing block hold partially updated values
@@ -34,6 +33,7 @@ namespace {
 
 constexpr int POTRF_NB = 64;
 constexpr int POTRF_BASE = 256;
+constexpr int kSideSms = 16;                      // left to the side stream
 
 // Unblocked right-looking Cholesky of the jb x jb (jb <= 64) diagonal block
 // at A, whose lower-view element (i, c), i >= c, is A[i*rs + c*cs] (rs = 1,
@@ -183,49 +183,94 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
         set_last_error("cudaMallocHost of the INFO readback failed");
         return kErrAlloc;
     }
-    // rows below (lower) or columns right of (upper) a factored block of width w at
-    // j, `rest` of them, and their update of what follows
-    auto trailing = [&](int j, int w, int rest) -> int {
-        double *A11 = A + j + (size_t)j * ldA, *A22 = A11 + w + (size_t)w * ldA;
-        int st;
-        if (lower) {
-            double *A21 = A11 + w;
-            if ((st = dtrsm_launch('R', 'L', 'T', 'N', rest, w, 1.0, A11, ldA, A21, ldA, s)) != kOk) return st;
-            return dsyrk_launch('L', 'N', rest, w, -1.0, A21, ldA, 1.0, A22, ldA, s);
-        }
-        double *A12 = A11 + (size_t)w * ldA;
-        if ((st = dtrsm_launch('L', 'U', 'T', 'N', w, rest, 1.0, A11, ldA, A12, ldA, s)) != kOk) return st;
-        return dsyrk_launch('U', 'T', rest, w, -1.0, A12, ldA, 1.0, A22, ldA, s);
+    auto at = [&](int i, int j) { return lower ? A + i + (size_t)j * ldA : A + j + (size_t)i * ldA; };   // element (i, j) of L
+    // Of a factored block of width w at j: rows r0 .. r0 + nr - 1 of L below it ...
+    auto solve_rows = [&](int j, int w, int r0, int nr, cudaStream_t q) -> int {
+        return lower ? dtrsm_launch('R', 'L', 'T', 'N', nr, w, 1.0, at(j, j), ldA, at(r0, j), ldA, q)
+                     : dtrsm_launch('L', 'U', 'T', 'N', w, nr, 1.0, at(j, j), ldA, at(r0, j), ldA, q);
     };
-    // Halved down to blocks of POTRF_BASE columns, so that the updates are as deep
-    // as wide (tensor cores, mod_gemm.cu); those blocks go right-looking in steps
-    // of 64.  *failed: a pivot failed (read back once per base block, as
-    // potrf.tcc:104-107 stops there; inside a base block the remaining steps skip).
-    auto factor = [&](auto &&self, int j, int w, bool last, bool *failed) -> int {
-        int st;
-        if (w > POTRF_BASE) {
-            const int h = ceil_div(ceil_div(w, 2), POTRF_NB) * POTRF_NB;
-            if ((st = self(self, j, h, false, failed)) != kOk || *failed) return st;
-            if ((st = trailing(j, h, w - h)) != kOk) return st;
-            return self(self, j + h, w - h, last, failed);
-        }
+    // ... their update of the triangle at c0, nc wide, and of the rows r0 .. below it
+    auto update_diag = [&](int j, int w, int c0, int nc, cudaStream_t q) -> int {
+        return dsyrk_launch(lower ? 'L' : 'U', lower ? 'N' : 'T', nc, w, -1.0, at(c0, j), ldA, 1.0, at(c0, c0), ldA, q);
+    };
+    auto update_below = [&](int j, int w, int c0, int nc, int r0, int nr, cudaStream_t q) -> int {
+        return lower ? dgemm_launch('N', 'T', nr, nc, w, -1.0, at(r0, j), ldA, at(c0, j), ldA, 1.0, at(r0, c0), ldA, q)
+                     : dgemm_launch('T', 'N', nc, nr, w, -1.0, at(c0, j), ldA, at(r0, j), ldA, 1.0, at(r0, c0), ldA, q);
+    };
+    // A diagonal block of up to POTRF_BASE columns, right-looking in steps of 64 (after
+    // a failed pivot the remaining steps skip).
+    auto diagonal = [&](int j, int w, cudaStream_t q) -> int {
         for (int c = 0; c < w; c += POTRF_NB) {
-            const int jb = w - c < POTRF_NB ? w - c : POTRF_NB;
+            const int jb = w - c < POTRF_NB ? w - c : POTRF_NB, rest = w - c - jb;
             {
-                KTimer kt(kFamPanel, s, (double)jb * jb * jb / 3.0, 16.0 * jb * jb);
-                potf2_kernel<<<1, POTF2_THREADS, 0, s>>>(jb, A + (j + c) + (size_t)(j + c) * ldA, rs, cs, j + c, info);
+                KTimer kt(kFamPanel, q, (double)jb * jb * jb / 3.0, 16.0 * jb * jb);
+                potf2_kernel<<<1, POTF2_THREADS, 0, q>>>(jb, at(j + c, j + c), rs, cs, j + c, info);
                 FG_CUDA(cudaGetLastError());
             }
-            if (c + jb < w && (st = trailing(j + c, jb, w - c - jb)) != kOk) return st;
+            int st;
+            if (rest > 0 && (st = solve_rows(j + c, jb, j + c + jb, rest, q)) != kOk) return st;
+            if (rest > 0 && (st = update_diag(j + c, jb, j + c + jb, rest, q)) != kOk) return st;
         }
-        if (last) return kOk;
-        FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, s));
-        FG_CUDA(cudaStreamSynchronize(s));
-        *failed = *h != 0;
         return kOk;
     };
-    bool failed = false;
-    const int st = factor(factor, 0, n, true, &failed);
+    if (n <= 2 * POTRF_BASE) {
+        // few blocks: one after the other; INFO is read back after each but the last
+        for (int j = 0; j < n; j += POTRF_BASE) {
+            const int w = n - j < POTRF_BASE ? n - j : POTRF_BASE, rest = n - j - w;
+            int st = diagonal(j, w, s);
+            if (st != kOk || rest == 0) return st;
+            FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, s));
+            FG_CUDA(cudaStreamSynchronize(s));
+            if (*h != 0) return kOk;           // as potrf.tcc:104-107 stops
+            if ((st = solve_rows(j, w, j + w, rest, s)) != kOk) return st;
+            if ((st = update_diag(j, w, j + w, rest, s)) != kOk) return st;
+        }
+        return kOk;
+    }
+    // Look-ahead: a diagonal block is a chain of small launches (330 us for 256
+    // columns), so the next one is updated first and factored on the side stream
+    // while the rest of the update, whose persistent products leave it 16 SMs, runs
+    // here.  n = 4000 with one right-hand side: 11.1 ms without.
+    Workspace *wo = workspace_side(s);
+    if (!wo) return kErrCuda;
+    cudaStream_t side = wo->side;
+    bool open = false;                            // side-stream work not yet joined
+    auto start = [&](int j, int w) -> int {       // diagonal block and its INFO, after what s has
+        FG_CUDA(cudaEventRecord(wo->ev_fwd, s));
+        FG_CUDA(cudaStreamWaitEvent(side, wo->ev_fwd, 0));
+        open = true;
+        const int st = diagonal(j, w, side);
+        if (st == kOk) FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, side));
+        FG_CUDA(cudaEventRecord(wo->ev_back, side));
+        return st;
+    };
+    auto run = [&]() -> int {
+        int st = start(0, POTRF_BASE);
+        for (int j = 0, w = POTRF_BASE; st == kOk;) {
+            const int e = j + w;
+            FG_CUDA(cudaStreamWaitEvent(s, wo->ev_back, 0));
+            open = false;
+            if (e == n) break;
+            FG_CUDA(cudaEventSynchronize(wo->ev_back));
+            if (*h != 0) break;                   // as potrf.tcc:104-107 stops
+            const int w2 = n - e < POTRF_BASE ? n - e : POTRF_BASE, e2 = e + w2;
+            if ((st = solve_rows(j, w, e, w2, s)) != kOk) return st;
+            if ((st = update_diag(j, w, e, w2, s)) != kOk) return st;
+            if ((st = start(e, w2)) != kOk) return st;
+            if (n > e2) {
+                SpareSms spare(kSideSms);
+                if ((st = solve_rows(j, w, e2, n - e2, s)) != kOk) return st;
+                if ((st = update_below(j, w, e, w2, e2, n - e2, s)) != kOk) return st;
+                if ((st = update_diag(j, w, e2, n - e2, s)) != kOk) return st;
+            }
+            j = e;
+            w = w2;
+        }
+        return st;
+    };
+    const int st = run();
+    // never leave side-stream work unjoined, also on an error path
+    if (open) cudaStreamWaitEvent(s, wo->ev_back, 0);
     if (st != kOk) return st;
     trace("potrf %c n=%d", uplo, n);
     return kOk;
