@@ -114,13 +114,22 @@ split_stats_kernel(int R, int K, const double *__restrict__ X, int ld, int *__re
         const int r = blockIdx.x * 32 + tx;
         unsigned long long mb = 0ull;
         if (r < R) {
-            for (int k = ty; k < K; k += 8) {
-                const unsigned long long b = abs_bits(X[(size_t)r + (size_t)k * ld]);
+            auto take = [&](double x) {
+                const unsigned long long b = abs_bits(x);
                 bad |= b >= kInfBits;
                 mb = b > mb ? b : mb;
                 sum += __longlong_as_double((long long)b);
                 nnz += b != 0ull;
+            };
+            int k = ty;
+            for (; k + 120 < K; k += 128) {          // 16 loads in flight
+                double x[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = X[(size_t)r + (size_t)(k + 8 * i) * ld];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) take(x[i]);
             }
+            for (; k < K; k += 8) take(X[(size_t)r + (size_t)k * ld]);
         }
         amax = __longlong_as_double((long long)mb);
         s_max[ty][tx] = amax;
@@ -143,13 +152,22 @@ split_stats_kernel(int R, int K, const double *__restrict__ X, int ld, int *__re
         if (r >= R) return;
         const double *x = X + (size_t)r * ld;
         unsigned long long mb = 0ull;
-        for (int k = lane; k < K; k += 32) {
-            const unsigned long long b = abs_bits(x[k]);
+        auto take = [&](double v) {
+            const unsigned long long b = abs_bits(v);
             bad |= b >= kInfBits;
             mb = b > mb ? b : mb;
             sum += __longlong_as_double((long long)b);
             nnz += b != 0ull;
+        };
+        int k = lane;
+        for (; k + 224 < K; k += 256) {              // 8 loads in flight
+            double v[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = x[k + 32 * i];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) take(v[i]);
         }
+        for (; k < K; k += 32) take(x[k]);
         amax = __longlong_as_double((long long)mb);
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) {
@@ -213,44 +231,46 @@ struct DigitGen {
     }
 };
 
+// The digits of two entries of a row, neighbours along k, as one store per slice.
 template <bool REVERSE>
-__device__ __forceinline__ void emit_digits(double v, int e, int S, int bits, size_t Kp,
+__device__ __forceinline__ void emit_digits(double v0, double v1, int e, int S, int bits, size_t Kp,
                                             __nv_bfloat16 *__restrict__ out) {
-    DigitGen gen(v, e, bits);
-    for (int s = 0; s < S; ++s)
-        out[(size_t)(REVERSE ? S - 1 - s : s) * Kp] = __float2bfloat16_rn((float)gen.next());
+    DigitGen g0(v0, e, bits), g1(v1, e, bits);
+    for (int s = 0; s < S; ++s) {
+        const float d0 = (float)g0.next(), d1 = (float)g1.next();
+        *(__nv_bfloat162 *)(out + (size_t)(REVERSE ? S - 1 - s : s) * Kp) = __floats2bfloat162_rn(d0, d1);
+    }
 }
 
 // Digits of op(X) (R x K) into a K-major BF16 buffer of R rows x (S*Kp);
-// columns K..Kp-1 of every slice are zero.  Grid (ceil(R/32), Kp/32), 256
-// threads.  RCONTIG as for the stats: a 32 x 32 tile is staged through shared
-// memory so that both the FP64 reads and the BF16 writes are coalesced.
+// columns K..Kp-1 of every slice are zero.  Grid (ceil(R/32), Kp/64), 256
+// threads.  RCONTIG as for the stats: a 32 x 64 tile is staged through shared
+// memory, 8 loads in flight per thread, so that the FP64 reads are coalesced and
+// a warp writes 128 bytes per slice (one row of the tile).
 template <bool RCONTIG, bool REVERSE>
 __global__ void __launch_bounds__(256)
 split_digits_kernel(int R, int K, int Kp, int S, int bits, const double *__restrict__ X, int ld,
                     const int *__restrict__ e_row, __nv_bfloat16 *__restrict__ out) {
-    __shared__ double tile[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+    __shared__ __align__(16) double tile[32][66];
+    const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
+    const int r0 = blockIdx.x * 32, k0 = blockIdx.y * 64;
     const size_t ldS = (size_t)S * Kp;
-    if (RCONTIG) {
-        for (int kk = ty; kk < 32; kk += 8) {
-            const int r = r0 + tx, k = k0 + kk;
-            tile[kk][tx] = (r < R && k < K) ? X[(size_t)r + (size_t)k * ld] : 0.0;
-        }
-    } else {
-        for (int rr = ty; rr < 32; rr += 8) {
-            const int r = r0 + rr, k = k0 + tx;
-            tile[tx][rr] = (r < R && k < K) ? X[(size_t)k + (size_t)r * ld] : 0.0;
-        }
+    double v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = r0 + (RCONTIG ? lane : wy + 8 * (i >> 1)), k = k0 + (RCONTIG ? wy + 8 * i : lane + 32 * (i & 1));
+        v[i] = (r < R && k < K) ? X[RCONTIG ? (size_t)r + (size_t)k * ld : (size_t)k + (size_t)r * ld] : 0.0;
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        tile[RCONTIG ? lane : wy + 8 * (i >> 1)][RCONTIG ? wy + 8 * i : lane + 32 * (i & 1)] = v[i];
     __syncthreads();
-    for (int rr = ty; rr < 32; rr += 8) {
-        const int r = r0 + rr, k = k0 + tx;
-        if (r < R && k < Kp) {
-            emit_digits<REVERSE>(tile[tx][rr], e_row[r], S, bits, (size_t)Kp,
-                                 out + (size_t)r * ldS + k);
-        }
+#pragma unroll 1
+    for (int rr = wy; rr < 32; rr += 8) {
+        const int r = r0 + rr;
+        if (r >= R) break;
+        const double2 d = *(const double2 *)&tile[rr][2 * lane];
+        emit_digits<REVERSE>(d.x, d.y, e_row[r], S, bits, (size_t)Kp, out + (size_t)r * ldS + (k0 + 2 * lane));
     }
 }
 
@@ -508,7 +528,7 @@ int dgemm_split_launch_at(char transA, char transB, int m, int n, int k, double 
     __nv_bfloat16 *Ad = (__nv_bfloat16 *)dig, *Bd = (__nv_bfloat16 *)(dig + bytesA);
     {
         KTimer kt(kFamAux, s, 0.0, (8.0 + 2.0 * S) * ((double)m + n) * geo.Kp);
-        const dim3 ga(ceil_div(m, 32), geo.Kp / 32), gb(ceil_div(n, 32), geo.Kp / 32);
+        const dim3 ga(ceil_div(m, 32), geo.Kp / 64), gb(ceil_div(n, 32), geo.Kp / 64);
         if (!ta) split_digits_kernel<true, false><<<ga, 256, 0, s>>>(m, k, geo.Kp, S, bits, A, ldA, ea, Ad);
         else split_digits_kernel<false, false><<<ga, 256, 0, s>>>(m, k, geo.Kp, S, bits, A, ldA, ea, Ad);
         if (tb) split_digits_kernel<true, true><<<gb, 256, 0, s>>>(n, k, geo.Kp, S, bits, B, ldB, eb, Bd);
