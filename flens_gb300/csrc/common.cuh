@@ -236,14 +236,15 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
 // The product on the tensor cores by exact residues (mod_gemm.cu), tri 0 all
 // of C, 1/2 its lower/upper triangle; kErrUnsupported (nothing launched) when
 // mod_gemm_wins is false, the stream is being captured or no scratch memory
-// is to be had.  dgemm_flagged_launch: the FP64 kernel on the blocks it
+// is to be had; kr as dgemm_kr_launch, for the tiles it refuses.  dgemm_flagged_launch: the FP64 kernel on the blocks it
 // refused.
 bool mod_gemm_wins(int m, int n, int k, int tri);
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
-                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s);
+                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s,
+                    int kr = 0);
 int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
                          int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
-                         const uint8_t *flag, int flag_ld, cudaStream_t stream);
+                         const uint8_t *flag, int flag_ld, int kr, cudaStream_t stream);
 
 // dgemm with one triangular operand stored full (explicit zeros): kr 1/2 =
 // op(A) upper/lower, 3/4 = op(B) upper/lower; the zero k blocks are skipped.

@@ -704,6 +704,10 @@ int dgemm_kr_launch(char transA, char transB, int m, int n, int k, double alpha,
                                      stream);
     if (m == 0 || n == 0) return kOk;
     if (alpha == 0.0) return scal_matrix_launch_t<double>(m, n, beta, C, ldC, stream);
+    // (the whole product on the tensor cores is far cheaper than half of it here;
+    // its refused tiles come back with the same k ranges)
+    const int mst = mod_gemm_launch(transA, transB, m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, 0, stream, kr);
+    if (mst != kErrUnsupported) return mst;
     const bool ta = !(transA == 'N' || transA == 'n');
     const bool tb = !(transB == 'N' || transB == 'n');
     const dim3 grid(ceil_div(m, BM), ceil_div(n, BN));
@@ -805,14 +809,16 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
 }
 
 // The FP64 kernel on the flagged 128 x 256 blocks of C only (tri 1/2: within
-// the lower/upper triangle): the tiles a residue product refused.
+// the lower/upper triangle; kr as dgemm_kr_launch): the tiles a residue product
+// refused.
 int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
                          int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
-                         const uint8_t *flag, int flag_ld, cudaStream_t stream) {
+                         const uint8_t *flag, int flag_ld, int kr, cudaStream_t stream) {
     const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
     KTimer kt(kFamGemm, stream, 0.0, 0.0);
     const dim3 g64(ceil_div(m, BM), ceil_div(n, BN)), g32(ceil_div(m, 32), ceil_div(n, 32));
-    const bool small = (long long)g64.x * g64.y < 4LL * num_sms();
+    // (k ranges depend on the tile: the one dgemm_kr_launch takes)
+    const bool small = !kr && (long long)g64.x * g64.y < 4LL * num_sms();
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -822,18 +828,34 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-#define FG_FL(TA_, TB_, TRI_)                                                                              \
+#define FG_FLK(TA_, TB_, TRI_, KR_)                                                                        \
     FG_CUDA(cudaLaunchKernelEx(&cfg,                                                                       \
-                               small ? dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32, true>           \
-                                     : dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, BM, BN, true>,          \
+                               small ? dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, 32, 32, true>         \
+                                     : dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, BM, BN, true>,        \
                                m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld))
+#define FG_FL(TA_, TB_, TRI_) FG_FLK(TA_, TB_, TRI_, 0)
+#define FG_FLK64(TA_, TB_, KR_)                                                                            \
+    FG_CUDA(cudaLaunchKernelEx(&cfg, dgemm_fma_kernel<double, TA_, TB_, 0, KR_, BM, BN, true>,             \
+                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld))
+#define FG_FLR(TA_, TB_) switch (kr) { case 1: FG_FLK64(TA_, TB_, 1); break; case 2: FG_FLK64(TA_, TB_, 2); break; \
+                                       case 3: FG_FLK64(TA_, TB_, 3); break; default: FG_FLK64(TA_, TB_, 4); }
+    if (kr) {
+        if (!ta && !tb) { FG_FLR(false, false) }
+        else if (ta && !tb) { FG_FLR(true, false) }
+        else if (!ta && tb) { FG_FLR(false, true) }
+        else { FG_FLR(true, true) }
+        return kOk;
+    }
 #define FG_FLT(TA_, TB_) do { if (tri == 1) FG_FL(TA_, TB_, 1); else if (tri == 2) FG_FL(TA_, TB_, 2); else FG_FL(TA_, TB_, 0); } while (0)
     if (!ta && !tb) FG_FL(false, false, 0);      // a triangle's product has one transposed operand
     else if (ta && !tb) FG_FLT(true, false);
     else if (!ta && tb) FG_FLT(false, true);
     else FG_FL(true, true, 0);
 #undef FG_FLT
+#undef FG_FLR
+#undef FG_FLK64
 #undef FG_FL
+#undef FG_FLK
     return kOk;
 }
 

@@ -781,8 +781,8 @@ constexpr int kBlkK = 4096, kBlkMN = 4096;        // one block product at most: 
 
 // One block product in the scratch `ws` (layout_for(m, n, Kp, tiles).total bytes).
 int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int ldA,
-              const double *B, int ldB, double beta, double *C, int ldC, int tri, char *ws, int *status,
-              cudaStream_t s) {
+              const double *B, int ldB, double beta, double *C, int ldC, int tri, int kr, char *ws,
+              int *status, cudaStream_t s) {
     const Consts &cs = consts();
     const int Kp = ceil_div(k, KBLK) * KBLK;
     const TileMap tiles = make_tiles(m, n, tri);
@@ -842,7 +842,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     }
     // tiles the check refused
     return dgemm_flagged_launch(ta ? 'T' : 'N', tb ? 'T' : 'N', m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, tri,
-                                a.flag, tiles.tm, s);
+                                a.flag, tiles.tm, kr, s);
 }
 
 int g_mode = -1;
@@ -878,7 +878,7 @@ bool mod_gemm_wins(int m, int n, int k, int tri) {
 // (a stream under capture, no scratch memory, or the FP64 route is faster):
 // nothing has been launched then and the caller takes the FP64 kernel.
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
-                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s) {
+                    const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s, int kr) {
     if (!mod_gemm_wins(m, n, k, tri)) return kErrUnsupported;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
@@ -893,13 +893,15 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
         const int parts = ceil_div(x, cap_);
         return ceil_div(ceil_div(x, parts), unit) * unit;
     };
-    const int kb = part(k, kBlkK, KBLK);
+    // (k ranges of refused tiles are counted from the whole operand: one block)
+    const int kb = kr ? ceil_div(k, KBLK) * KBLK : part(k, kBlkK, KBLK);
     // a shallow product may take larger blocks of C for the same scratch
     const int capMN = kb <= 1024 ? 2 * kBlkMN : kBlkMN;
-    const int mb = part(m, capMN, NT), nb = part(n, capMN, NT);
+    const int mb = kr ? ceil_div(m, NT) * NT : part(m, capMN, NT), nb = kr ? ceil_div(n, NT) * NT : part(n, capMN, NT);
     const int mm = mb < m ? mb : m, nn = nb < n ? nb : n, kk = kb < k ? kb : k;
     const Layout l = layout_for(mm, nn, ceil_div(kk, KBLK) * KBLK,
                                 make_tiles(mm, nn, tri && mb >= m && nb >= n ? tri : 0));
+    if (kr && l.total > ((size_t)4 << 30)) return kErrUnsupported;
     int *status = nullptr;
     char *ws = (char *)scratch_acquire(l.total, s, &status);
     if (!ws) return kErrUnsupported;
@@ -917,7 +919,7 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
                 const int bk = k - k0 < kb ? k - k0 : kb;
                 rc = mod_block(ta, tb, bm, bn, bk, alpha, A + (ta ? k0 + (size_t)i0 * ldA : i0 + (size_t)k0 * ldA),
                                ldA, B + (tb ? j0 + (size_t)k0 * ldB : k0 + (size_t)j0 * ldB), ldB,
-                               k0 == 0 ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, ws, status, s);
+                               k0 == 0 ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, kr, ws, status, s);
             }
     scratch_release(ws, s);
     return rc;
