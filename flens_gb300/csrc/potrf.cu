@@ -240,7 +240,9 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
         FG_CUDA(cudaStreamWaitEvent(side, wo->ev_fwd, 0));
         open = true;
         const int st = diagonal(j, w, side);
-        if (st == kOk) FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, side));
+        // (not after the last block: a copy in flight when the call returns could land
+        // in a later call's readback)
+        if (st == kOk && j + w < n) FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, side));
         FG_CUDA(cudaEventRecord(wo->ev_back, side));
         return st;
     };
@@ -271,7 +273,10 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
     const int st = run();
     // never leave side-stream work unjoined, also on an error path
     if (open) cudaStreamWaitEvent(s, wo->ev_back, 0);
-    if (st != kOk) return st;
+    if (st != kOk) {
+        cudaStreamSynchronize(side);              // its readback, too
+        return st;
+    }
     trace("potrf %c n=%d", uplo, n);
     return kOk;
 }

@@ -62,3 +62,25 @@ def test_info_and_leading_part(cuda, uplo, f, bad):
     assert np.array_equal(tri(a[:f, :f]), tri(w[:f, :f]))
     other = np.triu(np.ones((n, n), dtype=bool), 1) if uplo == "L" else np.tril(np.ones((n, n), dtype=bool), -1)
     assert np.array_equal(a[other], A0[other])
+
+
+def test_failure_in_the_last_block_stays_with_its_call(cuda):
+    """Calls on two streams by one thread share the host's INFO word: a failure in one
+    call's last block does not stop the other."""
+    import torch
+    n = 700
+    good = _spd(n, 5)
+    bad = good.copy()
+    bad[n - 3, n - 3] = -1.0
+    want, _ = _potrf(cuda, "L", good)
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for _ in range(20):
+        A = [fg.to_colmajor(torch.from_numpy(x).to(cuda)) for x in (bad, good)]
+        info = [torch.zeros(1, dtype=torch.int32, device=cuda) for _ in A]
+        torch.cuda.synchronize()
+        for s, a, i in zip(streams, A, info):
+            with torch.cuda.stream(s):
+                fg.dpotrf_dev("L", a, i)
+        torch.cuda.synchronize()
+        assert [int(i.item()) for i in info] == [n - 2, 0]
+        assert torch.equal(torch.tril(A[1]), torch.tril(want))
