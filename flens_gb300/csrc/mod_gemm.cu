@@ -25,15 +25,15 @@
 //
 // No less accurate than FP64 arithmetic, by a check on the data: an 18th
 // product of the magnitudes (rounded down to BF16) bounds Q_ij = sum_k
-// |a_ik||b_kj| 2^(-e_i-f_j) from below.  Rounding the operands changes c_ij by
-// at most 2^-beta k 2^(e_i+f_j); a tile is accepted only if k/Q_ij <= 2^(beta-51)
-// for all its elements with Q_ij != 0, that is, if that change is below
-// 4 * 2^-53 * (|A||B|)_ij -- FP64's own bound is k * 2^-53 * (|A||B|)_ij.
-// Uniform data needs k/Q = 2^2, LU and Cholesky updates up to 2^7, the limit
-// is 2^8 to 2^10.  Tiles of graded data beyond that, and tiles with
-// non-finite rows or exponents outside +-450, are left to the FP64 kernel,
-// which runs last and skips all others: no readback, the call stays
-// asynchronous.
+// |a_ik||b_kj| 2^(-e_i-f_j) from below, and their sums s_i, t_j over k are taken with
+// the residues.  Rounding the operands changes c_ij by at most
+// 2^(-beta-1) (s_i + t_j) 2^(e_i+f_j); a tile is accepted only if that is below
+// 4 * 2^-53 * (|A||B|)_ij for all its elements with Q_ij != 0 -- FP64's own bound is
+// k * 2^-53 * (|A||B|)_ij.  Uniform entries and LU and Cholesky updates keep 4 to 6 bits
+// of margin, entries u 2^e with e in [-16, 16] about one.  Tiles of data graded beyond
+// that, and tiles with non-finite rows or exponents outside +-450, are left to
+// the FP64 kernel, which runs last and skips all others: no readback, the
+// call stays asynchronous.
 #include "tcgen05.cuh"
 
 #include <cuda_bf16.h>
@@ -129,6 +129,7 @@ struct Operand {
     const double *X;
     int ld, R, rcontig;                      // rcontig: element (r, k) at X[r + k ld], else X[k + r ld]
     unsigned *key;                           // row maxima: high word of |x|
+    unsigned *sum;                           // row sums of the magnitudes, in 2^-16
     __nv_bfloat16 *planes;                   // NP planes of R rows x Kp
 };
 
@@ -271,7 +272,7 @@ __device__ __forceinline__ unsigned bf16x2(unsigned long long a) {
 // a residue is 4 FMAs (exact: |sum| < 2^24) and 3 operations of reduction, two
 // entries per instruction.  Bound: 8 bytes read and 36 written per element,
 // about 60 paired FP32 instructions.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ Operand ob, int K, int Kp,
                    int bits, int blocksA, const __grid_constant__ ResConst rc) {
     __shared__ __align__(16) double tile[32][66];
@@ -319,13 +320,22 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
                 v = (v - piece) >> 16;
             }
         }
+        __nv_bfloat16 *out = o.planes + (size_t)r * Kp + (k0 + kq);
+        // (integer sums: the same in any order)
+        unsigned sum = __float2uint_ru(((mg[0] + mg[1]) + (mg[2] + mg[3])) * 65536.0f);
+#pragma unroll
+        for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFu << (lane & 16), sum, off);
+        if ((lane & 15) == 0 && sum) atomicAdd(&o.sum[r], sum);
+        uint2 w0;
+        w0.x = bf16x2(f2(make_float2(mg[0], mg[1])));
+        w0.y = bf16x2(f2(make_float2(mg[2], mg[3])));
+        *(uint2 *)(out + NM * plane) = w0;
         unsigned long long xl[4], xh[4];          // entries 0 and 1, 2 and 3
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
             xl[t] = f2(make_float2(x[t][0], x[t][1]));
             xh[t] = f2(make_float2(x[t][2], x[t][3]));
         }
-        __nv_bfloat16 *out = o.planes + (size_t)r * Kp + (k0 + kq);
         const unsigned long long magic = f2(make_float2(kMagic, kMagic)), unmagic = f2(make_float2(-kMagic, -kMagic));
 #pragma unroll
         for (int j = 0; j < NM; ++j) {
@@ -340,10 +350,6 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
             *(uint2 *)out = w;
             out += plane;
         }
-        uint2 w;
-        w.x = bf16x2(f2(make_float2(mg[0], mg[1])));
-        w.y = bf16x2(f2(make_float2(mg[2], mg[3])));
-        *(uint2 *)out = w;
     }
 }
 
@@ -383,10 +389,10 @@ __device__ __forceinline__ void tile_at(const TileMap &tm, int t, int &m0, int &
 struct ModArgs {
     TileMap tiles;
     int nkb;                                  // 64-deep k blocks
-    float qmin;                               // smallest accepted Q
+    float qscale;                             // smallest accepted Q: this times (s_i + t_j)
     uint8_t *res;                             // residues [modulus][tile][4-column group][row][4]
     uint8_t *flag;                            // per tile (row tile + tm * column tile): 1 = left to FP64
-    const unsigned *keyA, *keyB;
+    const unsigned *keyA, *keyB, *sumA, *sumB;
     float p[NM], ip[NM];
 };
 
@@ -540,6 +546,24 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                                : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 4;
             uint32_t st[MULTI ? 32 : 1];
             bool bad = false;
+            float si = 0.0f, tj[2] = {0.0f, 0.0f};
+            if (mag) {                               // rows' and columns' data, before the wait
+                bool ok = true;
+                if (m0 + rl < M) {
+                    key_exp(a.keyA[m0 + rl], ok);
+                    bad |= !ok;
+                    si = (float)a.sumA[m0 + rl];
+                }
+#pragma unroll
+                for (int cc = 0; cc < 2; ++cc) {
+                    const int col = n0 + cq * 64 + cc * 32 + lane;
+                    if (col < N) {
+                        key_exp(a.keyB[col], ok);
+                        bad |= !ok;
+                        tj[cc] = (float)a.sumB[col];
+                    }
+                }
+            }
             for (int c = 0; c < chunks; ++c, ++i) {
                 const int b = i & 1;
                 if (!mbar_wait(&tfull[b], (uint32_t)(i >> 1) & 1u, status)) {
@@ -557,16 +581,11 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     uint32_t r[32];
                     tmem_ld32(base + (uint32_t)c0, r);
                     if (mag) {
-                        bool okr = true, okc = true;
-                        if (m0 + rl < M) key_exp(a.keyA[m0 + rl], okr);
-                        if (n0 + c0 + lane < N) key_exp(a.keyB[n0 + c0 + lane], okc);
-                        bad |= !okr | !okc;
-                        if (m0 + rl < M) {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                const float q = __uint_as_float(r[j]);
-                                bad |= n0 + c0 + j < N && q < a.qmin && q != 0.0f;
-                            }
+                        for (int j = 0; j < 32; ++j) {
+                            const float q = __uint_as_float(r[j]);
+                            const float qmin = (si + __shfl_sync(0xffffffffu, tj[cc], j)) * a.qscale;
+                            bad |= m0 + rl < M && n0 + c0 + j < N && q < qmin && q != 0.0f;
                         }
                     } else {
 #pragma unroll
@@ -762,13 +781,15 @@ static_assert(NM % 4 == 1, "the last residue group holds one modulus");
 size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Layout {
-    size_t keyA, keyB, flag, zeroed, planesA, planesB, res, total;
+    size_t keyA, keyB, sumA, sumB, flag, zeroed, planesA, planesB, res, total;
 };
 Layout layout_for(int m, int n, int Kp, const TileMap &t) {
     Layout l{};
     l.keyA = 0;
     l.keyB = up256((size_t)m * 4);
-    l.flag = l.keyB + up256((size_t)n * 4);
+    l.sumA = l.keyB + up256((size_t)n * 4);
+    l.sumB = l.sumA + up256((size_t)m * 4);
+    l.flag = l.sumB + up256((size_t)n * 4);
     l.zeroed = l.flag + up256((size_t)t.tm * t.tn);
     l.planesA = l.zeroed;
     l.planesB = l.planesA + up256((size_t)NP * m * Kp * 2);
@@ -791,8 +812,10 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     while ((1 << lk) < k) ++lk;
     int bits = (cs.log2P - 2 - lk) / 2;
     if (bits > 61) bits = 61;
-    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (__nv_bfloat16 *)(ws + l.planesA)};
-    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (__nv_bfloat16 *)(ws + l.planesB)};
+    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (unsigned *)(ws + l.sumA),
+                     (__nv_bfloat16 *)(ws + l.planesA)};
+    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (unsigned *)(ws + l.sumB),
+                     (__nv_bfloat16 *)(ws + l.planesB)};
     FG_CUDA(cudaMemsetAsync(ws, 0, l.zeroed, s));
     {
         KTimer kt(kFamAux, s, 0.0, 8.0 * k * ((double)m + n));
@@ -812,11 +835,14 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     ModArgs a{};
     a.tiles = tiles;
     a.nkb = Kp / KBLK;
-    a.qmin = (float)(k * ldexp(1.0, 51 - bits));
+    // 2^(-bits-1) (s + t) <= 2^-51 Q; the magnitudes were rounded down by up to 2^-7
+    a.qscale = (float)(1.01 * ldexp(1.0, 50 - bits - 16));
     a.res = (uint8_t *)(ws + l.res);
     a.flag = (uint8_t *)(ws + l.flag);
     a.keyA = oa.key;
     a.keyB = ob.key;
+    a.sumA = oa.sum;
+    a.sumB = ob.sum;
     for (int i = 0; i < NM; ++i) {
         a.p[i] = -cs.res.p[i].x;
         a.ip[i] = cs.res.ip[i].x;

@@ -76,6 +76,24 @@ def test_accuracy_sampled(cuda, m, n, k, spread):
         assert abs(Fraction(got[i, j]) - ex) <= Fraction(4 * U * mag + U * abs(float(ex)))
 
 
+@pytest.mark.parametrize("E", [4, 8, 12, 16, 24])
+def test_wide_entries(cuda, E):
+    """Entries u 2^e, e uniform in [-E, E]: accurate whether a tile is accepted or
+    refused (the bound of the FP64 sum, with 4 for the operands' rounding)."""
+    r = np.random.default_rng(E)
+    m, n, k = 300, 520, 1500
+    A = np.ldexp(r.uniform(-1, 1, (m, k)), r.integers(-E, E + 1, (m, k)))
+    B = np.ldexp(r.uniform(-1, 1, (k, n)), r.integers(-E, E + 1, (k, n)))
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, np.zeros((m, n)))
+    assert used >= 5
+    L = np.longdouble
+    for i in r.integers(0, m, 12):
+        ex = A[i].astype(L) @ B.astype(L)
+        mag = np.abs(A[i]) @ np.abs(B)
+        err = np.abs(got[i].astype(L) - ex).astype(np.float64) / (U * mag)
+        assert err.max() <= (4.5 if E <= 8 else np.sqrt(k) + 4.5)
+
+
 def _refused(cuda, A, B, C, alpha=1.0, beta=1.0):
     k = A.shape[1]
     got, used = _gemm(cuda, "N", "N", alpha, A, B, beta, C)
