@@ -193,7 +193,12 @@ void xerbla_(const char *SRNAME, const int *INFO, int SRNAME_LEN);
 /* ---------------------------------------- device-pointer entry points --- */
 
 /* dgemm on device memory (same semantics as dgemm_: beta scaling first,
- * alpha==0 returns without reading A or B).  Async on stream. */
+ * alpha==0 returns without reading A or B).  Async on stream.  Large products are
+ * formed on the tensor cores from exact residues, where a check on the data, on
+ * the device, keeps the rounding of the operands below 4 * 2^-53 * |A||B|; tiles
+ * it refuses, small products, streams under capture and calls without memory for
+ * the scratch (at most about 2.7 GB, from a pool in stream order) take the FP64
+ * kernel.  FLENS_GB300_DGEMM=fma in the environment selects that for all. */
 int flens_gb300_dgemm(char transA, char transB, int m, int n, int k,
                       double alpha, const double *A, int ldA,
                       const double *B, int ldB, double beta, double *C,
@@ -278,10 +283,10 @@ int flens_gb300_dgesvx(char fact, char trans, int n, int nrhs, double *A,
                        int ldX, double *rcond, double *ferr, double *berr,
                        double *rpvgrw, int *info, void *stream);
 
-/* dpotrf on device memory; info is a device int.  Blocked right-looking
- * (64-column steps: potf2 of the diagonal block, trsm, syrk of the trailing
- * triangle); waits for the stream once per step to stop at the first
- * non-positive pivot. */
+/* dpotrf on device memory; info is a device int.  Blocked right-looking by 256
+ * columns (64-column steps inside: potf2 of the diagonal block, trsm, syrk), the
+ * next diagonal block factored beside the rest of the update; waits once per
+ * block to stop at the first non-positive pivot. */
 int flens_gb300_dpotrf(char uplo, int n, double *A, int ldA, int *info,
                        void *stream);
 
