@@ -44,29 +44,40 @@ constexpr int kSideSms = 16;                      // left to the side stream
 // Bound: the chain of the pivots, as one FP64 instruction holds a scheduler's
 // pipe for 64 clocks and takes about 100.  The elimination therefore runs on the
 // unscaled columns, a_ic -= (a_it p_t) a_ct with p_t = 1 / pivot: two FP64
-// instructions and a reciprocal (three, see recip) per step.  Warps 0 and 1
+// instructions and a reciprocal per step.  Warps 0 and 1
 // (thread per row) run that chain: in step t they bring column t + 1 up to date
 // with columns t - 1 and t, and the warp that owns the next pivot takes its
 // reciprocal.  The other 14 apply column t - 1 to the columns from t + 2 on, one
 // barrier per step.  The columns are scaled by 1 / sqrt(pivot) and the diagonal's
 // square roots taken at the end, together.  (With sqrt, divide and three barriers
-// per column on the chain a block took 93 us; this takes 55.)
+// per column on the chain a block took 93 us; this takes 57.)
 constexpr int POTF2_THREADS = 512, UPD = POTF2_THREADS / 32 - 2;
 
-// 1 / d for a normal d within 2^+-1000, to about an ulp: the FP32 reciprocal r of
-// its significand, then the third-order iteration r + r (e + e^2), e = 1 - d r.
-__device__ __forceinline__ double recip(double d) {
-    const long long b = __double_as_longlong(d);
-    const int ex = (int)(b >> 52) & 0x7FF;
-    if (ex < 23 || ex > 2023) return 1.0 / d;
-    // significand in [1, 2) as FP32 (its leading 23 bits), and d scaled to it
-    const float f = __uint_as_float(0x3F800000u | (unsigned)((b >> 29) & 0x7FFFFF));
-    const unsigned r = __float_as_uint(__fdividef(1.0f, f));           // in [0.5, 1]
-    const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);
-    const double x = __longlong_as_double(((long long)((r >> 23) + 896) << 52) | ((long long)(r & 0x7FFFFFu) << 29));
-    const double e = fma(-m, x, 1.0);
-    const double y = fma(x, fma(e, e, e), x);
-    return __longlong_as_double(__double_as_longlong(y) - ((long long)(ex - 1023) << 52));
+// The block with each column scaled by 1 / sqrt(pivot) as it is reached, for pivots
+// whose reciprocal could overflow or lose bits (beyond 2^+-1000).  Returns the
+// failing column + 1, or 0.
+__device__ __noinline__ int potf2_plain(double (*S)[POTRF_NB + 1], int jb, const double *A, size_t rs, size_t cs) {
+    const int tid = threadIdx.x;
+    __syncthreads();
+    for (int e = tid; e < POTRF_NB * POTRF_NB; e += POTF2_THREADS) {
+        const int i = e % POTRF_NB, c = e / POTRF_NB;
+        S[c][i] = (i >= c && i < jb) ? A[(size_t)i * rs + (size_t)c * cs] : 0.0;
+    }
+    __syncthreads();
+    for (int t = 0; t < jb; ++t) {
+        const double a = S[t][t];
+        if (!(a > 0.0)) return t + 1;
+        const double d = sqrt(a), r = 1.0 / d;
+        __syncthreads();
+        if (tid >= t && tid < POTRF_NB) S[t][tid] = tid > t ? S[t][tid] * r : d;
+        __syncthreads();
+        for (int e = tid; e < POTRF_NB * POTRF_NB; e += POTF2_THREADS) {
+            const int i = e % POTRF_NB, c = e / POTRF_NB;
+            if (c > t && i >= c) S[c][i] = fma(-S[t][i], S[t][c], S[c][i]);
+        }
+        __syncthreads();
+    }
+    return 0;
 }
 
 __global__ void __launch_bounds__(POTF2_THREADS)
@@ -89,11 +100,11 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
     __syncthreads();
     if (s_skip) return;
     auto pivot = [&](double a, int j) {               // by a whole warp
-        const long long b = __double_as_longlong(a);
-        if (b <= 0 || b > 0x7FF0000000000000ll) {     // a <= 0 or NaN
+        // in [2^-1000, 2^1001), by its exponent and sign
+        if ((unsigned)((__double_as_longlong(a) >> 52) & 0xFFF) - 23u > 2000u) {
             if (lane == 0) s_fail = j + 1;
         } else {
-            const double p = recip(a);
+            const double p = 1.0 / a;
             if (lane == 0) s_p[j] = p;
         }
     };
@@ -101,7 +112,8 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
     __syncthreads();
     int fail = 0;
     for (int t = 0; t < jb; ++t) {
-        fail = s_fail;
+        // (a warp may see the failure of pivot t + 1, found in this step: not yet)
+        fail = s_fail == t + 1 ? t + 1 : 0;
         if (fail) break;
         if (warp < 2) {
             const int i = tid;
@@ -141,8 +153,13 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
         }
         __syncthreads();
     }
+    // a positive pivot beyond that range: the block starts again
+    const bool plain = fail && S[fail - 1][fail - 1] > 0.0;
+    if (plain) fail = potf2_plain(S, jb, A, rs, cs);
     const int ncol = fail ? fail - 1 : jb;
-    if (tid < ncol) {
+    if (plain) {
+        if (tid < POTRF_NB) s_p[tid] = 1.0;
+    } else if (tid < ncol) {
         const double a = S[tid][tid];
         S[tid][tid] = sqrt(a);
         s_p[tid] = rsqrt(a);

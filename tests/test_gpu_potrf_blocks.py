@@ -84,3 +84,41 @@ def test_failure_in_the_last_block_stays_with_its_call(cuda):
         torch.cuda.synchronize()
         assert [int(i.item()) for i in info] == [n - 2, 0]
         assert torch.equal(torch.tril(A[1]), torch.tril(want))
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("n", [2, 64, 130])
+@pytest.mark.parametrize("e", [-1064, -1020, 0, 1016])
+def test_pivots_at_the_ends_of_the_range(cuda, uplo, n, e):
+    """2^e M, M of small integers: pivots whose reciprocal overflows (e = -1064) or
+    is subnormal (e = 1016).  Same bound, plus n units of the last subnormal."""
+    r = np.random.default_rng(n)
+    M = r.integers(-1, 2, (n, n)) * (r.random((n, n)) < 0.2)
+    M = (np.tril(M, -1) + np.tril(M, -1).T + np.diag(r.integers(100, 127, n))).astype(np.float64)
+    A, info = _potrf(cuda, uplo, np.ldexp(M, e))
+    assert info == 0
+    L = A.cpu().numpy()
+    L = np.ldexp(np.tril(L) if uplo == "L" else np.triu(L).T, -(e // 2))
+    tol = 4 * n * U * (np.abs(L) @ np.abs(L).T) + n * 2.0 ** (-1074 - e)
+    assert np.all(np.abs(L @ L.T - M) <= tol)
+
+
+@pytest.mark.parametrize("uplo", "LU")
+def test_reciprocal_of_the_pivot(cuda, uplo):
+    """Blocks [d 1; 1 c] with c a little above 1/d: L22^2 = c - 1/d shows the
+    reciprocal's own error, bounded by its rounding plus the root's 2^-52 L22^2."""
+    from fractions import Fraction
+    n = 128
+    d = np.random.default_rng(3).uniform(1.0, 4.0, n // 2)
+    c = (1.0 / d) * (1.0 + 2.0 ** -20)
+    A0 = np.zeros((n, n))
+    A0[0::2, 0::2] = np.diag(d)
+    A0[1::2, 1::2] = np.diag(c)
+    A0[0::2, 1::2] = A0[1::2, 0::2] = np.eye(n // 2)
+    A, info = _potrf(cuda, uplo, A0)
+    assert info == 0
+    L22 = np.diagonal(A.cpu().numpy())[1::2]
+    for di, ci, li in zip(d, c, L22):
+        want = 1 / Fraction(float(di))
+        got = Fraction(float(ci)) - Fraction(float(li)) ** 2
+        assert abs(got - want) <= want * Fraction(1, 2 ** 53) + Fraction(float(li)) ** 2 / 2 ** 51
