@@ -41,20 +41,29 @@ constexpr int kSideSms = 16;                      // left to the side stream
 // column f it stores that pivot, writes back columns < f only and sets
 // *info = j0 + f + 1.  Does nothing when *info is already set.
 //
-// Bound: the chain of the pivots, as one FP64 instruction holds a scheduler's
-// pipe for 64 clocks and takes about 100.  The elimination therefore runs on the
-// unscaled columns, a_ic -= (a_it p_t) a_ct with p_t = 1 / pivot: two FP64
-// instructions and a reciprocal per step.  Warps 0 and 1
-// (thread per row) run that chain: in step t they bring column t + 1 up to date
-// with columns t - 1 and t, and the warp that owns the next pivot takes its
-// reciprocal.  The other 14 apply column t - 1 to the columns from t + 2 on, one
-// barrier per step.  The columns are scaled by 1 / sqrt(pivot) and the diagonal's
-// square roots taken at the end, together.  (With sqrt, divide and three barriers
-// per column on the chain a block took 93 us; this takes 57.)
-constexpr int POTF2_THREADS = 512, UPD = POTF2_THREADS / 32 - 2;
+// Bound: the chain of the pivots and the FP64 pipe behind it (a dependent FP64
+// instruction takes about 100 clocks, a warp's instruction 16 of the SM's pipe).  The
+// elimination therefore runs on the unscaled columns, a_ic -= (a_it p_t) a_ct with
+// p_t = 1 / pivot, in three stages beside each other, one barrier per step t:
+//   warp 0        column t + 1 (the half that holds its pivot) with column t, as
+//                 (a_it a_ct) p_t: the product is formed while the reciprocal before
+//                 is under way, so that one FMA and a reciprocal stand on the chain;
+//                 warp 3 its other half;
+//   warps 1, 2    column t + 2 with columns t - 1 and t;
+//   the other 8   column t - 1 to the columns from t + 3 on, which they hold in
+//                 registers in 8 x 4 tiles and store as each becomes column t + 3.
+// The columns are scaled by 1 / sqrt(pivot) and the diagonal's square roots taken at
+// the end, together.  A block takes 43 us: 4 of launch, load and store, 9 of
+// divisions.  93 with sqrt, divide and three barriers per column on the chain; 57 with
+// the trailing block in shared memory, whose masked lanes took 2560 warp FMAs instead
+// of 1500, and two FMAs and a multiplication on the chain.  More warps only lengthen
+// the barriers (512 threads: 45).
+constexpr int POTF2_THREADS = 384, UPD = POTF2_THREADS / 32 - 4;
+constexpr int TILES = 72, UPD_TILES = (TILES + UPD - 1) / UPD;      // 8 x 4 tiles that meet the triangle
 
 // The block with each column scaled by 1 / sqrt(pivot) as it is reached, for pivots
-// whose reciprocal could overflow or lose bits (beyond 2^+-1000).  Returns the
+// beyond 2^+-250: inside it neither a reciprocal nor a product of two entries of a
+// column can overflow or lose bits that matter to the rows below.  Returns the
 // failing column + 1, or 0.
 __device__ __noinline__ int potf2_plain(double (*S)[POTRF_NB + 1], int jb, const double *A, size_t rs, size_t cs) {
     const int tid = threadIdx.x;
@@ -92,68 +101,84 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
         s_skip = *info != 0;
     }
 #pragma unroll
-    for (int h = 0; h < POTRF_NB * POTRF_NB / POTF2_THREADS; ++h) {
+    for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
         const int e = h * POTF2_THREADS + tid, lo = e % POTRF_NB, hi = e / POTRF_NB;
+        if (hi >= POTRF_NB) break;
         const int i = rs == 1 ? lo : hi, c = rs == 1 ? hi : lo;
         S[c][i] = (i >= c && i < jb) ? A[(size_t)i * rs + (size_t)c * cs] : 0.0;
     }
     __syncthreads();
     if (s_skip) return;
-    auto pivot = [&](double a, int j) {               // by a whole warp
-        // in [2^-1000, 2^1001), by its exponent and sign
-        if ((unsigned)((__double_as_longlong(a) >> 52) & 0xFFF) - 23u > 2000u) {
+    // Warp 0's: p = 1 / pivot of column t, w = column t times its row t + 1
+    double p = 0.0, w = 0.0;
+    auto pivot = [&](double a, int j) {               // by warp 0
+        // in [2^-250, 2^251), by its exponent and sign
+        if ((unsigned)((__double_as_longlong(a) >> 52) & 0xFFF) - 773u > 500u) {
             if (lane == 0) s_fail = j + 1;
         } else {
-            const double p = 1.0 / a;
+            p = 1.0 / a;
             if (lane == 0) s_p[j] = p;
         }
     };
-    if (warp == 0) pivot(S[0][0], 0);
+    // the updating warps' tiles: 8 rows x 4 columns, the last columns first, so that
+    // the tiles still open in a step are the first of the list
+    double v[UPD_TILES];
+    int ti[UPD_TILES], tc[UPD_TILES];
+    if (warp >= 4) {
+#pragma unroll
+        for (int h = 0; h < UPD_TILES; ++h) {
+            const int idx = warp - 4 + UPD * h;
+            int q = 0;
+            while ((q + 1) * (q + 2) <= idx) ++q;
+            const int r = idx - q * (q + 1), far = r > q;
+            ti[h] = 8 * (7 - (far ? r - q - 1 : r)) + (lane & 7);
+            tc[h] = 4 * (15 - 2 * q - far) + (lane >> 3);
+            v[h] = idx < TILES ? S[tc[h]][ti[h]] : 0.0;
+        }
+    } else if (warp == 0) {
+        pivot(S[0][0], 0);
+    }
     __syncthreads();
     int fail = 0;
     for (int t = 0; t < jb; ++t) {
         // (a warp may see the failure of pivot t + 1, found in this step: not yet)
         fail = s_fail == t + 1 ? t + 1 : 0;
         if (fail) break;
-        if (warp < 2) {
-            const int i = tid;
+        if (warp == 0) {
             if (t + 1 < jb) {
-                const double at = S[t][t + 1];
-                double v = S[t + 1][i];
-                if (t > 0) v = fma(-Lp[(t - 1) & 1][i], S[t - 1][t + 1], v);
-                const double l = S[t][i] * s_p[t];
-                v = fma(-l, at, v);
-                if (((t + 1) >> 5) == warp) pivot(__shfl_sync(0xffffffffu, v, (t + 1) & 31), t + 1);
-                Lp[t & 1][i] = l;
-                if (i > t) S[t + 1][i] = v;
+                const int i = lane + (t + 1 < 32 ? 0 : 32);
+                if (t == 0 || t == 31) w = S[t][i] * S[t][t + 1];      // (rows 32 .. 63 from t = 31 on)
+                const double x = fma(-w, p, S[t + 1][i]);
+                pivot(__shfl_sync(0xffffffffu, x, (t + 1) & 31), t + 1);
+                if (i > t) S[t + 1][i] = x;
+                w = x * __shfl_sync(0xffffffffu, x, (t + 2) & 31);
+            }
+        } else if (warp == 3) {
+            if (t + 1 < 32) {
+                const int i = lane + 32;
+                S[t + 1][i] = fma(-(S[t][i] * s_p[t]), S[t][t + 1], S[t + 1][i]);
+            }
+        } else if (warp < 3) {
+            const int i = lane + 32 * (warp - 1);
+            const double l = S[t][i] * s_p[t];
+            Lp[t & 1][i] = l;
+            if (i >= t + 2) {
+                double y = S[t + 2][i];
+                if (t > 0) y = fma(-Lp[(t - 1) & 1][i], S[t - 1][t + 2], y);
+                S[t + 2][i] = fma(-l, S[t][t + 2], y);
             }
         } else if (t > 0) {
-            // units (column, row half) round robin over the other warps, four in
-            // flight: the loads do not wait for the stores before them
-            const int n1 = POTRF_NB - t - 2, n = n1 + (t + 2 < 32 ? 30 - t : 0);
-            const double l0 = Lp[(t - 1) & 1][lane], l1 = Lp[(t - 1) & 1][lane + 32];
-            for (int u = warp - 2; u < n; u += 4 * UPD) {
-                double *e[4], v[4], a[4];
-                bool in[4];
+            const int k = 16 - ((t + 3) >> 2), q = k >> 1, open = q * (q + 1) + (k & 1) * (q + 1);
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int w = u + UPD * h, lo = w >= n1, c = t + 2 + (lo ? w - n1 : w), i = (lo ? 0 : 32) + lane;
-                    in[h] = w < n && i >= c;
-                    e[h] = &S[in[h] ? c : 0][in[h] ? i : 0];
-                    a[h] = in[h] ? S[t - 1][c] : 0.0;
-                    v[h] = *e[h];
-                }
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    if (u + UPD * h >= n) break;
-                    v[h] = fma(-(u + UPD * h >= n1 ? l0 : l1), a[h], v[h]);
-                    if (in[h]) *e[h] = v[h];
-                }
+            for (int h = 0; h < UPD_TILES; ++h) {
+                if (warp - 4 + UPD * h >= open) break;
+                v[h] = fma(-Lp[(t - 1) & 1][ti[h]], S[t - 1][tc[h]], v[h]);
+                if (tc[h] == t + 3 && ti[h] >= t + 3) S[t + 3][ti[h]] = v[h];
             }
         }
         __syncthreads();
     }
-    // a positive pivot beyond that range: the block starts again
+    // a positive pivot beyond the range: the block starts again
     const bool plain = fail && S[fail - 1][fail - 1] > 0.0;
     if (plain) fail = potf2_plain(S, jb, A, rs, cs);
     const int ncol = fail ? fail - 1 : jb;
@@ -166,8 +191,9 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
     }
     __syncthreads();
 #pragma unroll
-    for (int h = 0; h < POTRF_NB * POTRF_NB / POTF2_THREADS; ++h) {
+    for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
         const int e = h * POTF2_THREADS + tid, lo = e % POTRF_NB, hi = e / POTRF_NB;
+        if (hi >= POTRF_NB) break;
         const int i = rs == 1 ? lo : hi, c = rs == 1 ? hi : lo;
         if (i >= c && i < jb && c < ncol)
             A[(size_t)i * rs + (size_t)c * cs] = i > c ? S[c][i] * s_p[c] : S[c][i];
@@ -244,7 +270,7 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
         }
         return kOk;
     }
-    // Look-ahead: a diagonal block is a chain of small launches (330 us for 256
+    // Look-ahead: a diagonal block is a chain of small launches (240 us for 256
     // columns), so the next one is updated first and factored on the side stream
     // while the rest of the update, whose persistent products leave it 16 SMs, runs
     // here.  n = 4000 with one right-hand side: 11.1 ms without.

@@ -122,3 +122,17 @@ def test_reciprocal_of_the_pivot(cuda, uplo):
         want = 1 / Fraction(float(di))
         got = Fraction(float(ci)) - Fraction(float(li)) ** 2
         assert abs(got - want) <= want * Fraction(1, 2 ** 53) + Fraction(float(li)) ** 2 / 2 ** 51
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("n,first", [(64, 0), (64, 1), (64, 33), (40, 39), (150, 70), (700, 300)])
+@pytest.mark.parametrize("e", [-200, 124, 126, 300])
+def test_pivots_that_cross_the_range(cuda, uplo, n, first, e):
+    """D A D with D = 2^e from row `first` on: the bound is that of A, entry by entry."""
+    d = np.where(np.arange(n) < first, 0, e)
+    A0 = np.ldexp(_spd(n, n), d[:, None] + d[None, :])
+    A, info = _potrf(cuda, uplo, A0)
+    assert info == 0
+    L = A.cpu().numpy()
+    L = np.ldexp(np.tril(L) if uplo == "L" else np.triu(L).T, -d[:, None])
+    assert np.all(np.abs(L @ L.T - np.ldexp(A0, -(d[:, None] + d[None, :]))) <= 4 * n * U * (np.abs(L) @ np.abs(L).T))
