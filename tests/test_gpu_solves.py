@@ -97,3 +97,32 @@ def test_solve_with_interchanges(cuda, n, trans, nrhs):
     op = (lambda M: M) if trans == "N" else (lambda M: M.t())  # noqa: E731
     R = (op(A0) @ X - B0).abs()
     assert bool((R <= 12 * n * U * (op(LU) @ X.abs()) + 4 * n * U * (op(A0).abs() @ X.abs())).all())
+
+
+@pytest.mark.parametrize("side,uplo,trans,diag", [("L", "L", "N", "N"), ("L", "U", "N", "U"), ("L", "L", "T", "U"),
+                                                  ("R", "U", "N", "N"), ("R", "L", "T", "N"), ("R", "L", "N", "U")])
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 33, 57, 64])
+def test_many_vectors_both_row_layouts(cuda, side, uplo, trans, diag, k):
+    """2561 vectors (cyclic rows) and the same among 6000 (consecutive rows): equal
+    bits, and the substitution's own bound."""
+    import torch
+    g = torch.Generator(device=cuda)
+    g.manual_seed(k)
+    T0 = torch.rand((k, k), generator=g, dtype=torch.float64, device=cuda) - 0.5 + 2 * torch.eye(k, dtype=torch.float64, device=cuda)
+    if k > 1:
+        T0[0, k - 1] = 0.0                             # (off the diagonal)
+    M = fg.to_colmajor(T0)
+    B = torch.rand((6000, k), generator=g, dtype=torch.float64, device=cuda) - 0.5
+    B = B if side == "R" else B.t()
+    few = B[37:2598] if side == "R" else B[:, 37:2598]
+    X, Y = fg.to_colmajor(B.clone()), fg.to_colmajor(few.clone())
+    fg.dtrsm_dev(side, uplo, trans, diag, 1.0, M, X)
+    fg.dtrsm_dev(side, uplo, trans, diag, 1.0, M, Y)
+    fg.sync()
+    assert torch.equal(Y, X[37:2598] if side == "R" else X[:, 37:2598])
+    T = torch.tril(T0) if uplo == "L" else torch.triu(T0)
+    if diag == "U":
+        T = T - torch.diag(torch.diagonal(T)) + torch.eye(k, dtype=torch.float64, device=cuda)
+    T = T.t() if trans == "T" else T
+    P, Q = (Y @ T, Y.abs() @ T.abs()) if side == "R" else (T @ Y, T.abs() @ Y.abs())
+    assert bool(((P - few).abs() <= 4 * (k + 1) * 2.0 ** -53 * (Q + few.abs())).all())
