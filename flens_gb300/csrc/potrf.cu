@@ -18,7 +18,7 @@
 // block first, which is then factored beside the rest; a diagonal block takes the
 // same three steps 64 columns at a time with potf2 of the 64 x 64 block in one CTA.
 // n = 4000 with one right-hand side: 31.6 ms with right-looking 64-column steps on
-// the FP64 pipe, 11.1 one after the other, 8.5 in this order.
+// the FP64 pipe, 11.1 one after the other, 8.3 in this order.
 //
 // Pivots, INFO and the factor agree with the reference to rounding; when
 // INFO > 0 the columns after the failing block hold partially updated values
