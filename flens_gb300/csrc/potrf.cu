@@ -25,6 +25,8 @@
 // (the reference leaves them as they were), as LAPACK leaves them undefined.
 #include "common.cuh"
 
+#include <math_constants.h>
+
 #include <cmath>
 
 namespace fg {
@@ -61,10 +63,12 @@ constexpr int kSideSms = 16;                      // left to the side stream
 constexpr int POTF2_THREADS = 384, UPD = POTF2_THREADS / 32 - 4;
 constexpr int TILES = 72, UPD_TILES = (TILES + UPD - 1) / UPD;      // 8 x 4 tiles that meet the triangle
 
-// The block with each column scaled by 1 / sqrt(pivot) as it is reached, for pivots
-// beyond 2^+-250: inside it neither a reciprocal nor a product of two entries of a
-// column can overflow or lose bits that matter to the rows below.  Returns the
-// failing column + 1, or 0.
+// The block with each column scaled by 1 / sqrt(pivot) as it is reached, so that no
+// product exceeds the square root of two diagonal entries: for pivots beyond 2^+-250,
+// and where the elimination above left an infinity or NaN.  (Between pivots in that
+// range a reciprocal is a normal number, but the unscaled product a_it a_ct of a large
+// row still overflows: [2^200 2^600; 2^600 2^1001].)  Returns the failing column + 1,
+// or 0.
 __device__ __noinline__ int potf2_plain(double (*S)[POTRF_NB + 1], int jb, const double *A, size_t rs, size_t cs) {
     const int tid = threadIdx.x;
     __syncthreads();
@@ -178,8 +182,17 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
         }
         __syncthreads();
     }
-    // a positive pivot beyond the range: the block starts again
-    const bool plain = fail && S[fail - 1][fail - 1] > 0.0;
+    // a positive pivot beyond the range, or an overflow, which stays where it arose: as
+    // an infinity or NaN in a column to be stored, -infinity on the diagonal (a NaN there
+    // alone was in A): the block starts again
+    bool redo = fail && (S[fail - 1][fail - 1] > 0.0 || S[fail - 1][fail - 1] == -CUDART_INF);
+#pragma unroll
+    for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
+        const int e = h * POTF2_THREADS + tid, i = e % POTRF_NB, c = min(e / POTRF_NB, POTRF_NB - 1);
+        const bool odd = (__double2hiint(S[c][i]) & 0x7FF00000) == 0x7FF00000;
+        redo |= odd && i >= c && (!fail || c < fail - 1);
+    }
+    const bool plain = __syncthreads_or(redo);
     if (plain) fail = potf2_plain(S, jb, A, rs, cs);
     const int ncol = fail ? fail - 1 : jb;
     if (plain) {

@@ -136,3 +136,30 @@ def test_pivots_that_cross_the_range(cuda, uplo, n, first, e):
     L = A.cpu().numpy()
     L = np.ldexp(np.tril(L) if uplo == "L" else np.triu(L).T, -d[:, None])
     assert np.all(np.abs(L @ L.T - np.ldexp(A0, -(d[:, None] + d[None, :]))) <= 4 * n * U * (np.abs(L) @ np.abs(L).T))
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("n,first", [(2, 1), (64, 1), (64, 33), (130, 20), (130, 64), (700, 300)])
+def test_rows_whose_products_overflow(cuda, uplo, n, first):
+    """D A D with D = 2^100, from row `first` on 2^500: the pivots before it are in the
+    middle of the range, the product of two entries below them is not.  The bound is
+    that of A, entry by entry."""
+    d = np.where(np.arange(n) < first, 100, 500)
+    A0 = np.ldexp(_spd(n, n), d[:, None] + d[None, :])
+    A, info = _potrf(cuda, uplo, A0)
+    assert info == 0
+    L = A.cpu().numpy()
+    L = np.ldexp(np.tril(L) if uplo == "L" else np.triu(L).T, -d[:, None])
+    assert np.all(np.abs(L @ L.T - np.ldexp(A0, -(d[:, None] + d[None, :]))) <= 4 * n * U * (np.abs(L) @ np.abs(L).T))
+
+
+@pytest.mark.parametrize("uplo", "LU")
+def test_overflow_is_not_a_failed_pivot(cuda, uplo):
+    """[2^200 2^600; 2^600 c]: positive definite for c = 2^1001, not for c = 2^999, whose
+    pivot -2^999 is stored."""
+    for c, want in ((2.0 ** 1001, 0), (2.0 ** 999, 2)):
+        A, info = _potrf(cuda, uplo, np.array([[2.0 ** 200, 2.0 ** 600], [2.0 ** 600, c]]))
+        got = A.cpu().numpy()
+        assert info == want
+        assert got[1, 1] == (2.0 ** 500 if want == 0 else -2.0 ** 999)
+        assert got[0, 0] == 2.0 ** 100 and (got[1, 0] if uplo == "L" else got[0, 1]) == 2.0 ** 500
