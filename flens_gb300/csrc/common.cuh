@@ -269,20 +269,28 @@ int dtrsm_launch_fixed(char side, char upLo, char transA, char diag, int m, int 
                        double alpha, const double *A, int ldA, double *B, int ldB,
                        const ChainFixed &fx, cudaStream_t stream);
 
+// The solve with one diagonal block (at most 64 x 64), left undone where the
+// device word *skip is set (nullptr: never).
+int dtrsm_block_launch(char side, char upLo, char transA, char diag, int m, int n,
+                       double alpha, const double *A, int ldA, double *B, int ldB,
+                       const int *skip, cudaStream_t stream);
+
 int dscal_matrix_launch(int m, int n, double alpha, double *B, int ldB,
                         cudaStream_t stream);
 
 // C <- beta*C + alpha*op(A)*op(A)^T on the uplo triangle ('L'/'U') of C,
-// trans 'N' (A n x k) or 'T' (A k x n).
+// trans 'N' (A n x k) or 'T' (A k x n); left undone where the device word *skip
+// is set (nullptr: never).
 int dsyrk_launch(char uplo, char trans, int n, int k, double alpha,
                  const double *A, int ldA, double beta, double *C, int ldC,
-                 cudaStream_t stream);
+                 cudaStream_t stream, const int *skip = nullptr);
 
 // C <- beta*C + alpha*op(A)*op(B)^T on the uplo triangle of C (trans 'N':
 // A, B n x k; 'T': k x n).
 int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha,
                     const double *A, int ldA, const double *B, int ldB,
-                    double beta, double *C, int ldC, cudaStream_t stream);
+                    double beta, double *C, int ldC, cudaStream_t stream,
+                    const int *skip = nullptr);
 
 // Level-3 BLAS on the GEMM engine (blas3.cu): trmm (B <- alpha op(A) B or
 // alpha B op(A), A triangular), symm (C <- beta C + alpha A B or alpha B A,
@@ -331,7 +339,7 @@ int dgesvx_launch(char fact, char trans, int n, int nrhs, double *A, int ldA,
 
 // Cholesky (uplo 'L': A = L L^T, 'U': A = U^T U) of the n x n uplo triangle
 // in place; *info (device) = first non-positive pivot (1-based) or 0.
-// Synchronises once per 64-column block to stop at the first failure.
+// Synchronises once per 256-column block to stop at the first failure.
 int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info,
                   cudaStream_t stream);
 

@@ -82,13 +82,15 @@ struct SlabLoader {
 // FLAG: only the tiles of the 128 x 256 blocks of C whose byte in `flag`
 // (column-major, flag_ld block rows) is set: what the residue product
 // (mod_gemm.cu) left to FP64.
+// skip (triangles only): a device word that, when set, leaves C as it is; read
+// first, tested last, so that its latency is hidden.
 template <typename T, bool TA, bool TB, int TRI = 0, int KR = 0, int TM = BM, int TN = BN, bool FLAG = false>
 __global__ void __launch_bounds__(TM < 16 ? 64 : 256)
 dgemm_fma_kernel(int m, int n, int k, T alpha,
                  const T *__restrict__ A, int ldA,
                  const T *__restrict__ B, int ldB,
                  T beta, T *__restrict__ C, int ldC, const uint8_t *__restrict__ flag = nullptr,
-                 int flag_ld = 0) {
+                 int flag_ld = 0, const int *__restrict__ skip = nullptr) {
     constexpr int TX = TM < 16 ? TM : 16, TY = TN < 16 ? TN : 16, NT = TX * TY;   // threads
     constexpr int RI = TM / TX, RJ = TN / TY;
     __shared__ T As[2][BK][TM + PAD];
@@ -102,6 +104,7 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     }
     if (TRI == 1 && m0 + TM <= n0) return;       // tile strictly above the diagonal
     if (TRI == 2 && n0 + TN <= m0) return;       // tile strictly below the diagonal
+    const bool stop = TRI && !FLAG && skip && *skip;
 
     SlabLoader<T, !TA, TM, NT> la;
     SlabLoader<T, TB, TN, NT> lb;
@@ -151,6 +154,7 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     // included, so the multiply is skipped -- one FP64 instruction fewer per
     // element on a pipe that bounds the kernel
     const bool beta1 = beta == T(1);
+    if (stop) return;
 #pragma unroll
     for (int j = 0; j < RJ; ++j) {
         const int gj = n0 + ty + TY * j;
@@ -735,9 +739,11 @@ int dgemm_kr_launch(char transA, char transB, int m, int n, int k, double alpha,
 // C <- beta*C + alpha*op(A)*op(B)^T on the uplo triangle of the n x n C, op
 // = identity (trans 'N': A, B n x k) or transpose ('T': A, B k x n); only the
 // uplo triangle of C is read or written.  k == 0 only scales (unless beta ==
-// 1).  No alpha == 0 shortcut: the reference's syrk/syr2k have none.
+// 1).  No alpha == 0 shortcut: the reference's syrk/syr2k have none.  skip: a
+// device word that leaves C as it is when it is set (FP64 kernel only).
 int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const double *A, int ldA,
-                    const double *B, int ldB, double beta, double *C, int ldC, cudaStream_t stream) {
+                    const double *B, int ldB, double beta, double *C, int ldC, cudaStream_t stream,
+                    const int *skip) {
     if (n == 0) return kOk;
     if (k == 0) {
         if (beta == 1.0) return kOk;
@@ -745,7 +751,7 @@ int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const dou
     }
     const bool lower = uplo == 'L' || uplo == 'l';
     const bool nt = trans == 'N' || trans == 'n';
-    if (k > 0 && alpha != 0.0) {
+    if (k > 0 && alpha != 0.0 && !skip) {
         const int st = mod_gemm_launch(nt ? 'N' : 'T', nt ? 'T' : 'N', n, n, k, alpha, A, ldA, B, ldB, beta, C, ldC,
                                        lower ? 1 : 2, stream);
         if (st != kErrUnsupported) return st;
@@ -766,10 +772,10 @@ int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const dou
     const dim3 gt(ceil_div(n, tile), ceil_div(n, tile));
 #define FG_TRI(TA_, TB_, TRI_)                                                                                 \
     do {                                                                                                       \
-        if (tile == 8) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 8, 8><<<gt, 64, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
-        else if (tile == 16) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 16, 16><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
-        else if (tile == 32) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
-        else dgemm_fma_kernel<double, TA_, TB_, TRI_><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC); \
+        if (tile == 8) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 8, 8><<<gt, 64, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC, nullptr, 0, skip); \
+        else if (tile == 16) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 16, 16><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC, nullptr, 0, skip); \
+        else if (tile == 32) dgemm_fma_kernel<double, TA_, TB_, TRI_, 0, 32, 32><<<gt, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC, nullptr, 0, skip); \
+        else dgemm_fma_kernel<double, TA_, TB_, TRI_><<<grid, 256, 0, stream>>>(n, n, k, alpha, Ak, lda, Bk, ldb, beta, C, ldC, nullptr, 0, skip); \
     } while (0)
     if (lower) {
         if (nt) FG_TRI(false, true, 1);
@@ -786,9 +792,9 @@ int tri_gemm_launch(char uplo, char trans, int n, int k, double alpha, const dou
 // C <- beta*C + alpha*op(A)*op(A)^T on the uplo triangle of the n x n C
 // (cxxblas/level3/syrk.tcc:42-90): op(A) = A (n x k, trans 'N') or A^T.
 int dsyrk_launch(char uplo, char trans, int n, int k, double alpha, const double *A, int ldA,
-                 double beta, double *C, int ldC, cudaStream_t stream) {
+                 double beta, double *C, int ldC, cudaStream_t stream, const int *skip) {
     trace("syrk %c%c n=%d k=%d", uplo, trans, n, k);
-    return tri_gemm_launch(uplo, trans, n, k, alpha, A, ldA, A, ldA, beta, C, ldC, stream);
+    return tri_gemm_launch(uplo, trans, n, k, alpha, A, ldA, A, ldA, beta, C, ldC, stream, skip);
 }
 
 int dgemm_launch(char transA, char transB, int m, int n, int k, double alpha,
@@ -832,11 +838,11 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
     FG_CUDA(cudaLaunchKernelEx(&cfg,                                                                       \
                                small ? dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, 32, 32, true>         \
                                      : dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, BM, BN, true>,        \
-                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld))
+                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld, (const int *)nullptr))
 #define FG_FL(TA_, TB_, TRI_) FG_FLK(TA_, TB_, TRI_, 0)
 #define FG_FLK64(TA_, TB_, KR_)                                                                            \
     FG_CUDA(cudaLaunchKernelEx(&cfg, dgemm_fma_kernel<double, TA_, TB_, 0, KR_, BM, BN, true>,             \
-                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld))
+                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld, (const int *)nullptr))
 #define FG_FLR(TA_, TB_) switch (kr) { case 1: FG_FLK64(TA_, TB_, 1); break; case 2: FG_FLK64(TA_, TB_, 2); break; \
                                        case 3: FG_FLK64(TA_, TB_, 3); break; default: FG_FLK64(TA_, TB_, 4); }
     if (kr) {

@@ -21,8 +21,9 @@
 // the FP64 pipe, 11.1 one after the other, 8.3 in this order.
 //
 // Pivots, INFO and the factor agree with the reference to rounding; when
-// INFO > 0 the columns after the failing block hold partially updated values
-// (the reference leaves them as they were), as LAPACK leaves them undefined.
+// INFO > 0 the columns from the failing 64-column step on hold the updates of all
+// whole steps before it and nothing else but the columns of its own 64 x 64 block
+// before the pivot (the reference leaves them as they were, LAPACK undefined).
 #include "common.cuh"
 
 #include <math_constants.h>
@@ -253,8 +254,9 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
         return lower ? dgemm_launch('N', 'T', nr, nc, w, -1.0, at(r0, j), ldA, at(c0, j), ldA, 1.0, at(r0, c0), ldA, q)
                      : dgemm_launch('T', 'N', nc, nr, w, -1.0, at(c0, j), ldA, at(r0, j), ldA, 1.0, at(r0, c0), ldA, q);
     };
-    // A diagonal block of up to POTRF_BASE columns, right-looking in steps of 64 (after
-    // a failed pivot the remaining steps skip).
+    // A diagonal block of up to POTRF_BASE columns, right-looking in steps of 64.  After
+    // a failed pivot its step's solve and update, and the steps behind it, leave the
+    // matrix as it is (by *info, on the device).
     auto diagonal = [&](int j, int w, cudaStream_t q) -> int {
         for (int c = 0; c < w; c += POTRF_NB) {
             const int jb = w - c < POTRF_NB ? w - c : POTRF_NB, rest = w - c - jb;
@@ -263,11 +265,27 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
                 potf2_kernel<<<1, POTF2_THREADS, 0, q>>>(jb, at(j + c, j + c), rs, cs, j + c, info);
                 FG_CUDA(cudaGetLastError());
             }
-            int st;
-            if (rest > 0 && (st = solve_rows(j + c, jb, j + c + jb, rest, q)) != kOk) return st;
-            if (rest > 0 && (st = update_diag(j + c, jb, j + c + jb, rest, q)) != kOk) return st;
+            if (rest <= 0) break;
+            const int c0 = j + c, r0 = c0 + jb;
+            int st = lower ? dtrsm_block_launch('R', 'L', 'T', 'N', rest, jb, 1.0, at(c0, c0), ldA, at(r0, c0), ldA, info, q)
+                           : dtrsm_block_launch('L', 'U', 'T', 'N', jb, rest, 1.0, at(c0, c0), ldA, at(r0, c0), ldA, info, q);
+            if (st != kOk) return st;
+            if ((st = dsyrk_launch(lower ? 'L' : 'U', lower ? 'N' : 'T', rest, jb, -1.0, at(r0, c0), ldA, 1.0,
+                                   at(r0, r0), ldA, q, info)) != kOk)
+                return st;
         }
         return kOk;
+    };
+    // The block of width w at j failed in column f: what its whole 64-column steps
+    // before f mean for the rows below it and the columns behind them, so that the
+    // matrix is left as if the step of f had been the first not taken.
+    auto finish = [&](int j, int w, int f) -> int {
+        const int w0 = (f - j) / POTRF_NB * POTRF_NB, e = j + w, c0 = j + w0;
+        if (w0 == 0 || e == n) return kOk;
+        int st = solve_rows(j, w0, e, n - e, s);
+        if (st == kOk) st = update_below(j, w0, c0, e - c0, e, n - e, s);
+        if (st == kOk) st = update_diag(j, w0, e, n - e, s);
+        return st;
     };
     if (n <= 2 * POTRF_BASE) {
         // few blocks: one after the other; INFO is read back after each but the last
@@ -277,7 +295,7 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
             if (st != kOk || rest == 0) return st;
             FG_CUDA(cudaMemcpyAsync(h, info, sizeof(int), cudaMemcpyDeviceToHost, s));
             FG_CUDA(cudaStreamSynchronize(s));
-            if (*h != 0) return kOk;           // as potrf.tcc:104-107 stops
+            if (*h != 0) return finish(j, w, *h - 1);           // as potrf.tcc:104-107 stops
             if ((st = solve_rows(j, w, j + w, rest, s)) != kOk) return st;
             if ((st = update_diag(j, w, j + w, rest, s)) != kOk) return st;
         }
@@ -310,7 +328,7 @@ int dpotrf_launch(char uplo, int n, double *A, int ldA, int *info, cudaStream_t 
             open = false;
             if (e == n) break;
             FG_CUDA(cudaEventSynchronize(wo->ev_back));
-            if (*h != 0) break;                   // as potrf.tcc:104-107 stops
+            if (*h != 0) return finish(j, w, *h - 1);           // as potrf.tcc:104-107 stops
             const int w2 = n - e < POTRF_BASE ? n - e : POTRF_BASE, e2 = e + w2;
             if ((st = solve_rows(j, w, e, w2, s)) != kOk) return st;
             if ((st = update_diag(j, w, e, w2, s)) != kOk) return st;

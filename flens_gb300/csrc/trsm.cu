@@ -347,9 +347,11 @@ int trsm_warp_max() {
 template <typename T, bool LOWER, bool UNIT>
 __global__ void __launch_bounds__(32 * TRSM_WARP_VECS)
 trsm_diag_warp_kernel(int nb, const T *__restrict__ M0, long long mi, long long mp,
-                      T *__restrict__ X0, long long xs, long long vs, int nvec) {
+                      T *__restrict__ X0, long long xs, long long vs, int nvec,
+                      const int *__restrict__ skip) {
     __shared__ T Ms[TRSM_NB][TRSM_NB + 1];     // Ms[i][r] = M(r, i)
     __shared__ T rinv[TRSM_NB];
+    const bool stop = skip && *skip;           // (tested at the end: its latency is hidden)
     const int lane = threadIdx.x & 31;
     const long long v = (long long)blockIdx.x * TRSM_WARP_VECS + (threadIdx.x >> 5);
     T *x = X0 + v * vs;
@@ -374,6 +376,7 @@ trsm_diag_warp_kernel(int nb, const T *__restrict__ M0, long long mi, long long 
         xb = fma(-Ms[oa + i][ob + lane], __shfl_sync(0xffffffffu, xa, i), xb);
     }
     solve32<LOWER, !UNIT>(xb, Ms, ob, rinv);
+    if (stop) return;
     if (r0 < nb) x[r0 * xs] = x0;
     if (r1 < nb) x[r1 * xs] = x1;
 }
@@ -607,11 +610,11 @@ bool chain_enabled() {
 
 template <typename T>
 int launch_diag(int kb, const T *M0, long long mi, long long mp, bool lowerM, bool unit,
-                T *X0, long long xs, long long vs, int nvec, cudaStream_t stream) {
+                T *X0, long long xs, long long vs, int nvec, const int *skip, cudaStream_t stream) {
     KTimer kt(kFamTrsm, stream, (double)kb * kb * nvec, 16.0 * (double)kb * nvec);
-    if (nvec <= trsm_warp_max()) {
+    if (nvec <= trsm_warp_max() || skip) {     // (only this kernel looks at skip)
         const int grid = ceil_div(nvec, TRSM_WARP_VECS);
-#define FG_WARP(L, U) trsm_diag_warp_kernel<T, L, U><<<grid, 32 * TRSM_WARP_VECS, 0, stream>>>(kb, M0, mi, mp, X0, xs, vs, nvec)
+#define FG_WARP(L, U) trsm_diag_warp_kernel<T, L, U><<<grid, 32 * TRSM_WARP_VECS, 0, stream>>>(kb, M0, mi, mp, X0, xs, vs, nvec, skip)
         if (lowerM) { if (unit) FG_WARP(true, true); else FG_WARP(true, false); }
         else { if (unit) FG_WARP(false, true); else FG_WARP(false, false); }
 #undef FG_WARP
@@ -656,7 +659,7 @@ int gemm_t<float>(char ta, char tb, int m, int n, int k, float alpha, const floa
 template <typename T>
 int trsm_launch_t(char side, char upLo, char transA, char diag, int m, int n,
                   T alpha, const T *A, int ldA, T *B, int ldB, cudaStream_t stream,
-                  const ChainFixed *fx = nullptr) {
+                  const ChainFixed *fx = nullptr, const int *skip = nullptr) {
     if (m == 0 || n == 0) return kOk;
     const bool left = (side == 'L' || side == 'l');
     const bool lowerA = (upLo == 'L' || upLo == 'l');
@@ -724,7 +727,7 @@ int trsm_launch_t(char side, char upLo, char transA, char diag, int m, int n,
         const int k0 = bi * TRSM_NB;
         const int kb = (ka - k0) < TRSM_NB ? (ka - k0) : TRSM_NB;
         int st0 = launch_diag<T>(kb, A + k0 * mi + k0 * mp, mi, mp, lowerM, unit != 0, B + k0 * xs, xs,
-                              vs, nvec, stream);
+                              vs, nvec, skip, stream);
         if (st0 != kOk) return st0;
         // rows still to solve: below the block (lower) or above it (upper)
         const int r0 = lowerM ? k0 + kb : 0;
@@ -756,6 +759,12 @@ int trsm_launch_t(char side, char upLo, char transA, char diag, int m, int n,
 int dtrsm_launch(char side, char upLo, char transA, char diag, int m, int n, double alpha,
                  const double *A, int ldA, double *B, int ldB, cudaStream_t stream) {
     return trsm_launch_t<double>(side, upLo, transA, diag, m, n, alpha, A, ldA, B, ldB, stream);
+}
+
+int dtrsm_block_launch(char side, char upLo, char transA, char diag, int m, int n, double alpha,
+                       const double *A, int ldA, double *B, int ldB, const int *skip, cudaStream_t stream) {
+    if (((side == 'L' || side == 'l') ? m : n) > TRSM_NB || alpha != 1.0) return kErrUnsupported;
+    return trsm_launch_t<double>(side, upLo, transA, diag, m, n, alpha, A, ldA, B, ldB, stream, nullptr, skip);
 }
 
 int dtrsm_launch_fixed(char side, char upLo, char transA, char diag, int m, int n, double alpha,

@@ -163,3 +163,32 @@ def test_overflow_is_not_a_failed_pivot(cuda, uplo):
         assert info == want
         assert got[1, 1] == (2.0 ** 500 if want == 0 else -2.0 ** 999)
         assert got[0, 0] == 2.0 ** 100 and (got[1, 0] if uplo == "L" else got[0, 1]) == 2.0 ** 500
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("n,f", [(64, 10), (200, 0), (200, 70), (256, 255), (300, 130), (500, 200), (513, 300),
+                                 (700, 63), (700, 64), (700, 250), (700, 400), (700, 699)])
+def test_what_a_failed_pivot_leaves(cuda, uplo, n, f):
+    """A(f, f) = -2: rows and columns behind the failing 64-column step hold A minus the
+    updates of the whole steps before it, its own block's columns behind f are as they
+    were, and no quotient by the failing pivot is anywhere.  Each entry is one sum of at
+    most n products: 2 n 2^-53 (|A| + |L||L^T|)."""
+    A0 = _spd(n, 7)
+    A0[f, f] = -2.0
+    A, info = _potrf(cuda, uplo, A0)
+    assert info == f + 1
+    got = A.cpu().numpy()
+    got = np.tril(got) if uplo == "L" else np.triu(got).T
+    c = f // 64 * 64
+    b = min(c + 64, n)                                 # the failing step's block: rows and columns c .. b - 1
+    L = got[:, :c]
+    want = np.tril(A0 - L @ L.T)
+    want[:, :c] = 0.0
+    tol = 2 * n * U * (np.abs(A0) + np.abs(L) @ np.abs(L).T)
+    rest = np.tril(np.ones((n, n), dtype=bool))
+    rest[:, :c] = False
+    rest[c:b, c:f + 1] = False                         # written by the step itself
+    assert np.all(np.abs(got - want)[rest] <= tol[rest])
+    # the leading columns: L L^T = A in all rows before the step's, and below
+    lead = np.tril(np.ones((n, n), dtype=bool))[:, :c]
+    assert np.all((np.abs(L @ L.T - A0)[:, :c] <= tol[:, :c])[lead])
