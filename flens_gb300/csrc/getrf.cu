@@ -1542,6 +1542,20 @@ int panel_ctas(int sms) {
     return cap;
 }
 
+// Rows per CTA of a grid panel of mp rows, and its width: the reference's 64,
+// narrowed only if a CTA's rows would not fit in shared memory (very tall
+// matrices, few CTAs); 0 when no column does.
+int grid_panel_rows(int mp, int gcap) {
+    const int R = ceil_div(mp, gcap);
+    return R < PANEL_RMIN ? PANEL_RMIN : R;
+}
+int grid_panel_width(int mp, int gcap, size_t elem_bytes) {
+    const size_t R = (size_t)grid_panel_rows(mp, gcap);
+    int nb = PANEL_NB;
+    while (nb > 0 && R * nb * elem_bytes > PANEL_SMEM_MAX) nb >>= 1;
+    return nb;
+}
+
 // SMs left to the side stream's cluster panel.
 constexpr int kClusterSms = CP_CS;
 
@@ -1708,15 +1722,25 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
     const bool fp64_split = split_nb > 0 && tc_kind < 0;
     // look-ahead over outer blocks: its lists of row moves and the side stream's
     // operands, after ours too.  The blocks of the tensor-core LU are split_nb wide:
-    // tc_buf is sized for updates of that depth.  (onb bounded: the lists have room
-    // for 32 panels of a block, 32 wide at least; m, because beyond 8192 rows, FP32
-    // 16,384, panels need the whole grid and nothing runs beside them.)
-    int onb = !recursive ? 0 : tc_kind >= 0 ? split_nb : lookahead_nb(mn);
-    if (m > 20000 || onb > 1024) onb = 0;
+    // tc_buf is sized for updates of that depth.  (m bounded: panels of more than 8192
+    // rows, FP32 16,384, need the whole grid and nothing runs beside them.  onb bounded
+    // by the lists: a block has room for kLists panels, and the narrowest are those of
+    // the whole height, half of 64 columns as a cluster's or what a grid's CTAs hold.)
+    int sms = num_sms();
+    if (sms <= 0) {
+        set_last_error("no CUDA device");
+        return kErrNoDevice;
+    }
+    const int gcap = panel_ctas(sms);
     const bool f32 = std::is_same<T, float>::value && panel32_enabled();   // FP32 panels, else FP64 arithmetic
     const bool cluster = !(std::is_same<T, float>::value && !f32) && cluster_fits<T>();
-    const bool ahead_blocks = onb > 0 && mn > 2 * onb && cluster && lookahead_enabled();
+    // (panel_kernel holds the panel in FP64, panel32_kernel in FP32)
+    const size_t panel_es = f32 ? sizeof(float) : sizeof(double);
     constexpr int kLists = 1024 / CP_NARROW, kListInts = 2 + 4 * PANEL_NB;
+    int onb = !recursive ? 0 : tc_kind >= 0 ? split_nb : lookahead_nb(mn);
+    const int narrowest = std::min(grid_panel_width(m, gcap, panel_es), CP_NARROW);
+    if (m > 20000 || narrowest == 0 || onb > kLists * narrowest) onb = 0;
+    const bool ahead_blocks = onb > 0 && mn > 2 * onb && cluster && lookahead_enabled();
     const size_t list_bytes = ((size_t)2 * kLists * kListInts * sizeof(int) + 255) / 256 * 256;
     const size_t side_bytes = tc_kind >= 0 ? tc_update_workspace_bytes(tc_kind, m, onb, PANEL_NB) : 0;
     Workspace *w = workspace_for(stream, fp64_split     ? split_off + split_ws0_bytes(m, n)
@@ -1736,12 +1760,6 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
         if (st0 == kOk) st0 = set_smem_once(f32 ? once_fd : once_d, panel_fn[1], (int)PANEL_SMEM_MAX);
         if (st0 != kOk) return st0;
     }
-    int sms = num_sms();
-    if (sms <= 0) {
-        set_last_error("no CUDA device");
-        return kErrNoDevice;
-    }
-    const int gcap = panel_ctas(sms);
     // look-ahead (CUDA-core updates only: the tensor-core update is a
     // persistent kernel that leaves no SM free for a concurrent panel; with
     // its operand ring cut to 3 stages so that a panel CTA fits beside it, the
@@ -1783,15 +1801,9 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
             *jb_out = jb;
             return kOk;
         }
-        int R = ceil_div(mp, gcap);
-        if (R < PANEL_RMIN) R = PANEL_RMIN;
-        // panel width: the reference's 64, narrowed only if a CTA's rows
-        // would not fit in shared memory (very tall matrices)
-        // (panel_kernel holds the panel in FP64, panel32_kernel in FP32)
-        const size_t es = f32 ? sizeof(float) : sizeof(double);
-        int nb = PANEL_NB;
-        while (nb > 1 && (size_t)R * nb * es > PANEL_SMEM_MAX) nb >>= 1;
-        if ((size_t)R * nb * es > PANEL_SMEM_MAX) {
+        int R = grid_panel_rows(mp, gcap);
+        const int nb = grid_panel_width(mp, gcap, panel_es);
+        if (nb == 0) {
             set_last_error("getrf: m=%d too tall for the shared-memory panel", m);
             return kErrUnsupported;
         }
@@ -1801,7 +1813,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
         T *Ap = A + j + (size_t)j * ldA;
         int *status = w->status;
         int j0 = j;
-        size_t smem = (size_t)R * jb * es;
+        size_t smem = (size_t)R * jb * panel_es;
         ++epoch;
         void *args[] = {&Ap, &ldA, &mp, &jb, &j0, &ipiv, &info, &status, &ps, &R, &epoch};
         KTimer ktp(kFamPanel, s, (double)mp * jb * jb - (double)jb * jb * jb / 3.0,
@@ -1856,6 +1868,10 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
         if (w <= PANEL_NB || std::is_same<T, float>::value) {
             // (a panel of a very tall matrix comes out narrower)
             ob_end = j + w;
+            if (k.lists && k.nl >= kLists) {
+                set_last_error("getrf: more than %d panels in a block", kLists);
+                return kErrUnsupported;
+            }
             const PanelScratch &pl = k.lists ? k.lists[k.nl] : ps;
             if ((st = panel_at(j, k.s, &jb, true, pl, k.beside)) != kOk) return st;
             ++k.nl;
