@@ -61,12 +61,13 @@ __device__ __forceinline__ void stage_block(T (*D)[TRSM_NB + 1], const T *__rest
 // solve, the only user, the error of a solve (n = 100 to 1000, against extended
 // precision) is 0.8 to 0.9 of the unscaled kernel's it replaced.  Only where no scaled entry leaves [2^-900, 2^900]
 // (or is zero already): `scaled` is false otherwise and the block stays as it was.
+// Only the solved triangle decides (LOWER: r > p): the other one may hold anything.
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
 __device__ __forceinline__ bool mid_range(double x) {
     const int e = exp_field(x);
     return e >= 1023 - 900 && e <= 1023 + 900;
 }
-template <int NT, typename T>
+template <int NT, bool LOWER, typename T>
 __device__ __forceinline__ bool scale_rows(T (*D)[TRSM_NB + 1], const T *rinv) {
     if (sizeof(T) != 8) return false;
     constexpr int PER = TRSM_NB * TRSM_NB / NT;
@@ -77,7 +78,7 @@ __device__ __forceinline__ bool scale_rows(T (*D)[TRSM_NB + 1], const T *rinv) {
         const int e = j * NT + threadIdx.x, r = e % TRSM_NB, p = e / TRSM_NB;
         v[j] = D[p][r] * rinv[r];
         ok &= mid_range((double)rinv[r]);
-        if (p != r) ok &= mid_range((double)v[j]) || (__double_as_longlong((double)D[p][r]) << 1) == 0;
+        if (LOWER ? r > p : r < p) ok &= mid_range((double)v[j]) || (__double_as_longlong((double)D[p][r]) << 1) == 0;
     }
     if (!__syncthreads_and(ok)) return false;
 #pragma unroll
@@ -459,7 +460,7 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
     if (!UNIT) {
         if (tid < CH_NB) rinv[tid] = tid < kb ? T(1) / Md[tid][tid] : T(1);
         __syncthreads();
-        scaled = scale_rows<CH_THREADS>(Md, rinv);
+        scaled = scale_rows<CH_THREADS, LOWER>(Md, rinv);
     }
 
     for (int s2 = 0; s2 < s; ++s2) {

@@ -46,6 +46,20 @@ def test_trsm_few(cuda, n, nvec, uplo, kind):
         _residual_ok(A if trans == "N" else A.T, X, B)
 
 
+@pytest.mark.parametrize("n", [65, 130, 200])
+@pytest.mark.parametrize("nvec", [1, 4])
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("other", [np.nan, 5e-324, 2.0 ** -950, -2.0 ** 1000])
+def test_other_triangle_decides_nothing(cuda, n, nvec, uplo, other):
+    for trans in "NT":
+        A = _tri(n, uplo, "plain", n)
+        B = oracle.uniform(n + 9, n, nvec)
+        want = fg.dtrsm("L", uplo, trans, "N", 1.0, A, B.copy(order="F"))
+        low = np.tril(np.ones((n, n), dtype=bool))
+        A[~low if uplo == "L" else ~low.T] = other
+        assert np.array_equal(fg.dtrsm("L", uplo, trans, "N", 1.0, A, B.copy(order="F")), want)
+
+
 def test_large_right_hand_side_that_cancels(cuda):
     """b / diagonal overflows, the solution does not."""
     n = 100
