@@ -114,22 +114,27 @@ __device__ __forceinline__ void solve32_any(T &x, const T (*D)[TRSM_NB + 1], int
     else solve32<LOWER, true>(x, D, o, rinv);
 }
 
-// Right-hand sides of a warp's vector for the scaled block: b' = rinv b.  Where
-// that could overflow although x does not (|b'| >= 2^1000), the vector is solved
-// times 2^-200; returns what x is to be multiplied by.
+// Finite in all lanes (FP64: the exponents of two values, below 2^(limit + 1)).
 template <typename T>
-__device__ __forceinline__ T scale_rhs(T &x0, T &x1, T r0, T r1) {
-    const T y0 = x0 * r0, y1 = x1 * r1;
-    const bool ok = exp_field((double)y0) <= 1023 + 1000 && exp_field((double)y1) <= 1023 + 1000;
-    if (__all_sync(0xffffffffu, ok)) {
-        x0 = y0;
-        x1 = y1;
-        return T(1);
+__device__ __forceinline__ bool all_below(T a, T b, int limit) {
+    return __all_sync(0xffffffffu, exp_field((double)a) <= 1023 + limit && exp_field((double)b) <= 1023 + limit);
+}
+
+// One warp's vector by the plain substitution with the block as it is in memory: for
+// a finite right-hand side that the scaled block takes beyond the range, in b' = rinv b
+// (then at least 2^1001) or in a sum.  x0, x1: rows lane and lane + 32.
+template <bool LOWER, typename T>
+__device__ __noinline__ void solve_unscaled(T &x0, T &x1, const T *M, long long mi, long long mp, int kb,
+                                            const T *rinv) {
+    const int lane = threadIdx.x & 31;
+    for (int s = 0; s < kb; ++s) {
+        const int i = LOWER ? s : kb - 1 - s;
+        const T xi = __shfl_sync(0xffffffffu, i < 32 ? x0 : x1, i & 31) * rinv[i];
+        if (lane == (i & 31)) (i < 32 ? x0 : x1) = xi;
+        if ((LOWER ? lane > i : lane < i) && lane < kb) x0 = fma(-M[lane * mi + i * mp], xi, x0);
+        const int r = lane + 32;
+        if ((LOWER ? r > i : r < i) && r < kb) x1 = fma(-M[r * mi + i * mp], xi, x1);
     }
-    const double sc = 6.223015277861142e-61;      // 2^-200
-    x0 = (T)(((double)x0 * sc) * (double)r0);
-    x1 = (T)(((double)x1 * sc) * (double)r1);
-    return (T)1.6069380442589903e60;              // 2^200
 }
 
 // Solves the kb x kb (kb <= 64) diagonal block M for 32 vectors per CTA.
@@ -509,7 +514,8 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
     // instructions per step on one scheduler's pipe: 11.5 us a block, now about 6.)
     const int warp = tid >> 5, lane = tid & 31;
     const int oa = LOWER ? 0 : 32, ob = 32 - oa;
-    T xa = T(0), xb = T(0), back = T(1);
+    T xa = T(0), xb = T(0), ba = T(0), bb = T(0);      // solution, right-hand side
+    bool plain = false;
     if (warp < nvec) {
         const T *x = X0 + warp * vs + (long long)R0 * xs;
         auto rhs = [&](int rr) -> T {
@@ -518,7 +524,13 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
         };
         xa = rhs(oa + lane);
         xb = rhs(ob + lane);
-        if (scaled) back = scale_rhs(xa, xb, rinv[oa + lane], rinv[ob + lane]);
+        ba = xa;
+        bb = xb;
+        if (scaled) {
+            xa *= rinv[oa + lane];
+            xb *= rinv[ob + lane];
+            plain = !all_below(xa, xb, 1000) && all_below(ba, bb, 1023);
+        }
         solve32_any<LOWER, UNIT>(xa, Md, oa, rinv, scaled);
         xk[warp][oa + lane] = xa;
     }
@@ -536,8 +548,14 @@ trsv_chain_kernel(int ka, const T *__restrict__ M0, long long mi, long long mp, 
         xb -= (part[0][warp][lane] + part[1][warp][lane]) + (part[2][warp][lane] + part[3][warp][lane]);
         solve32_any<LOWER, UNIT>(xb, Md, ob, rinv, scaled);
         T *x = X0 + warp * vs + (long long)R0 * xs;
-        if (oa + lane < kb) x[(oa + lane) * xs] = back != T(1) ? xa * back : xa;
-        if (ob + lane < kb) x[(ob + lane) * xs] = back != T(1) ? xb * back : xb;
+        if (scaled && (plain || (!all_below(xa, xb, 1023) && all_below(ba, bb, 1023)))) {
+            T &lo = LOWER ? ba : bb, &hi = LOWER ? bb : ba;
+            solve_unscaled<LOWER>(lo, hi, M0 + R0 * (mi + mp), mi, mp, kb, rinv);
+            xa = ba;
+            xb = bb;
+        }
+        if (oa + lane < kb) x[(oa + lane) * xs] = xa;
+        if (ob + lane < kb) x[(ob + lane) * xs] = xb;
     }
     __syncthreads();
     if (tid == 0) ch_release(&flags[s], epoch);

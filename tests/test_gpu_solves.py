@@ -78,6 +78,36 @@ def test_large_right_hand_side_that_cancels(cuda):
     _residual_ok(A, X, B)
 
 
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("at", [0, 40, 64, 100])
+def test_small_entries_beside_a_large_quotient(cuda, uplo, at):
+    """Diagonal matrix, exact quotients: one of 2^1010, the others near 2^-900."""
+    n = 130
+    d, x = np.ones(n), np.full(n, 2.0 ** -900)
+    d[at], x[at] = 2.0 ** -500, 2.0 ** 1010
+    x *= 1.0 + np.arange(n) / 1024.0
+    X = fg.dtrsm("L", uplo, "N", "N", 1.0, np.asfortranarray(np.diag(d)), (d * x)[:, None].copy(order="F"))
+    assert np.array_equal(X[:, 0], x)
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("row,cols", [(20, (3, 7)), (50, (3, 7)), (50, (7, 40)), (90, (66, 70)), (127, (66, 120))])
+def test_terms_that_cancel_beyond_the_scaled_range(cuda, uplo, row, cols):
+    """2^250 (2^200 - 2^200) + 2^-600 x = 2^399, exact in FP64 in any order: no sum
+    overflows but in the rows over their diagonal (2^1050)."""
+    n = 130
+    A, B, want = np.eye(n), np.ones((n, 2)), np.ones((n, 2))
+    A[row, row] = 2.0 ** -600
+    A[row, cols[0]], A[row, cols[1]] = 2.0 ** 250, -2.0 ** 250
+    B[list(cols)] = want[list(cols)] = 2.0 ** 200
+    B[row] = 2.0 ** 399
+    want[row] = 2.0 ** 999
+    if uplo == "U":
+        A, B, want = A[::-1, ::-1], B[::-1], want[::-1]
+    X = fg.dtrsm("L", uplo, "N", "N", 1.0, np.asfortranarray(A), np.asfortranarray(B))
+    assert np.array_equal(X, want)
+
+
 def test_infinite_right_hand_side(cuda):
     n = 96
     A = _tri(n, "L", "plain", 5)
