@@ -94,6 +94,28 @@ def test_wide_entries(cuda, E):
         assert err.max() <= (4.5 if E <= 8 else np.sqrt(k) + 4.5)
 
 
+@pytest.mark.parametrize("m,n,k", [(300, 300, 1024), (300, 300, 513), (257, 300, 1025), (200, 270, 2048), (150, 300, 3072)])
+def test_sums_at_the_edge_of_fp32(cuda, m, n, k):
+    """Rows and columns constant but for their last entry, with odd significands of as
+    many bits (53, from k = 1025 on 52) as make every residue modulo 256 one of 128: a
+    full chunk's sum is 2^24 in magnitude.  The operands are exact, the result is the
+    sum rounded once."""
+    r = np.random.default_rng(k)
+    bits = 53 if k <= 1024 else 52
+
+    def odd(size):
+        v = (r.integers(1 << (bits - 2), 1 << (bits - 1), size) * 2 + 1).astype(np.float64)
+        return v * 2.0 ** -bits * np.where(r.random(size) < 0.5, -1.0, 1.0)
+
+    A, B = np.repeat(odd((m, 1)), k, 1), np.repeat(odd((1, n)), k, 0)
+    A[:, -1], B[-1] = odd(m), odd(n)
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, np.zeros((m, n)))
+    assert used >= 5
+    a, a1, b, b1 = ([Fraction(x) for x in v.tolist()] for v in (A[:, 0], A[:, -1], B[0], B[-1]))
+    for i in range(m):
+        assert got[i].tolist() == [float((k - 1) * a[i] * b[j] + a1[i] * b1[j]) for j in range(n)]
+
+
 def _refused(cuda, A, B, C, alpha=1.0, beta=1.0):
     k = A.shape[1]
     got, used = _gemm(cuda, "N", "N", alpha, A, B, beta, C)
