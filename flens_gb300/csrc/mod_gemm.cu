@@ -12,8 +12,8 @@
 //  2. residues: a_ik is rounded to the integer X_ik = rint(a_ik 2^(beta-e_i)),
 //     |X| <= 2^beta, and stored as its NM = 17 centred residues modulo
 //     pairwise coprime p <= 256 (exact in BF16); likewise op(B).  beta is the
-//     largest with 2^(2 beta) k <= P/4, P = prod p ~ 2^133, at most 61: 61 for
-//     k <= 512, 59 for k = 4096 -- 6 to 8 bits more than FP64's significand.
+//     largest with 2^(2 beta) k <= P/4, P = prod p ~ 2^132, at most 61: 61 for
+//     k <= 256, 59 for k = 4096 -- 6 to 8 bits more than FP64's significand.
 //  3. products: one BF16 tensor-core GEMM per modulus.  |r r'| <= 2^14, so the
 //     FP32 sums of 1024 products are exact integers; longer k is cut into such
 //     chunks whose residues are added.  17 products where the digit form
@@ -28,8 +28,14 @@
 // |a_ik||b_kj| 2^(-e_i-f_j) from below, and their sums s_i, t_j over k are taken with
 // the residues.  Rounding the operands changes c_ij by at most
 // 2^(-beta-1) (s_i + t_j) 2^(e_i+f_j); a tile is accepted only if that is below
-// 4 * 2^-53 * (|A||B|)_ij for all its elements with Q_ij != 0 -- FP64's own bound is
-// k * 2^-53 * (|A||B|)_ij.  Uniform entries and LU and Cholesky updates keep 4 to 6 bits
+// 4 * 2^-53 * (|A||B|)_ij for all its elements with Q_ij != 0, and below 2^-53 *
+// (|A||B|)_ij where the nonzeros of row i and column j do not make sure that five terms
+// of the sum are nonzero.  With the rounding of the sum that is never more than FP64's
+// own bound, (number of nonzero terms) * 2^-53 * (|A||B|)_ij; and a product of one
+// term is exact but for that rounding, as in FP64: an entry that beta bits do not hold
+// is below 2^(52-beta) of its row's range, its product with b_kj below 2^(52-beta)
+// |b_kj| <= 2^(52-beta) t_j, and the second condition fails.
+// Uniform entries and LU and Cholesky updates keep 4 to 6 bits
 // of margin, entries u 2^e with e in [-16, 16] about one.  Tiles of data graded beyond
 // that, and tiles with non-finite rows or exponents outside +-450, are left to
 // the FP64 kernel, which runs last and skips all others: no readback, the
@@ -38,6 +44,7 @@
 
 #include <cuda_bf16.h>
 
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 
@@ -129,7 +136,7 @@ struct Operand {
     const double *X;
     int ld, R, rcontig;                      // rcontig: element (r, k) at X[r + k ld], else X[k + r ld]
     unsigned *key;                           // row maxima: high word of |x|
-    unsigned *sum;                           // row sums of the magnitudes, in 2^-16
+    unsigned long long *sum;                 // rows: sum of the magnitudes in 2^-16, nonzeros << 32
     __nv_bfloat16 *planes;                   // NP planes of R rows x Kp
 };
 
@@ -321,11 +328,15 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
             }
         }
         __nv_bfloat16 *out = o.planes + (size_t)r * Kp + (k0 + kq);
-        // (integer sums: the same in any order)
+        // (integer sums: the same in any order; 64 entries: the sum below 2^23, their
+        // number above it)
         unsigned sum = __float2uint_ru(((mg[0] + mg[1]) + (mg[2] + mg[3])) * 65536.0f);
 #pragma unroll
+        for (int i = 0; i < 4; ++i) sum += mg[i] != 0.0f ? 1u << 24 : 0u;
+#pragma unroll
         for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFu << (lane & 16), sum, off);
-        if ((lane & 15) == 0 && sum) atomicAdd(&o.sum[r], sum);
+        if ((lane & 15) == 0 && sum)
+            atomicAdd(&o.sum[r], ((unsigned long long)(sum >> 24) << 32) | (sum & 0xFFFFFFu));
         uint2 w0;
         w0.x = bf16x2(f2(make_float2(mg[0], mg[1])));
         w0.y = bf16x2(f2(make_float2(mg[2], mg[3])));
@@ -389,10 +400,12 @@ __device__ __forceinline__ void tile_at(const TileMap &tm, int t, int &m0, int &
 struct ModArgs {
     TileMap tiles;
     int nkb;                                  // 64-deep k blocks
-    float qscale;                             // smallest accepted Q: this times (s_i + t_j)
+    float qscale;                             // smallest accepted Q: this times (s_i + t_j), or 4
+    int dense;                                // times it: fewer nonzeros in row and column together
     uint8_t *res;                             // residues [modulus][tile][4-column group][row][4]
     uint8_t *flag;                            // per tile (row tile + tm * column tile): 1 = left to FP64
-    const unsigned *keyA, *keyB, *sumA, *sumB;
+    const unsigned *keyA, *keyB;
+    const unsigned long long *sumA, *sumB;
     float p[NM], ip[NM];
 };
 
@@ -547,12 +560,15 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             uint32_t st[MULTI ? 32 : 1];
             bool bad = false;
             float si = 0.0f, tj[2] = {0.0f, 0.0f};
+            int ni = INT_MAX / 2, nj[2] = {INT_MAX / 2, INT_MAX / 2};        // (no nonzero: Q = 0)
             if (mag) {                               // rows' and columns' data, before the wait
                 bool ok = true;
                 if (m0 + rl < M) {
                     key_exp(a.keyA[m0 + rl], ok);
                     bad |= !ok;
-                    si = (float)a.sumA[m0 + rl];
+                    const unsigned long long w = a.sumA[m0 + rl];
+                    si = (float)(unsigned)w;
+                    if (w) ni = (int)(w >> 32);
                 }
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
@@ -560,7 +576,9 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     if (col < N) {
                         key_exp(a.keyB[col], ok);
                         bad |= !ok;
-                        tj[cc] = (float)a.sumB[col];
+                        const unsigned long long w = a.sumB[col];
+                        tj[cc] = (float)(unsigned)w;
+                        if (w) nj[cc] = (int)(w >> 32);
                     }
                 }
             }
@@ -581,10 +599,13 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     uint32_t r[32];
                     tmem_ld32(base + (uint32_t)c0, r);
                     if (mag) {
+                        // (the sparsest of the 32 columns decides for all)
+                        const int nmin = ni + (int)__reduce_min_sync(0xffffffffu, (unsigned)nj[cc]);
+                        const float qs = nmin >= a.dense ? a.qscale : 4.0f * a.qscale;
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float q = __uint_as_float(r[j]);
-                            const float qmin = (si + __shfl_sync(0xffffffffu, tj[cc], j)) * a.qscale;
+                            const float qmin = (si + __shfl_sync(0xffffffffu, tj[cc], j)) * qs;
                             bad |= m0 + rl < M && n0 + c0 + j < N && q < qmin && q != 0.0f;
                         }
                     } else {
@@ -788,8 +809,8 @@ Layout layout_for(int m, int n, int Kp, const TileMap &t) {
     l.keyA = 0;
     l.keyB = up256((size_t)m * 4);
     l.sumA = l.keyB + up256((size_t)n * 4);
-    l.sumB = l.sumA + up256((size_t)m * 4);
-    l.flag = l.sumB + up256((size_t)n * 4);
+    l.sumB = l.sumA + up256((size_t)m * 8);
+    l.flag = l.sumB + up256((size_t)n * 8);
     l.zeroed = l.flag + up256((size_t)t.tm * t.tn);
     l.planesA = l.zeroed;
     l.planesB = l.planesA + up256((size_t)NP * m * Kp * 2);
@@ -812,9 +833,9 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     while ((1 << lk) < k) ++lk;
     int bits = (cs.log2P - 2 - lk) / 2;
     if (bits > 61) bits = 61;
-    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (unsigned *)(ws + l.sumA),
+    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (unsigned long long *)(ws + l.sumA),
                      (__nv_bfloat16 *)(ws + l.planesA)};
-    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (unsigned *)(ws + l.sumB),
+    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (unsigned long long *)(ws + l.sumB),
                      (__nv_bfloat16 *)(ws + l.planesB)};
     FG_CUDA(cudaMemsetAsync(ws, 0, l.zeroed, s));
     {
@@ -837,6 +858,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     a.nkb = Kp / KBLK;
     // 2^(-bits-1) (s + t) <= 2^-51 Q; the magnitudes were rounded down by up to 2^-7
     a.qscale = (float)(1.01 * ldexp(1.0, 50 - bits - 16));
+    a.dense = k + 5;
     a.res = (uint8_t *)(ws + l.res);
     a.flag = (uint8_t *)(ws + l.flag);
     a.keyA = oa.key;

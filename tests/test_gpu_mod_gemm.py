@@ -116,6 +116,40 @@ def test_sums_at_the_edge_of_fp32(cuda, m, n, k):
         assert got[i].tolist() == [float((k - 1) * a[i] * b[j] + a1[i] * b1[j]) for j in range(n)]
 
 
+@pytest.mark.parametrize("k", [200, 300, 1000, 1500])
+@pytest.mark.parametrize("e", [-13, -11, -10, -9, -8, -7, -6, -5, -1])
+@pytest.mark.parametrize("swap", [False, True])
+def test_products_of_one_term_are_exact(cuda, k, e, swap):
+    """A I and I A for A bidiagonal, 1 on the diagonal and 53-bit entries in [2^e,
+    2^(e+1)) beside it: the FP64 sum is A itself."""
+    r = np.random.default_rng(k - e)
+    A = np.eye(k)
+    A[np.arange(k - 1), np.arange(1, k)] = np.ldexp(1.0 + r.integers(0, 1 << 52, k - 1) * 2.0 ** -52, e)
+    A, B = (np.eye(k), A) if swap else (A, np.eye(k))
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, np.zeros((k, k)))
+    assert used >= 5 or k < 300
+    assert np.array_equal(got, B if swap else A)
+
+
+def test_few_terms_keep_the_fp64_bound(cuda):
+    """Rows of A with 1 to 6 nonzeros in a 300^3 product: n nonzero terms, n * 2^-53 *
+    |A||B| in each element."""
+    r = np.random.default_rng(11)
+    m = n = k = 300
+    B = r.uniform(0.25, 1.0, (k, n))
+    A = np.zeros((m, k))
+    for i in range(m):
+        at = r.choice(k, 1 + i % 6, replace=False)
+        A[i, at] = r.uniform(0.5, 1.0, at.size) * 2.0 ** -r.integers(0, 10, at.size)
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, 0.0, np.zeros((m, n)))
+    assert used >= 5
+    for i in range(m):
+        at = np.flatnonzero(A[i])
+        for j in range(0, n, 7):
+            terms = [Fraction(float(A[i, x])) * Fraction(float(B[x, j])) for x in at]
+            assert abs(Fraction(float(got[i, j])) - sum(terms)) <= at.size * Fraction(1, 1 << 53) * sum(terms)
+
+
 def _refused(cuda, A, B, C, alpha=1.0, beta=1.0):
     k = A.shape[1]
     got, used = _gemm(cuda, "N", "N", alpha, A, B, beta, C)
