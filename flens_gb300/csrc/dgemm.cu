@@ -816,35 +816,36 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
 
 // The FP64 kernel on the flagged 128 x 256 blocks of C only (tri 1/2: within
 // the lower/upper triangle; kr as dgemm_kr_launch): the tiles a residue product
-// refused.
+// refused, in the tiles that the whole product would take (512 x 64 x 512 with all
+// refused: 171 us in 32 x 32 tiles; the FP64 product alone takes 47).
 int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
                          int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
                          const uint8_t *flag, int flag_ld, int kr, cudaStream_t stream) {
     const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
     KTimer kt(kFamGemm, stream, 0.0, 0.0);
-    const dim3 g64(ceil_div(m, BM), ceil_div(n, BN)), g32(ceil_div(m, 32), ceil_div(n, 32));
     // (k ranges depend on the tile: the one dgemm_kr_launch takes)
-    const bool small = !kr && (long long)g64.x * g64.y < 4LL * num_sms();
+    const int tile = kr ? BM : fp64_tile(m, n, tri ? 0.5 : 1.0);
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = small ? g32 : g64;
-    cfg.blockDim = dim3(256);
+    cfg.gridDim = dim3(ceil_div(m, tile), ceil_div(n, tile));
+    cfg.blockDim = dim3(tile < 16 ? 64 : 256);
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-#define FG_FLK(TA_, TB_, TRI_, KR_)                                                                        \
-    FG_CUDA(cudaLaunchKernelEx(&cfg,                                                                       \
-                               small ? dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, 32, 32, true>         \
-                                     : dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, BM, BN, true>,        \
-                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld, (const int *)nullptr))
-#define FG_FL(TA_, TB_, TRI_) FG_FLK(TA_, TB_, TRI_, 0)
-#define FG_FLK64(TA_, TB_, KR_)                                                                            \
-    FG_CUDA(cudaLaunchKernelEx(&cfg, dgemm_fma_kernel<double, TA_, TB_, 0, KR_, BM, BN, true>,             \
-                               m, n, k, alpha, A, ldA, B, ldB, beta, C, ldC, flag, flag_ld, (const int *)nullptr))
-#define FG_FLR(TA_, TB_) switch (kr) { case 1: FG_FLK64(TA_, TB_, 1); break; case 2: FG_FLK64(TA_, TB_, 2); break; \
-                                       case 3: FG_FLK64(TA_, TB_, 3); break; default: FG_FLK64(TA_, TB_, 4); }
+#define FG_FLK(TA_, TB_, TRI_, KR_, T_)                                                                    \
+    FG_CUDA(cudaLaunchKernelEx(&cfg, dgemm_fma_kernel<double, TA_, TB_, TRI_, KR_, T_, T_, true>, m, n, k, alpha, A, \
+                               ldA, B, ldB, beta, C, ldC, flag, flag_ld, (const int *)nullptr))
+#define FG_FL(TA_, TB_, TRI_)                                                                              \
+    switch (tile) {                                                                                        \
+        case 8: FG_FLK(TA_, TB_, TRI_, 0, 8); break;                                                       \
+        case 16: FG_FLK(TA_, TB_, TRI_, 0, 16); break;                                                     \
+        case 32: FG_FLK(TA_, TB_, TRI_, 0, 32); break;                                                     \
+        default: FG_FLK(TA_, TB_, TRI_, 0, 64);                                                            \
+    }
+#define FG_FLR(TA_, TB_) switch (kr) { case 1: FG_FLK(TA_, TB_, 0, 1, 64); break; case 2: FG_FLK(TA_, TB_, 0, 2, 64); break; \
+                                       case 3: FG_FLK(TA_, TB_, 0, 3, 64); break; default: FG_FLK(TA_, TB_, 0, 4, 64); }
     if (kr) {
         if (!ta && !tb) { FG_FLR(false, false) }
         else if (ta && !tb) { FG_FLR(true, false) }
@@ -852,14 +853,13 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
         else { FG_FLR(true, true) }
         return kOk;
     }
-#define FG_FLT(TA_, TB_) do { if (tri == 1) FG_FL(TA_, TB_, 1); else if (tri == 2) FG_FL(TA_, TB_, 2); else FG_FL(TA_, TB_, 0); } while (0)
-    if (!ta && !tb) FG_FL(false, false, 0);      // a triangle's product has one transposed operand
+#define FG_FLT(TA_, TB_) do { if (tri == 1) FG_FL(TA_, TB_, 1) else if (tri == 2) FG_FL(TA_, TB_, 2) else FG_FL(TA_, TB_, 0) } while (0)
+    if (!ta && !tb) FG_FL(false, false, 0)       // a triangle's product has one transposed operand
     else if (ta && !tb) FG_FLT(true, false);
     else if (!ta && tb) FG_FLT(false, true);
-    else FG_FL(true, true, 0);
+    else FG_FL(true, true, 0)
 #undef FG_FLT
 #undef FG_FLR
-#undef FG_FLK64
 #undef FG_FL
 #undef FG_FLK
     return kOk;
