@@ -27,7 +27,8 @@
 // product of the magnitudes (rounded down to BF16) bounds Q_ij = sum_k
 // |a_ik||b_kj| 2^(-e_i-f_j) from below, and their sums s_i, t_j over k are taken with
 // the residues.  Rounding the operands changes c_ij by at most
-// 2^(-beta-1) (s_i + t_j) 2^(e_i+f_j); a tile is accepted only if that is below
+// 2^(-beta-1) (s_i + t_j) 2^(e_i+f_j), s_i and t_j at most the number of nonzeros of
+// column j and row i (the other entries meet zeros); a tile is accepted only if that is below
 // 4 * 2^-53 * (|A||B|)_ij for all its elements with Q_ij != 0, and below 2^-53 *
 // (|A||B|)_ij where the nonzeros of row i and column j do not make sure that five terms
 // of the sum are nonzero.  With the rounding of the sum that is never more than FP64's
@@ -560,7 +561,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
             uint32_t st[MULTI ? 32 : 1];
             bool bad = false;
             float si = 0.0f, tj[2] = {0.0f, 0.0f};
-            int ni = INT_MAX / 2, nj[2] = {INT_MAX / 2, INT_MAX / 2};        // (no nonzero: Q = 0)
+            int ni = 0, nj[2] = {0, 0};              // nonzeros
             if (mag) {                               // rows' and columns' data, before the wait
                 bool ok = true;
                 if (m0 + rl < M) {
@@ -568,7 +569,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     bad |= !ok;
                     const unsigned long long w = a.sumA[m0 + rl];
                     si = (float)(unsigned)w;
-                    if (w) ni = (int)(w >> 32);
+                    ni = (int)(w >> 32);
                 }
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
@@ -578,7 +579,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                         bad |= !ok;
                         const unsigned long long w = a.sumB[col];
                         tj[cc] = (float)(unsigned)w;
-                        if (w) nj[cc] = (int)(w >> 32);
+                        nj[cc] = (int)(w >> 32);
                     }
                 }
             }
@@ -599,13 +600,16 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     uint32_t r[32];
                     tmem_ld32(base + (uint32_t)c0, r);
                     if (mag) {
-                        // (the sparsest of the 32 columns decides for all)
-                        const int nmin = ni + (int)__reduce_min_sync(0xffffffffu, (unsigned)nj[cc]);
-                        const float qs = nmin >= a.dense ? a.qscale : 4.0f * a.qscale;
+                        // (the sparsest of the 32 columns, but for those of zeros, and the
+                        // densest decide for all)
+                        const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)nj[cc]);
+                        const int least = (int)__reduce_min_sync(0xffffffffu, nj[cc] ? (unsigned)nj[cc] : 1u << 30);
+                        const float qs = ni + least >= a.dense ? a.qscale : 4.0f * a.qscale;
+                        const float sx = fminf(si, 65536.0f * (float)most), tx = 65536.0f * (float)ni;
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float q = __uint_as_float(r[j]);
-                            const float qmin = (si + __shfl_sync(0xffffffffu, tj[cc], j)) * qs;
+                            const float qmin = (sx + fminf(__shfl_sync(0xffffffffu, tj[cc], j), tx)) * qs;
                             bad |= m0 + rl < M && n0 + c0 + j < N && q < qmin && q != 0.0f;
                         }
                     } else {
