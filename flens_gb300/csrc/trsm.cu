@@ -591,6 +591,11 @@ int launch_chain(int ka, const T *M0, long long mi, long long mp, bool lowerM, b
     } else {
         int st = workspace_flags(stream, nblk, &flags, &epoch);
         if (st != kOk) return st;
+        // a recorded launch publishes the same epoch at every replay: cleared before each
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) cudaGetLastError();
+        if (cap != cudaStreamCaptureStatusNone)
+            FG_CUDA(cudaMemsetAsync(flags, 0, sizeof(unsigned long long) * nblk, stream));
         Workspace *w = workspace_for(stream, 0);
         if (!w) return kErrAlloc;
         status = w->status;
