@@ -823,7 +823,9 @@ Layout layout_for(int m, int n, int Kp, const TileMap &t) {
     return l;
 }
 
-constexpr int kBlkK = 4096, kBlkMN = 4096;        // one block product at most: 1.5 GB of scratch
+// One block product at most: 1.5 GB of scratch (two operands' planes 1.2 GB, residues
+// 0.3), or 8192 x 8192 with k = 1024: 1.8 GB (0.6 and 1.1).
+constexpr int kBlkK = 4096, kBlkMN = 4096;
 
 // One block product in the scratch `ws` (layout_for(m, n, Kp, tiles).total bytes).
 int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int ldA,
@@ -945,15 +947,15 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
         const int parts = ceil_div(x, cap_);
         return ceil_div(ceil_div(x, parts), unit) * unit;
     };
-    // (k ranges of refused tiles are counted from the whole operand: one block)
-    const int kb = kr ? ceil_div(k, KBLK) * KBLK : part(k, kBlkK, KBLK);
+    // (a triangular operand in the same parts along both its dimensions: its blocks are
+    // zero, triangles, or full)
+    const int kb = part(k, kBlkK, kr ? NT : KBLK);
     // a shallow product may take larger blocks of C for the same scratch
-    const int capMN = kb <= 1024 ? 2 * kBlkMN : kBlkMN;
-    const int mb = kr ? ceil_div(m, NT) * NT : part(m, capMN, NT), nb = kr ? ceil_div(n, NT) * NT : part(n, capMN, NT);
+    const int capMN = !kr && kb <= 1024 ? 2 * kBlkMN : kBlkMN;
+    const int mb = kr == 1 || kr == 2 ? kb : part(m, capMN, NT), nb = kr >= 3 ? kb : part(n, capMN, NT);
     const int mm = mb < m ? mb : m, nn = nb < n ? nb : n, kk = kb < k ? kb : k;
     const Layout l = layout_for(mm, nn, ceil_div(kk, KBLK) * KBLK,
                                 make_tiles(mm, nn, tri && mb >= m && nb >= n ? tri : 0));
-    if (kr && l.total > ((size_t)4 << 30)) return kErrUnsupported;
     int *status = nullptr;
     char *ws = (char *)scratch_acquire(l.total, s, &status);
     if (!ws) return kErrUnsupported;
@@ -968,10 +970,19 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
                     if ((tri == 1) != (i0 > j0)) continue;     // the other triangle
                     bt = 0;
                 }
+                int bkr = 0;
+                bool first = k0 == 0;
+                if (kr) {
+                    const int t0 = kr <= 2 ? i0 : j0;
+                    const bool from = kr == 1 || kr == 4;      // nonzero for k >= the row or column, else k <=
+                    if (from ? k0 < t0 : k0 > t0) continue;
+                    bkr = k0 == t0 ? kr : 0;
+                    if (from) first = k0 == t0;
+                }
                 const int bk = k - k0 < kb ? k - k0 : kb;
                 rc = mod_block(ta, tb, bm, bn, bk, alpha, A + (ta ? k0 + (size_t)i0 * ldA : i0 + (size_t)k0 * ldA),
                                ldA, B + (tb ? j0 + (size_t)k0 * ldB : k0 + (size_t)j0 * ldB), ldB,
-                               k0 == 0 ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, kr, ws, status, s);
+                               first ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, bkr, ws, status, s);
             }
     scratch_release(ws, s);
     return rc;

@@ -63,3 +63,24 @@ def test_infinities_reach_what_they_reached(cuda, tmp_path):
     want, got = np.load(path), run_special()
     for k in got:
         assert np.array_equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("side", "LR")
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("trans", "NT")
+def test_triangle_in_parts_is_exact(cuda, side, uplo, trans):
+    """4200 rows: two parts of the triangle, whose blocks are zero, triangles or full.
+    Integers, so the result is the product itself; what lies in the other triangle is
+    never part of it."""
+    ka, other = 4200, 300
+    r = np.random.default_rng(ka)
+    A = np.asfortranarray(r.integers(-999, 1000, (ka, ka)).astype(np.float64))
+    B = np.asfortranarray(r.integers(-999, 1000, (ka, other) if side == "L" else (other, ka)).astype(np.float64))
+    T = np.tril(A) if uplo == "L" else np.triu(A)
+    T = T if trans == "N" else T.T
+    want = T @ B if side == "L" else B @ T
+    A[~(np.tril(np.ones((ka, ka), dtype=bool)) if uplo == "L" else np.triu(np.ones((ka, ka), dtype=bool)))] = np.nan
+    before = fg.lib().flens_gb300_launch_count()
+    fg.dtrmm(side, uplo, trans, "N", 1.0, A, B)
+    assert fg.lib().flens_gb300_launch_count() - before >= 10
+    assert np.array_equal(B, want)
