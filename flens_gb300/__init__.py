@@ -542,5 +542,12 @@ def dgesv_dev(A, ipiv, B, info, stream=None):
     return B
 
 
+def scratch_trim(keep: int = 0) -> None:
+    """Give the product scratch that no call is using back to the device, but for `keep` bytes."""
+    f = lib().flens_gb300_scratch_trim
+    f.restype, f.argtypes = ctypes.c_int, [ctypes.c_size_t]
+    _check(f(keep), "flens_gb300_scratch_trim")
+
+
 def sync(stream=None) -> None:
     _check(lib().flens_gb300_sync(_stream(stream)), "flens_gb300_sync")

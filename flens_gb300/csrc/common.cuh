@@ -94,9 +94,10 @@ int workspace_flags(cudaStream_t stream, int n, unsigned long long **flags,
 
 // Scratch for one sequence of launches on `stream`, taken from and given back
 // to a device's memory pool in stream order (cudaMallocAsync), so calls on the
-// same stream from several threads have their own.  The pool keeps at most
-// kScratchKeep bytes between synchronisations and is destroyed at unload.
-// nullptr when there is no memory (the last error is not set: the callers have
+// same stream from several threads have their own.  At a synchronisation the pool
+// gives back what is free beyond kScratchKeep bytes; those it keeps until
+// flens_gb300_scratch_trim or unload.  (No call takes more than 1.8 GB: repeated calls
+// between synchronisations find their memory there.)  nullptr when there is no memory (the last error is not set: the callers have
 // a way without).  *status: the stream's device status word.
 constexpr size_t kScratchKeep = (size_t)2 << 30;
 void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status);

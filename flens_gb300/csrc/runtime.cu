@@ -294,6 +294,15 @@ void scratch_release(void *p, cudaStream_t stream) {
     if (p && cudaFreeAsync(p, stream) != cudaSuccess) cudaGetLastError();
 }
 
+// Free memory of the pools beyond `keep` bytes each back to the devices.
+static int scratch_trim(size_t keep) {
+    Registry &r = registry();
+    std::lock_guard<std::mutex> lock(r.mu);
+    for (auto &kv : r.pools)
+        if (kv.second) FG_CUDA(cudaMemPoolTrimTo(kv.second, keep));
+    return kOk;
+}
+
 int set_smem_once(DeviceOnce &once, const void *fn, int bytes) {
     if (!once.pending()) return kOk;
     FG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
@@ -376,6 +385,8 @@ FG_API const char *flens_gb300_last_error(void) { return fg::t_last_error; }
 
 // Device allocations (cudaMalloc) the library has made since load.
 FG_API long long flens_gb300_device_alloc_count(void) { return fg::g_dev_allocs.load(); }
+
+FG_API int flens_gb300_scratch_trim(size_t keep) { return fg::scratch_trim(keep); }
 
 // Test hook: the next `count` device allocations of the library fail as an
 // out-of-memory cudaMalloc would (count <= 0 clears the hook).

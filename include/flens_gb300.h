@@ -197,8 +197,8 @@ void xerbla_(const char *SRNAME, const int *INFO, int SRNAME_LEN);
  * formed on the tensor cores from exact residues, where a check on the data, on
  * the device, keeps the rounding of the operands below 4 * 2^-53 * |A||B|; tiles
  * it refuses, small products, streams under capture and calls without memory for
- * the scratch (at most about 2.7 GB, from a pool in stream order) take the FP64
- * kernel.  FLENS_GB300_DGEMM=fma in the environment selects that for all. */
+ * the scratch (at most 1.8 GB, from a pool in stream order: see
+ * flens_gb300_scratch_trim) take the FP64 kernel.  FLENS_GB300_DGEMM=fma in the environment selects that for all. */
 int flens_gb300_dgemm(char transA, char transB, int m, int n, int k,
                       double alpha, const double *A, int ldA,
                       const double *B, int ldB, double beta, double *C,
@@ -453,6 +453,12 @@ int flens_gb300_blas_status(void);
 /* Diagnostics, no counterpart in the reference.  Device allocations
  * (cudaMalloc) the library has made since it was loaded. */
 long long flens_gb300_device_alloc_count(void);
+
+/* The products' scratch comes from a memory pool per device, which at a
+ * synchronisation keeps up to 2 GiB of it for the next call.  This gives what no call
+ * is using back to the devices, but for `keep` bytes of each pool, for a program
+ * that shares the GPU; work still running keeps its own.  Any thread, any time. */
+int flens_gb300_scratch_trim(size_t keep);
 
 /* Test hook for the allocation-failure paths: the next `count` device
  * allocations of the library fail as an out-of-memory cudaMalloc would, so

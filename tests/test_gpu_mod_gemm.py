@@ -272,3 +272,21 @@ def test_threads_on_one_stream(cuda):
     s.synchronize()
     for (a, b), (_, _, c) in zip(ops, dev):
         assert np.array_equal(c.cpu().numpy(), a @ b)
+
+
+def test_scratch_given_back(cuda):
+    """After a synchronisation the pool keeps the scratch of a product (512 MB and more
+    at 3000^3); trimmed, that is free again, and the next call takes it anew."""
+    import torch
+    r = np.random.default_rng(12)
+    A, B = (_dev(cuda, r.integers(-9, 10, (3000, 3000)).astype(float)) for _ in range(2))
+    C = [_dev(cuda, np.zeros((3000, 3000))) for _ in range(2)]
+    fg.dgemm_dev("N", "N", 1.0, A, B, 0.0, C[0])
+    fg.sync()
+    kept = torch.cuda.mem_get_info()[0]
+    fg.scratch_trim()
+    assert torch.cuda.mem_get_info()[0] - kept >= 500 << 20
+    fg.dgemm_dev("N", "N", 1.0, A, B, 0.0, C[1])
+    fg.scratch_trim()                                 # the running call keeps its own
+    fg.sync()
+    assert torch.equal(C[0], C[1])
