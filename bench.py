@@ -262,6 +262,47 @@ def gemm_subbench(torch, fg, dev, reps=10):
             "tflops": 2.0 * n ** 3 / (ms * 1e-3) / 1e12, "l2": "flushed between reps"}
 
 
+def roofline(fam, steps, ms, n, pipe_peak, cublas_peak):
+    """The family that takes most of a step's time, against what bounds it; and the
+    residue products (all their kernels: exponents, residues, products, reconstruction,
+    refused tiles) against the BF16 peak over the 18 products that make one."""
+    if not fam:
+        return None
+    dom, d = max(fam.items(), key=lambda kv: kv[1]["ms"])
+    ratios = {}
+    path = os.path.join(ROOT, "profiles", "traffic.json")
+    if os.path.exists(path):
+        with open(path) as f:
+            ratios = json.load(f)
+    bf16, bf16_src = measured_peak("bf16_tflops")
+
+    def entry(name, bound, peak, peak_source):
+        e = fam[name]
+        achieved = e["flops"] / (e["ms"] * 1e-3) / 1e12
+        # DRAM bytes per launch: the measured DRAM / algorithmic ratio of this
+        # family times its algorithmic bytes per launch in this run
+        ratio = ratios.get(name, {}).get("dram_over_algorithmic")
+        return {"kernel": name, "bound": bound, "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+                "frac": achieved / peak if peak else None, "share_of_step": e["ms"] / ms,
+                "traffic": ratio * e["bytes"] / e["launches"] if ratio and e["launches"] else None,
+                "peak_source": peak_source}
+
+    fp64_src = (f"FP64 pipe, 2 DFMA/clk/SM at the sampled clock ({pipe_peak:.3f}); cuBLAS dgemm 8192^3 in this "
+                f"run {cublas_peak}")
+    residues_src = f"{bf16_src} bf16_tflops {bf16} / 18"
+    if dom == "dgemm_residues":
+        out = entry(dom, "bf16_tensor_18_products", bf16 / 18.0, residues_src)
+    elif dom == "lu_panel":
+        # one column after another: the pipe's rate is not what bounds it
+        out = entry(dom, "latency", pipe_peak, fp64_src)
+        out["us_per_column"] = d["ms"] * 1e3 / (steps * n)
+    else:
+        out = entry(dom, "fp64_pipe", max(p for p in (cublas_peak, pipe_peak) if p), fp64_src)
+    if "dgemm_residues" in fam and dom != "dgemm_residues":
+        out["residues"] = entry("dgemm_residues", "bf16_tensor_18_products", bf16 / 18.0, residues_src)
+    return out
+
+
 def our_arm(args, rank: int, world: int) -> None:
     import numpy as np
     import torch
@@ -373,36 +414,7 @@ def our_arm(args, rank: int, world: int) -> None:
         sm_mhz = result["clocks"].get("sm_mhz") or 2070.0
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         pipe_peak = 2 * 2 * sms * sm_mhz * 1e6 / 1e12
-        peak = max(p for p in (cublas_peak, pipe_peak) if p)
-        dom = max(fam.items(), key=lambda kv: kv[1]["ms"])[0] if fam else None
-        if dom:
-            d = fam[dom]
-            achieved = d["flops"] / (d["ms"] * 1e-3) / 1e12
-            # DRAM bytes per launch: the ncu-measured DRAM/algorithmic ratio of
-            # this kernel (profiles/traffic.json) times its per-launch
-            # algorithmic bytes in this run
-            traffic = None
-            tpath = os.path.join(ROOT, "profiles", "traffic.json")
-            if os.path.exists(tpath):
-                ratio = json.load(open(tpath)).get(dom, {}).get("dram_over_algorithmic")
-                if ratio and d["launches"]:
-                    traffic = ratio * d["bytes"] / d["launches"]
-            # FP64 products by exact residues: 18 BF16 products per FP64 one
-            residues = dom == "dgemm_fp64" and not os.environ.get("FLENS_GB300_DGEMM")
-            bf16, bf16_src = measured_peak("bf16_tflops")
-            if residues:
-                peak = bf16 / 18.0
-            result["roofline"] = {
-                "kernel": dom, "bound": "bf16_tensor_18_products" if residues else "fp64_pipe",
-                "achieved": achieved, "peak": peak,
-                "unit": "TFLOP/s", "frac": (achieved / peak) if peak else None,
-                "traffic": traffic,
-                "peak_source": (f"{bf16_src} bf16_tflops {bf16} / 18 (MEASURED_PEAKS.json)") if residues else ("max of cuBLAS FP64 dgemm 8192^3 measured in this run "
-                                f"({cublas_peak}) and the FP64 pipe issue rate 2 DFMA/clk/SM x "
-                                f"{sms} SMs x {sm_mhz} MHz ({pipe_peak:.3f}); MEASURED_PEAKS.json "
-                                "has no FP64 entry and tcgen05 has no f64 kind"),
-                "share_of_step": d["ms"] / ms_fam,
-                "algorithmic": "2*m*n*k flops per trailing-update/trsm GEMM launch"}
+        result["roofline"] = roofline(fam, fam_steps, ms_fam, n, pipe_peak, cublas_peak)
         if not args.quick:
             result["gemm_fp64_config1"] = gemm_subbench(torch, fg, dev)
         if not args.quick and not args.no_mixed:

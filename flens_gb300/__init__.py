@@ -163,7 +163,7 @@ def last_error() -> str:
 
 
 # ------------------------------------------------------ instrumentation ---
-N_FAMILIES = 12
+N_FAMILIES = 13
 
 
 def launch_count() -> int:

@@ -143,7 +143,7 @@ void trace(const char *fmt, ...);
 // CUDA event pair around it on the launching stream together with the
 // launch's algorithmic flops and bytes.
 enum Family : int {
-    kFamGemm = 0,     // FP64 GEMM (trailing updates, trsm off-diagonal blocks)
+    kFamGemm = 0,     // FP64 GEMM on the FP64 pipe (small products, trsm off-diagonal blocks)
     kFamPanel = 1,    // LU panel (pivot search, swap, scale, rank-1)
     kFamLaswp = 2,    // row interchanges
     kFamTrsm = 3,     // triangular diagonal-block solves
@@ -155,7 +155,8 @@ enum Family : int {
     kFamTrsv = 9,     // chained triangular solves with few vectors (trs, refinement)
     kFamKrylov = 10,  // GMRES: permutation, Gram-Schmidt, norms, updates
     kFamPrecond = 11, // GMRES preconditioner: block inverses and chained solves
-    kFamCount = 12
+    kFamResidue = 12, // FP64 GEMM by residues: all its kernels, the flops with the product's
+    kFamCount = 13
 };
 
 struct KTimer {

@@ -847,7 +847,7 @@ int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double a
                          int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
                          const uint8_t *flag, int flag_ld, int kr, cudaStream_t stream) {
     const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
-    KTimer kt(kFamGemm, stream, 0.0, 0.0);
+    KTimer kt(kFamResidue, stream, 0.0, 0.0);
     // (k ranges depend on the tile: the one dgemm_kr_launch takes)
     const int tile = kr ? BM : fp64_tile(m, n, tri ? 0.5 : 1.0);
     cudaLaunchAttribute attr;

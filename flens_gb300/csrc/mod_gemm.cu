@@ -845,13 +845,13 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
                      (__nv_bfloat16 *)(ws + l.planesB)};
     FG_CUDA(cudaMemsetAsync(ws, 0, l.zeroed, s));
     {
-        KTimer kt(kFamAux, s, 0.0, 8.0 * k * ((double)m + n));
+        KTimer kt(kFamResidue, s, 0.0, 8.0 * k * ((double)m + n));
         const int ba = exp_blocks(m, k, oa.rcontig), bb = exp_blocks(n, k, ob.rcontig);
         mod_exp_kernel<<<ba + bb, 256, 0, s>>>(oa, ob, k, ba);
         FG_CUDA(cudaGetLastError());
     }
     {
-        KTimer kt(kFamAux, s, 0.0, (8.0 + 2.0 * NP) * Kp * ((double)m + n));
+        KTimer kt(kFamResidue, s, 0.0, (8.0 + 2.0 * NP) * Kp * ((double)m + n));
         const int ba = ceil_div(m, 32) * (Kp / KBLK), bb = ceil_div(n, 32) * (Kp / KBLK);
         FG_CUDA(launch_early(mod_residue_kernel, ba + bb, 256, 0, s, oa, ob, k, Kp, bits, ba, cs.res));
     }
@@ -878,7 +878,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     const int items = tiles.ntiles * NP, sms = num_sms() - spare_sms();
     const int grid = items < sms ? items : sms;
     {
-        KTimer kt(kFamGemm, s, 2.0 * (tri ? 0.5 : 1.0) * m * (double)n * k,
+        KTimer kt(kFamResidue, s, 2.0 * (tri ? 0.5 : 1.0) * m * (double)n * k,
                   8.0 * ((double)m * k + (double)k * n + 2.0 * m * n));
         static DeviceOnce once1, onceN;
         if (Kp <= CHUNK) {
@@ -890,7 +890,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
         }
     }
     {
-        KTimer kt(kFamAux, s, 0.0, (NM + 16.0) * m * (double)n);
+        KTimer kt(kFamResidue, s, 0.0, (NM + 16.0) * m * (double)n);
         FG_CUDA(launch_early(mod_crt_kernel, tiles.ntiles * CRT_PARTS, 256, 0, s, tiles, (const uint8_t *)a.res,
                              (const uint8_t *)a.flag, a.keyA, a.keyB, 2 * bits, alpha, beta, C, ldC, cs.crt));
     }

@@ -426,6 +426,6 @@ FG_API const char *flens_gb300_family_name(int family) {
     static const char *names[fg::kFamCount] = {"dgemm_fp64", "lu_panel", "laswp", "trsm_diag",
                                                "aux", "tc_gemm", "refine", "batched_lu",
                                                "split_gemm", "trsv_chain", "krylov",
-                                               "precond_chain"};
+                                               "precond_chain", "dgemm_residues"};
     return (family >= 0 && family < fg::kFamCount) ? names[family] : "";
 }

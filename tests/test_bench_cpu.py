@@ -80,3 +80,13 @@ def test_reference_arm_json_line():
     e2e = line["e2e"]
     assert e2e["value"] == line["value"] and e2e["h2d_bytes_per_step"] == 0
     assert e2e["d2h_bytes_per_step"] == 0
+
+
+def test_roofline_of_a_latency_bound_step():
+    fam = {"lu_panel": {"ms": 68.0, "launches": 326, "flops": 3.3e9, "bytes": 4.4e9},
+           "dgemm_residues": {"ms": 40.0, "launches": 600, "flops": 7.3e11, "bytes": 5.0e10}}
+    r = bench.roofline(fam, 2, 104.0, 8192, 1.2586, 1.1)
+    assert r["kernel"] == "lu_panel" and r["bound"] == "latency"
+    assert r["us_per_column"] == pytest.approx(68.0e3 / (2 * 8192))
+    assert r["residues"]["achieved"] == pytest.approx(7.3e11 / 40.0e-3 / 1e12)
+    assert r["residues"]["traffic"] > 0
