@@ -303,6 +303,31 @@ def roofline(fam, steps, ms, n, pipe_peak, cublas_peak):
     return out
 
 
+def _short(x):
+    """Floats to six digits, all the way down."""
+    if isinstance(x, float):
+        return float(f"{x:.6g}")
+    if isinstance(x, dict):
+        return {k: _short(v) for k, v in x.items()}
+    return [_short(v) for v in x] if isinstance(x, list) else x
+
+
+LINE_KEYS = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+             "vs_baseline", "dtype", "data", "config", "gpu_launches", "clocks")
+
+
+def headline(result):
+    """The line on stdout, short enough for readers that keep the end of a log: what
+    identifies and qualifies the number.  Everything else is in the record on stderr."""
+    line = {k: result[k] for k in LINE_KEYS}
+    for k, keep in (("accuracy", ("info", "backward_error_normwise", "forward_error_vs_x_true")),
+                    ("e2e", ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ok")),
+                    ("roofline", ("kernel", "bound", "achieved", "peak", "unit", "frac", "share_of_step", "traffic"))):
+        if result.get(k):
+            line[k] = {a: result[k][a] for a in keep if a in result[k]}
+    return {k: v if k in ("value", "ms_per_step") else _short(v) for k, v in line.items()}
+
+
 def our_arm(args, rank: int, world: int) -> None:
     import numpy as np
     import torch
@@ -431,7 +456,9 @@ def our_arm(args, rank: int, world: int) -> None:
         # -- CPU baseline (oracle C restatement, 1 thread, bounded sample)
         if not args.no_cpu:
             result["cpu_baseline"] = cpu_baseline(n)
-        print(json.dumps(result), flush=True)
+        # the whole record goes to stderr (22 KB of it: readers of the line keep less)
+        print(json.dumps(result), file=sys.stderr, flush=True)
+        print(json.dumps(headline(result)), flush=True)
     if dist:
         dist.destroy_process_group()
 

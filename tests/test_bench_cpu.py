@@ -90,3 +90,21 @@ def test_roofline_of_a_latency_bound_step():
     assert r["us_per_column"] == pytest.approx(68.0e3 / (2 * 8192))
     assert r["residues"]["achieved"] == pytest.approx(7.3e11 / 40.0e-3 / 1e12)
     assert r["residues"]["traffic"] > 0
+
+
+def test_line_is_short_and_complete():
+    fam = {"lu_panel": {"ms": 68.0, "launches": 326, "flops": 3.3e9, "bytes": 4.4e9},
+           "dgemm_residues": {"ms": 40.0, "launches": 600, "flops": 7.3e11, "bytes": 5.0e10}}
+    result = {k: 1.0 for k in bench.LINE_KEYS}
+    result.update(metric=bench.METRIC, data="x" * 90, config={"workload": "y" * 120}, value=19.17445677736412,
+                  clocks={"sm_mhz": 2070.0, "sm_max_mhz": 2070.0, "reasons": [], "samples": 3},
+                  accuracy={"info": 0, "backward_error_normwise": 8.967343784302304e-16},
+                  e2e={"value": 17.3715697611948, "unit": "solves/s", "h2d_bytes_per_step": 536936448,
+                       "d2h_bytes_per_step": 536969216, "ok": True, "ms_steps": [1.0] * 100},
+                  roofline=bench.roofline(fam, 2, 104.0, 8192, 1.2586, 1.1), mixed_config3={"cases": ["z" * 20000]})
+    text = json.dumps(bench.headline(result))
+    line = json.loads(text)
+    assert len(text) < 2000
+    assert set(bench.LINE_KEYS) <= set(line) and line["value"] == result["value"]
+    assert {"value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"} <= set(line["e2e"])
+    assert line["roofline"]["kernel"] == "lu_panel" and line["roofline"]["bound"] == "latency"
