@@ -803,6 +803,21 @@ mod_crt_kernel(const __grid_constant__ TileMap tiles, const uint8_t *__restrict_
 }
 static_assert(NM % 4 == 1, "the last residue group holds one modulus");
 
+// C <- beta*C + alpha*W (tri 1/2: the lower/upper triangle), W the sum of a block's
+// products over the parts of k: C is read and rounded once, as by the FP64 kernel.
+__global__ void __launch_bounds__(256)
+mod_finish_kernel(int m, int n, int tri, double alpha, const double *__restrict__ W, double beta,
+                  double *__restrict__ C, int ldC) {
+    const bool beta1 = beta == 1.0;
+    const size_t total = (size_t)m * n;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+        const int i = (int)(e % m), j = (int)(e / m);
+        if ((tri == 1 && i < j) || (tri == 2 && i > j)) continue;
+        double *c = &C[(size_t)i + (size_t)j * ldC];
+        *c = fma(alpha, W[e], beta1 ? *c : beta * *c);
+    }
+}
+
 size_t up256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Layout {
@@ -823,9 +838,9 @@ Layout layout_for(int m, int n, int Kp, const TileMap &t) {
     return l;
 }
 
-// One block product at most: 1.5 GB of scratch (two operands' planes 1.2 GB, residues
-// 0.3), or 8192 x 8192 with k = 1024: 1.8 GB (0.6 and 1.1).
-constexpr int kBlkK = 4096, kBlkMN = 4096;
+// One block product at most: 1.8 GB of scratch (two operands' planes 1.4 GB, residues
+// 0.3, the sum over parts of k 0.1), or 8192 x 8192 with k = 1024 (0.6 and 1.1 GB).
+constexpr int kBlkK = 4608, kBlkMN = 4096;
 
 // One block product in the scratch `ws` (layout_for(m, n, Kp, tiles).total bytes).
 int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int ldA,
@@ -949,7 +964,7 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
     };
     // (a triangular operand in the same parts along both its dimensions: its blocks are
     // zero, triangles, or full)
-    const int kb = part(k, kBlkK, kr ? NT : KBLK);
+    const int kb = kr ? part(k, kBlkMN, NT) : part(k, kBlkK, KBLK);
     // a shallow product may take larger blocks of C for the same scratch
     const int capMN = !kr && kb <= 1024 ? 2 * kBlkMN : kBlkMN;
     const int mb = kr == 1 || kr == 2 ? kb : part(m, capMN, NT), nb = kr >= 3 ? kb : part(n, capMN, NT);
@@ -957,33 +972,46 @@ int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha,
     const Layout l = layout_for(mm, nn, ceil_div(kk, KBLK) * KBLK,
                                 make_tiles(mm, nn, tri && mb >= m && nb >= n ? tri : 0));
     int *status = nullptr;
-    char *ws = (char *)scratch_acquire(l.total, s, &status);
+    // more than one part of k: their products are summed here, then added to C
+    const size_t sum_off = up256(l.total), sum_bytes = kb < k ? (size_t)mm * nn * sizeof(double) : 0;
+    char *ws = (char *)scratch_acquire(sum_off + sum_bytes, s, &status);
     if (!ws) return kErrUnsupported;
     trace("dgemm: m=%d n=%d k=%d engine=residues blocks of %d x %d x %d", m, n, k, mm, nn, kk);
-    int rc = kOk;
-    for (int k0 = 0; k0 < k && rc == kOk; k0 += kb)
-        for (int i0 = 0; i0 < m && rc == kOk; i0 += mb)
-            for (int j0 = 0; j0 < n && rc == kOk; j0 += nb) {
-                int bt = tri;
-                const int bm = m - i0 < mb ? m - i0 : mb, bn = n - j0 < nb ? n - j0 : nb;
-                if (tri && i0 != j0) {
-                    if ((tri == 1) != (i0 > j0)) continue;     // the other triangle
-                    bt = 0;
-                }
-                int bkr = 0;
-                bool first = k0 == 0;
-                if (kr) {
-                    const int t0 = kr <= 2 ? i0 : j0;
-                    const bool from = kr == 1 || kr == 4;      // nonzero for k >= the row or column, else k <=
-                    if (from ? k0 < t0 : k0 > t0) continue;
-                    bkr = k0 == t0 ? kr : 0;
-                    if (from) first = k0 == t0;
-                }
-                const int bk = k - k0 < kb ? k - k0 : kb;
-                rc = mod_block(ta, tb, bm, bn, bk, alpha, A + (ta ? k0 + (size_t)i0 * ldA : i0 + (size_t)k0 * ldA),
-                               ldA, B + (tb ? j0 + (size_t)k0 * ldB : k0 + (size_t)j0 * ldB), ldB,
-                               first ? beta : 1.0, C + i0 + (size_t)j0 * ldC, ldC, bt, bkr, ws, status, s);
+    double *W = sum_bytes ? (double *)(ws + sum_off) : nullptr;
+    auto block = [&](int i0, int j0) -> int {
+        int bt = tri;
+        const int bm = m - i0 < mb ? m - i0 : mb, bn = n - j0 < nb ? n - j0 : nb;
+        if (tri && i0 != j0) {
+            if ((tri == 1) != (i0 > j0)) return kOk;          // the other triangle
+            bt = 0;
+        }
+        double *Cb = C + i0 + (size_t)j0 * ldC;
+        if (W) FG_CUDA(cudaMemsetAsync(W, 0, (size_t)bm * bn * sizeof(double), s));
+        for (int k0 = 0; k0 < k; k0 += kb) {
+            int bkr = 0;
+            if (kr) {
+                const int t0 = kr <= 2 ? i0 : j0;             // nonzero for k >= the row or column, else k <=
+                if (kr == 1 || kr == 4 ? k0 < t0 : k0 > t0) continue;
+                bkr = k0 == t0 ? kr : 0;
             }
+            const int bk = k - k0 < kb ? k - k0 : kb;
+            const int rc = mod_block(ta, tb, bm, bn, bk, W ? 1.0 : alpha,
+                                     A + (ta ? k0 + (size_t)i0 * ldA : i0 + (size_t)k0 * ldA), ldA,
+                                     B + (tb ? j0 + (size_t)k0 * ldB : k0 + (size_t)j0 * ldB), ldB, W ? 1.0 : beta,
+                                     W ? W : Cb, W ? bm : ldC, bt, bkr, ws, status, s);
+            if (rc != kOk) return rc;
+        }
+        if (W) {
+            KTimer kt(kFamResidue, s, 0.0, 24.0 * bm * (double)bn);
+            const size_t blocks = ((size_t)bm * bn + 255) / 256, cap = (size_t)num_sms() * 16;
+            mod_finish_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, s>>>(bm, bn, bt, alpha, W, beta, Cb, ldC);
+            FG_CUDA(cudaGetLastError());
+        }
+        return kOk;
+    };
+    int rc = kOk;
+    for (int i0 = 0; i0 < m && rc == kOk; i0 += mb)
+        for (int j0 = 0; j0 < n && rc == kOk; j0 += nb) rc = block(i0, j0);
     scratch_release(ws, s);
     return rc;
 }

@@ -131,6 +131,42 @@ def test_products_of_one_term_are_exact(cuda, k, e, swap):
     assert np.array_equal(got, B if swap else A)
 
 
+@pytest.mark.parametrize("beta", [1.0, -0.5])
+def test_c_is_rounded_once_whatever_the_depth(cuda, beta):
+    """k = 8200 is summed in parts; C is 2^30 times the product: one rounding of
+    the result, one of beta*C (exact here), and 8 * 2^-53 |A||B|."""
+    r = np.random.default_rng(13)
+    m, n, k = 130, 140, 8200
+    A, B = r.uniform(-1, 1, (m, k)), r.uniform(-1, 1, (k, n))
+    C = r.uniform(-1, 1, (m, n)) * 2.0 ** 30
+    got, used = _gemm(cuda, "N", "N", 1.0, A, B, beta, C)
+    assert used >= 10
+    for i, j in zip(r.integers(0, m, 60), r.integers(0, n, 60)):
+        ex = Fraction(beta) * Fraction(float(C[i, j])) + sum(
+            Fraction(a) * Fraction(b) for a, b in zip(A[i].tolist(), B[:, j].tolist()))
+        mag = float(np.abs(A[i]) @ np.abs(B[:, j]))
+        assert abs(Fraction(float(got[i, j])) - ex) <= Fraction(U) * abs(ex) + Fraction(8 * U * mag)
+
+
+@pytest.mark.parametrize("uplo", "LU")
+def test_deep_triangle(cuda, uplo):
+    """syrk with k in two parts and C in four blocks: integers, the other triangle kept."""
+    import torch
+    n, k = 4200, 5000
+    g = torch.Generator(device=cuda)
+    g.manual_seed(2)
+    A = torch.randint(-9, 10, (k, n), generator=g, device=cuda).double().t()
+    C0 = torch.randint(-9, 10, (n, n), generator=g, device=cuda).double().t()
+    C = fg.to_colmajor(C0.clone())
+    fg.dsyrk_dev(uplo, "N", 2.0, A, -1.0, C)
+    fg.sync()
+    want = 2 * (A @ A.t()) - C0
+    tri = torch.tril if uplo == "L" else torch.triu
+    assert torch.equal(tri(C), tri(want))
+    other = torch.triu(C0, 1) if uplo == "L" else torch.tril(C0, -1)
+    assert torch.equal(torch.triu(C, 1) if uplo == "L" else torch.tril(C, -1), other)
+
+
 def test_few_terms_keep_the_fp64_bound(cuda):
     """Rows of A with 1 to 6 nonzeros in a 300^3 product: n nonzero terms, n * 2^-53 *
     |A||B| in each element."""
