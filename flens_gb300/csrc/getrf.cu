@@ -1561,16 +1561,19 @@ constexpr int kClusterSms = CP_CS;
 
 // Outer block of the FP64 order with look-ahead (FLENS_GB300_LOOKAHEAD_NB, a
 // multiple of 64).  A narrow block gets the next panel started sooner, a wide one
-// makes the updates deeper.  Factorisations of n = 2000, 4096, 5000, 8192 in ms: 64
-// columns 5.9, 16.9, 25.4, -; 128 columns 6.6, 17.2, 23.5, 55.5; 256 columns
-// -, 18.2, 24.3, 50.2; halved without look-ahead 7.7 (2048), 20.6, 28.5, 60.0.
+// makes the updates deeper.  Factorisations in ms with 64, 128 and 256 columns:
+//   n    2000   3000   4000   4300   4600   5000   5500   6000   6500   7000   8192
+//    64  5.92   10.1   16.0   18.4   20.9   24.9   30.3   36.7   44.4   53.2   78.1
+//   128  6.47   11.1   16.6   18.5   20.4   23.5   27.2   31.1   35.9   41.2   56.0
+//   256  6.95   11.8   17.3   19.2   21.1   23.7   27.4   30.6   34.6   39.1   50.8
+// (halved without look-ahead: 7.7 at 2048, 28.5 at 5000, 60.0 at 8192).
 int lookahead_nb(int mn) {
     static int nb = [] {
         const char *e = getenv("FLENS_GB300_LOOKAHEAD_NB");
         const int v = e ? atoi(e) : 0;
         return (v >= 64 && v <= 1024 && v % 64 == 0) ? v : 0;
     }();
-    return nb > 0 ? nb : mn < 4500 ? 64 : mn < 6500 ? 128 : 256;
+    return nb > 0 ? nb : mn < 4400 ? 64 : mn < 5700 ? 128 : 256;
 }
 
 // Whether the FP64 LU takes outer blocks with look-ahead, or halves the columns
