@@ -1,4 +1,4 @@
-// blas3.cu -- the remaining level-3 BLAS for double on the FP64 GEMM engine.
+// blas3.cu -- the remaining level-3 BLAS for double on the GEMM engine.
 //
 //   dtrmm  B <- alpha*op(A)*B (side 'L') or alpha*B*op(A) ('R'), A triangular
 //          (cxxblas/level3/trmm.tcc:40-70: trmv per vector, alpha applied at
@@ -11,7 +11,7 @@
 // The triangular or symmetric operand is first written out as a full ka x ka
 // matrix in the workspace (zeros outside the triangle, ones on a unit
 // diagonal; or both triangles from the stored one), so the product runs on
-// the tiled FP64 GEMM.  trmm computes T*B (or B*T) into a workspace buffer and
+// the FP64 GEMM (large ones by residues).  trmm computes T*B (or B*T) into a workspace buffer and
 // writes alpha*result back over B.  syr2k is two triangle-restricted GEMMs
 // (tri_gemm_launch).  Results agree with the reference to rounding.
 #include "common.cuh"

@@ -7,8 +7,9 @@
 // multiply, so NaN/Inf in C propagate even when beta==0); alpha==0 returns
 // after that scaling without reading A or B.
 //
-// GB300 has no FP64 tensor-core kind in tcgen05, so FP64 runs on the FP64
-// pipe either as DFMA (dgemm_fma_kernel) or as the legacy FP64 mma.sync
+// Large products go to the tensor cores by exact residues (mod_gemm.cu); what is
+// left to this file -- small products, tiles that the residues' check refuses,
+// streams under capture -- runs on the FP64 pipe (tcgen05 has no FP64 kind) either as DFMA (dgemm_fma_kernel) or as the legacy FP64 mma.sync
 // m8n8k4 (dgemm_dmma_kernel).  Both are register-tiled with shared-memory
 // staging; the FP64 issue rate, not memory, bounds them.  Which one runs is
 // picked by measured speed (FLENS_GB300_DGEMM=fma|dmma overrides).

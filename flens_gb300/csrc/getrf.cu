@@ -7,10 +7,18 @@
 //   laswp               -> generic::laswp_impl flens/lapack/la/laswp.tcc:54-93
 //   trs                 -> generic::trs_impl   flens/lapack/ge/trs.tcc:59-109
 //
-// Structure (one stream, all asynchronous):
-//   for each block column j (width jb <= 64, the reference's ilaenv GETRF
-//   block size, flens/lapack/la/ilaenv.tcc:93-99):
-//     panel_kernel      cooperative grid, up to one CTA per SM; the (m-j) x jb
+// Orders (all asynchronous; the panel's width is the reference's ilaenv GETRF block
+// size, flens/lapack/la/ilaenv.tcc:93-99):
+//   - FP64 from 1024 columns on: outer blocks of 64 to 256 columns with look-ahead; a
+//     block is factored by halves on a side stream while the previous block's update
+//     runs (lookahead_nb).  FP32 storage from 2048 columns on: its outer blocks so.
+//   - FP64, taller than 20,000 rows: the columns by halves, on one stream.
+//   - smaller, and under stream capture: right-looking steps of 64 columns, the next
+//     panel on the side stream beside the update.
+// The pieces of each:
+//     panel_cluster_kernel  panels of up to 6000 (FP32 13,300) rows: one cluster of 16
+//                       CTAs, exchange by st.async (below).
+//     panel_kernel      taller ones: cooperative grid, up to one CTA per SM; the (m-j) x jb
 //                       panel lives in shared memory split by rows.  Per
 //                       column each CTA finds its best candidate (warp-shuffle
 //                       argmax, first maximum wins), publishes it with the
@@ -26,7 +34,7 @@
 //     laswp_pairs_kernel applies those moves to every column outside the
 //                       panel, one warp per column (loads, then stores).
 //     dtrsm_launch      U12 = L11^-1 A12
-//     dgemm_launch      A22 -= A21 * U12
+//     dgemm_launch      A22 -= A21 * U12 (large ones by residues, mod_gemm.cu)
 //
 // Unlike the reference, the GPU path always uses the blocked algorithm (the
 // reference switches to tf2 when nb >= min(m,n), trf.tcc:87-91); the pivots and

@@ -5,8 +5,8 @@
 // GB300's FP64 pipe issues 2 FMAs per clock per SM (1.26 TFLOP/s); its tensor
 // cores have no FP64 kind but add BF16 products of small integers exactly.
 // The product is therefore formed in a residue number system (the scheme of
-// Ozaki, Uchino and Imamura, "Ozaki Scheme II", 2025, with moduli and bounds
-// of our own):
+// Ozaki, Uchino and Imamura, "Ozaki Scheme II", 2025; the moduli are the
+// largest pairwise coprime numbers up to 256, bounds and data check our own):
 //
 //  1. exponents: 2^e_i bounds row i of op(A), 2^f_j column j of op(B).
 //  2. residues: a_ik is rounded to the integer X_ik = rint(a_ik 2^(beta-e_i)),

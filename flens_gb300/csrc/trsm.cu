@@ -8,10 +8,12 @@
 // All eight side/uplo/trans variants reduce to one description: an effective
 // triangle M (op(A) for side=Left, op(A)^T for side=Right) addressed as
 // M(i,p) = A[i*mi + p*mp], and a set of vectors (columns of B for Left, rows
-// of B for Right).  The blocked, right-looking driver solves 64x64 diagonal
-// blocks (trsm_diag_tile_kernel: 32 vectors per CTA, 8 rows per thread;
+// of B for Right).  Up to four vectors against more than one block take the chained
+// solve (trsv_chain_kernel).  Large solves are halved while the product between the
+// halves goes to the tensor cores (mod_gemm.cu).  The blocked, right-looking driver
+// solves 64x64 diagonal blocks (trsm_diag_tile_kernel: 32 vectors per CTA, 8 rows per thread;
 // trsm_diag_warp_kernel: a warp per vector for up to 2560 vectors) and applies
-// each solved block to the rest of B with the FP64 GEMM.  The
+// each solved block to the rest of B with a GEMM.  The
 // diagonal solve uses the column-sweep (axpy) form rather than the
 // reference's dot form, and multiplies by the reciprocal of the diagonal
 // instead of dividing; the result agrees to rounding.

@@ -1,5 +1,5 @@
-"""Cholesky at the edges of its blocks (64-column steps, 256-column bases, the
-halving above), the other triangle untouched, and INFO at every kind of
+"""Cholesky at the edges of its blocks (64-column steps, 256-column blocks, the
+look-ahead above), the other triangle untouched, and INFO at every kind of
 position.  Bound of the backward error: 4 * n * 2^-53 * |L||L^T|."""
 from __future__ import annotations
 
