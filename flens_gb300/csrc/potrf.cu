@@ -68,7 +68,8 @@ constexpr int TILES = 72, UPD_TILES = (TILES + UPD - 1) / UPD;      // 8 x 4 til
 // product exceeds the square root of two diagonal entries: for pivots beyond 2^+-250,
 // and where the elimination above left an infinity or NaN.  (Between pivots in that
 // range a reciprocal is a normal number, but the unscaled product a_it a_ct of a large
-// row still overflows: [2^200 2^600; 2^600 2^1001].)  Returns the failing column + 1,
+// row still overflows: [2^200 2^600; 2^600 2^1001]; and one of two entries below 2^-480
+// may lose bits that the reciprocal of a pivot below 2^-50 brings back into range.)  Returns the failing column + 1,
 // or 0.
 __device__ __noinline__ int potf2_plain(double (*S)[POTRF_NB + 1], int jb, const double *A, size_t rs, size_t cs) {
     const int tid = threadIdx.x;
@@ -99,11 +100,12 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
     __shared__ double S[POTRF_NB][POTRF_NB + 1];      // S[c][i] = element (i, c), unscaled
     __shared__ double Lp[2][POTRF_NB];                // column t times p_t
     __shared__ double s_p[POTRF_NB];                  // 1 / pivot, later 1 / sqrt(pivot)
-    __shared__ int s_fail, s_skip;
+    __shared__ int s_fail, s_skip, s_odd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) {
         s_fail = 0;
         s_skip = *info != 0;
+        s_odd = 0;
     }
 #pragma unroll
     for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
@@ -183,17 +185,27 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
         }
         __syncthreads();
     }
-    // a positive pivot beyond the range, or an overflow, which stays where it arose: as
-    // an infinity or NaN in a column to be stored, -infinity on the diagonal (a NaN there
-    // alone was in A): the block starts again
-    bool redo = fail && (S[fail - 1][fail - 1] > 0.0 || S[fail - 1][fail - 1] == -CUDART_INF);
+    // The block starts again after a positive pivot beyond the range (bit 0), an overflow,
+    // which stays where it arose: as an infinity or NaN in a column to be stored,
+    // -infinity on the diagonal (a NaN there alone was in A), and where bits may be lost:
+    // an entry below 2^-480 (bit 1) and a pivot below 2^-50 (bit 2).
+    // (High words only; the entries above the diagonal are zeros.)
+    const int lim = (fail ? fail - 1 : POTRF_NB) * POTRF_NB;
+    unsigned most = 0u, least = ~0u;                  // of |entry|, least: of the nonzeros, less one
 #pragma unroll
     for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
-        const int e = h * POTF2_THREADS + tid, i = e % POTRF_NB, c = min(e / POTRF_NB, POTRF_NB - 1);
-        const bool odd = (__double2hiint(S[c][i]) & 0x7FF00000) == 0x7FF00000;
-        redo |= odd && i >= c && (!fail || c < fail - 1);
+        const int e = h * POTF2_THREADS + tid;
+        const unsigned u = e < lim ? (unsigned)__double2hiint(S[e / POTRF_NB][e % POTRF_NB]) & 0x7FFFFFFFu : 0u;
+        most = max(most, u);
+        least = min(least, u - 1u);
     }
-    const bool plain = __syncthreads_or(redo);
+    unsigned odd = (most >= 0x7FFu << 20 ? 1u : 0u) | (least < (1023u - 480u) << 20 ? 2u : 0u);
+    if (tid < lim / POTRF_NB && (unsigned)__double2hiint(S[tid][tid]) - 1u < (1023u - 50u) << 20) odd |= 4u;
+    if (fail && (S[fail - 1][fail - 1] > 0.0 || S[fail - 1][fail - 1] == -CUDART_INF)) odd |= 1u;
+    odd = __reduce_or_sync(0xffffffffu, odd);
+    if (odd && lane == 0) atomicOr(&s_odd, (int)odd);
+    __syncthreads();
+    const bool plain = (s_odd & 1) || (s_odd & 6) == 6;
     if (plain) fail = potf2_plain(S, jb, A, rs, cs);
     const int ncol = fail ? fail - 1 : jb;
     if (plain) {

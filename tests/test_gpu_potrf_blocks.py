@@ -192,3 +192,24 @@ def test_what_a_failed_pivot_leaves(cuda, uplo, n, f):
     # the leading columns: L L^T = A in all rows before the step's, and below
     lead = np.tril(np.ones((n, n), dtype=bool))[:, :c]
     assert np.all((np.abs(L @ L.T - A0)[:, :c] <= tol[:, :c])[lead])
+
+
+@pytest.mark.parametrize("uplo", "LU")
+@pytest.mark.parametrize("at", [0, 1, 29, 30, 40, 60])
+@pytest.mark.parametrize("a,b", [(-540, -540), (-500, -520), (-560, -480)])
+def test_products_below_the_range(cuda, uplo, at, a, b):
+    """A pivot 2^-240 at `at`, 2^a and 2^b beside it, ones and zeros otherwise: the fill-in
+    -2^(a + b + 240) is a normal number, the product of the two entries is not."""
+    n = 64
+    A0 = np.eye(n)
+    A0[at, at] = 2.0 ** -240
+    A0[at + 1, at] = A0[at, at + 1] = 2.0 ** a
+    A0[at + 2, at] = A0[at, at + 2] = 2.0 ** b
+    A, info = _potrf(cuda, uplo, A0)
+    assert info == 0
+    L = A.cpu().numpy()
+    L = np.tril(L) if uplo == "L" else np.triu(L).T
+    want = np.eye(n)
+    want[at, at], want[at + 1, at], want[at + 2, at] = 2.0 ** -120, 2.0 ** (a + 120), 2.0 ** (b + 120)
+    want[at + 2, at + 1] = -2.0 ** (a + b + 240)
+    assert np.array_equal(L, want)
