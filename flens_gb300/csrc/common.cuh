@@ -103,17 +103,14 @@ constexpr size_t kScratchKeep = (size_t)2 << 30;
 void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status);
 void scratch_release(void *p, cudaStream_t stream);
 
-// While a SpareSms lives, the launches of this thread run beside a kernel on another
-// stream (beside_kernel, unless told that nothing does), and its persistent
-// tensor-core kernels leave n SMs free for that.
+// SMs that the persistent tensor-core kernels launched by this thread leave free
+// while a SpareSms lives: for a kernel that runs beside them on another stream.
 int spare_sms();
-bool beside_kernel();
 struct SpareSms {
-    explicit SpareSms(int n, bool beside = true);
+    explicit SpareSms(int n);
     ~SpareSms();
     SpareSms(const SpareSms &) = delete;
     int before;
-    bool before_beside;
 };
 
 int num_sms();                 // SM count of the current device

@@ -639,7 +639,7 @@ static int fp64_tile(int m, int n, double part = 1.0, double *units = nullptr) {
 // smaller tiles' estimate).
 double dgemm_fp64_us(int m, int n, int k, int tri, int kr) {
     double units = 0.0;
-    if (kr || beside_kernel()) {
+    if (kr || spare_sms() > 0) {
         const int sms = num_sms() > 0 ? num_sms() : 1;
         units = ceil(ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 16;
     } else {

@@ -1948,7 +1948,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
                     }
                     if (e < mn && (st = start(i + 1, e)) != kOk) return st;
                     // the rest, beside that block's panels
-                    SpareSms spare(e < mn && cluster_width<T>(m - e, true) > 0 ? kClusterSms : 0, e < mn);
+                    SpareSms spare(e < mn && cluster_width<T>(m - e, true) > 0 ? kClusterSms : 0);
                     for (int l = 0; l < b.nl; ++l) {
                         if ((st = interchange_on(b.lists[l], 0, j, j, 0, stream)) != kOk) return st;
                         if ((st = interchange_on(b.lists[l], e2, n, n, 0, stream)) != kOk) return st;
@@ -2010,7 +2010,7 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
                             set_last_error("getrf: look-ahead panel wider than its update");
                             return kErrUnsupported;
                         }
-                        // (beside that panel: a cluster's SMs stay free)
+                        // (beside a cluster panel, whose SMs and FP64 work it spares)
                         SpareSms spare(cluster && cluster_width<T>(m - nx, false) > 0 ? kClusterSms : 0);
                         if (nr > w2 && (st = update(j, jb, nx + w2, nr - w2)) != kOk) return st;
                     } else if ((st = update(j, jb, j + jb, nr)) != kOk) {

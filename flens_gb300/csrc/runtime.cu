@@ -241,17 +241,9 @@ void *workspace_slot(cudaStream_t stream, int slot, size_t bytes) {
 }
 
 static thread_local int t_spare_sms = 0;
-static thread_local bool t_beside = false;
 int spare_sms() { return t_spare_sms; }
-bool beside_kernel() { return t_beside; }
-SpareSms::SpareSms(int n, bool beside) : before(t_spare_sms), before_beside(t_beside) {
-    t_spare_sms = n;
-    t_beside = beside;
-}
-SpareSms::~SpareSms() {
-    t_spare_sms = before;
-    t_beside = before_beside;
-}
+SpareSms::SpareSms(int n) : before(t_spare_sms) { t_spare_sms = n; }
+SpareSms::~SpareSms() { t_spare_sms = before; }
 
 void *scratch_acquire(size_t bytes, cudaStream_t stream, int **status) {
     Workspace *w = workspace_for(stream, 0);
