@@ -235,16 +235,12 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
                       int ldA, const double *B, int ldB, double beta, double *C, int ldC,
                       cudaStream_t stream);
 
-// Estimated microseconds of that kernel on the whole of C (tri 1/2: one triangle; kr
-// as dgemm_kr_launch).
-double dgemm_fp64_us(int m, int n, int k, int tri, int kr);
-
 // The product on the tensor cores by exact residues (mod_gemm.cu), tri 0 all
 // of C, 1/2 its lower/upper triangle; kErrUnsupported (nothing launched) when
 // mod_gemm_wins is false, the stream is being captured or no scratch memory
 // is to be had; kr as dgemm_kr_launch, for the tiles it refuses.  dgemm_flagged_launch: the FP64 kernel on the blocks it
 // refused.
-bool mod_gemm_wins(int m, int n, int k, int tri, int kr = 0);
+bool mod_gemm_wins(int m, int n, int k, int tri);
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
                     const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s,
                     int kr = 0);

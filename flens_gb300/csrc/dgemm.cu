@@ -15,8 +15,6 @@
 // picked by measured speed (FLENS_GB300_DGEMM=fma|dmma overrides).
 #include "common.cuh"
 
-#include <cmath>
-
 #include <stdlib.h>
 #include <string.h>
 
@@ -618,35 +616,12 @@ int sscal_matrix_launch(int m, int n, float alpha, float *X, int ld, cudaStream_
 // SMs, and smaller ones on until every SM has a tile: the waves of tiles over the
 // SMs times a tile's pipe time (16, 4, 1) decide.  64 x 48 x 80 took 21 us of one
 // SM's pipe per 32x32 tile, 1.3 us per 8x8 tile.
-static int fp64_tile(int m, int n, double part = 1.0, double *units = nullptr) {
+static int fp64_tile(int m, int n, double part = 1.0) {
     const int sms = num_sms() > 0 ? num_sms() : 1;
-    auto cost = [&](int t) { return ceil(ceil_div(m, t) * (double)ceil_div(n, t) * part / sms - 0.001) * (t * t / 64); };
-    int tile = 64;
-    if ((double)ceil_div(m, BM) * ceil_div(n, BN) * part < 4.0 * sms) {
-        const double c32 = cost(32), c16 = cost(16), c8 = cost(8);
-        tile = c8 * 2 <= c16 && c8 * 4 <= c32 ? 8 : c16 * 4 <= c32 * 3 ? 16 : 32;
-    }
-    if (units) *units = cost(tile);
-    return tile;
-}
-
-// Estimated microseconds of the FP64 kernel, fitted to measurements from 100^3 to
-// 4096^3 (within 15%): an SM takes 0.0166 us of its pipe per unit of k and 8 x 8 tile.
-// Of a triangle's tiles some SM holds one more than the mean (syrk 200, 300, 512,
-// 1000: 25, 57, 257, 1270 us).  kr: 64 x 64 tiles over half of k in the mean, counted as
-// 32 x 32 tiles over all of it; so are products beside another stream's kernel
-// (SpareSms), which wants the FP64 pipes too (dpotrf, n = 700: 900 us, and 920 with the
-// smaller tiles' estimate).
-double dgemm_fp64_us(int m, int n, int k, int tri, int kr) {
-    double units = 0.0;
-    if (kr || spare_sms() > 0) {
-        const int sms = num_sms() > 0 ? num_sms() : 1;
-        units = ceil(ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 16;
-    } else {
-        const int tile = fp64_tile(m, n, tri ? 0.5 : 1.0, &units);
-        if (tri) units += tile * tile / 64;
-    }
-    return 5.0 + 0.0166 * units * k;
+    if ((double)ceil_div(m, BM) * ceil_div(n, BN) * part >= 4.0 * sms) return 64;
+    auto cost = [&](int t) { return (int)(ceil_div(m, t) * (double)ceil_div(n, t) * part / sms + 0.999) * (t * t / 64); };
+    const int c32 = cost(32), c16 = cost(16), c8 = cost(8);
+    return c8 * 2 <= c16 && c8 * 4 <= c32 ? 8 : c16 * 4 <= c32 * 3 ? 16 : 32;
 }
 
 template <typename T>

@@ -2010,8 +2010,6 @@ int getrf_t(int m, int n, T *A, int ldA, int *ipiv, int *info, int tc_kind, int 
                             set_last_error("getrf: look-ahead panel wider than its update");
                             return kErrUnsupported;
                         }
-                        // (beside a cluster panel, whose SMs and FP64 work it spares)
-                        SpareSms spare(cluster && cluster_width<T>(m - nx, false) > 0 ? kClusterSms : 0);
                         if (nr > w2 && (st = update(j, jb, nx + w2, nr - w2)) != kOk) return st;
                     } else if ((st = update(j, jb, j + jb, nr)) != kOk) {
                         return st;

@@ -926,20 +926,20 @@ bool mod_enabled() {
 
 }  // namespace
 
-// Estimated microseconds of the two routes, fitted to measurements from 100^3 to
-// 4096^3 and 1000 x 17 x 1000 to 8192 x 256 x 256 (within 15%).  FP64: dgemm_fp64_us.
-// Residues: the launches, the work items in waves (1.2 us + 5.5 ns per unit of k), the
-// operands and C.  FP64 and residues at, say, 128 x 128 x 256: 26 and 33 us of a call;
-// 200^3: 39 and 34; 300^3: 70 and 39; 4032 x 64 x 64: 45 and 46; 4096 x 128 x 128: 143
-// and 45.  A product whose tiles are all refused takes both.
-bool mod_gemm_wins(int m, int n, int k, int tri, int kr) {
+// Estimated microseconds of the two routes, fitted to measurements from 256^3 to
+// 4096^3 and 1000 x 100 x 1000 to 8192 x 256 x 256 (within 15%).  FP64: an SM
+// takes 0.265 us of its pipe per unit of k and 32 x 32 tile, in waves over the
+// SMs.  Residues: the launches, the work items in waves (1.2 us + 5.5 ns per unit
+// of k), the operands and C.  Both at, say, 300^3: 85 and 28 us; 4032 x 64 x 64: 38 and 37;
+// 4096 x 128 x 128: 134 and 44.
+bool mod_gemm_wins(int m, int n, int k, int tri) {
     if (n <= 16 || m <= 16 || k < 32 || !mod_enabled()) return false;
     const double half = tri ? 0.5 : 1.0, mn = half * m * (double)n;
     const int sms = num_sms() > 0 ? num_sms() : 1;
+    const double fp64 = 5.0 + ceil(half * ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 0.265 * k;
     const double items = ceil(half * ceil_div(m, MT) * (double)ceil_div(n, NT) * NP / sms);
     const double mod = 24.0 + items * (1.2 + 0.0055 * k) + 1.0e-5 * k * ((double)m + n) + 1.5e-5 * mn;
-    // (a triangular operand has rows of few terms, whose tiles are refused)
-    return mod < (kr ? 0.75 : 0.9) * dgemm_fp64_us(m, n, k, tri, kr);
+    return mod < 0.9 * fp64;
 }
 
 // C <- beta*C + alpha*op(A)*op(B) (tri 1/2: only the lower/upper triangle of a
@@ -948,7 +948,7 @@ bool mod_gemm_wins(int m, int n, int k, int tri, int kr) {
 // nothing has been launched then and the caller takes the FP64 kernel.
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
                     const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s, int kr) {
-    if (!mod_gemm_wins(m, n, k, tri, kr)) return kErrUnsupported;
+    if (!mod_gemm_wins(m, n, k, tri)) return kErrUnsupported;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
         cudaGetLastError();
