@@ -240,7 +240,7 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
 // mod_gemm_wins is false, the stream is being captured or no scratch memory
 // is to be had; kr as dgemm_kr_launch, for the tiles it refuses.  dgemm_flagged_launch: the FP64 kernel on the blocks it
 // refused.
-bool mod_gemm_wins(int m, int n, int k, int tri);
+bool mod_gemm_wins(int m, int n, int k, int tri, int kr = 0);
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
                     const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s,
                     int kr = 0);

@@ -931,15 +931,21 @@ bool mod_enabled() {
 // takes 0.265 us of its pipe per unit of k and 32 x 32 tile, in waves over the
 // SMs.  Residues: the launches, the work items in waves (1.2 us + 5.5 ns per unit
 // of k), the operands and C.  Both at, say, 300^3: 85 and 28 us; 4032 x 64 x 64: 38 and 37;
-// 4096 x 128 x 128: 134 and 44.
-bool mod_gemm_wins(int m, int n, int k, int tri) {
+// 4096 x 128 x 128: 134 and 44.  (The FP64 kernel's 8 x 8 tiles beat that estimate: 128
+// x 128 x 256 takes 26 us of a call there and 33 here, 100^3 19 and 33.  The residues
+// stay: they are the more exact, and inside solves it shows.  With the smaller tiles'
+// estimate LU and solve with 40 right-hand sides were 1.4 times as far off at n = 700 to
+// 2500.)
+bool mod_gemm_wins(int m, int n, int k, int tri, int kr) {
     if (n <= 16 || m <= 16 || k < 32 || !mod_enabled()) return false;
     const double half = tri ? 0.5 : 1.0, mn = half * m * (double)n;
     const int sms = num_sms() > 0 ? num_sms() : 1;
     const double fp64 = 5.0 + ceil(half * ceil_div(m, 32) * (double)ceil_div(n, 32) / sms) * 0.265 * k;
     const double items = ceil(half * ceil_div(m, MT) * (double)ceil_div(n, NT) * NP / sms);
     const double mod = 24.0 + items * (1.2 + 0.0055 * k) + 1.0e-5 * k * ((double)m + n) + 1.5e-5 * mn;
-    return mod < 0.9 * fp64;
+    // (a triangular operand has rows of few terms, whose tiles are refused: trmm 100 x 100
+    // 138 us on the FP64 kernel, 160 with both; 200 x 200 236 and 184)
+    return mod < (kr ? 0.75 : 0.9) * fp64;
 }
 
 // C <- beta*C + alpha*op(A)*op(B) (tri 1/2: only the lower/upper triangle of a
@@ -948,7 +954,7 @@ bool mod_gemm_wins(int m, int n, int k, int tri) {
 // nothing has been launched then and the caller takes the FP64 kernel.
 int mod_gemm_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A, int ldA,
                     const double *B, int ldB, double beta, double *C, int ldC, int tri, cudaStream_t s, int kr) {
-    if (!mod_gemm_wins(m, n, k, tri)) return kErrUnsupported;
+    if (!mod_gemm_wins(m, n, k, tri, kr)) return kErrUnsupported;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
         cudaGetLastError();
