@@ -818,14 +818,20 @@ int dgemm_fp64_launch(char transA, char transB, int m, int n, int k, double alph
 // The FP64 kernel on the flagged 128 x 256 blocks of C only (tri 1/2: within
 // the lower/upper triangle; kr as dgemm_kr_launch): the tiles a residue product
 // refused, in the tiles that the whole product would take (512 x 64 x 512 with all
-// refused: 171 us in 32 x 32 tiles; the FP64 product alone takes 47).
+// refused: 171 us in 32 x 32 tiles, 69 in 16 x 16; the FP64 product alone takes 46), but
+// 32 x 32 rather than smaller ones beyond four blocks an SM, and 64 x 64 where those of
+// the whole of C are four an SM: where nothing is refused, the usual case, 3000 blocks that
+// exit at once cost 3 us more than 800 (3% of a Cholesky of n = 2048).
 int dgemm_flagged_launch(char transA, char transB, int m, int n, int k, double alpha, const double *A,
                          int ldA, const double *B, int ldB, double beta, double *C, int ldC, int tri,
                          const uint8_t *flag, int flag_ld, int kr, cudaStream_t stream) {
     const bool ta = !(transA == 'N' || transA == 'n'), tb = !(transB == 'N' || transB == 'n');
     KTimer kt(kFamResidue, stream, 0.0, 0.0);
     // (k ranges depend on the tile: the one dgemm_kr_launch takes)
-    const int tile = kr ? BM : fp64_tile(m, n, tri ? 0.5 : 1.0);
+    int tile = kr ? BM : fp64_tile(m, n, tri ? 0.5 : 1.0);
+    const double most = 4.0 * num_sms();
+    if (tile < 32 && (double)ceil_div(m, tile) * ceil_div(n, tile) > most) tile = 32;
+    if (tile == 32 && (double)ceil_div(m, BM) * ceil_div(n, BN) >= most) tile = BM;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;

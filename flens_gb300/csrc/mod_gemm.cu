@@ -137,9 +137,16 @@ struct Operand {
     const double *X;
     int ld, R, rcontig;                      // rcontig: element (r, k) at X[r + k ld], else X[k + r ld]
     unsigned *key;                           // row maxima: high word of |x|
-    unsigned long long *sum;                 // rows: sum of the magnitudes in 2^-16, nonzeros << 32
+    unsigned *sum;                           // rows: sum of the magnitudes and nonzeros (row_sum, ...)
     __nv_bfloat16 *planes;                   // NP planes of R rows x Kp
 };
+
+// The word of a row: sum of its magnitudes, rounded up to 2^-6 per 64 entries, in the low
+// 19 bits, its nonzeros above them (32 bits as one atomic; 64 made every product 1.4 us
+// longer).  Both hold up to 4608 entries.
+constexpr unsigned kSumOne = 1u << 19;
+__device__ __forceinline__ float row_sum(unsigned w) { return (float)(w & (kSumOne - 1u)) * 0.015625f; }
+__device__ __forceinline__ unsigned row_nonzeros(unsigned w) { return w / kSumOne; }
 
 // e with max|x| < 2^e from the row key; ok = false: non-finite or out of range.
 __device__ __forceinline__ int key_exp(unsigned key, bool &ok) {
@@ -337,7 +344,7 @@ mod_residue_kernel(const __grid_constant__ Operand oa, const __grid_constant__ O
 #pragma unroll
         for (int off = 8; off > 0; off >>= 1) sum += __shfl_xor_sync(0xFFFFu << (lane & 16), sum, off);
         if ((lane & 15) == 0 && sum)
-            atomicAdd(&o.sum[r], ((unsigned long long)(sum >> 24) << 32) | (sum & 0xFFFFFFu));
+            atomicAdd(&o.sum[r], (sum >> 24) * kSumOne + (((sum & 0xFFFFFFu) + 1023u) >> 10));
         uint2 w0;
         w0.x = bf16x2(f2(make_float2(mg[0], mg[1])));
         w0.y = bf16x2(f2(make_float2(mg[2], mg[3])));
@@ -402,11 +409,11 @@ struct ModArgs {
     TileMap tiles;
     int nkb;                                  // 64-deep k blocks
     float qscale;                             // smallest accepted Q: this times (s_i + t_j), or 4
-    int dense;                                // times it: fewer nonzeros in row and column together
+    unsigned dense;                           // times it: fewer nonzeros in row and column together
     uint8_t *res;                             // residues [modulus][tile][4-column group][row][4]
     uint8_t *flag;                            // per tile (row tile + tm * column tile): 1 = left to FP64
     const unsigned *keyA, *keyB;
-    const unsigned long long *sumA, *sumB;
+    const unsigned *sumA, *sumB;
     float p[NM], ip[NM];
 };
 
@@ -560,16 +567,13 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                                : a.res + ((size_t)(pl - 1) * ntiles + t) * (MT * NT) + (size_t)rl * 4;
             uint32_t st[MULTI ? 32 : 1];
             bool bad = false;
-            float si = 0.0f, tj[2] = {0.0f, 0.0f};
-            int ni = 0, nj[2] = {0, 0};              // nonzeros
+            unsigned wi = 0u, wj[2] = {0u, 0u};      // sums and nonzeros
             if (mag) {                               // rows' and columns' data, before the wait
                 bool ok = true;
                 if (m0 + rl < M) {
                     key_exp(a.keyA[m0 + rl], ok);
                     bad |= !ok;
-                    const unsigned long long w = a.sumA[m0 + rl];
-                    si = (float)(unsigned)w;
-                    ni = (int)(w >> 32);
+                    wi = a.sumA[m0 + rl];
                 }
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
@@ -577,9 +581,7 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     if (col < N) {
                         key_exp(a.keyB[col], ok);
                         bad |= !ok;
-                        const unsigned long long w = a.sumB[col];
-                        tj[cc] = (float)(unsigned)w;
-                        nj[cc] = (int)(w >> 32);
+                        wj[cc] = a.sumB[col];
                     }
                 }
             }
@@ -600,17 +602,18 @@ mod_product_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
                     uint32_t r[32];
                     tmem_ld32(base + (uint32_t)c0, r);
                     if (mag) {
-                        // (the sparsest of the 32 columns, but for those of zeros, and the
-                        // densest decide for all)
-                        const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)nj[cc]);
-                        const int least = (int)__reduce_min_sync(0xffffffffu, nj[cc] ? (unsigned)nj[cc] : 1u << 30);
-                        const float qs = ni + least >= a.dense ? a.qscale : 4.0f * a.qscale;
-                        const float sx = fminf(si, 65536.0f * (float)most), tx = 65536.0f * (float)ni;
+                        // (The sparsest of the 32 columns, but for those of zeros, and the
+                        // densest decide for all.  A smallest Q of -inf: no such row or column.)
+                        const unsigned ni = row_nonzeros(wi), nj = row_nonzeros(wj[cc]);
+                        const unsigned most = __reduce_max_sync(0xffffffffu, nj);
+                        const unsigned least = __reduce_min_sync(0xffffffffu, nj ? nj : 1u << 30);
+                        const float qs = ni + least >= a.dense ? a.qscale : 4.0f * a.qscale, ti = (float)ni;
+                        const float pi = m0 + rl < M ? fminf(row_sum(wi), (float)most) * qs : -INFINITY;
+                        const float tj = n0 + c0 + lane < N ? row_sum(wj[cc]) : -INFINITY;
 #pragma unroll
                         for (int j = 0; j < 32; ++j) {
                             const float q = __uint_as_float(r[j]);
-                            const float qmin = (sx + fminf(__shfl_sync(0xffffffffu, tj[cc], j), tx)) * qs;
-                            bad |= m0 + rl < M && n0 + c0 + j < N && q < qmin && q != 0.0f;
+                            bad |= q < fmaf(fminf(__shfl_sync(0xffffffffu, tj, j), ti), qs, pi) && q != 0.0f;
                         }
                     } else {
 #pragma unroll
@@ -828,8 +831,8 @@ Layout layout_for(int m, int n, int Kp, const TileMap &t) {
     l.keyA = 0;
     l.keyB = up256((size_t)m * 4);
     l.sumA = l.keyB + up256((size_t)n * 4);
-    l.sumB = l.sumA + up256((size_t)m * 8);
-    l.flag = l.sumB + up256((size_t)n * 8);
+    l.sumB = l.sumA + up256((size_t)m * 4);
+    l.flag = l.sumB + up256((size_t)n * 4);
     l.zeroed = l.flag + up256((size_t)t.tm * t.tn);
     l.planesA = l.zeroed;
     l.planesB = l.planesA + up256((size_t)NP * m * Kp * 2);
@@ -841,6 +844,7 @@ Layout layout_for(int m, int n, int Kp, const TileMap &t) {
 // One block product at most: 1.8 GB of scratch (two operands' planes 1.4 GB, residues
 // 0.3, the sum over parts of k 0.1), or 8192 x 8192 with k = 1024 (0.6 and 1.1 GB).
 constexpr int kBlkK = 4608, kBlkMN = 4096;
+static_assert(kBlkK * 64 < (int)kSumOne && kBlkMN <= kBlkK && kBlkK < 1 << 13, "a row's sum and nonzeros fit its word");
 
 // One block product in the scratch `ws` (layout_for(m, n, Kp, tiles).total bytes).
 int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double *A, int ldA,
@@ -854,9 +858,9 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     while ((1 << lk) < k) ++lk;
     int bits = (cs.log2P - 2 - lk) / 2;
     if (bits > 61) bits = 61;
-    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (unsigned long long *)(ws + l.sumA),
+    const Operand oa{A, ldA, m, ta ? 0 : 1, (unsigned *)(ws + l.keyA), (unsigned *)(ws + l.sumA),
                      (__nv_bfloat16 *)(ws + l.planesA)};
-    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (unsigned long long *)(ws + l.sumB),
+    const Operand ob{B, ldB, n, tb ? 1 : 0, (unsigned *)(ws + l.keyB), (unsigned *)(ws + l.sumB),
                      (__nv_bfloat16 *)(ws + l.planesB)};
     FG_CUDA(cudaMemsetAsync(ws, 0, l.zeroed, s));
     {
@@ -878,7 +882,7 @@ int mod_block(bool ta, bool tb, int m, int n, int k, double alpha, const double 
     a.tiles = tiles;
     a.nkb = Kp / KBLK;
     // 2^(-bits-1) (s + t) <= 2^-51 Q; the magnitudes were rounded down by up to 2^-7
-    a.qscale = (float)(1.01 * ldexp(1.0, 50 - bits - 16));
+    a.qscale = (float)(1.01 * ldexp(1.0, 50 - bits));
     a.dense = k + 5;
     a.res = (uint8_t *)(ws + l.res);
     a.flag = (uint8_t *)(ws + l.flag);
