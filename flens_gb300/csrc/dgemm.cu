@@ -105,7 +105,7 @@ dgemm_fma_kernel(int m, int n, int k, T alpha,
     }
     if (TRI == 1 && m0 + TM <= n0) return;       // tile strictly above the diagonal
     if (TRI == 2 && n0 + TN <= m0) return;       // tile strictly below the diagonal
-    const bool stop = TRI && !FLAG && skip && *skip;
+    const int stop = TRI && !FLAG && skip ? *skip : 0;
 
     SlabLoader<T, !TA, TM, NT> la;
     SlabLoader<T, TB, TN, NT> lb;

@@ -188,34 +188,36 @@ potf2_kernel(int jb, double *__restrict__ A, size_t rs, size_t cs, int j0, int *
     // The block starts again after a positive pivot beyond the range (bit 0), an overflow,
     // which stays where it arose: as an infinity or NaN in a column to be stored,
     // -infinity on the diagonal (a NaN there alone was in A), and where bits may be lost:
-    // an entry below 2^-480 (bit 1) and a pivot below 2^-50 (bit 2).
-    // (High words only; the entries above the diagonal are zeros.)
-    const int lim = (fail ? fail - 1 : POTRF_NB) * POTRF_NB;
+    // an entry below 2^-480 (bit 1) and a pivot below 2^-50 (bit 2).  High words only, and
+    // beside the roots, which the diagonal's threads take.
+    int ncol = fail ? fail - 1 : jb;
+    unsigned odd = fail && (S[fail - 1][fail - 1] > 0.0 || S[fail - 1][fail - 1] == -CUDART_INF) ? 1u : 0u;
     unsigned most = 0u, least = ~0u;                  // of |entry|, least: of the nonzeros, less one
 #pragma unroll
     for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
-        const int e = h * POTF2_THREADS + tid;
-        const unsigned u = e < lim ? (unsigned)__double2hiint(S[e / POTRF_NB][e % POTRF_NB]) & 0x7FFFFFFFu : 0u;
+        const int e = h * POTF2_THREADS + tid, i = e % POTRF_NB, c = e / POTRF_NB;
+        const unsigned u = i > c && c < ncol ? (unsigned)__double2hiint(S[c][i]) & 0x7FFFFFFFu : 0u;
         most = max(most, u);
         least = min(least, u - 1u);
     }
-    unsigned odd = (most >= 0x7FFu << 20 ? 1u : 0u) | (least < (1023u - 480u) << 20 ? 2u : 0u);
-    if (tid < lim / POTRF_NB && (unsigned)__double2hiint(S[tid][tid]) - 1u < (1023u - 50u) << 20) odd |= 4u;
-    if (fail && (S[fail - 1][fail - 1] > 0.0 || S[fail - 1][fail - 1] == -CUDART_INF)) odd |= 1u;
-    odd = __reduce_or_sync(0xffffffffu, odd);
-    if (odd && lane == 0) atomicOr(&s_odd, (int)odd);
-    __syncthreads();
-    const bool plain = (s_odd & 1) || (s_odd & 6) == 6;
-    if (plain) fail = potf2_plain(S, jb, A, rs, cs);
-    const int ncol = fail ? fail - 1 : jb;
-    if (plain) {
-        if (tid < POTRF_NB) s_p[tid] = 1.0;
-    } else if (tid < ncol) {
+    if (tid < ncol) {
         const double a = S[tid][tid];
+        const unsigned u = (unsigned)__double2hiint(a);
+        most = max(most, u);
+        if (u < (1023u - 50u) << 20) odd |= 4u;
         S[tid][tid] = sqrt(a);
         s_p[tid] = rsqrt(a);
     }
+    odd |= (most >= 0x7FFu << 20 ? 1u : 0u) | (least < (1023u - 480u) << 20 ? 2u : 0u);
+    odd = __reduce_or_sync(0xffffffffu, odd);
+    if (odd && lane == 0) atomicOr(&s_odd, (int)odd);
     __syncthreads();
+    if ((s_odd & 1) || (s_odd & 6) == 6) {
+        fail = potf2_plain(S, jb, A, rs, cs);
+        ncol = fail ? fail - 1 : jb;
+        if (tid < POTRF_NB) s_p[tid] = 1.0;
+        __syncthreads();
+    }
 #pragma unroll
     for (int h = 0; h < (POTRF_NB * POTRF_NB + POTF2_THREADS - 1) / POTF2_THREADS; ++h) {
         const int e = h * POTF2_THREADS + tid, lo = e % POTRF_NB, hi = e / POTRF_NB;

@@ -359,7 +359,7 @@ trsm_diag_warp_kernel(int nb, const T *__restrict__ M0, long long mi, long long 
                       const int *__restrict__ skip) {
     __shared__ T Ms[TRSM_NB][TRSM_NB + 1];     // Ms[i][r] = M(r, i)
     __shared__ T rinv[TRSM_NB];
-    const bool stop = skip && *skip;           // (tested at the end: its latency is hidden)
+    const int stop = skip ? *skip : 0;         // (tested at the end: its latency is hidden)
     const int lane = threadIdx.x & 31;
     const long long v = (long long)blockIdx.x * TRSM_WARP_VECS + (threadIdx.x >> 5);
     T *x = X0 + v * vs;
